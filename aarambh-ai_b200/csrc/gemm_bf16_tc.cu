@@ -159,22 +159,19 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
             if (!bar_wait(&sh->accempty[ab], ((tuse >> 1) & 1) ^ 1, failed)) break;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const uint32_t tacc = tmem + (uint32_t)(ab * ACC_COLS);
-            for (int ks = 0; ks < KS && !*failed; ++ks, ++use) {
+            for (int ks = 0; ks < KS; ++ks, ++use) {
                 const int s = use % STAGES;
-                if (!bar_wait(&sh->full[s], (use / STAGES) & 1, failed)) break;
-                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                if (lane == 0) {
-                    const uint32_t a0 = sptr(ring + s * STAGE_BYTES), b0 = a0 + (DUAL ? 2 : 1) * GB_A_BYTES;
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        umma_bf16(tacc, umma_desc(a0 + k * 32), umma_desc(b0 + k * 32), IDESC, (ks | k) != 0);
-                        if (DUAL) umma_bf16(tacc + NTOK, umma_desc(a0 + GB_A_BYTES + k * 32), umma_desc(b0 + k * 32), IDESC, (ks | k) != 0);
-                    }
+                if (!warp_wait(&sh->full[s], (use / STAGES) & 1, failed)) break;  // no tensor memory in a stage: no tcgen05 fence
+                if (elect_one()) {
+                    const uint32_t a0 = sptr(ring + s * STAGE_BYTES);
+                    const uint64_t xd = umma_desc(a0 + (DUAL ? 2 : 1) * GB_A_BYTES);
+                    umma_stage(tacc, umma_desc(a0), xd, IDESC, ks == 0);
+                    if (DUAL) umma_stage(tacc + NTOK, umma_desc(a0 + GB_A_BYTES), xd, IDESC, ks == 0);
                     umma_commit(&sh->empty[s]);  // the stage is free when the MMAs retire
                 }
                 __syncwarp();
             }
-            if (lane == 0) umma_commit(&sh->accfull[ab]);
+            if (elect_one()) umma_commit(&sh->accfull[ab]);
             __syncwarp();
         }
     } else {

@@ -12,12 +12,10 @@
 //   warp 0      one lane loads a 128-channel x 128-K tile of codes per ring slot with one TMA
 //               tile copy (128-byte swizzle, so that the row-per-thread reads below do not
 //               collide on shared-memory banks)
-//   warps 2-9   two threads per channel turn 32 codes each into bf16 per stage: a byte b is
-//               b + 128 after one XOR, PRMT puts it under the exponent of 2^23, one subtract
-//               gives float(b) exactly, and since |b| <= 127 needs at most 7 significant bits the
-//               bf16 is the upper half of that float (one PRMT per pair).  The codes enter the
-//               MMA unscaled and exact;
-//   warps 10-13 the epilogue multiplies the f32 accumulator by the channel's f32 scale - the
+//   warps 2-17  thread = channel: two codes at a time go into the low bytes of 16-bit halves (PRMT); the low
+//               7 bits and the sign bit are each the mantissa of a bf16 between 128 and 256 (two logic ops),
+//               whose difference is the code, exactly.  The codes enter the MMA unscaled;
+//   warps 18-21 the epilogue multiplies the f32 accumulator by the channel's f32 scale - the
 //               product is rounded once, where the reference rounds q * scale to the model
 //               dtype before its matmul.
 // Every wait on an mbarrier is bounded; on a time-out the CTA records AB2_ERR_TIMEOUT, stops
@@ -37,39 +35,40 @@ int device_status_word(int **out);
 int device_sm_count();
 namespace {
 
-constexpr int TC_STAGES = 4;          // operand-A (unpacked weight) stages of 64 K-elements
-constexpr int TC_MAX_XSTAGES = 6;     // operand-B (activation) stages: a ring of its own, 128 KB deep, because an
-                                      // activation tile takes about three stage times to arrive from L2
-constexpr int TC_WSLOTS = 2;          // code ring slots (128 channels x 128 K, 16 KB each)
+constexpr int TC_MAX_STAGES = 6, TC_MAX_WSLOTS = 6;
 constexpr int TC_WSLOT_BYTES = 128 * 128;  // 128 channels x 128 codes
 constexpr int TC_A_BYTES = 128 * 128;  // 128 channels x 64 bf16
-constexpr int TC_THREADS = 480;  // 1 weight producer, 1 MMA, 8 convert, 4 epilogue, 1 activation producer
+constexpr int TC_SETS = 4;  // sets of four convert warps on stages of their own
+constexpr int TC_THREADS = (2 + 4 * TC_SETS + 4 + 1) * 32;  // weight producer, MMA, convert, epilogue, activation producer
 
 struct TcShared {
-    uint64_t wfull[TC_WSLOTS], wempty[TC_WSLOTS];
-    uint64_t xfull[TC_MAX_XSTAGES], xempty[TC_MAX_XSTAGES], afull[TC_STAGES], sempty[TC_STAGES];
+    uint64_t wfull[TC_MAX_WSLOTS], wempty[TC_MAX_WSLOTS];
+    uint64_t full[TC_MAX_STAGES], empty[TC_MAX_STAGES];
     uint64_t accfull[2], accempty[2];  // two accumulators: the epilogue of a tile overlaps the next tile's MMAs
     uint32_t tmem_base;
     int failed;
 };
 
+// Stages of 64 K-elements: a converted weight tile and an activation tile that share one pair of barriers, so that
+// the issuing warp waits once per stage (a wait costs it about 150 cycles even when the stage is ready, and four MMAs
+// of 32 tokens only 160).  What they leave of shared memory goes to the slots of codes, 128 channels x 128 K each.
 template <int NTOK>
-__host__ __device__ constexpr int tc_xstages() {
-    return NTOK > 128 ? TC_STAGES : TC_MAX_XSTAGES;
-}
+__host__ __device__ constexpr int tc_stages() { return NTOK > 128 ? 4 : 6; }
+template <int NTOK>
+__host__ __device__ constexpr int tc_wslots() { return NTOK > 32 ? 2 : TC_MAX_WSLOTS; }
 
 template <int NTOK>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const float *__restrict__ scales,
                   const __grid_constant__ CUtensorMap xmap, __nv_bfloat16 *__restrict__ y, int N, int K, int M, int *status) {
     constexpr int B_BYTES = NTOK * 128;
-    constexpr int XST = tc_xstages<NTOK>();
+    constexpr int TC_STAGES = tc_stages<NTOK>(), TC_WSLOTS = tc_wslots<NTOK>();
     constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NTOK >> 3) << 17) | ((128u >> 4) << 24);
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t *a_st = smem;                                   // [TC_STAGES][TC_A_BYTES]
-    uint8_t *b_st = a_st + TC_STAGES * TC_A_BYTES;          // [XST][B_BYTES]
-    uint8_t *w_ring = b_st + XST * B_BYTES;                 // [TC_WSLOTS][TC_WSLOT_BYTES]
+    uint8_t *b_st = a_st + TC_STAGES * TC_A_BYTES;          // [TC_STAGES][B_BYTES]
+    uint8_t *w_ring = b_st + TC_STAGES * B_BYTES;                 // [TC_WSLOTS][TC_WSLOT_BYTES]
     TcShared *sh = (TcShared *)(w_ring + TC_WSLOTS * TC_WSLOT_BYTES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -79,9 +78,8 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const float *__restr
     volatile int *failed = &sh->failed;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < TC_WSLOTS; ++i) { bar_init(&sh->wfull[i], 1); bar_init(&sh->wempty[i], 256); }
-        for (int i = 0; i < TC_STAGES; ++i) { bar_init(&sh->afull[i], 256); bar_init(&sh->sempty[i], 1); }
-        for (int i = 0; i < XST; ++i) { bar_init(&sh->xfull[i], 1); bar_init(&sh->xempty[i], 1); }
+        for (int i = 0; i < TC_WSLOTS; ++i) { bar_init(&sh->wfull[i], 1); bar_init(&sh->wempty[i], 8); }
+        for (int i = 0; i < TC_STAGES; ++i) { bar_init(&sh->full[i], 4 + 1); bar_init(&sh->empty[i], 1); }
         for (int i = 0; i < 2; ++i) { bar_init(&sh->accfull[i], 1); bar_init(&sh->accempty[i], 4); }
         sh->failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -117,11 +115,10 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const float *__restr
             for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x) {
                 const int mt = it % m_tiles;
                 for (int ks = 0; ks < 2 * G && !*failed; ++ks, ++suse) {
-                    const int xs = suse % XST;
-                    // rings of equal depth share one "stage free" barrier (one commit per stage instead of two)
-                    if (!bar_wait(XST == TC_STAGES ? &sh->sempty[xs] : &sh->xempty[xs], ((suse / XST) & 1) ^ 1, failed)) break;
-                    bar_expect_tx(&sh->xfull[xs], B_BYTES);
-                    tma_load_2d(b_st + xs * B_BYTES, &xmap, ks * 64, mt * NTOK, &sh->xfull[xs]);
+                    const int st = suse % TC_STAGES;
+                    if (!bar_wait(&sh->empty[st], ((suse / TC_STAGES) & 1) ^ 1, failed)) break;
+                    bar_expect_tx(&sh->full[st], B_BYTES);
+                    tma_load_2d(b_st + st * B_BYTES, &xmap, ks * 64, mt * NTOK, &sh->full[st]);
                 }
             }
         }
@@ -133,73 +130,60 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const float *__restr
             if (!bar_wait(&sh->accempty[ab], ((tuse >> 1) & 1) ^ 1, failed)) break;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const uint32_t tacc = tmem + (uint32_t)(ab * NTOK);
-            for (int ks = 0; ks < 2 * G && !*failed; ++ks, ++suse) {
-                const int s = suse % TC_STAGES, xs = suse % XST;
-                if (!bar_wait(&sh->xfull[xs], (suse / XST) & 1, failed)) break;
-                if (!bar_wait(&sh->afull[s], (suse / TC_STAGES) & 1, failed)) break;
-                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                if (lane == 0) {
-                    const uint32_t a0 = sptr(a_st + s * TC_A_BYTES), b0 = sptr(b_st + xs * B_BYTES);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        umma_bf16(tacc, umma_desc(a0 + k * 32), umma_desc(b0 + k * 32), IDESC, (ks | k) != 0);
-                    umma_commit(&sh->sempty[s]);  // the operand stages are free when the MMAs retire
-                    if (XST != TC_STAGES) umma_commit(&sh->xempty[xs]);
+            for (int ks = 0; ks < 2 * G; ++ks, ++suse) {
+                const int st = suse % TC_STAGES;
+                if (!warp_wait(&sh->full[st], (suse / TC_STAGES) & 1, failed)) break;  // no tensor memory in a stage: no tcgen05 fence
+                if (elect_one()) {
+                    umma_stage(tacc, umma_desc(sptr(a_st + st * TC_A_BYTES)), umma_desc(sptr(b_st + st * B_BYTES)), IDESC, ks == 0);
+                    umma_commit(&sh->empty[st]);  // the stage is free when the MMAs retire
                 }
                 __syncwarp();
             }
-            if (lane == 0) umma_commit(&sh->accfull[ab]);
+            if (elect_one()) umma_commit(&sh->accfull[ab]);
             __syncwarp();
         }
-    } else if (warp < 10) {
+    } else if (warp < 2 + 4 * TC_SETS) {
         // ---------------------------------------------------------- codes -> bf16
-        const int u = threadIdx.x - 64;    // 0..255
-        const int t = u & 127;             // output channel within the 128-channel tile
-        const int hsel = u >> 7;           // which 32 of a stage's 64 K-elements this thread converts
-        uint32_t wuse = 0, suse = 0;
+        // a set of four warps takes the same half (64 K-elements, one stage) of every second group
+        const int t = (threadIdx.x - 64) & 127, set = (threadIdx.x - 64) >> 7, half = set & 1;
+        uint32_t gbase = 0;  // groups before this tile
         for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x) {
-            for (int g = 0; g < G && !*failed; ++g, ++wuse) {
+            for (uint32_t wuse = gbase + ((set >> 1) + TC_SETS - gbase % (TC_SETS / 2)) % (TC_SETS / 2); wuse < gbase + (uint32_t)G && !*failed; wuse += TC_SETS / 2) {
                 const int ws = wuse % TC_WSLOTS;
                 if (!bar_wait(&sh->wfull[ws], (wuse / TC_WSLOTS) & 1, failed)) break;
                 // row t of the slot: 128 codes in eight 16-byte chunks, chunk c stored at c ^ (t & 7)
                 const uint8_t *wrow = w_ring + ws * TC_WSLOT_BYTES + t * 128;
-                uint4 raw[2][2];
+                uint4 raw[4];
 #pragma unroll
-                for (int half = 0; half < 2; ++half)
+                for (int i = 0; i < 4; ++i) raw[i] = *reinterpret_cast<const uint4 *>(wrow + (((4 * half + i) ^ (t & 7)) << 4));
+                // one arrival per warp, fed by the loads of all its lanes
+                const uint32_t held = __reduce_or_sync(0xffffffffu, raw[0].x ^ raw[1].x ^ raw[2].x ^ raw[3].x);
+                if (lane == 0) bar_arrive_after(&sh->wempty[ws], held, (uint32_t)K & 1u);
+                const uint32_t suse = 2 * wuse + half;
+                const int s = suse % TC_STAGES;
+                if (!bar_wait(&sh->empty[s], ((suse / TC_STAGES) & 1) ^ 1, failed)) break;
+                uint8_t *arow = a_st + s * TC_A_BYTES + t * 128;
 #pragma unroll
-                    for (int i = 0; i < 2; ++i)
-                        raw[half][i] = *reinterpret_cast<const uint4 *>(wrow + (((4 * half + 2 * hsel + i) ^ (t & 7)) << 4));
-                bar_arrive_after(&sh->wempty[ws], raw[0][0].x ^ raw[0][1].x ^ raw[1][0].x ^ raw[1][1].x, (uint32_t)K & 1u);
+                for (int i = 0; i < 4; ++i) {  // 16 codes -> two chunks of 8 bf16
+                    const uint32_t w4[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+                    uint32_t o[8];
 #pragma unroll
-                for (int half = 0; half < 2; ++half, ++suse) {
-                    const int s = suse % TC_STAGES;
-                    if (!bar_wait(&sh->sempty[s], ((suse / TC_STAGES) & 1) ^ 1, failed)) break;
-                    uint8_t *arow = a_st + s * TC_A_BYTES + t * 128;
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) {  // 16 codes -> two chunks of 8 bf16
-                        const uint32_t w4[4] = {raw[half][i].x, raw[half][i].y, raw[half][i].z, raw[half][i].w};
-                        uint32_t o[8];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const uint32_t ub = w4[j] ^ 0x80808080u;  // b + 128 as unsigned bytes
-                            const float f0 = __uint_as_float(__byte_perm(ub, 0x4B000000u, 0x7540)) - 8388736.0f;
-                            const float f1 = __uint_as_float(__byte_perm(ub, 0x4B000000u, 0x7541)) - 8388736.0f;
-                            const float f2 = __uint_as_float(__byte_perm(ub, 0x4B000000u, 0x7542)) - 8388736.0f;
-                            const float f3 = __uint_as_float(__byte_perm(ub, 0x4B000000u, 0x7543)) - 8388736.0f;
-                            // exact small integers: the bf16 is the upper half of the float
-                            o[2 * j] = __byte_perm(__float_as_uint(f0), __float_as_uint(f1), 0x7632);
-                            o[2 * j + 1] = __byte_perm(__float_as_uint(f2), __float_as_uint(f3), 0x7632);
-                        }
-                        const int oc = 4 * hsel + 2 * i;  // chunk = 8 consecutive k of the stage row
-                        *reinterpret_cast<uint4 *>(arow + ((oc ^ (t & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-                        *reinterpret_cast<uint4 *>(arow + (((oc + 1) ^ (t & 7)) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
+                    for (int j = 0; j < 8; ++j) {
+                        // two codes into the low bytes of 16-bit halves; code = (128 + its low 7 bits) - (128 + its
+                        // sign's 128), both of which are a bf16 with those bits as mantissa: exact
+                        const uint32_t p = __byte_perm(w4[j >> 1], 0u, j & 1 ? 0x4342 : 0x4140);
+                        o[j] = bf16x2_add_((p & 0x007F007Fu) | 0x43004300u, (p & 0x00800080u) | 0xC300C300u);
                     }
-                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-                    bar_arrive(&sh->afull[s]);
+                    *reinterpret_cast<uint4 *>(arow + (((2 * i) ^ (t & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+                    *reinterpret_cast<uint4 *>(arow + (((2 * i + 1) ^ (t & 7)) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
                 }
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                __syncwarp();
+                if (lane == 0) bar_arrive(&sh->full[s]);
             }
+            gbase += (uint32_t)G;
         }
-    } else if (warp < 14) {
+    } else if (warp < TC_THREADS / 32 - 1) {
         // ---------------------------------------------------------- epilogue
         const int quad = warp & 3;
         uint32_t tuse = 0;
@@ -278,7 +262,7 @@ int launch_i8_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaStream
     if (rc != AB2_OK) return rc;
     rc = make_w8_map(&wmap, w->codes, w->N, w->K);
     if (rc != AB2_OK) return rc;
-    const size_t smem = 1024 + TC_STAGES * TC_A_BYTES + tc_xstages<NTOK>() * NTOK * 128 + TC_WSLOTS * TC_WSLOT_BYTES + sizeof(TcShared);
+    const size_t smem = 1024 + tc_stages<NTOK>() * (TC_A_BYTES + NTOK * 128) + tc_wslots<NTOK>() * TC_WSLOT_BYTES + sizeof(TcShared);
     static bool configured[64] = {false};  // the attribute is per device
     int dev = 0;
     AB2_CUDA(cudaGetDevice(&dev));

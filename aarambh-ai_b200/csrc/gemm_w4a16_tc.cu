@@ -10,7 +10,7 @@
 // persistent over tiles, warp-specialised:
 //   warp 0      producer of the packed weights: one ring slot per quantisation
 //               group, lane b issues the bulk copy of 16-channel block b
-//   warp 10     producer of the activations: TMA tile loads of X (128-byte
+//   warp 22     producer of the activations: TMA tile loads of X (128-byte
 //               swizzle) into the operand-B stages
 //   warp 1      allocates tensor memory, issues tcgen05.mma (K = 16 per
 //               instruction, 64 per stage), commits stage / accumulator barriers.
@@ -19,11 +19,11 @@
 //               tiles are 256 tokens wide where the token count allows, and the
 //               operand rings of that tile size have equal depth so that one
 //               commit per stage frees both operands
-//   warps 2-5   dequantise: thread = output channel; nibbles -> bf16 (128 + q by
+//   warps 2-17  dequantise, four sets of four warps on stages of their own; thread = output channel; nibbles -> bf16 (128 + q by
 //               one logic op, minus (128 + z) exactly, times the bf16 scale, i.e.
 //               the round-to-nearest bf16 of (q - z) * s) written into the
 //               operand-A stage in the canonical K-major 128-byte-swizzle layout
-//   warps 6-9   epilogue: tcgen05.ld of the accumulator, bf16 stores of Y
+//   warps 18-21 epilogue: tcgen05.ld of the accumulator, bf16 stores of Y
 // Every wait on an mbarrier is bounded; on a time-out the CTA records
 // AB2_ERR_TIMEOUT, stops issuing work, still frees its tensor memory and returns.
 #include <cuda.h>
@@ -42,40 +42,43 @@ int device_status_word(int **out);
 int device_sm_count();
 namespace {
 
-constexpr int TC_STAGES = 4;          // operand-A (unpacked weight) stages of 64 K-elements
-constexpr int TC_MAX_XSTAGES = 8;     // operand-B (activation) stages: a ring of its own, 128 KB deep, because an
-                                      // activation tile takes about three stage times to arrive from L2
-constexpr int TC_WSLOTS = 3;          // packed-weight ring slots (one quantisation group each)
+constexpr int TC_MAX_STAGES = 6, TC_MAX_WSLOTS = 10;
 constexpr int TC_BLOCK_WORDS = 272;   // 16 rows x 16 code words + 16 parameter words
 constexpr int TC_WSLOT_BYTES = 8 * TC_BLOCK_WORDS * 4;  // 8 row tiles of 16 = 128 channels
 constexpr int TC_A_BYTES = 128 * 128;  // 128 channels x 64 bf16
-constexpr int TC_THREADS = 352;
+constexpr int TC_SETS = 4;  // sets of four unpack warps; a set takes every TC_SETS-th stage
+constexpr int TC_UNPACK_WARPS = 4 * TC_SETS;
+constexpr int TC_THREADS = (2 + TC_UNPACK_WARPS + 4 + 1) * 32;
 
 struct TcShared {
-    uint64_t wfull[TC_WSLOTS], wempty[TC_WSLOTS];
-    uint64_t xfull[TC_MAX_XSTAGES], xempty[TC_MAX_XSTAGES], afull[TC_STAGES], sempty[TC_STAGES];
+    uint64_t wfull[TC_MAX_WSLOTS], wempty[TC_MAX_WSLOTS];
+    uint64_t full[TC_MAX_STAGES], empty[TC_MAX_STAGES];
     uint64_t accfull[2], accempty[2];  // two accumulators: the epilogue of a tile overlaps the next tile's MMAs
     uint32_t tmem_base;
     int failed;
 };
 
+// Stages of 64 K-elements: an unpacked weight tile and an activation tile that share one pair of barriers, so that
+// the issuing warp waits once per stage (a wait costs it about 150 cycles even when the stage is ready, and four MMAs
+// of 32 tokens only 160).  What they leave of shared memory goes to the packed-weight slots, one quantisation group
+// each.
 template <int NTOK>
-__host__ __device__ constexpr int tc_xstages() {
-    return NTOK > 128 ? TC_STAGES : TC_MAX_XSTAGES;
-}
+__host__ __device__ constexpr int tc_stages() { return NTOK > 128 ? 4 : 6; }
+template <int NTOK>
+__host__ __device__ constexpr int tc_wslots() { return NTOK > 32 ? 3 : TC_MAX_WSLOTS; }
 
 template <int NTOK>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CUtensorMap xmap,
                      __nv_bfloat16 *__restrict__ y, int N, int K, int M, int *status, int ksplit, float *part) {
     constexpr int B_BYTES = NTOK * 128;
-    constexpr int XST = tc_xstages<NTOK>();
+    constexpr int TC_STAGES = tc_stages<NTOK>(), TC_WSLOTS = tc_wslots<NTOK>();
     constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NTOK >> 3) << 17) | ((128u >> 4) << 24);
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t *a_st = smem;                                   // [TC_STAGES][TC_A_BYTES]
-    uint8_t *b_st = a_st + TC_STAGES * TC_A_BYTES;          // [XST][B_BYTES]
-    uint8_t *w_ring = b_st + XST * B_BYTES;                 // [TC_WSLOTS][TC_WSLOT_BYTES]
+    uint8_t *b_st = a_st + TC_STAGES * TC_A_BYTES;          // [TC_STAGES][B_BYTES]
+    uint8_t *w_ring = b_st + TC_STAGES * B_BYTES;                 // [TC_WSLOTS][TC_WSLOT_BYTES]
     TcShared *sh = (TcShared *)(w_ring + TC_WSLOTS * TC_WSLOT_BYTES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -92,9 +95,8 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
     volatile int *failed = &sh->failed;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < TC_WSLOTS; ++i) { bar_init(&sh->wfull[i], 1); bar_init(&sh->wempty[i], 128); }
-        for (int i = 0; i < TC_STAGES; ++i) { bar_init(&sh->afull[i], 128); bar_init(&sh->sempty[i], 1); }
-        for (int i = 0; i < XST; ++i) { bar_init(&sh->xfull[i], 1); bar_init(&sh->xempty[i], 1); }
+        for (int i = 0; i < TC_WSLOTS; ++i) { bar_init(&sh->wfull[i], 1); bar_init(&sh->wempty[i], 8); }
+        for (int i = 0; i < TC_STAGES; ++i) { bar_init(&sh->full[i], 4 + 1); bar_init(&sh->empty[i], 1); }
         for (int i = 0; i < 2; ++i) { bar_init(&sh->accfull[i], 1); bar_init(&sh->accempty[i], 4); }
         sh->failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -138,11 +140,10 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
             for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x) {
                 TC_ITEM(it)
                 for (int ks = 2 * g0; ks < 2 * g1 && !*failed; ++ks, ++suse) {
-                    const int xs = suse % XST;
-                    // rings of equal depth share one "stage free" barrier (one commit per stage instead of two)
-                    if (!bar_wait(XST == TC_STAGES ? &sh->sempty[xs] : &sh->xempty[xs], ((suse / XST) & 1) ^ 1, failed)) break;
-                    bar_expect_tx(&sh->xfull[xs], B_BYTES);
-                    tma_load_2d(b_st + xs * B_BYTES, &xmap, ks * 64, mt * NTOK, &sh->xfull[xs]);
+                    const int st = suse % TC_STAGES;
+                    if (!bar_wait(&sh->empty[st], ((suse / TC_STAGES) & 1) ^ 1, failed)) break;
+                    bar_expect_tx(&sh->full[st], B_BYTES);
+                    tma_load_2d(b_st + st * B_BYTES, &xmap, ks * 64, mt * NTOK, &sh->full[st]);
                 }
             }
         }
@@ -155,69 +156,64 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const uint32_t tacc = tmem + (uint32_t)(ab * NTOK);
             TC_ITEM(it)
-            for (int ks = 2 * g0; ks < 2 * g1 && !*failed; ++ks, ++suse) {
-                const int s = suse % TC_STAGES, xs = suse % XST;
-                if (!bar_wait(&sh->xfull[xs], (suse / XST) & 1, failed)) break;
-                if (!bar_wait(&sh->afull[s], (suse / TC_STAGES) & 1, failed)) break;
-                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                if (lane == 0) {
-                    const uint32_t a0 = sptr(a_st + s * TC_A_BYTES), b0 = sptr(b_st + xs * B_BYTES);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        umma_bf16(tacc, umma_desc(a0 + k * 32), umma_desc(b0 + k * 32), IDESC, ((ks - 2 * g0) | k) != 0);
-                    umma_commit(&sh->sempty[s]);  // the operand stages are free when the MMAs retire
-                    if (XST != TC_STAGES) umma_commit(&sh->xempty[xs]);
+            for (int ks = 2 * g0; ks < 2 * g1; ++ks, ++suse) {
+                const int st = suse % TC_STAGES;
+                if (!warp_wait(&sh->full[st], (suse / TC_STAGES) & 1, failed)) break;  // no tensor memory in a stage: no tcgen05 fence
+                if (elect_one()) {
+                    umma_stage(tacc, umma_desc(sptr(a_st + st * TC_A_BYTES)), umma_desc(sptr(b_st + st * B_BYTES)), IDESC, ks == 2 * g0);
+                    umma_commit(&sh->empty[st]);  // the stage is free when the MMAs retire
                 }
                 __syncwarp();
             }
-            if (lane == 0) umma_commit(&sh->accfull[ab]);
+            if (elect_one()) umma_commit(&sh->accfull[ab]);
             __syncwarp();
         }
-    } else if (warp < 6) {
+    } else if (warp < 2 + TC_UNPACK_WARPS) {
         // ---------------------------------------------------------- dequantise
-        const int t = threadIdx.x - 64;  // output channel within the 128-channel tile
-        const int blk = t >> 4, r = t & 15;
-        uint32_t wuse = 0, suse = 0;
+        const int t = (threadIdx.x - 64) & 127, set = (threadIdx.x - 64) >> 7;  // output channel within the 128-channel tile
+        const int blk = t >> 4, r = t & 15, half = set & 1;
+        uint32_t gbase = 0;  // groups before this tile
         uint32_t k_mask = 0x000F000Fu, k_magic = 0x43004300u;
         asm volatile("" : "+r"(k_mask), "+r"(k_magic));
         for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x) {
             TC_ITEM(it)
-            for (int g = g0; g < g1 && !*failed; ++g, ++wuse) {
+            // the set's groups: every (TC_SETS / 2)-th of the CTA's sequence of groups
+            for (uint32_t wuse = gbase + ((set >> 1) + TC_SETS - gbase % (TC_SETS / 2)) % (TC_SETS / 2); wuse < gbase + (uint32_t)(g1 - g0) && !*failed; wuse += TC_SETS / 2) {
                 const int ws = wuse % TC_WSLOTS;
                 if (!bar_wait(&sh->wfull[ws], (wuse / TC_WSLOTS) & 1, failed)) break;
                 const uint32_t *bw = (const uint32_t *)(w_ring + ws * TC_WSLOT_BYTES) + blk * TC_BLOCK_WORDS;
-                uint4 pw[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) pw[i] = *reinterpret_cast<const uint4 *>(bw + r * 16 + i * 4);
+                const uint4 pw[2] = {*reinterpret_cast<const uint4 *>(bw + r * 16 + half * 8), *reinterpret_cast<const uint4 *>(bw + r * 16 + half * 8 + 4)};
                 const uint32_t pr = bw[256 + r];
-                bar_arrive_after(&sh->wempty[ws], pw[0].x ^ pw[1].x ^ pw[2].x ^ pw[3].x ^ pr, (uint32_t)K & 1u);
+                // one arrival per warp, fed by the loads of all its lanes
+                const uint32_t held = __reduce_or_sync(0xffffffffu, pw[0].x ^ pw[1].x ^ pr);
+                if (lane == 0) bar_arrive_after(&sh->wempty[ws], held, (uint32_t)K & 1u);
                 const uint32_t sc2 = __byte_perm(pr, pr, 0x1010);  // bf16x2 (scale, scale)
                 const uint32_t nz2 = __byte_perm(pr, pr, 0x3232);  // bf16x2 -(128 + z)
+                const uint32_t suse = 2 * wuse + half;
+                const int s = suse % TC_STAGES;
+                if (!bar_wait(&sh->empty[s], ((suse / TC_STAGES) & 1) ^ 1, failed)) break;
+                uint8_t *arow = a_st + s * TC_A_BYTES + t * 128;
 #pragma unroll
-                for (int half = 0; half < 2; ++half, ++suse) {
-                    const int s = suse % TC_STAGES;
-                    if (!bar_wait(&sh->sempty[s], ((suse / TC_STAGES) & 1) ^ 1, failed)) break;
-                    uint8_t *arow = a_st + s * TC_A_BYTES + t * 128;
+                for (int c = 0; c < 8; ++c) {  // chunk c = 8 consecutive k = one code word
+                    const uint4 q4 = pw[c >> 2];
+                    const uint32_t word = (c & 3) == 0 ? q4.x : (c & 3) == 1 ? q4.y : (c & 3) == 2 ? q4.z : q4.w;
+                    uint32_t o[4];
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) {  // chunk c = 8 consecutive k = one code word
-                        const uint4 q4 = pw[half * 2 + (c >> 2)];
-                        const uint32_t word = (c & 3) == 0 ? q4.x : (c & 3) == 1 ? q4.y : (c & 3) == 2 ? q4.z : q4.w;
-                        uint32_t o[4];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            uint32_t v;
-                            const uint32_t shv = j ? (word >> (4 * j)) : word;
-                            asm("lop3.b32 %0, %1, %2, %3, 0xEA;\n" : "=r"(v) : "r"(shv), "r"(k_mask), "r"(k_magic));
-                            o[j] = bf16x2_mul_(bf16x2_add_(v, nz2), sc2);
-                        }
-                        *reinterpret_cast<uint4 *>(arow + ((c ^ (t & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+                    for (int j = 0; j < 4; ++j) {
+                        uint32_t v;
+                        const uint32_t shv = j ? (word >> (4 * j)) : word;
+                        asm("lop3.b32 %0, %1, %2, %3, 0xEA;\n" : "=r"(v) : "r"(shv), "r"(k_mask), "r"(k_magic));
+                        o[j] = bf16x2_mul_(bf16x2_add_(v, nz2), sc2);
                     }
-                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-                    bar_arrive(&sh->afull[s]);
+                    *reinterpret_cast<uint4 *>(arow + ((c ^ (t & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
                 }
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                __syncwarp();
+                if (lane == 0) bar_arrive(&sh->full[s]);
             }
+            gbase += (uint32_t)(g1 - g0);
         }
-    } else if (warp < 10) {
+    } else if (warp < TC_THREADS / 32 - 1) {
         // ---------------------------------------------------------- epilogue
         const int quad = warp & 3;
         uint32_t tuse = 0;
@@ -312,7 +308,7 @@ int launch_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t 
     CUtensorMap map;
     rc = make_x_map(&map, x, M, w->K, NTOK);
     if (rc != AB2_OK) return rc;
-    const size_t smem = 1024 + TC_STAGES * TC_A_BYTES + tc_xstages<NTOK>() * NTOK * 128 + TC_WSLOTS * TC_WSLOT_BYTES + sizeof(TcShared);
+    const size_t smem = 1024 + tc_stages<NTOK>() * (TC_A_BYTES + NTOK * 128) + tc_wslots<NTOK>() * TC_WSLOT_BYTES + sizeof(TcShared);
     static bool configured[64] = {false};  // the attribute is per device
     int dev = 0;
     AB2_CUDA(cudaGetDevice(&dev));

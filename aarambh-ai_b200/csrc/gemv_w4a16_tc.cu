@@ -208,20 +208,15 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
             for (int half = 0; half < 2 && !*failed; ++half) {
                 const uint32_t suse = 2 * use + half;
                 const int s = suse % DG_STAGES, xs = suse % DG_XSTAGES;
-                if (!bar_wait(&sh->xfull[xs], (suse / DG_XSTAGES) & 1, failed)) break;
-                if (!bar_wait(&sh->afull[s], (suse / DG_STAGES) & 1, failed)) break;
-                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                if (lane == 0) {
-                    const uint32_t a0 = sptr(a_st + s * DG_A_BYTES), b0 = sptr(b_st + xs * B_BYTES);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        umma_bf16(td, umma_desc(a0 + k * 32), umma_desc(b0 + k * 32), IDESC, (half | k) != 0);
+                if (!warp_wait(&sh->xfull[xs], (suse / DG_XSTAGES) & 1, failed) || !warp_wait(&sh->afull[s], (suse / DG_STAGES) & 1, failed)) break;
+                if (elect_one()) {
+                    umma_stage(td, umma_desc(sptr(a_st + s * DG_A_BYTES)), umma_desc(sptr(b_st + xs * B_BYTES)), IDESC, half == 0);
                     umma_commit(&sh->sempty[s]);  // the operand stages are free when the MMAs retire
                     umma_commit(&sh->xempty[xs]);
                 }
                 __syncwarp();
             }
-            if (lane == 0) umma_commit(&sh->accfull[ab]);
+            if (elect_one()) umma_commit(&sh->accfull[ab]);
             __syncwarp();
         }
     } else if (warp < 10) {
@@ -245,9 +240,9 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
             const uint32_t pr = bw[256 + r];
             if (half == 0) sh->params[use % DG_PARAM_BUFS][t] = pr;
             const uint32_t nz2 = __byte_perm(pr, pr, 0x3232);  // bf16x2 -(128 + zero) of this channel
-            // one arrival per warp: arrivals on one mbarrier serialise on its word
-            __syncwarp();
-            if (lane == 0) bar_arrive_after(&sh->wempty[q][ws], p0.x ^ p1.x ^ pr, (uint32_t)K & 1u);
+            // one arrival per warp (arrivals on one mbarrier serialise on its word), fed by the loads of all its lanes
+            const uint32_t held = __reduce_or_sync(0xffffffffu, p0.x ^ p1.x ^ pr);
+            if (lane == 0) bar_arrive_after(&sh->wempty[q][ws], held, (uint32_t)K & 1u);
             const uint32_t suse = 2 * use + half;
             const int s = suse % DG_STAGES;
             if (!bar_wait(&sh->sempty[s], ((suse / DG_STAGES) & 1) ^ 1, failed)) break;

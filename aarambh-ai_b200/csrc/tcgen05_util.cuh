@@ -108,6 +108,13 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n selp.u32 %0, 1, 0, e;\n}\n" : "=r"(p));
     return p;
 }
+// The four K = 16 steps of a stage of 64 K-elements, by one thread.  Its branch is taken with elect_one(): behind
+// `lane == 0` the compiler cannot know that a single thread is active and feeds the instruction's uniform operands
+// lane by lane.  Descriptors count in 16 bytes.
+__device__ __forceinline__ void umma_stage(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, bool first) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) umma_bf16(tmem_d, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, !first || k > 0);
+}
 // A wait of a whole warp, with one answer for it.
 __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volatile int *failed) { return __all_sync(0xffffffffu, bar_wait(bar, parity, failed)); }
 
