@@ -65,6 +65,18 @@ struct ab2_qweight {
 
 namespace ab2 {
 
+// Device memory for the kernels that a call launches on `stream`: taken and given back in the stream's order, so calls
+// on several threads and streams may overlap (scratch.cu).
+struct ScratchLease {
+    cudaStream_t stream;
+    void *ptr = nullptr;
+    explicit ScratchLease(cudaStream_t s) : stream(s) {}
+    ScratchLease(const ScratchLease &) = delete;
+    ScratchLease &operator=(const ScratchLease &) = delete;
+    ~ScratchLease();
+    int take(size_t bytes);
+};
+
 static inline size_t ceil_div(size_t a, size_t b) { return (a + b - 1) / b; }
 
 template <typename T> struct ActType;

@@ -231,27 +231,6 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const float *__restr
     }
 }
 
-// Tensor map of the codes: [N][K] bytes, tiles of 128 K x 128 channels, 128-byte swizzle.
-static int make_w8_map(CUtensorMap *map, const void *codes, int N, int K) {
-    static EncodeTiledFn encode = nullptr;
-    if (!encode) {
-        void *fn = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        AB2_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres));
-        AB2_REQUIRE(fn != nullptr && qres == cudaDriverEntryPointSuccess, AB2_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled is unavailable");
-        encode = (EncodeTiledFn)fn;
-    }
-    cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)N};
-    cuuint64_t strides[1] = {(cuuint64_t)K};
-    cuuint32_t box[2] = {128, 128};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(codes), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    AB2_REQUIRE(r == CUDA_SUCCESS, AB2_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
-    return AB2_OK;
-}
-
 template <int NTOK>
 int launch_i8_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t s) {
     int *status = nullptr;
@@ -260,7 +239,7 @@ int launch_i8_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaStream
     CUtensorMap xmap, wmap;
     rc = make_x_map(&xmap, x, M, w->K, NTOK);
     if (rc != AB2_OK) return rc;
-    rc = make_w8_map(&wmap, w->codes, w->N, w->K);
+    rc = make_bytes_map(&wmap, w->codes, w->N, w->K);
     if (rc != AB2_OK) return rc;
     const size_t smem = 1024 + tc_stages<NTOK>() * (TC_A_BYTES + NTOK * 128) + tc_wslots<NTOK>() * TC_WSLOT_BYTES + sizeof(TcShared);
     static bool configured[64] = {false};  // the attribute is per device

@@ -1,0 +1,351 @@
+// Q4_K_M-style block weights (256 values per block, 4-bit codes, f16 scale and minimum,
+// crates/aarambh-studio-quant/src/gguf_quant.rs:39-49: w = q * scale + min), bf16 activations, many tokens: the
+// prompts and larger batches of a GGUF-loaded model on the 5th-generation tensor cores.
+//
+//   y[t][n] = sum over blocks b of  scale[n][b] * (sum_k q[n][k] x[t][k]) + min[n][b] * X[t][b],
+//
+// X the sum of a token's activations over a block.  The codes enter the MMA as exact small integers; a block is 256
+// steps of K, after which its accumulator leaves tensor memory and the scale and the minimum are applied in f32, so
+// no weight is rounded.  A first kernel forms X and a copy of the activations whose groups of 8 are ordered
+// 0,4,1,5,2,6,3,7, the order in which one shift and one mask take codes out of a word of the reference's layout.
+//
+// As in the other tcgen05 kernels the 128 channels of a tile are the M dimension of the MMA and NTOK tokens its N
+// dimension, one persistent CTA per SM:
+//   warp 0       producer of the codes: a TMA tile of 128 channels x one block per slot
+//   warp 1       MMA issue; two accumulators, a block each in turn
+//   warps 2-9    unpack, two sets of four warps on alternate stages of 64 K-elements, thread = channel
+//   warps 10-17  epilogue, thread = channel and half of the tokens, running sums in registers
+//   warp 18      producer of the activation tiles and of X
+// With fewer tiles than SMs the blocks of a tile are divided over several CTAs; their f32 sums meet in a reduce pass.
+// What bounds it is the unpack and the per-block epilogue (about 450 cycles a stage against the MMA's 257 at 128
+// tokens).  14336 x 4096 at 300 tokens: 3329 us on CUDA cores,
+// 88 us here (400 TFLOP/s); 3072 x 2048: 421 -> 20 us, at 9 tokens 17 -> 11.
+// Every wait on an mbarrier is bounded; on a time-out the CTA records AB2_ERR_TIMEOUT, stops issuing work, frees its
+// tensor memory and returns.
+#include <cuda.h>
+
+#include <algorithm>
+
+#include "common.cuh"
+#include "tcgen05_util.cuh"
+
+using namespace ab2;
+using namespace ab2::tc;
+
+namespace ab2 {
+int device_status_word(int **out);
+int device_sm_count();
+void launch_splitk_reduce(const float *part, __nv_bfloat16 *y, int M, int N, int ksplit, cudaStream_t s);
+namespace {
+
+constexpr int QB_MAX_STAGES = 6, QB_MAX_WSLOTS = 6;
+constexpr int QB_A_BYTES = 128 * 128;      // 128 channels x 64 bf16
+constexpr int QB_WSLOT_BYTES = 128 * 128;  // 128 channels x 256 codes
+constexpr int QB_UNPACK_WARPS = 8, QB_EPI_WARPS = 8;
+constexpr int QB_THREADS = (2 + QB_UNPACK_WARPS + QB_EPI_WARPS + 1) * 32;
+
+template <int NTOK>
+__host__ __device__ constexpr int qb_stages() { return NTOK > 64 ? 5 : 6; }
+template <int NTOK>
+__host__ __device__ constexpr int qb_wslots() { return NTOK > 64 ? 3 : NTOK > 32 ? 4 : QB_MAX_WSLOTS; }
+
+struct QbShared {
+    uint64_t wfull[QB_MAX_WSLOTS], wempty[QB_MAX_WSLOTS];
+    uint64_t full[QB_MAX_STAGES], empty[QB_MAX_STAGES];
+    uint64_t accfull[2], accempty[2], xsfull[2];
+    uint32_t tmem_base;
+    int failed;
+    alignas(16) float xsum[2][128];
+};
+
+struct QbArgs {
+    const uint32_t *params;  // [N][KB]
+    const float *xsum;       // [KB][Mp]
+    __nv_bfloat16 *y;
+    float *part;             // [ksplit][M][N] with a K split
+    int N, KB, M, Mp, ksplit;
+};
+
+// A warp per (token, block): the block's sum and its activations in the order of the unpacked codes.
+__global__ void __launch_bounds__(256) q4km_prepare_kernel(const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__restrict__ xp, float *__restrict__ xsum,
+                                                           int M, int Mp, int K) {
+    const int b = blockIdx.x, t = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (t >= Mp) return;
+    float sum = 0.f;
+    if (t < M) {
+        const size_t at = (size_t)t * K + b * 256 + lane * 8;
+        const uint4 v = *reinterpret_cast<const uint4 *>(x + at);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sum += __uint_as_float(w[j] << 16) + __uint_as_float(w[j] & 0xffff0000u);
+        *reinterpret_cast<uint4 *>(xp + at) = make_uint4(__byte_perm(v.x, v.z, 0x5410), __byte_perm(v.x, v.z, 0x7632),
+                                                         __byte_perm(v.y, v.w, 0x5410), __byte_perm(v.y, v.w, 0x7632));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) xsum[(size_t)b * Mp + t] = sum;
+}
+
+template <int NTOK>
+__global__ void __launch_bounds__(QB_THREADS, 1)
+gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, QbArgs a, int *status) {
+    constexpr int STAGES = qb_stages<NTOK>(), WSLOTS = qb_wslots<NTOK>(), B_BYTES = NTOK * 128;
+    constexpr uint32_t TMEM_COLS = 2 * NTOK;
+    constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NTOK >> 3) << 17) | ((128u >> 4) << 24);
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *a_st = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);  // [STAGES][QB_A_BYTES]
+    uint8_t *b_st = a_st + STAGES * QB_A_BYTES;                                    // [STAGES][B_BYTES]
+    uint8_t *w_ring = b_st + STAGES * B_BYTES;                                     // [WSLOTS][QB_WSLOT_BYTES]
+    QbShared *sh = (QbShared *)(w_ring + WSLOTS * QB_WSLOT_BYTES);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n_tiles = (a.N + 127) >> 7, m_tiles = (a.M + NTOK - 1) / NTOK, items = n_tiles * m_tiles * a.ksplit;
+    volatile int *failed = &sh->failed;
+    // item: (channel tile, token tile, share of the blocks)
+    auto item = [&](int it, int &nt, int &mt, int &sp, int &b0, int &b1) {
+        sp = it % a.ksplit;
+        mt = it / a.ksplit % m_tiles;
+        nt = it / a.ksplit / m_tiles;
+        b0 = (int)((long long)sp * a.KB / a.ksplit);
+        b1 = (int)((long long)(sp + 1) * a.KB / a.ksplit);
+    };
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < WSLOTS; ++i) { bar_init(&sh->wfull[i], 1); bar_init(&sh->wempty[i], QB_UNPACK_WARPS); }
+        for (int i = 0; i < STAGES; ++i) { bar_init(&sh->full[i], 4 + 1); bar_init(&sh->empty[i], 1); }
+        for (int i = 0; i < 2; ++i) { bar_init(&sh->accfull[i], 1); bar_init(&sh->accempty[i], QB_EPI_WARPS); bar_init(&sh->xsfull[i], 1); }
+        sh->failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    }
+    if (warp == 1) {  // tensor-memory allocation is a whole-warp operation
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(sptr(&sh->tmem_base)), "r"(TMEM_COLS));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tmem = sh->tmem_base;
+    int nt, mt, sp, b0, b1;
+
+    if (warp == 0) {
+        // ---------------------------------------------------------- producer of the codes
+        if (lane == 0) {
+            uint32_t wuse = 0;
+            for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x) {
+                item(it, nt, mt, sp, b0, b1);
+                for (int b = b0; b < b1 && !*failed; ++b, ++wuse) {
+                    const int ws = wuse % WSLOTS;
+                    if (!bar_wait(&sh->wempty[ws], ((wuse / WSLOTS) & 1) ^ 1, failed)) break;
+                    bar_expect_tx(&sh->wfull[ws], QB_WSLOT_BYTES);  // rows past N arrive as zeros and count
+                    tma_load_2d(w_ring + ws * QB_WSLOT_BYTES, &wmap, b * 128, nt * 128, &sh->wfull[ws]);
+                }
+            }
+        }
+    } else if (warp == QB_THREADS / 32 - 1) {
+        // ---------------------------------------------------------- producer of the activation tiles and their sums
+        if (lane == 0) {
+            uint32_t suse = 0, buse = 0;
+            for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x) {
+                item(it, nt, mt, sp, b0, b1);
+                for (int b = b0; b < b1 && !*failed; ++b, ++buse) {
+                    const int ab = buse & 1;
+                    if (!bar_wait(&sh->accempty[ab], ((buse >> 1) & 1) ^ 1, failed)) break;
+                    bar_expect_tx(&sh->xsfull[ab], NTOK * 4);
+                    bulk_copy(sh->xsum[ab], a.xsum + (size_t)b * a.Mp + mt * NTOK, NTOK * 4, &sh->xsfull[ab]);
+                    for (int q = 0; q < 4; ++q, ++suse) {
+                        const int st = suse % STAGES;
+                        if (!bar_wait(&sh->empty[st], ((suse / STAGES) & 1) ^ 1, failed)) break;
+                        bar_expect_tx(&sh->full[st], B_BYTES);
+                        tma_load_2d(b_st + st * B_BYTES, &xmap, b * 256 + q * 64, mt * NTOK, &sh->full[st]);
+                    }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ---------------------------------------------------------- MMA issue
+        uint32_t suse = 0, buse = 0;
+        bool ok = true;
+        for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+            item(it, nt, mt, sp, b0, b1);
+            for (int b = b0; b < b1 && ok; ++b, ++buse) {
+                const int ab = buse & 1;
+                ok = warp_wait(&sh->accempty[ab], ((buse >> 1) & 1) ^ 1, failed);
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                for (int q = 0; q < 4 && ok; ++q, ++suse) {
+                    const int st = suse % STAGES;
+                    ok = warp_wait(&sh->full[st], (suse / STAGES) & 1, failed);
+                    if (!ok) break;
+                    if (elect_one()) {
+                        umma_stage(tmem + (uint32_t)(ab * NTOK), umma_desc(sptr(a_st + st * QB_A_BYTES)), umma_desc(sptr(b_st + st * B_BYTES)), IDESC, q == 0);
+                        umma_commit(&sh->empty[st]);
+                        if (q == 3) umma_commit(&sh->accfull[ab]);
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+    } else if (warp < 2 + QB_UNPACK_WARPS) {
+        // ---------------------------------------------------------- unpack: codes -> bf16 integers
+        const int t = (threadIdx.x - 64) & 127, set = (threadIdx.x - 64) >> 7;
+        uint32_t wuse = 0;
+        uint32_t k_mask = 0x000F000Fu, k_magic = 0x43004300u, k_off = 0xC300C300u;  // -128
+        asm volatile("" : "+r"(k_mask), "+r"(k_magic), "+r"(k_off));
+        for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x) {
+            item(it, nt, mt, sp, b0, b1);
+            for (int b = b0; b < b1 && !*failed; ++b, ++wuse) {
+                const int ws = wuse % WSLOTS;
+                if (!bar_wait(&sh->wfull[ws], (wuse / WSLOTS) & 1, failed)) break;
+                // row t of the slot: 256 codes in eight 16-byte chunks, chunk c stored at c ^ (t & 7); the set takes quarters
+                // set and set + 2 of the block
+                const uint8_t *wrow = w_ring + ws * QB_WSLOT_BYTES + t * 128;
+                uint4 raw[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) raw[i] = *reinterpret_cast<const uint4 *>(wrow + (((2 * set + (i & 1) + 4 * (i >> 1)) ^ (t & 7)) << 4));
+                const uint32_t held = __reduce_or_sync(0xffffffffu, raw[0].x ^ raw[1].x ^ raw[2].x ^ raw[3].x);
+                if (lane == 0) bar_arrive_after(&sh->wempty[ws], held, (uint32_t)a.KB >> 30);
+#pragma unroll 1
+                for (int h = 0; h < 2; ++h) {
+                    const uint32_t suse = 4 * wuse + set + 2 * h;
+                    const int st = suse % STAGES;
+                    if (!bar_wait(&sh->empty[st], ((suse / STAGES) & 1) ^ 1, failed)) break;
+                    uint8_t *arow = a_st + st * QB_A_BYTES + t * 128;
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        const uint4 q4 = h ? raw[2 + (c >> 2)] : raw[c >> 2];
+                        const uint32_t word = (c & 3) == 0 ? q4.x : (c & 3) == 1 ? q4.y : (c & 3) == 2 ? q4.z : q4.w;
+                        uint32_t o[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {  // codes j and j + 4
+                            uint32_t v;
+                            const uint32_t shv = j ? (word >> (4 * j)) : word;
+                            asm("lop3.b32 %0, %1, %2, %3, 0xEA;\n" : "=r"(v) : "r"(shv), "r"(k_mask), "r"(k_magic));
+                            o[j] = bf16x2_add_(v, k_off);
+                        }
+                        *reinterpret_cast<uint4 *>(arow + ((c ^ (t & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) bar_arrive(&sh->full[st]);
+                }
+            }
+        }
+    } else {
+        // ---------------------------------------------------------- epilogue
+        constexpr int COLS = NTOK / 2;  // tokens of a thread
+        const int quad = warp & 3, half = (warp - 2 - QB_UNPACK_WARPS) >> 2;
+        uint32_t buse = 0;
+        bool ok = true;
+        for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+            item(it, nt, mt, sp, b0, b1);
+            const int n = nt * 128 + quad * 32 + lane;
+            const uint32_t *prm = a.params + (size_t)min(n, a.N - 1) * a.KB;
+            float acc[COLS];
+#pragma unroll
+            for (int j = 0; j < COLS; ++j) acc[j] = 0.f;
+            uint32_t next = __ldg(prm + b0);
+            for (int b = b0; b < b1; ++b, ++buse) {
+                const int ab = buse & 1;
+                const float s = f16_bits_to_f32((uint16_t)(next & 0xffffu)), m = f16_bits_to_f32((uint16_t)(next >> 16));
+                if (b + 1 < b1) next = __ldg(prm + b + 1);
+                ok = warp_wait(&sh->xsfull[ab], (buse >> 1) & 1, failed) && warp_wait(&sh->accfull[ab], (buse >> 1) & 1, failed);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                const float *xs = sh->xsum[ab] + half * COLS;
+                const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(ab * NTOK + half * COLS);
+#pragma unroll
+                for (int c = 0; c < COLS / 8; ++c) {
+                    uint32_t v[8];
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                        : "r"(taddr + 8 * c));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+                    for (int j = 0; j < 8; j += 4) {
+                        const float4 X = *reinterpret_cast<const float4 *>(xs + 8 * c + j);
+                        acc[8 * c + j] += fmaf(s, __uint_as_float(v[j]), m * X.x);
+                        acc[8 * c + j + 1] += fmaf(s, __uint_as_float(v[j + 1]), m * X.y);
+                        acc[8 * c + j + 2] += fmaf(s, __uint_as_float(v[j + 2]), m * X.z);
+                        acc[8 * c + j + 3] += fmaf(s, __uint_as_float(v[j + 3]), m * X.w);
+                    }
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                // the arrival also gives X's slot back: its loads have fed the sums
+                uint32_t held = 0;
+#pragma unroll
+                for (int j = 0; j < COLS; j += 4) held ^= __float_as_uint(acc[j]);
+                held = __reduce_or_sync(0xffffffffu, held);
+                if (lane == 0) bar_arrive_after(&sh->accempty[ab], held, (uint32_t)a.KB >> 30);
+            }
+            const int t0 = mt * NTOK + half * COLS;
+#pragma unroll
+            for (int j = 0; j < COLS; ++j)
+                if (ok && n < a.N && t0 + j < a.M) {
+                    if (a.ksplit > 1) a.part[((size_t)sp * a.M + t0 + j) * a.N + n] = acc[j];
+                    else a.y[(size_t)(t0 + j) * a.N + n] = __float2bfloat16_rn(acc[j]);
+                }
+            __syncwarp();
+        }
+    }
+
+    // ---- teardown: every warp arrives here (all waits are bounded)
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x == 0 && sh->failed) atomicExch(status, (int)AB2_ERR_TIMEOUT);
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS));
+    }
+}
+
+template <int NTOK>
+int launch_qb(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t s) {
+    int *status = nullptr;
+    int rc = device_status_word(&status);
+    if (rc != AB2_OK) return rc;
+    const int N = w->N, K = w->K, KB = K / 256, Mp = (M + NTOK - 1) / NTOK * NTOK;
+    const size_t smem = 1024 + qb_stages<NTOK>() * (QB_A_BYTES + NTOK * 128) + qb_wslots<NTOK>() * QB_WSLOT_BYTES + sizeof(QbShared);
+    static_assert(1024 + qb_stages<NTOK>() * (QB_A_BYTES + NTOK * 128) + qb_wslots<NTOK>() * QB_WSLOT_BYTES + sizeof(QbShared) <= 227 * 1024, "shared memory of a CTA");
+    static bool configured[64] = {false};  // the attribute is per device
+    int dev = 0;
+    AB2_CUDA(cudaGetDevice(&dev));
+    AB2_REQUIRE(dev >= 0 && dev < 64, AB2_ERR_BAD_ARG, "device index %d out of range", dev);
+    if (!configured[dev]) {
+        AB2_CUDA(cudaFuncSetAttribute(gemm_q4km_tc_kernel<NTOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        configured[dev] = true;
+    }
+    // as many shares of K as make one wave of items, at least two blocks each
+    const int tiles = ((N + 127) / 128) * (Mp / NTOK), sms = device_sm_count();
+    const int ksplit = N % 8 == 0 ? std::max(1, std::min(std::min(8, KB / 2), sms / tiles)) : 1;
+    const size_t xp_bytes = ((size_t)M * K * 2 + 255) & ~(size_t)255, xs_bytes = ((size_t)KB * Mp * 4 + 255) & ~(size_t)255;
+    const size_t part_bytes = ksplit > 1 ? (size_t)ksplit * M * N * 4 : 0;
+    ScratchLease ws(s);
+    rc = ws.take(xp_bytes + xs_bytes + part_bytes);
+    if (rc != AB2_OK) return rc;
+    __nv_bfloat16 *xp = (__nv_bfloat16 *)ws.ptr;
+    float *xsum = (float *)((char *)ws.ptr + xp_bytes), *part = (float *)((char *)ws.ptr + xp_bytes + xs_bytes);
+    CUtensorMap wmap, xmap;
+    rc = make_x_map(&xmap, xp, M, K, NTOK);
+    if (rc == AB2_OK) rc = make_bytes_map(&wmap, w->codes, N, K / 2);
+    if (rc != AB2_OK) return rc;
+    q4km_prepare_kernel<<<dim3(KB, (Mp + 7) / 8), 256, 0, s>>>((const __nv_bfloat16 *)x, xp, xsum, M, Mp, K);
+    const QbArgs a = {w->block_params, xsum, (__nv_bfloat16 *)y, part, N, KB, M, Mp, ksplit};
+    gemm_q4km_tc_kernel<NTOK><<<std::min(tiles * ksplit, sms), QB_THREADS, smem, s>>>(wmap, xmap, a, status);
+    if (ksplit > 1) launch_splitk_reduce(part, (__nv_bfloat16 *)y, M, N, ksplit, s);
+    AB2_LAUNCH_CHECK();
+    return AB2_OK;
+}
+
+}  // namespace
+
+bool qlinear_q4km_tc_eligible(const ab2_qweight *w, ab2_dtype dtype) { return w->fmt == FMT_Q4KM && dtype == AB2_BF16 && w->K % 256 == 0; }
+
+int qlinear_q4km_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t s) {
+    // the token tile that leaves the fewest padded tokens in the fewest waves, larger tiles unpacking less
+    if (M <= 32) return launch_qb<32>(w, x, M, y, s);
+    if (M <= 64) return launch_qb<64>(w, x, M, y, s);
+    return launch_qb<128>(w, x, M, y, s);
+}
+
+}  // namespace ab2

@@ -40,6 +40,7 @@ using namespace ab2::tc;
 namespace ab2 {
 int device_status_word(int **out);
 int device_sm_count();
+void launch_splitk_reduce(const float *part, __nv_bfloat16 *y, int M, int N, int ksplit, cudaStream_t s);
 namespace {
 
 constexpr int TC_MAX_STAGES = 6, TC_MAX_WSLOTS = 10;
@@ -282,23 +283,7 @@ __global__ void splitk_reduce_kernel(const float *__restrict__ part, __nv_bfloat
     reinterpret_cast<uint4 *>(y)[i] = make_uint4(o[0], o[1], o[2], o[3]);
 }
 
-// Workspace of the K split, one per device, grown on demand (prefill passes are not captured in graphs;
-// a capture in progress simply runs without the split).
 constexpr size_t TC_SPLIT_MAX_BYTES = (size_t)128 << 20;
-static float *g_split_ws[64] = {nullptr};
-static size_t g_split_bytes[64] = {0};
-static float *split_workspace(int dev, size_t bytes, cudaStream_t s) {
-    if (g_split_bytes[dev] >= bytes) return g_split_ws[dev];
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return nullptr;
-    if (cudaDeviceSynchronize() != cudaSuccess) return nullptr;
-    if (g_split_ws[dev]) cudaFree(g_split_ws[dev]);
-    g_split_ws[dev] = nullptr;
-    g_split_bytes[dev] = 0;
-    if (cudaMalloc((void **)&g_split_ws[dev], bytes) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-    g_split_bytes[dev] = bytes;
-    return g_split_ws[dev];
-}
 
 template <int NTOK>
 int launch_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t s) {
@@ -323,26 +308,34 @@ int launch_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t 
     const int sms = device_sm_count(), G = w->K / 128;
     int ksplit = 1;
     float *part = nullptr;
+    ScratchLease ws(s);
     static const bool no_split = getenv("AB2_GEMM_NO_SPLITK") != nullptr;
     if (!no_split && tiles * 2 <= sms + sms / 4 && G >= 8 && w->N % 8 == 0) {
         ksplit = std::max(1, std::min(4, std::min(G / 4, sms / tiles)));  // all items in one wave
         const size_t bytes = (size_t)ksplit * M * w->N * sizeof(float);
-        part = ksplit > 1 && bytes <= TC_SPLIT_MAX_BYTES ? split_workspace(dev, bytes, s) : nullptr;
-        if (!part) ksplit = 1;
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (bytes > TC_SPLIT_MAX_BYTES || cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) ksplit = 1;
+        if (ksplit > 1) {
+            rc = ws.take(bytes);
+            if (rc != AB2_OK) return rc;
+            part = (float *)ws.ptr;
+        }
     }
     const int items = tiles * ksplit;
     const int grid = std::min(items, sms);
     gemm_w4a16_tc_kernel<NTOK><<<grid, TC_THREADS, smem, s>>>((const uint32_t *)w->codes, map, (__nv_bfloat16 *)y, w->N, w->K, M, status, ksplit, part);
+    if (ksplit > 1) launch_splitk_reduce(part, (__nv_bfloat16 *)y, M, w->N, ksplit, s);
     AB2_LAUNCH_CHECK();
-    if (ksplit > 1) {
-        const size_t n8 = (size_t)M * w->N / 8;
-        splitk_reduce_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, s>>>(part, (__nv_bfloat16 *)y, n8, (size_t)M * w->N, ksplit);
-        AB2_LAUNCH_CHECK();
-    }
     return AB2_OK;
 }
 
 }  // namespace
+
+// y[M][N] = bf16(sum of the splits' part[ksplit][M][N]); N is a multiple of 8
+void launch_splitk_reduce(const float *part, __nv_bfloat16 *y, int M, int N, int ksplit, cudaStream_t s) {
+    const size_t n8 = (size_t)M * N / 8;
+    splitk_reduce_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, s>>>(part, y, n8, (size_t)M * N, ksplit);
+}
 
 // Y[M][N] = X[M][K] . W^T on the tcgen05 path (W4A16, group 128, bf16).
 int qlinear_w4a16_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t s) {

@@ -5,7 +5,7 @@
 #include <utility>
 
 #include "common.cuh"
-#include "gemv_generic.cuh"
+#include "gemm_generic.cuh"
 #include "tp.cuh"
 #include "gemv_w4a16_mma.cuh"
 #include "gemv_w4a16_warp.cuh"
@@ -16,6 +16,8 @@
 using namespace ab2;
 
 namespace ab2 {
+
+int device_sm_count();
 
 GemvArgs gemv_args_of(const ab2_qweight *w) {
     GemvArgs a;
@@ -29,6 +31,16 @@ template <int FMT, typename T>
 static int launch_generic(const ab2_qweight *w, const T *x, int M, T *y, cudaStream_t s) {
     GemvArgs a = gemv_args_of(w);
     dim3 grid((w->N + 7) / 8), block(256);
+    // From 9 tokens on, tiles: a warp per row would read its row from the caches once for every 4 tokens.
+    if (M > 8) {
+        // 64 x 64 outputs where that gives at least a tile per SM, else 32 x 32
+        if (((size_t)(w->N + 63) / 64) * ((M + 63) / 64) >= (size_t)device_sm_count())
+            gemm_generic_kernel<FMT, T, 64, 64><<<dim3((w->N + 63) / 64, (M + 63) / 64), 256, 0, s>>>(a, x, y, M);
+        else
+            gemm_generic_kernel<FMT, T, 32, 32><<<dim3((w->N + 31) / 32, (M + 31) / 32), 64, 0, s>>>(a, x, y, M);
+        AB2_LAUNCH_CHECK();
+        return AB2_OK;
+    }
     // one launch whatever the token count: the kernel walks the tokens in groups of MT
     if (M == 1) gemv_generic_kernel<FMT, T, 1><<<grid, block, 0, s>>>(a, x, y, M);
     else if (M == 2) gemv_generic_kernel<FMT, T, 2><<<grid, block, 0, s>>>(a, x, y, M);
@@ -405,6 +417,8 @@ int qlinear_w4a16_norm_peer(const ab2_qweight *w, const void *x, const float *no
 int qlinear_w4a16_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t s);
 bool qlinear_i8_stream_eligible(const ab2_qweight *w, ab2_dtype dtype, int M);
 bool qlinear_q4km_stream_eligible(const ab2_qweight *w, ab2_dtype dtype, int M);
+bool qlinear_q4km_tc_eligible(const ab2_qweight *w, ab2_dtype dtype);
+int qlinear_q4km_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t s);
 int qlinear_q4km_stream(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t s);
 int qlinear_i8_stream(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t s);
 bool qlinear_i8_tc_eligible(const ab2_qweight *w, ab2_dtype dtype, int M);
@@ -425,6 +439,8 @@ int qlinear_dispatch(const ab2_qweight *w, const void *x, int M, ab2_dtype dtype
     if (qlinear_i8_tc_eligible(w, dtype, M)) return qlinear_i8_tc(w, x, M, y, s);
     // Q4_K_M blocks (GGUF-loaded models), bf16 activations, a few tokens: the streaming GEMV over the two planes
     if (qlinear_q4km_stream_eligible(w, dtype, M)) return qlinear_q4km_stream(w, x, M, y, s);
+    // more tokens: tcgen05 GEMM, scale and minimum applied in f32 per block
+    if (qlinear_q4km_tc_eligible(w, dtype)) return qlinear_q4km_tc(w, x, M, y, s);
     return qlinear_generic(w, x, M, dtype, y, s);
 }
 

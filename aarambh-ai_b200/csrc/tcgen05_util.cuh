@@ -69,6 +69,13 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
             "r"(sptr(dst)), "l"(map), "r"(sptr(bar)), "r"(x), "r"(y) : "memory");
 }
 
+// 3-D tile load: coordinates (element, row, matrix).
+__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int x, int y, int z, uint64_t *bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n" ::
+            "r"(sptr(dst)), "l"(map), "r"(sptr(bar)), "r"(x), "r"(y), "r"(z) : "memory");
+}
+
 // Shared-memory matrix descriptor, K-major, 128-byte swizzle: 8-row groups are
 // 1024 bytes apart, the start address advances by 32 bytes per K = 16 step.
 __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
@@ -134,8 +141,7 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-// Tensor map of a [M][K] bf16 matrix whose rows lie `ld` elements apart (0: K), read in boxes of 64 x ntok.
-inline int make_x_map(CUtensorMap *map, const void *x, int M, int K, int ntok, long long ld = 0) {
+inline int tensor_map_encoder(EncodeTiledFn *out) {
     static EncodeTiledFn encode = nullptr;
     if (!encode) {
         void *fn = nullptr;
@@ -144,15 +150,50 @@ inline int make_x_map(CUtensorMap *map, const void *x, int M, int K, int ntok, l
         AB2_REQUIRE(fn != nullptr && qres == cudaDriverEntryPointSuccess, AB2_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled is unavailable");
         encode = (EncodeTiledFn)fn;
     }
-    cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)M};
-    cuuint64_t strides[1] = {(cuuint64_t)(ld > 0 ? ld : K) * 2};
-    cuuint32_t box[2] = {64, (cuuint32_t)ntok};
+    *out = encode;
+    return AB2_OK;
+}
+
+// Tensor map of `rows` rows of `cols` elements that lie `ld` elements apart, read in boxes of 128 bytes x box_rows
+// (128-byte swizzle).
+inline int make_rows_map(CUtensorMap *map, CUtensorMapDataType type, int elem, const void *p, int rows, int cols, long long ld, int box_rows) {
+    EncodeTiledFn encode;
+    int rc = tensor_map_encoder(&encode);
+    if (rc != AB2_OK) return rc;
+    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)ld * elem};
+    cuuint32_t box[2] = {(cuuint32_t)(128 / elem), (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
-    CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(x), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    CUresult r = encode(map, type, 2, const_cast<void *>(p), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     AB2_REQUIRE(r == CUDA_SUCCESS, AB2_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
     return AB2_OK;
+}
+
+// Tensor map of a [M][K] bf16 matrix whose rows lie `ld` elements apart (0: K), read in boxes of 64 x ntok.
+inline int make_x_map(CUtensorMap *map, const void *x, int M, int K, int ntok, long long ld = 0) {
+    return make_rows_map(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, M, K, ld > 0 ? ld : K, ntok);
+}
+
+// Tensor map of `mats` bf16 matrices of `rows` rows x `cols`, rows `ld` and matrices `z` elements apart, read in boxes
+// of 64 x box_rows of one matrix.
+inline int make_mats_map(CUtensorMap *map, const void *p, int mats, int rows, int cols, long long ld, long long z, int box_rows) {
+    EncodeTiledFn encode;
+    int rc = tensor_map_encoder(&encode);
+    if (rc != AB2_OK) return rc;
+    cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)mats};
+    cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)z * 2};
+    cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(p), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    AB2_REQUIRE(r == CUDA_SUCCESS, AB2_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
+    return AB2_OK;
+}
+
+// Tensor map of [N][bytes] bytes, read in boxes of 128 x 128.
+inline int make_bytes_map(CUtensorMap *map, const void *p, int N, int bytes) {
+    return make_rows_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p, N, bytes, bytes, 128);
 }
 
 

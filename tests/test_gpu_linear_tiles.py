@@ -1,0 +1,77 @@
+"""Linears of many tokens over the reference's formats: the tcgen05 GEMM over Q4_K_M-style blocks (bf16, from 9 tokens
+on) and the tiled CUDA-core GEMM (every other format and type from 9 tokens on), against the product with the
+dequantised weight in 64 bits.  An f32 sum of n terms is within n 2^-24 of the sum of their magnitudes, a bf16
+output within 2^-8 of itself."""
+import pytest
+import torch
+
+from helpers import pkg
+
+pytestmark = pytest.mark.gpu
+
+
+def check(lin, x, terms):
+    y = lin(x).double()
+    w = lin.dequantise().double()
+    ref, size = x.double() @ w.T, x.double().abs() @ w.abs().T
+    rounding = {torch.float32: 0.0, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[x.dtype]
+    assert torch.isfinite(y).all()
+    assert bool(((y - ref).abs() <= rounding * ref.abs() + terms * 2.0 ** -24 * size + 1e-30).all())
+    assert pkg().device_status() == 0
+
+
+# tiles of 128 channels and 32, 64 or 128 tokens, one and several blocks of 256 per row, K split or not (N % 8)
+@pytest.mark.parametrize("M", [9, 31, 33, 64, 65, 128, 129, 300])
+@pytest.mark.parametrize("N,K", [(128, 256), (7, 512), (1028, 768), (200, 5632), (2048, 2048)])
+def test_q4km_many_tokens(M, N, K):
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    w = torch.randn((N, K), generator=g, device="cuda") * torch.rand((N, 1), generator=g, device="cuda") + 0.1
+    lin = pkg().QuantLinear.quantise(w, "q4_k_m")
+    x = (torch.randn((M, K), generator=g, device="cuda") * 3 + 0.5).to(torch.bfloat16)
+    # the sums of a block and of its activations are within 256 terms each, the blocks' within K / 256, and the part
+    # with the minimum enters beside the codes': both are at most 16 times the sum of the weights' magnitudes here
+    check(lin, x, 16 * (512 + K // 256))
+    assert torch.equal(lin(x), lin(x))
+
+
+def test_q4km_many_tokens_streams_and_capture():
+    """Two streams at once and a captured call give the bits of a call alone."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    lin = pkg().QuantLinear.quantise(torch.randn((1024, 1024), generator=g, device="cuda"), "q4_k_m")
+    xs = [torch.randn((40, 1024), generator=g, device="cuda").to(torch.bfloat16) for _ in range(2)]
+    alone = [lin(x).clone() for x in xs]
+    streams = [torch.cuda.Stream() for _ in xs]
+    torch.cuda.synchronize()
+    for _ in range(20):
+        outs = []
+        for x, s in zip(xs, streams):
+            with torch.cuda.stream(s):
+                outs.append(lin(x))
+        torch.cuda.synchronize()
+        assert all(torch.equal(o, a) for o, a in zip(outs, alone))
+    with torch.cuda.stream(streams[0]):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=streams[0]):
+            y = lin(xs[0])
+        for _ in range(3):
+            graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, alone[0])
+
+
+# tiles of 64 x 64 and 32 x 32 outputs, steps of 32 columns
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("method", ["int8_channel", "int4", "q4_k_m", "w4a16"])
+@pytest.mark.parametrize("M,N,K", [(9, 33, 128), (32, 384, 384), (70, 1000, 256), (200, 8192, 384)])
+def test_generic_tiles(dtype, method, M, N, K):
+    g = torch.Generator(device="cuda").manual_seed(K)
+    lin = pkg().QuantLinear.quantise(torch.randn((N, K), generator=g, device="cuda"), method, 64 if method == "w4a16" else 128)
+    check(lin, torch.randn((M, K), generator=g, device="cuda").to(dtype), 16 * (K // 32 + 34))
+
+
+@pytest.mark.parametrize("method", ["int8_channel", "int4"])
+def test_generic_tiles_short_rows(method):
+    """Rows that end inside a step, and groups that straddle rows."""
+    g = torch.Generator(device="cuda").manual_seed(1)
+    lin = pkg().QuantLinear.quantise(torch.randn((50, 72), generator=g, device="cuda"), method, 16)
+    check(lin, torch.randn((35, 72), generator=g, device="cuda"), 64)
