@@ -16,6 +16,7 @@
 
 #include "common.cuh"
 #include "kv_cache.cuh"
+#include "stack.cuh"
 
 using namespace ab2;
 
@@ -311,10 +312,13 @@ int attention_cached_device(const ab2_kv *kv, int layer, const void *q, void *ou
         return AB2_OK;
     }
     if (S > 1) {
-        // prefill chunk over an INT8 cache: the tensor-core causal kernel (attention_mma.cu)
+        // prefill chunk of a bf16 model: the tcgen05 kernel (attention_prompt_tc.cu); few queries, or a recorded launch,
+        // over an INT8 cache: the warp-level tensor-core kernel (attention_mma.cu)
         static const bool scalar_prefill = getenv("AB2_SCALAR_PREFILL_ATTN") != nullptr;  // measurement switch
         if (!scalar_prefill) {
-            int rc = attention_prefill_mma_device(kv, layer, q, out, S, pending, row0, nrows, scale, dtype, st, s);
+            int rc = prompt_tc_cached(kv, layer, q, out, S, pending, row0, nrows, scale, dtype, st, s);
+            if (rc != AB2_ERR_UNSUPPORTED) return rc;
+            rc = attention_prefill_mma_device(kv, layer, q, out, S, pending, row0, nrows, scale, dtype, st, s);
             if (rc != AB2_ERR_UNSUPPORTED) return rc;
         }
     }

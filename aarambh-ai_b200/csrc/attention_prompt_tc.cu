@@ -1,6 +1,7 @@
 // Causal attention of a prompt portion in bf16 on the 5th-generation tensor cores, over keys and values laid
-// out position by position (PromptAttnArgs).  A CTA owns 128 queries of a head and walks the keys 128 at
-// a time:
+// out position by position (PromptAttnArgs): projected latents, the cache of a dense decoder (bf16 rows as they are,
+// INT8 codes after one pass that widens them), the ring of a window layer (copied straight where it wraps).  A CTA
+// owns 128 queries of a head and walks the keys in its sight 128 at a time:
 //
 //   S[128 queries][128 keys] = Q . K^T         both K-major in shared memory
 //   O[128 queries][vdim]    += (P_hi + P_lo) . V   P in tensor memory, V N-major in shared memory
@@ -15,10 +16,15 @@
 // Tensor memory: S_0, S_1 (128 columns each; the weights take the place of the scores), O_0, O_1.  The
 // weights are relative to a maximum per query that moves only when a score exceeds it by 2^8; then the query's
 // sums are rescaled in tensor memory.
+// The chain scores - softmax - sums of a half bounds it, about 2 us a tile of 128 x 128 against the 0.8 us of its
+// MMAs.  32 / 8 heads of 128: 3001 tokens over an INT8 cache 787 us on the warp-level tensor cores, 222 + 11 (widening) here;
+// 1000 tokens behind 500 over a bf16 cache 1344 us on CUDA cores, 50 here; 2048 tokens of 16 / 4 heads with a window of
+// 1024: 114 -> 48.  Below 16 queries a CTA would be nearly empty.
 // Every wait on an mbarrier is bounded; on a time-out the CTA records AB2_ERR_TIMEOUT, stops issuing
 // work, frees its tensor memory and returns.
 #include <algorithm>
 
+#include "kv_cache.cuh"
 #include "stack.cuh"
 #include "tcgen05_util.cuh"
 
@@ -31,6 +37,7 @@ namespace {
 
 constexpr int PT_Q = 128, PT_KEYS = 128, PT_THREADS = 384, PT_BOX = 128 * 128;  // a box is 128 rows of 64 elements
 constexpr int PT_SMEM = 227 * 1024;
+constexpr int PT_MIN_QUERIES = 16;  // fewer go to the kernels that read the cache as it is
 constexpr float PT_SLACK = 8.f;  // powers of two a score may exceed the query's maximum by
 
 struct PtShared {
@@ -38,6 +45,8 @@ struct PtShared {
     uint32_t tmem_base;
     int failed;
     float top[2][PT_Q], sum[2][PT_Q];
+    // scales of a tile's keys and values: a half's tile is read from one buffer while its next is written to the other
+    alignas(16) float ks[2][2][PT_KEYS], vs[2][2][PT_KEYS];
 };
 
 struct PtArgs {
@@ -81,9 +90,11 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, u
 }
 
 // One tile of keys for the warp's 32 queries, a lane each: scores to weights in tensor memory.  With EDGE the keys
-// past `lim` are out of sight.  o_blocks blocks of 32 columns hold sums so far.
-template <bool EDGE>
-__device__ __forceinline__ void softmax_tile(uint32_t s_addr, uint32_t o_addr, float sl, int lim, int o_blocks, float &top, float &sum) {
+// before `lo` and past `lim` are out of sight.  With SCALED a score is multiplied by its key's scale and a weight, after it has been
+// counted, by its value's.  o_blocks blocks of 32 columns hold sums so far.
+template <bool EDGE, bool SCALED>
+__device__ __forceinline__ void softmax_tile(uint32_t s_addr, uint32_t o_addr, float sl, int lo, int lim, const float *ks, const float *vs, int o_blocks, float &top,
+                                             float &sum) {
     // two buffers: the next 32 scores are on their way while these are looked at
     uint32_t v[2][32];
     float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -93,7 +104,15 @@ __device__ __forceinline__ void softmax_tile(uint32_t s_addr, uint32_t o_addr, f
         tmem_ld32_wait(v[c & 1]);
         tmem_ld32_start(v[(c + 1) & 1], s_addr + 32 * ((c + 1) & 3));  // the last one fetches the first again
 #pragma unroll
-        for (int k = 0; k < 32; ++k) mx[k & 3] = fmaxf(mx[k & 3], EDGE && 32 * c + k > lim ? -INFINITY : __uint_as_float(v[c & 1][k]));
+        for (int k = 0; k < 32; k += 4) {
+            float f[4] = {__uint_as_float(v[c & 1][k]), __uint_as_float(v[c & 1][k + 1]), __uint_as_float(v[c & 1][k + 2]), __uint_as_float(v[c & 1][k + 3])};
+            if (SCALED) {
+                const float4 q = *reinterpret_cast<const float4 *>(ks + 32 * c + k);
+                f[0] *= q.x; f[1] *= q.y; f[2] *= q.z; f[3] *= q.w;
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) mx[e] = fmaxf(mx[e], EDGE && (32 * c + k + e > lim || 32 * c + k + e < lo) ? -INFINITY : f[e]);
+        }
     }
     tmem_ld32_wait(v[0]);
     const float best = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sl;  // the scale is positive
@@ -119,21 +138,38 @@ __device__ __forceinline__ void softmax_tile(uint32_t s_addr, uint32_t o_addr, f
         if (c < 3) tmem_ld32_start(v[(c + 1) & 1], s_addr + 32 * (c + 1));
         uint32_t w[32];
 #pragma unroll
-        for (int k = 0; k < 32; k += 2) {
-            float x = ex2(fmaf(__uint_as_float(v[c & 1][k]), sl, -top)), y = ex2(fmaf(__uint_as_float(v[c & 1][k + 1]), sl, -top));
-            if (EDGE && 32 * c + k > lim) x = 0.f;
-            if (EDGE && 32 * c + k + 1 > lim) y = 0.f;
-            part_sum[(k >> 1) & 3] += x + y;
-            const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-            w[k >> 1] = *reinterpret_cast<const uint32_t *>(&h);
-            const __nv_bfloat162 l = __floats2bfloat162_rn(x - __uint_as_float(w[k >> 1] << 16), y - __uint_as_float(w[k >> 1] & 0xffff0000u));
-            w[16 + (k >> 1)] = *reinterpret_cast<const uint32_t *>(&l);
+        for (int k = 0; k < 32; k += 4) {
+            float f[4] = {__uint_as_float(v[c & 1][k]), __uint_as_float(v[c & 1][k + 1]), __uint_as_float(v[c & 1][k + 2]), __uint_as_float(v[c & 1][k + 3])};
+            if (SCALED) {
+                const float4 q = *reinterpret_cast<const float4 *>(ks + 32 * c + k);
+                f[0] *= q.x; f[1] *= q.y; f[2] *= q.z; f[3] *= q.w;
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                f[e] = ex2(fmaf(f[e], sl, -top));
+                if (EDGE && (32 * c + k + e > lim || 32 * c + k + e < lo)) f[e] = 0.f;
+            }
+            part_sum[(k >> 1) & 3] += f[0] + f[1];
+            part_sum[((k >> 1) + 1) & 3] += f[2] + f[3];
+            if (SCALED) {
+                const float4 q = *reinterpret_cast<const float4 *>(vs + 32 * c + k);
+                f[0] *= q.x; f[1] *= q.y; f[2] *= q.z; f[3] *= q.w;
+            }
+#pragma unroll
+            for (int e = 0; e < 4; e += 2) {
+                const int i = (k + e) >> 1;
+                const __nv_bfloat162 h = __floats2bfloat162_rn(f[e], f[e + 1]);
+                w[i] = *reinterpret_cast<const uint32_t *>(&h);
+                const __nv_bfloat162 l = __floats2bfloat162_rn(f[e] - __uint_as_float(w[i] << 16), f[e + 1] - __uint_as_float(w[i] & 0xffff0000u));
+                w[16 + i] = *reinterpret_cast<const uint32_t *>(&l);
+            }
         }
         tmem_st32(s_addr + 32 * c, w);
     }
     sum += (part_sum[0] + part_sum[1]) + (part_sum[2] + part_sum[3]);
 }
 
+template <bool SCALED>
 __global__ void __launch_bounds__(PT_THREADS, 1)
 prompt_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap vmap, PtArgs p, int *status) {
     extern __shared__ uint8_t smem_raw[];
@@ -142,21 +178,24 @@ prompt_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
     const int kboxes = p.main_boxes + p.tail_boxes;
     uint8_t *kbuf = qbuf + kboxes * PT_BOX, *vbuf = kbuf + 2 * kboxes * PT_BOX;
     PtShared *sh = (PtShared *)(vbuf + 2 * p.v_boxes * PT_BOX);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, head = blockIdx.y;
-    const int q_lo = ((int)gridDim.x - 1 - (int)blockIdx.x) * PT_Q;  // the longest walks first
-    const int tiles = (a.first + min(a.S, q_lo + PT_Q) + PT_KEYS - 1) / PT_KEYS;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, head = blockIdx.x;
+    const int q_lo = ((int)gridDim.y - 1 - (int)blockIdx.y) * PT_Q;  // the longest walks of every head first
+    const int kv_head = a.rep > 1 ? head / a.rep : head, z = a.k_z ? kv_head : 0, first = a.first - a.base;  // positions count from row 0 of the keys
+    // tiles of keys in sight of the first query (from t0 on) to that of the last
+    const int t0 = a.window ? max(0, first + q_lo - a.window + 1) / PT_KEYS : 0;
+    const int tiles = (first + min(a.S, q_lo + PT_Q) + PT_KEYS - 1) / PT_KEYS - t0;
     volatile int *failed = &sh->failed;
 
     auto load_k = [&](int j) {
         uint8_t *dst = kbuf + (j & 1) * kboxes * PT_BOX;
         bar_expect_tx(&sh->kfull[j & 1], (uint32_t)(kboxes * PT_BOX));
-        for (int b = 0; b < p.main_boxes; ++b) tma_load_2d(dst + b * PT_BOX, &kmap, head * a.k_head + b * 64, j * PT_KEYS, &sh->kfull[j & 1]);
-        for (int b = 0; b < p.tail_boxes; ++b) tma_load_2d(dst + (p.main_boxes + b) * PT_BOX, &tmap, b * 64, j * PT_KEYS, &sh->kfull[j & 1]);
+        for (int b = 0; b < p.main_boxes; ++b) tma_load_3d(dst + b * PT_BOX, &kmap, kv_head * a.k_head + b * 64, (t0 + j) * PT_KEYS, z, &sh->kfull[j & 1]);
+        for (int b = 0; b < p.tail_boxes; ++b) tma_load_2d(dst + (p.main_boxes + b) * PT_BOX, &tmap, b * 64, (t0 + j) * PT_KEYS, &sh->kfull[j & 1]);
     };
     auto load_v = [&](int j) {
         uint8_t *dst = vbuf + (j & 1) * p.v_boxes * PT_BOX;
         bar_expect_tx(&sh->vfull[j & 1], (uint32_t)(p.v_boxes * PT_BOX));
-        for (int b = 0; b < p.v_boxes; ++b) tma_load_2d(dst + b * PT_BOX, &vmap, head * a.v_head + b * 64, j * PT_KEYS, &sh->vfull[j & 1]);
+        for (int b = 0; b < p.v_boxes; ++b) tma_load_3d(dst + b * PT_BOX, &vmap, kv_head * a.v_head + b * 64, (t0 + j) * PT_KEYS, z, &sh->vfull[j & 1]);
     };
 
     if (threadIdx.x == 0) {
@@ -243,19 +282,33 @@ prompt_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
     } else if (warp >= 4) {
         // ---------------------------------------------------------- softmax
         const int part = (warp - 4) >> 2, quad = warp & 3, r = quad * 32 + lane;
-        const int pos = a.first + q_lo + r;
+        const int pos = first + q_lo + r;
         const uint32_t quad_addr = (uint32_t)(quad * 32) << 16, s_addr = tmem + quad_addr + (uint32_t)(part * PT_KEYS), o_addr = tmem_o + quad_addr + (uint32_t)(part * 128);
         const float sl = a.scale * 1.44269504088896341f;  // scores in powers of two
         float top = -1e30f, sum = 0.f;
         bool ok = true;
+        // the thread fetches the scales of key r of its half's next tile
+        const int rows = first + a.S;
+        auto scale_of = [&](const float *p, int j) { const int k = (t0 + j) * PT_KEYS + r; return j < tiles && k < rows ? __ldg(p + (size_t)kv_head * a.scale_z + k) : 0.f; };
+        float ks_next = SCALED ? scale_of(a.k_scale, part) : 0.f, vs_next = SCALED ? scale_of(a.v_scale, part) : 0.f;
         for (int j = part; j < tiles; j += 2) {
+            const int buf = (j >> 1) & 1;
+            if (SCALED) {
+                sh->ks[part][buf][r] = ks_next;
+                sh->vs[part][buf][r] = vs_next;
+                ks_next = scale_of(a.k_scale, j + 2);
+                vs_next = scale_of(a.v_scale, j + 2);
+                asm volatile("barrier.cta.sync %0, 128;\n" ::"r"(2 + part) : "memory");
+            }
             ok = warp_wait(&sh->sfull[part], (j >> 1) & 1, failed);
-            if (!ok) break;
+            if (!SCALED && !ok) break;  // with scales the warps go on to their barrier together; what they write is not read
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const bool edge = (j + 1) * PT_KEYS - 1 > a.first + q_lo;
-            const int lim = pos - j * PT_KEYS;  // the last key of the tile in sight
-            if (edge) softmax_tile<true>(s_addr, o_addr, sl, lim, j >= 2 ? p.v_boxes * 2 : 0, top, sum);
-            else softmax_tile<false>(s_addr, o_addr, sl, lim, j >= 2 ? p.v_boxes * 2 : 0, top, sum);
+            const int at = (t0 + j) * PT_KEYS;
+            const bool edge = at + PT_KEYS - 1 > first + q_lo || (a.window && at < first + q_lo + PT_Q - a.window);
+            const int lim = pos - at, lo = a.window ? lim - a.window + 1 : -0x40000000;  // keys of the tile in sight
+            const int o_blocks = j >= 2 ? p.v_boxes * 2 : 0;
+            if (edge) softmax_tile<true, SCALED>(s_addr, o_addr, sl, lo, lim, sh->ks[part][buf], sh->vs[part][buf], o_blocks, top, sum);
+            else softmax_tile<false, SCALED>(s_addr, o_addr, sl, lo, lim, sh->ks[part][buf], sh->vs[part][buf], o_blocks, top, sum);
             asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
             __syncwarp();
@@ -314,12 +367,83 @@ prompt_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
 
 size_t prompt_tc_smem(const PtArgs &p) { return 1024 + (size_t)(3 * (p.main_boxes + p.tail_boxes) + 2 * p.v_boxes) * PT_BOX + sizeof(PtShared); }
 
+template <bool SCALED>
+int launch_prompt(const PtArgs &p, const CUtensorMap &kmap, const CUtensorMap &tmap, const CUtensorMap &vmap, int *status, cudaStream_t s) {
+    static bool configured[64] = {false};  // the attribute is per device
+    int dev = 0;
+    AB2_CUDA(cudaGetDevice(&dev));
+    AB2_REQUIRE(dev >= 0 && dev < 64, AB2_ERR_BAD_ARG, "device index %d out of range", dev);
+    if (!configured[dev]) {
+        AB2_CUDA(cudaFuncSetAttribute(prompt_tc_kernel<SCALED>, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM));
+        configured[dev] = true;
+    }
+    cudaError_t e = launch_kernel(prompt_tc_kernel<SCALED>, dim3(p.a.heads, (p.a.S + PT_Q - 1) / PT_Q), dim3(PT_THREADS), prompt_tc_smem(p), s, kmap, tmap, vmap, p, status);
+    if (e != cudaSuccess) return fail(AB2_ERR_CUDA, "prompt attention launch failed: %s", cudaGetErrorString(e));
+    return AB2_OK;
+}
+
+// Rows [base, base + n) of every head, one after the other: INT8 codes as the bf16 integers they are, or the rows of
+// a ring of `cap` slots.  blockIdx.y is the head, z keys or values; 16 bytes of the output a thread.
+struct PtGather {
+    const void *src[2];
+    __nv_bfloat16 *dst[2];
+    int ld[2];            // elements of a row, a multiple of 8
+    long long src_z[2];   // elements between heads of the source
+    int base, n, cap;
+};
+template <bool INT8>
+__global__ void __launch_bounds__(256) prompt_gather_kernel(PtGather a) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int w = blockIdx.z, per = a.ld[w] >> 3;
+    const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+    if (i >= (size_t)a.n * per) return;
+    const int r = (int)(i / per), c = (int)(i % per) * 8;
+    const size_t from = (size_t)blockIdx.y * a.src_z[w] + (size_t)((a.base + r) % a.cap) * a.ld[w] + c;
+    uint4 v;
+    if (INT8) {
+        const uint2 q = *reinterpret_cast<const uint2 *>((const int8_t *)a.src[w] + from);
+        // a code is the difference of two bf16 between 128 and 256, as in the INT8 GEMM
+        auto pair = [](uint32_t x, uint32_t sel) {
+            const uint32_t b = __byte_perm(x, 0u, sel);
+            return bf16x2_add_((b & 0x007F007Fu) | 0x43004300u, (b & 0x00800080u) | 0xC300C300u);
+        };
+        v = make_uint4(pair(q.x, 0x4140), pair(q.x, 0x4342), pair(q.y, 0x4140), pair(q.y, 0x4342));
+    } else {
+        v = *reinterpret_cast<const uint4 *>((const __nv_bfloat16 *)a.src[w] + from);
+    }
+    *reinterpret_cast<uint4 *>(a.dst[w] + ((size_t)blockIdx.y * a.n + r) * a.ld[w] + c) = v;
+}
+
+// Fills in the gathered keys and values; `heads` of them.
+int gather_rows(PtGather g, bool int8, int heads, ScratchLease &ws, PromptAttnArgs &p, cudaStream_t s) {
+    const size_t kb = (size_t)heads * g.n * g.ld[0] * 2, vb = (size_t)heads * g.n * g.ld[1] * 2;
+    int rc = ws.take(kb + vb);  // both are multiples of 16 bytes
+    if (rc != AB2_OK) return rc;
+    g.dst[0] = (__nv_bfloat16 *)ws.ptr;
+    g.dst[1] = (__nv_bfloat16 *)((char *)ws.ptr + kb);
+    const dim3 grid((unsigned)(((size_t)g.n * (std::max(g.ld[0], g.ld[1]) / 8) + 255) / 256), heads, 2);
+    cudaError_t e = int8 ? launch_kernel(prompt_gather_kernel<true>, grid, dim3(256), 0, s, g) : launch_kernel(prompt_gather_kernel<false>, grid, dim3(256), 0, s, g);
+    if (e != cudaSuccess) return fail(AB2_ERR_CUDA, "prompt attention launch failed: %s", cudaGetErrorString(e));
+    p.k = g.dst[0]; p.v = g.dst[1];
+    p.k_stride = g.ld[0]; p.v_stride = g.ld[1];
+    p.k_z = (long long)g.n * g.ld[0]; p.v_z = (long long)g.n * g.ld[1];
+    return AB2_OK;
+}
+
+// The host's lengths are those of the rows when the launch runs, unless the launch is recorded to run again.
+bool lengths_known(cudaStream_t s) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+}
+
 }  // namespace
 
 bool prompt_tc_serves(const PromptAttnArgs &a) {
     const PtArgs p = {a, (a.dim + 63) / 64, (a.tail_dims + 63) / 64, (a.vdim + 63) / 64};
     return a.scale >= 0.f && a.dim % 8 == 0 && a.tail_dims % 8 == 0 && a.vdim % 8 == 0 && p.v_boxes <= 2 && prompt_tc_smem(p) <= PT_SMEM && a.q_stride % 8 == 0 &&
            a.k_stride % 8 == 0 && a.v_stride % 8 == 0 && a.tail_stride % 8 == 0 && a.k_head % 8 == 0 && a.v_head % 8 == 0 && a.out_stride % 8 == 0 &&
+           a.k_z % 8 == 0 && a.v_z % 8 == 0 &&
            (((uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.tail | (uintptr_t)a.out) & 15) == 0;
 }
 
@@ -328,21 +452,80 @@ int prompt_tc_attention(const PromptAttnArgs &a, cudaStream_t s) {
     int *status = nullptr;
     int rc = device_status_word(&status);
     CUtensorMap kmap, tmap, vmap;
-    const int L = a.first + a.S;
-    if (rc == AB2_OK) rc = make_x_map(&kmap, a.k, L, (a.heads - 1) * a.k_head + a.dim, PT_KEYS, a.k_stride);
+    const int L = a.first + a.S - a.base, heads = a.heads / std::max(1, a.rep);
+    const int mats = a.k_z ? heads : 1, kcols = a.k_z ? a.dim : (heads - 1) * a.k_head + a.dim, vcols = a.k_z ? a.vdim : (heads - 1) * a.v_head + a.vdim;
+    if (rc == AB2_OK) rc = make_mats_map(&kmap, a.k, mats, L, kcols, a.k_stride, a.k_z ? a.k_z : L * a.k_stride, PT_KEYS);
     if (rc == AB2_OK) rc = a.tail_dims > 0 ? make_x_map(&tmap, a.tail, L, a.tail_dims, PT_KEYS, a.tail_stride) : make_x_map(&tmap, a.k, L, a.dim, PT_KEYS, a.k_stride);
-    if (rc == AB2_OK) rc = make_x_map(&vmap, a.v, L, (a.heads - 1) * a.v_head + a.vdim, PT_KEYS, a.v_stride);
+    if (rc == AB2_OK) rc = make_mats_map(&vmap, a.v, mats, L, vcols, a.v_stride, a.k_z ? a.v_z : L * a.v_stride, PT_KEYS);
     if (rc != AB2_OK) return rc;
-    static bool configured[64] = {false};  // the attribute is per device
-    int dev = 0;
-    AB2_CUDA(cudaGetDevice(&dev));
-    AB2_REQUIRE(dev >= 0 && dev < 64, AB2_ERR_BAD_ARG, "device index %d out of range", dev);
-    if (!configured[dev]) {
-        AB2_CUDA(cudaFuncSetAttribute(prompt_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM));
-        configured[dev] = true;
+    return a.k_scale ? launch_prompt<true>(p, kmap, tmap, vmap, status, s) : launch_prompt<false>(p, kmap, tmap, vmap, status, s);
+}
+
+int prompt_tc_cached(const ab2_kv *kv, int layer, const void *q, void *out, int S, int pending, int row0, int nrows, float scale,
+                     ab2_dtype dtype, const AttnStrides &st, cudaStream_t s) {
+    const int hd = kv->hd;
+    const bool int8 = kv->dtype == AB2_KV_INT8;
+    if (S < PT_MIN_QUERIES || dtype != AB2_BF16 || kv->dtype == AB2_KV_F32 || st.q_h != hd || st.o_h != hd || !lengths_known(s)) return AB2_ERR_UNSUPPORTED;
+    const KvView v = kv_view(kv, layer);
+    for (int i = 0; i < nrows; ++i) {
+        const int row = kv_row_host(kv, row0, i), L = kv->lens_host[row] + pending;
+        const size_t head0 = (size_t)row * kv->kvh * kv->cap;
+        PromptAttnArgs p = {};
+        p.q = (const __nv_bfloat16 *)q + i * st.q_b; p.out = (__nv_bfloat16 *)out + i * st.o_b;
+        p.q_stride = st.q_s; p.out_stride = st.o_s;
+        p.S = S; p.heads = kv->h; p.rep = kv->h / kv->kvh; p.first = L - S; p.dim = p.vdim = hd; p.scale = scale;
+        p.k_stride = p.v_stride = hd;
+        p.k_z = p.v_z = (long long)kv->cap * hd;
+        if (!int8) {
+            p.k = (const __nv_bfloat16 *)v.k + head0 * hd;
+            p.v = (const __nv_bfloat16 *)v.v + head0 * hd;
+        }
+        if (p.first < 0 || !prompt_tc_serves(p)) return AB2_ERR_UNSUPPORTED;  // the same for every row
+        ScratchLease ws(s);
+        if (int8) {
+            PtGather g = {};
+            g.src[0] = (const int8_t *)v.k + head0 * hd; g.src[1] = (const int8_t *)v.v + head0 * hd;
+            g.ld[0] = g.ld[1] = hd; g.src_z[0] = g.src_z[1] = p.k_z;
+            g.n = g.cap = L;
+            int rc = gather_rows(g, true, kv->kvh, ws, p, s);
+            if (rc != AB2_OK) return rc;
+            p.k_scale = v.ks + head0; p.v_scale = v.vs + head0; p.scale_z = kv->cap;
+        }
+        int rc = prompt_tc_attention(p, s);
+        if (rc != AB2_OK) return rc;
     }
-    cudaError_t e = launch_kernel(prompt_tc_kernel, dim3((a.S + PT_Q - 1) / PT_Q, a.heads), dim3(PT_THREADS), prompt_tc_smem(p), s, kmap, tmap, vmap, p, status);
-    if (e != cudaSuccess) return fail(AB2_ERR_CUDA, "prompt attention launch failed: %s", cudaGetErrorString(e));
+    return AB2_OK;
+}
+
+int prompt_tc_window(const ab2_kv *kv, const WindowAttnArgs &a, int nrows, cudaStream_t s) {
+    const KvLayer &l = a.kv.l;
+    if (a.S < PT_MIN_QUERIES || !lengths_known(s)) return AB2_ERR_UNSUPPORTED;
+    for (int i = 0; i < nrows; ++i) {
+        const int row = kv_row_host(kv, a.row0, i), first = kv->lens_host[row];
+        const size_t kz = (size_t)l.cap * l.kds, vz = (size_t)l.cap * l.vds;
+        PromptAttnArgs p = {};
+        p.q = (const __nv_bfloat16 *)a.q + (size_t)i * a.S * a.q_stride; p.q_stride = a.q_stride;
+        p.out = (__nv_bfloat16 *)a.out + (size_t)i * a.S * a.H * a.vdim; p.out_stride = (long long)a.H * a.vdim;
+        p.S = a.S; p.heads = a.H; p.rep = a.rep; p.first = first; p.dim = a.dim; p.vdim = a.vdim; p.scale = a.scale;
+        p.window = l.window < first + a.S ? l.window : 0;
+        p.base = p.window ? std::max(0, first - l.window + 1) : 0;
+        const int n = first + a.S - p.base, slot = p.base % l.cap;
+        const __nv_bfloat16 *k = (const __nv_bfloat16 *)l.k + row * l.kvh * kz, *v = (const __nv_bfloat16 *)l.v + row * l.kvh * vz;
+        p.k = k + (size_t)slot * l.kds; p.v = v + (size_t)slot * l.vds;
+        p.k_stride = l.kds; p.v_stride = l.vds; p.k_z = kz; p.v_z = vz;
+        if (!prompt_tc_serves(p)) return AB2_ERR_UNSUPPORTED;  // the same for every row
+        ScratchLease ws(s);
+        if (slot + n > l.cap) {
+            PtGather g = {};
+            g.src[0] = k; g.src[1] = v;
+            g.ld[0] = l.kds; g.ld[1] = l.vds; g.src_z[0] = kz; g.src_z[1] = vz;
+            g.base = p.base; g.n = n; g.cap = l.cap;
+            int rc = gather_rows(g, false, l.kvh, ws, p, s);
+            if (rc != AB2_OK) return rc;
+        }
+        int rc = prompt_tc_attention(p, s);
+        if (rc != AB2_OK) return rc;
+    }
     return AB2_OK;
 }
 

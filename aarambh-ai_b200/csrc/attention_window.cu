@@ -767,6 +767,8 @@ int launch_window(const ab2_kv *kv, WindowAttnArgs a, int nrows, int max_len, cu
         if (e != cudaSuccess) return fail(AB2_ERR_CUDA, "window preparation launch failed: %s", cudaGetErrorString(e));
     }
     if (on_mma && a.S >= 16) {
+        const int rc = prompt_tc_window(kv, a, nrows, s);
+        if (rc != AB2_ERR_UNSUPPORTED) return rc;
         if (a.dim <= 64) e = a.vdim <= 64 ? launch_mma<64, 64>(a, a.H, nrows, s) : launch_mma<64, 128>(a, a.H, nrows, s);
         else e = a.vdim <= 64 ? launch_mma<128, 64>(a, a.H, nrows, s) : launch_mma<128, 128>(a, a.H, nrows, s);
         if (e != cudaSuccess) return fail(AB2_ERR_CUDA, "window attention launch failed: %s", cudaGetErrorString(e));

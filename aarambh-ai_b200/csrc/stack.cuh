@@ -95,9 +95,21 @@ struct PromptAttnArgs {
     __nv_bfloat16 *out;    // head h at h * vdim
     int S, heads, first, dim, tail_dims, vdim;   // `first`: position of the first query
     float scale;
+    // what only attention_prompt_tc.cu reads: `rep` query heads (0: one) share a head of keys and values, whose heads
+    // lie k_z and v_z elements apart (0: side by side in a row); row 0 of the keys is position `base`; a query sees
+    // `window` keys (0: all before it); with k_scale and v_scale the key of row j is that row times
+    // k_scale[head scale_z + j], the value times v_scale[...] (codes of an INT8 cache)
+    long long k_z, v_z, scale_z;
+    int rep, base, window;
+    const float *k_scale, *v_scale;
 };
 bool prompt_attention_serves(int dim, int tail, int vdim);
 bool prompt_tc_serves(const PromptAttnArgs &a);   // attention_prompt_tc.cu
+// The same over the cache of a dense decoder (attention_cached_device's arguments) and over the rings of window
+// layers, after the new tokens are stored; AB2_ERR_UNSUPPORTED where another kernel has to serve.
+int prompt_tc_cached(const ab2_kv *kv, int layer, const void *q, void *out, int S, int pending, int row0, int nrows, float scale,
+                     ab2_dtype dtype, const AttnStrides &st, cudaStream_t s);
+int prompt_tc_window(const ab2_kv *kv, const WindowAttnArgs &a, int nrows, cudaStream_t s);
 int prompt_tc_attention(const PromptAttnArgs &a, cudaStream_t s);
 int prompt_attention(const PromptAttnArgs &a, cudaStream_t s);
 
