@@ -125,8 +125,8 @@ __global__ void __launch_bounds__(128) attn_decode_fused_kernel(FusedArgs a) {
     // The cached K/V of older tokens do not depend on the preceding kernel: the
     // raw bytes of this warp's first chunk are requested before waiting for it,
     // all at once, so the chunk costs one memory round trip instead of a chain.
-    constexpr bool STAGED = (KVD != AB2_KV_F32) && HD == 128;
-    constexpr int ESZ = KVD == AB2_KV_INT8 ? 1 : 2;
+    constexpr bool STAGED = HD == 128 ? KVD != AB2_KV_F32 : HD == 64 && KVD != AB2_KV_INT8;
+    constexpr int ESZ = KVD == AB2_KV_INT8 ? 1 : KVD == AB2_KV_BF16 ? 2 : 4;
     constexpr int KW = STAGED ? HD * ESZ / 16 : 1;  // 16-byte words of one K row
     constexpr int VW = STAGED ? DPL * ESZ / 4 : 1;  // 4-byte words of one lane's V slice
     uint4 kraw[KW];
@@ -252,6 +252,13 @@ __global__ void __launch_bounds__(128) attn_decode_fused_kernel(FusedArgs a) {
                         i8x4(w4[i], t);
                         kf[4 * i] = t[0]; kf[4 * i + 1] = t[1]; kf[4 * i + 2] = t[2]; kf[4 * i + 3] = t[3];
                     }
+                } else if constexpr (KVD == AB2_KV_F32) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const uint4 r4 = kraw[d0 / 4 + q];
+                        kf[4 * q] = __uint_as_float(r4.x); kf[4 * q + 1] = __uint_as_float(r4.y);
+                        kf[4 * q + 2] = __uint_as_float(r4.z); kf[4 * q + 3] = __uint_as_float(r4.w);
+                    }
                 } else {
 #pragma unroll
                     for (int hv = 0; hv < 2; ++hv) {
@@ -309,8 +316,15 @@ __global__ void __launch_bounds__(128) attn_decode_fused_kernel(FusedArgs a) {
                 if constexpr (KVD == AB2_KV_INT8) {
                     i8x4(vraw[t][0], vf);
                 } else {
-                    vf[0] = __uint_as_float(vraw[t][0] << 16); vf[1] = __uint_as_float(vraw[t][0] & 0xffff0000u);
-                    vf[2] = __uint_as_float(vraw[t][1] << 16); vf[3] = __uint_as_float(vraw[t][1] & 0xffff0000u);
+#pragma unroll
+                    for (int i = 0; i < VW; ++i) {
+                        if constexpr (KVD == AB2_KV_F32) {
+                            vf[i] = __uint_as_float(vraw[t][i]);
+                        } else {
+                            vf[2 * i] = __uint_as_float(vraw[t][i] << 16);
+                            vf[2 * i + 1] = __uint_as_float(vraw[t][i] & 0xffff0000u);
+                        }
+                    }
                 }
 #pragma unroll
                 for (int hh = 0; hh < REP; ++hh) {

@@ -33,6 +33,9 @@ int qlinear_w4a16_mma_add(const ab2_qweight *w, const void *x, int M, void *y, c
 int qlinear_w4a16_mma_swiglu(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t s);
 int qlinear_w4a16_mma_f32(const ab2_qweight *w, const void *x, int M, float *y, cudaStream_t s);
 int qlinear_w4a16_mma_f32_peer(const ab2_qweight *w, const void *x, int M, ab2_tp *tp, cudaStream_t s);
+bool qlinear_step_eligible(const ab2_qweight *w, ab2_dtype dtype, int M);
+int qlinear_step_norm(const ab2_qweight *w, const void *x, const float *norm_w, float eps, int M, ab2_dtype dtype, bool swiglu, void *y, cudaStream_t s);
+int qlinear_step_add(const ab2_qweight *w, const void *x, const void *resid, int M, ab2_dtype dtype, void *y, cudaStream_t s);
 }
 extern "C" int ab2_qweight_interleave_gate_up(ab2_qweight **out, const ab2_qweight *gate, const ab2_qweight *up);
 
@@ -149,6 +152,7 @@ static int norm_linear(ab2_model *m, const ab2_qweight *w, const void *x, const 
                        int epi, cudaStream_t s, bool normed = false) {
     const ab2_model_config &c = m->cfg;
     if (normed) return qlinear_dispatch(w, m->xn, T, m->dtype, out, s);  // m->xn already holds RMSNorm(x; norm_w)
+    if (epi == 0 && qlinear_step_eligible(w, m->dtype, T)) return qlinear_step_norm(w, x, norm_w, c.rms_eps, T, m->dtype, false, out, s);
     if (m->fused_epilogues && qlinear_w4a16_norm_fusable(w, m->dtype, T))
         return qlinear_w4a16_norm(w, x, norm_w, c.rms_eps, out, epi, s);
     STEP(launch_rms_norm(x, norm_w, m->xn, T, c.d_model, c.rms_eps, m->dtype, s));
@@ -283,13 +287,27 @@ static int forward_launches(ab2_model *m, ab2_kv *kv, const uint32_t *ids, int S
             STEP(norm_linear(m, L.wgu, m->x, L.norm2, T, m->hid, 2, s));
             STEP(qlinear_w4a16_mma_add(L.part[6], m->hid, T, m->x, m->x, s));
         } else {
-            STEP(qlinear_dispatch(L.part[3], m->attn, T, m->dtype, m->proj, s));
-            STEP(launch_add(m->x, m->proj, m->x, (size_t)T * d, m->dtype, s));
-            STEP(launch_rms_norm(m->x, L.norm2, m->xn, T, d, c.rms_eps, m->dtype, s));
-            STEP(qlinear_dispatch(L.wgu, m->xn, T, m->dtype, m->gu, s));
-            STEP(launch_swiglu_fused(m->gu, m->hid, T, c.ffn_hidden, m->dtype, s));
-            STEP(qlinear_dispatch(L.part[6], m->hid, T, m->dtype, m->proj, s));
-            STEP(launch_add(m->x, m->proj, m->x, (size_t)T * d, m->dtype, s));
+            // a few tokens over weights without a GEMV of their own: the norm, the gated unit and the residual additions
+            // ride with the linears
+            if (qlinear_step_eligible(L.part[3], m->dtype, T)) {
+                STEP(qlinear_step_add(L.part[3], m->attn, m->x, T, m->dtype, m->x, s));
+            } else {
+                STEP(qlinear_dispatch(L.part[3], m->attn, T, m->dtype, m->proj, s));
+                STEP(launch_add(m->x, m->proj, m->x, (size_t)T * d, m->dtype, s));
+            }
+            if (qlinear_step_eligible(L.wgu, m->dtype, T)) {
+                STEP(qlinear_step_norm(L.wgu, m->x, L.norm2, c.rms_eps, T, m->dtype, true, m->hid, s));
+            } else {
+                STEP(launch_rms_norm(m->x, L.norm2, m->xn, T, d, c.rms_eps, m->dtype, s));
+                STEP(qlinear_dispatch(L.wgu, m->xn, T, m->dtype, m->gu, s));
+                STEP(launch_swiglu_fused(m->gu, m->hid, T, c.ffn_hidden, m->dtype, s));
+            }
+            if (qlinear_step_eligible(L.part[6], m->dtype, T)) {
+                STEP(qlinear_step_add(L.part[6], m->hid, m->x, T, m->dtype, m->x, s));
+            } else {
+                STEP(qlinear_dispatch(L.part[6], m->hid, T, m->dtype, m->proj, s));
+                STEP(launch_add(m->x, m->proj, m->x, (size_t)T * d, m->dtype, s));
+            }
         }
     }
     if (logits_mode == 0 && argmax_out == nullptr) return AB2_OK;
@@ -717,7 +735,9 @@ AB2_API int ab2_model_decode_step(ab2_model *m, ab2_kv *kv, const uint32_t *ids_
         if (!m->stack) rc = w4a16_prepare_stream(s);  // scratch of the GEMV is allocated outside the capture
         if (rc != AB2_OK) return rc;
         AB2_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        g_pdl_launch = m->fused_epilogues || m->stack;  // every kernel of the fast path takes part in the chain
+        // Chained launches: a kernel launched with the attribute waits for its predecessor itself, one launched without
+        // waits as a whole.  (Tensor parallel keeps plain launches unless the fast path is taken: its collectives are not ours.)
+        g_pdl_launch = m->fused_epilogues || m->stack || !m->tp;
         rc = forward_launches(m, kv, ids_dev, 1, row0, nrows, kv->lens_dev, logits_dev ? 1 : 0, logits_dev, argmax_dev, len_bound, s);
         if (rc == AB2_OK) {
             // lengths advance inside the graph; the host mirror is advanced per replay
