@@ -19,6 +19,8 @@ struct GemvArgs {
     int N, K, group;
 };
 
+GemvArgs gemv_args_of(const ab2_qweight *w);   // qlinear.cu
+
 template <typename T> struct Vec8;
 template <> struct Vec8<float> {
     static __device__ __forceinline__ void load(const float *p, float (&v)[8]) {
