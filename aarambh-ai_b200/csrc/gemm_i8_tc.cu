@@ -63,6 +63,7 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const float *__restr
                   const __grid_constant__ CUtensorMap xmap, __nv_bfloat16 *__restrict__ y, int N, int K, int M, int *status) {
     constexpr int B_BYTES = NTOK * 128;
     constexpr int TC_STAGES = tc_stages<NTOK>(), TC_WSLOTS = tc_wslots<NTOK>();
+    static_assert(TC_WSLOTS % (TC_SETS / 2) == 0 && TC_STAGES >= TC_SETS, "one pair of sets per slot; no set a lap ahead of a stage");
     constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NTOK >> 3) << 17) | ((128u >> 4) << 24);
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);

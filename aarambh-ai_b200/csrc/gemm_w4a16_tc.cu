@@ -62,11 +62,13 @@ struct TcShared {
 // Stages of 64 K-elements: an unpacked weight tile and an activation tile that share one pair of barriers, so that
 // the issuing warp waits once per stage (a wait costs it about 150 cycles even when the stage is ready, and four MMAs
 // of 32 tokens only 160).  What they leave of shared memory goes to the packed-weight slots, one quantisation group
-// each.
+// each.  The slots are even in number: a slot is then read by one pair of sets only.  With three, a pair could
+// reach its next use of a slot while the group between, the other pair's, was still on its way - copies may land out
+// of order - and take the barrier's older phase for the one it waits for.
 template <int NTOK>
-__host__ __device__ constexpr int tc_stages() { return NTOK > 128 ? 4 : 6; }
+__host__ __device__ constexpr int tc_stages() { return NTOK > 128 ? 4 : NTOK > 32 ? 5 : 6; }
 template <int NTOK>
-__host__ __device__ constexpr int tc_wslots() { return NTOK > 32 ? 3 : TC_MAX_WSLOTS; }
+__host__ __device__ constexpr int tc_wslots() { return NTOK > 128 ? 2 : NTOK > 32 ? 6 : TC_MAX_WSLOTS; }
 
 template <int NTOK>
 __global__ void __launch_bounds__(TC_THREADS, 1)
@@ -74,6 +76,7 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
                      __nv_bfloat16 *__restrict__ y, int N, int K, int M, int *status, int ksplit, float *part) {
     constexpr int B_BYTES = NTOK * 128;
     constexpr int TC_STAGES = tc_stages<NTOK>(), TC_WSLOTS = tc_wslots<NTOK>();
+    static_assert(TC_WSLOTS % (TC_SETS / 2) == 0 && TC_STAGES >= TC_SETS, "one pair of sets per slot; no set a lap ahead of a stage");
     constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NTOK >> 3) << 17) | ((128u >> 4) << 24);
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
