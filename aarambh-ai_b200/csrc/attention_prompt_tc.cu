@@ -54,41 +54,11 @@ struct PtArgs {
     int main_boxes, tail_boxes, v_boxes;
 };
 
-#define PT_REGS32(c, v) \
-    c(v[0]), c(v[1]), c(v[2]), c(v[3]), c(v[4]), c(v[5]), c(v[6]), c(v[7]), c(v[8]), c(v[9]), c(v[10]), c(v[11]), c(v[12]), c(v[13]), c(v[14]), c(v[15]), \
-    c(v[16]), c(v[17]), c(v[18]), c(v[19]), c(v[20]), c(v[21]), c(v[22]), c(v[23]), c(v[24]), c(v[25]), c(v[26]), c(v[27]), c(v[28]), c(v[29]), c(v[30]), c(v[31])
-// 32 columns of the warp's lanes; the registers pass through the wait, so that nothing computed from them can move
-// ahead of it.
-__device__ __forceinline__ void tmem_ld32_start(uint32_t (&v)[32], uint32_t addr) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
-        : PT_REGS32("=r", v) : "r"(addr));
-}
-__device__ __forceinline__ void tmem_ld32_wait(uint32_t (&v)[32]) { asm volatile("tcgen05.wait::ld.sync.aligned;\n" : PT_REGS32("+r", v)::"memory"); }
-__device__ __forceinline__ void tmem_ld32(uint32_t (&v)[32], uint32_t addr) {
-    tmem_ld32_start(v, addr);
-    tmem_ld32_wait(v);
-}
-__device__ __forceinline__ void tmem_st32(uint32_t addr, const uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31};\n" ::PT_REGS32("r", v), "r"(addr)
-        : "memory");
-}
 __device__ __forceinline__ float ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
     return y;
 }
-// The first operand in tensor memory: 128 lanes, two bf16 per column.
-__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::
-            "r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-
 // One tile of keys for the warp's 32 queries, a lane each: scores to weights in tensor memory.  With EDGE the keys
 // before `lo` and past `lim` are out of sight.  With SCALED a score is multiplied by its key's scale and a weight, after it has been
 // counted, by its value's.  o_blocks blocks of 32 columns hold sums so far.

@@ -9,7 +9,7 @@
 // bf16, not the dequantised weight: the unpack warps turn codes into 128 + q
 // (0x4300 | q, one shift and one logic op per pair of codes), add the channel's
 // -(128 + zero) as one packed bf16 add (exact: both are small integers) and write
-// the pair to the swizzled operand stage.  The scale is applied per quantisation
+// the pair to an operand stage in tensor memory.  The scale is applied per quantisation
 // group in f32 by the epilogue warps: after the MMAs of a group
 //   d[c][t] = sum_k x[t][k] (q[c][k] - zero[c])        (tensor memory)
 // and the group adds scale[c] * d[c][t] to the running f32 output kept in the
@@ -58,7 +58,7 @@ constexpr int DG_STAGES = 4;         // operand-A stages of 64 K-elements (two p
 constexpr int DG_XSTAGES = 8;        // operand-B (activation) stages: small, so the ring is deeper
 constexpr int DG_WSLOTS = 12;        // depth of a packed-weight ring (two blocks = 32 channels of one unit per slot)
 constexpr int DG_WSLOT_BYTES = 2 * W4_BLOCK_WORDS * 4;  // per ring; four rings (one per 32 channels) = ~100 KB in flight per SM
-constexpr int DG_A_BYTES = 128 * 128;  // 128 channels x 64 bf16
+constexpr int DG_A_COLS = 32;          // tensor-memory columns of 64 K-elements: two bf16 per column, a lane per channel
 constexpr int DG_MMA_WARPS = 2;        // MMA-issue warps, taking alternate units (warp 1 and the warps after the epilogue)
 constexpr int DG_THREADS = 448 + 32 * (DG_MMA_WARPS - 1) + 32;  // the last warp fetches the packed weights
 constexpr int DG_ACC = 4;             // accumulator pairs (D, S) in tensor memory
@@ -124,11 +124,11 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
                      int *counters, int *status) {
     constexpr int B_BYTES = NTOK * 128;
     constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NTOK >> 3) << 17) | ((128u >> 4) << 24);
-    constexpr uint32_t TMEM_COLS = NTOK == 16 ? 64u : 128u;  // DG_ACC accumulators of NTOK columns
+    constexpr uint32_t ACC_COLS = DG_ACC * NTOK, TMEM_COLS = 256u;
+    static_assert(ACC_COLS + DG_STAGES * DG_A_COLS <= TMEM_COLS, "accumulators and operand stages fit");
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t *a_st = smem;                                   // [DG_STAGES][DG_A_BYTES]
-    uint8_t *b_st = a_st + DG_STAGES * DG_A_BYTES;          // [DG_XSTAGES][B_BYTES]
+    uint8_t *b_st = smem;                                    // [DG_XSTAGES][B_BYTES]
     uint8_t *w_ring = b_st + DG_XSTAGES * B_BYTES;           // [4][DG_WSLOTS][DG_WSLOT_BYTES]
     DgShared *sh = (DgShared *)(w_ring + 4 * DG_WSLOTS * DG_WSLOT_BYTES);
 
@@ -153,7 +153,7 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = sh->tmem_base;
+    const uint32_t tmem = sh->tmem_base, tmem_a = tmem + ACC_COLS;
     pdl_launch_dependents();  // the next kernel may start fetching its constant weights
 
     if (warp == 0) {
@@ -209,8 +209,9 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
                 const uint32_t suse = 2 * use + half;
                 const int s = suse % DG_STAGES, xs = suse % DG_XSTAGES;
                 if (!warp_wait(&sh->xfull[xs], (suse / DG_XSTAGES) & 1, failed) || !warp_wait(&sh->afull[s], (suse / DG_STAGES) & 1, failed)) break;
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 if (elect_one()) {
-                    umma_stage(td, umma_desc(sptr(a_st + s * DG_A_BYTES)), umma_desc(sptr(b_st + xs * B_BYTES)), IDESC, half == 0);
+                    umma_stage_ts(td, tmem_a + (uint32_t)(s * DG_A_COLS), umma_desc(sptr(b_st + xs * B_BYTES)), IDESC, half == 0);
                     umma_commit(&sh->sempty[s]);  // the operand stages are free when the MMAs retire
                     umma_commit(&sh->xempty[xs]);
                 }
@@ -223,9 +224,9 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
         // ---------------------------------------------------------- unpack: codes -> bf16 128 + q
         // The two warps that share 32 channels (one per half of the group) read those channels'
         // two packed blocks from a ring of their own, filled by the producer warp.
-        const int t = (threadIdx.x - 64) & 127;   // channel within the 128-channel tile
-        const int half = (threadIdx.x - 64) >> 7;  // which 64 of the group's 128 K-elements
-        const int q = t >> 5;                      // ring: channels 32q .. 32q+31 = blocks 2q, 2q+1
+        const int q = warp & 3;                    // ring: channels 32q .. 32q+31 = blocks 2q, 2q+1, the warp's lanes of tensor memory
+        const int t = q * 32 + lane;               // channel within the 128-channel tile
+        const int half = (warp - 2) >> 2;          // which 64 of the group's 128 K-elements
         const int blk = t >> 4, r = t & 15;
         uint8_t *ring = w_ring + q * DG_WSLOTS * DG_WSLOT_BYTES;
         uint32_t k_mask = 0x000F000Fu, k_magic = 0x43004300u;
@@ -245,17 +246,17 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
             if (lane == 0) bar_arrive_after(&sh->wempty[q][ws], held, (uint32_t)K & 1u);
             const uint32_t suse = 2 * use + half;
             const int s = suse % DG_STAGES;
-            if (!bar_wait(&sh->sempty[s], ((suse / DG_STAGES) & 1) ^ 1, failed)) break;
-            uint8_t *arow = a_st + s * DG_A_BYTES + t * 128;
+            if (!warp_wait(&sh->sempty[s], ((suse / DG_STAGES) & 1) ^ 1, failed)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const uint32_t words[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+            uint32_t o[32];
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {  // chunk c = 8 consecutive k = one code word
-                uint32_t o[4];
+            for (int c = 0; c < 8; ++c)  // 8 consecutive k = one code word
 #pragma unroll
-                for (int j = 0; j < 4; ++j) o[j] = bf16x2_add(w4_pair_bf16(words[c], j, k_mask, k_magic), nz2);  // q - zero, exact
-                *reinterpret_cast<uint4 *>(arow + ((c ^ (t & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-            }
-            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                for (int j = 0; j < 4; ++j) o[4 * c + j] = bf16x2_add(w4_pair_bf16(words[c], j, k_mask, k_magic), nz2);  // q - zero, exact
+            tmem_st32(tmem_a + ((uint32_t)(q * 32) << 16) + (uint32_t)(s * DG_A_COLS), o);
+            asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
             __syncwarp();
             if (lane == 0) bar_arrive(&sh->afull[s]);
         }
@@ -361,7 +362,7 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
 
 template <int NTOK>
 constexpr size_t dg_smem_bytes() {
-    return 1024 + DG_STAGES * DG_A_BYTES + DG_XSTAGES * NTOK * 128 + 4 * DG_WSLOTS * DG_WSLOT_BYTES + sizeof(DgShared);
+    return 1024 + DG_XSTAGES * NTOK * 128 + 4 * DG_WSLOTS * DG_WSLOT_BYTES + sizeof(DgShared);
 }
 
 template <int NTOK, int EPI>
