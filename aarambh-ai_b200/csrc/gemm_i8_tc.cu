@@ -37,7 +37,8 @@ namespace {
 
 constexpr int TC_MAX_STAGES = 6, TC_MAX_WSLOTS = 6;
 constexpr int TC_WSLOT_BYTES = 128 * 128;  // 128 channels x 128 codes
-constexpr int TC_A_BYTES = 128 * 128;  // 128 channels x 64 bf16
+constexpr int TC_OUT_BYTES = 4 * 32 * 32 * 2;  // an epilogue warp's 32 tokens x 32 channels on their way out
+constexpr int TC_A_COLS = 32;  // tensor-memory columns of 64 K-elements: two bf16 per column, a lane per channel
 constexpr int TC_SETS = 4;  // sets of four convert warps on stages of their own
 constexpr int TC_THREADS = (2 + 4 * TC_SETS + 4 + 1) * 32;  // weight producer, MMA, convert, epilogue, activation producer
 
@@ -49,28 +50,35 @@ struct TcShared {
     int failed;
 };
 
-// Stages of 64 K-elements: a converted weight tile and an activation tile that share one pair of barriers, so that
-// the issuing warp waits once per stage (a wait costs it about 150 cycles even when the stage is ready, and four MMAs
-// of 32 tokens only 160).  What they leave of shared memory goes to the slots of codes, 128 channels x 128 K each.
+// Stages of 64 K-elements: the weight tile in tensor memory, the activation tile in shared memory, with one pair of
+// barriers, so that the issuing warp waits once per stage (a wait costs it about 150 cycles even when the stage is
+// ready).  A weight tile in shared memory would be written and read there besides the activations, at 256 tokens 112
+// KB a stage instead of 80.  256 tokens leave room for one accumulator: the MMAs of a tile wait for the last one's to be stored.
+// The slots hold 128 channels x 128 codes each.
 template <int NTOK>
-__host__ __device__ constexpr int tc_stages() { return NTOK > 128 ? 4 : 6; }
+__host__ __device__ constexpr int tc_stages() { return NTOK > 192 ? 5 : NTOK > 128 ? 4 : 6; }
 template <int NTOK>
-__host__ __device__ constexpr int tc_wslots() { return NTOK > 32 ? 2 : TC_MAX_WSLOTS; }
+__host__ __device__ constexpr int tc_wslots() { return NTOK > 192 ? 2 : TC_MAX_WSLOTS; }
+template <int NTOK>
+__host__ __device__ constexpr int tc_accs() { return NTOK > 192 ? 1 : 2; }
+template <int NTOK>
+__host__ __device__ constexpr uint32_t tc_cols() { return tc_accs<NTOK>() * NTOK + tc_stages<NTOK>() * TC_A_COLS > 256 ? 512 : 256; }
 
 template <int NTOK>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const float *__restrict__ scales,
                   const __grid_constant__ CUtensorMap xmap, __nv_bfloat16 *__restrict__ y, int N, int K, int M, int *status) {
     constexpr int B_BYTES = NTOK * 128;
-    constexpr int TC_STAGES = tc_stages<NTOK>(), TC_WSLOTS = tc_wslots<NTOK>();
+    constexpr int TC_STAGES = tc_stages<NTOK>(), TC_WSLOTS = tc_wslots<NTOK>(), ACCS = tc_accs<NTOK>();
+    static_assert(ACCS * NTOK + TC_STAGES * TC_A_COLS <= 512, "tensor memory");
     static_assert(TC_WSLOTS % (TC_SETS / 2) == 0 && TC_STAGES >= TC_SETS, "one pair of sets per slot; no set a lap ahead of a stage");
     constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NTOK >> 3) << 17) | ((128u >> 4) << 24);
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t *a_st = smem;                                   // [TC_STAGES][TC_A_BYTES]
-    uint8_t *b_st = a_st + TC_STAGES * TC_A_BYTES;          // [TC_STAGES][B_BYTES]
-    uint8_t *w_ring = b_st + TC_STAGES * B_BYTES;                 // [TC_WSLOTS][TC_WSLOT_BYTES]
-    TcShared *sh = (TcShared *)(w_ring + TC_WSLOTS * TC_WSLOT_BYTES);
+    uint8_t *b_st = smem;                            // [TC_STAGES][B_BYTES]
+    uint8_t *w_ring = b_st + TC_STAGES * B_BYTES;    // [TC_WSLOTS][TC_WSLOT_BYTES]
+    __nv_bfloat16 *stage = (__nv_bfloat16 *)(w_ring + TC_WSLOTS * TC_WSLOT_BYTES);  // [4 epilogue warps][32 tokens][32 channels]
+    TcShared *sh = (TcShared *)((uint8_t *)stage + TC_OUT_BYTES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = K >> 7;
@@ -87,13 +95,13 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const float *__restr
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     }
     if (warp == 1) {  // tensor-memory allocation is a whole-warp operation
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(sptr(&sh->tmem_base)), "r"((uint32_t)(2 * NTOK)));
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(sptr(&sh->tmem_base)), "r"(tc_cols<NTOK>()));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = sh->tmem_base;
+    const uint32_t tmem = sh->tmem_base, tmem_a = tmem + (uint32_t)(ACCS * NTOK);
 
     if (warp == 0) {
         // ---------------------------------------------------------- producer of the codes
@@ -127,15 +135,16 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const float *__restr
         // ---------------------------------------------------------- MMA issue
         uint32_t suse = 0, tuse = 0;
         for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x, ++tuse) {
-            const int ab = tuse & 1;
-            if (!bar_wait(&sh->accempty[ab], ((tuse >> 1) & 1) ^ 1, failed)) break;
+            const int ab = tuse % ACCS;
+            if (!bar_wait(&sh->accempty[ab], ((tuse / ACCS) & 1) ^ 1, failed)) break;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const uint32_t tacc = tmem + (uint32_t)(ab * NTOK);
             for (int ks = 0; ks < 2 * G; ++ks, ++suse) {
                 const int st = suse % TC_STAGES;
-                if (!warp_wait(&sh->full[st], (suse / TC_STAGES) & 1, failed)) break;  // no tensor memory in a stage: no tcgen05 fence
+                if (!warp_wait(&sh->full[st], (suse / TC_STAGES) & 1, failed)) break;
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 if (elect_one()) {
-                    umma_stage(tacc, umma_desc(sptr(a_st + st * TC_A_BYTES)), umma_desc(sptr(b_st + st * B_BYTES)), IDESC, ks == 0);
+                    umma_stage_ts(tacc, tmem_a + (uint32_t)(st * TC_A_COLS), umma_desc(sptr(b_st + st * B_BYTES)), IDESC, ks == 0);
                     umma_commit(&sh->empty[st]);  // the stage is free when the MMAs retire
                 }
                 __syncwarp();
@@ -146,7 +155,7 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const float *__restr
     } else if (warp < 2 + 4 * TC_SETS) {
         // ---------------------------------------------------------- codes -> bf16
         // a set of four warps takes the same half (64 K-elements, one stage) of every second group
-        const int t = (threadIdx.x - 64) & 127, set = (threadIdx.x - 64) >> 7, half = set & 1;
+        const int t = (warp & 3) * 32 + lane, set = (warp - 2) >> 2, half = set & 1;  // channel: the warp's lanes of tensor memory
         uint32_t gbase = 0;  // groups before this tile
         for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x) {
             for (uint32_t wuse = gbase + ((set >> 1) + TC_SETS - gbase % (TC_SETS / 2)) % (TC_SETS / 2); wuse < gbase + (uint32_t)G && !*failed; wuse += TC_SETS / 2) {
@@ -162,23 +171,23 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const float *__restr
                 if (lane == 0) bar_arrive_after(&sh->wempty[ws], held, (uint32_t)K & 1u);
                 const uint32_t suse = 2 * wuse + half;
                 const int s = suse % TC_STAGES;
-                if (!bar_wait(&sh->empty[s], ((suse / TC_STAGES) & 1) ^ 1, failed)) break;
-                uint8_t *arow = a_st + s * TC_A_BYTES + t * 128;
+                if (!warp_wait(&sh->empty[s], ((suse / TC_STAGES) & 1) ^ 1, failed)) break;
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                uint32_t o[32];  // two bf16 each
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {  // 16 codes -> two chunks of 8 bf16
+                for (int i = 0; i < 4; ++i) {  // 16 codes
                     const uint32_t w4[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
-                    uint32_t o[8];
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
                         // two codes into the low bytes of 16-bit halves; code = (128 + its low 7 bits) - (128 + its
                         // sign's 128), both of which are a bf16 with those bits as mantissa: exact
                         const uint32_t p = __byte_perm(w4[j >> 1], 0u, j & 1 ? 0x4342 : 0x4140);
-                        o[j] = bf16x2_add_((p & 0x007F007Fu) | 0x43004300u, (p & 0x00800080u) | 0xC300C300u);
+                        o[8 * i + j] = bf16x2_add_((p & 0x007F007Fu) | 0x43004300u, (p & 0x00800080u) | 0xC300C300u);
                     }
-                    *reinterpret_cast<uint4 *>(arow + (((2 * i) ^ (t & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-                    *reinterpret_cast<uint4 *>(arow + (((2 * i + 1) ^ (t & 7)) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
                 }
-                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                tmem_st32(tmem_a + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(s * TC_A_COLS), o);
+                asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
                 __syncwarp();
                 if (lane == 0) bar_arrive(&sh->full[s]);
             }
@@ -187,28 +196,28 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const float *__restr
     } else if (warp < TC_THREADS / 32 - 1) {
         // ---------------------------------------------------------- epilogue
         const int quad = warp & 3;
+        const bool aligned = (N & 7) == 0 && ((uintptr_t)y & 15) == 0;
         uint32_t tuse = 0;
         for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x, ++tuse) {
             const int nt = it / m_tiles, mt = it % m_tiles;
-            const int ab = tuse & 1;
-            if (!bar_wait(&sh->accfull[ab], (tuse >> 1) & 1, failed)) break;
+            const int ab = tuse % ACCS;
+            if (!bar_wait(&sh->accfull[ab], (tuse / ACCS) & 1, failed)) break;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const int n = nt * 128 + quad * 32 + lane;
             const float sc = n < N ? __ldg(scales + n) : 0.f;
 #pragma unroll 1
-            for (int c = 0; c < NTOK / 32; ++c) {
+            for (int c = 0; c < NTOK / 32 && mt * NTOK + c * 32 < M; ++c) {
                 uint32_t v[32];
                 const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(ab * NTOK + c * 32);
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                    "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
-                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                      "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-                      "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-                      "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                    : "r"(taddr));
-                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                if (n < N) {
+                __syncwarp();  // the tensor-memory load is a whole-warp operation
+                tmem_ld32(v, taddr);
+                if (aligned) {
+                    __nv_bfloat16 *out = stage + quad * 1024;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) out[j * 32 + lane] = __float2bfloat16_rn(__uint_as_float(v[j]) * sc);
+                    const int tok = mt * NTOK + c * 32, n0 = nt * 128 + quad * 32;
+                    flush_rows<32>(out, y + (size_t)tok * N + n0, N, M - tok, N - n0, lane);
+                } else if (n < N) {
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
                         const int tok = mt * NTOK + c * 32 + j;
@@ -228,7 +237,7 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const float *__restr
     if (threadIdx.x == 0 && sh->failed) atomicExch(status, (int)AB2_ERR_TIMEOUT);
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"((uint32_t)(2 * NTOK)));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(tc_cols<NTOK>()));
     }
 }
 
@@ -242,7 +251,7 @@ int launch_i8_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaStream
     if (rc != AB2_OK) return rc;
     rc = make_bytes_map(&wmap, w->codes, w->N, w->K);
     if (rc != AB2_OK) return rc;
-    const size_t smem = 1024 + tc_stages<NTOK>() * (TC_A_BYTES + NTOK * 128) + tc_wslots<NTOK>() * TC_WSLOT_BYTES + sizeof(TcShared);
+    const size_t smem = 1024 + tc_stages<NTOK>() * NTOK * 128 + tc_wslots<NTOK>() * TC_WSLOT_BYTES + TC_OUT_BYTES + sizeof(TcShared);
     static bool configured[64] = {false};  // the attribute is per device
     int dev = 0;
     AB2_CUDA(cudaGetDevice(&dev));
@@ -269,8 +278,15 @@ bool qlinear_i8_tc_eligible(const ab2_qweight *w, ab2_dtype dtype, int M) {
 // Y[M][N] = X[M][K] . W^T on the tcgen05 path (INT8 codes, f32 scale per channel, bf16 activations).
 int qlinear_i8_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t s) {
     AB2_REQUIRE(((uintptr_t)x & 15) == 0, AB2_ERR_BAD_ALIGN, "activations must be 16-byte aligned");
-    if (M <= 256) return launch_i8_tc<128>(w, x, M, y, s);  // as for the W4A16 GEMM: 256-token tiles from 257 tokens on
-    return launch_i8_tc<256>(w, x, M, y, s);
+    // Measured: rounds of 18 / 21 / 28 us of tiles of 128 / 192 / 256 tokens over K = 4096, 61 / 72 / 86 over K = 14336; a
+    // tile of 32 takes what one of 128 does but for its stores.
+    static const GemmTileCost costs[] = {{32, 0.5, 0.53}, {128, 1.0, 0.54}, {192, 1.5, 0.62}, {256, 6.0, 0.70}};
+    switch (choose_gemm_tile(costs, M, w->N, w->K / 128, device_sm_count(), 1).ntok) {
+    case 32: return launch_i8_tc<32>(w, x, M, y, s);
+    case 128: return launch_i8_tc<128>(w, x, M, y, s);
+    case 192: return launch_i8_tc<192>(w, x, M, y, s);
+    default: return launch_i8_tc<256>(w, x, M, y, s);
+    }
 }
 
 }  // namespace ab2

@@ -42,6 +42,7 @@ constexpr int QB_MAX_STAGES = 6, QB_MAX_WSLOTS = 6;
 constexpr int QB_A_BYTES = 128 * 128;      // 128 channels x 64 bf16
 constexpr int QB_WSLOT_BYTES = 128 * 128;  // 128 channels x 256 codes
 constexpr int QB_UNPACK_WARPS = 8, QB_EPI_WARPS = 8;
+constexpr int QB_OUT_BYTES = QB_EPI_WARPS * 16 * 32 * 2;  // an epilogue warp's 16 tokens x 32 channels on their way out
 constexpr int QB_THREADS = (2 + QB_UNPACK_WARPS + QB_EPI_WARPS + 1) * 32;
 
 template <int NTOK>
@@ -96,7 +97,8 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
     uint8_t *a_st = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);  // [STAGES][QB_A_BYTES]
     uint8_t *b_st = a_st + STAGES * QB_A_BYTES;                                    // [STAGES][B_BYTES]
     uint8_t *w_ring = b_st + STAGES * B_BYTES;                                     // [WSLOTS][QB_WSLOT_BYTES]
-    QbShared *sh = (QbShared *)(w_ring + WSLOTS * QB_WSLOT_BYTES);
+    __nv_bfloat16 *stage = (__nv_bfloat16 *)(w_ring + WSLOTS * QB_WSLOT_BYTES);  // [QB_EPI_WARPS][16][32]
+    QbShared *sh = (QbShared *)((uint8_t *)stage + QB_OUT_BYTES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_tiles = (a.N + 127) >> 7, m_tiles = (a.M + NTOK - 1) / NTOK, items = n_tiles * m_tiles * a.ksplit;
@@ -233,6 +235,7 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
     } else {
         // ---------------------------------------------------------- epilogue
         constexpr int COLS = NTOK / 2;  // tokens of a thread
+        const bool aligned = (a.N & 7) == 0 && ((uintptr_t)a.y & 15) == 0;  // rows go out in 16-byte pieces
         const int quad = warp & 3, half = (warp - 2 - QB_UNPACK_WARPS) >> 2;
         uint32_t buse = 0;
         bool ok = true;
@@ -279,6 +282,15 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                 if (lane == 0) bar_arrive_after(&sh->accempty[ab], held, (uint32_t)a.KB >> 30);
             }
             const int t0 = mt * NTOK + half * COLS;
+            if (aligned && a.ksplit == 1) {
+                __nv_bfloat16 *out = stage + (warp - 2 - QB_UNPACK_WARPS) * 512;
+#pragma unroll
+                for (int j = 0; j < COLS; ++j) {
+                    out[(j & 15) * 32 + lane] = __float2bfloat16_rn(acc[j]);
+                    if ((j & 15) == 15) flush_rows<16>(out, a.y + (size_t)(t0 + j - 15) * a.N + n - lane, a.N, ok ? a.M - t0 - (j - 15) : 0, a.N - (n - lane), lane);
+                }
+                continue;
+            }
 #pragma unroll
             for (int j = 0; j < COLS; ++j)
                 if (ok && n < a.N && t0 + j < a.M) {
@@ -305,8 +317,8 @@ int launch_qb(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t 
     int rc = device_status_word(&status);
     if (rc != AB2_OK) return rc;
     const int N = w->N, K = w->K, KB = K / 256, Mp = (M + NTOK - 1) / NTOK * NTOK;
-    const size_t smem = 1024 + qb_stages<NTOK>() * (QB_A_BYTES + NTOK * 128) + qb_wslots<NTOK>() * QB_WSLOT_BYTES + sizeof(QbShared);
-    static_assert(1024 + qb_stages<NTOK>() * (QB_A_BYTES + NTOK * 128) + qb_wslots<NTOK>() * QB_WSLOT_BYTES + sizeof(QbShared) <= 227 * 1024, "shared memory of a CTA");
+    const size_t smem = 1024 + qb_stages<NTOK>() * (QB_A_BYTES + NTOK * 128) + qb_wslots<NTOK>() * QB_WSLOT_BYTES + QB_OUT_BYTES + sizeof(QbShared);
+    static_assert(1024 + qb_stages<NTOK>() * (QB_A_BYTES + NTOK * 128) + qb_wslots<NTOK>() * QB_WSLOT_BYTES + QB_OUT_BYTES + sizeof(QbShared) <= 227 * 1024, "shared memory of a CTA");
     static bool configured[64] = {false};  // the attribute is per device
     int dev = 0;
     AB2_CUDA(cudaGetDevice(&dev));

@@ -14,16 +14,11 @@
 //               swizzle) into the operand-B stages
 //   warp 1      allocates tensor memory, issues tcgen05.mma (K = 16 per
 //               instruction, 64 per stage), commits stage / accumulator barriers.
-//               A tcgen05 instruction costs the issuing thread on the order of a
-//               hundred cycles, about what a 128 x 256 x 16 MMA takes to execute:
-//               tiles are 256 tokens wide where the token count allows, and the
-//               operand rings of that tile size have equal depth so that one
-//               commit per stage frees both operands
 //   warps 2-17  dequantise, four sets of four warps on stages of their own; thread = output channel; nibbles -> bf16 (128 + q by
 //               one logic op, minus (128 + z) exactly, times the bf16 scale, i.e.
-//               the round-to-nearest bf16 of (q - z) * s) written into the
-//               operand-A stage in the canonical K-major 128-byte-swizzle layout
-//   warps 18-21 epilogue: tcgen05.ld of the accumulator, bf16 stores of Y
+//               the round-to-nearest bf16 of (q - z) * s) written to the
+//               operand-A stage in tensor memory, a lane per channel
+//   warps 18-21 epilogue: tcgen05.ld of the accumulator, bf16 rows of Y by way of shared memory
 // Every wait on an mbarrier is bounded; on a time-out the CTA records
 // AB2_ERR_TIMEOUT, stops issuing work, still frees its tensor memory and returns.
 #include <cuda.h>
@@ -46,7 +41,8 @@ namespace {
 constexpr int TC_MAX_STAGES = 6, TC_MAX_WSLOTS = 10;
 constexpr int TC_BLOCK_WORDS = 272;   // 16 rows x 16 code words + 16 parameter words
 constexpr int TC_WSLOT_BYTES = 8 * TC_BLOCK_WORDS * 4;  // 8 row tiles of 16 = 128 channels
-constexpr int TC_A_BYTES = 128 * 128;  // 128 channels x 64 bf16
+constexpr int TC_OUT_BYTES = 4 * 32 * 32 * 2;  // an epilogue warp's 32 tokens x 32 channels on their way out
+constexpr int TC_A_COLS = 32;  // tensor-memory columns of 64 K-elements: two bf16 per column, a lane per channel
 constexpr int TC_SETS = 4;  // sets of four unpack warps; a set takes every TC_SETS-th stage
 constexpr int TC_UNPACK_WARPS = 4 * TC_SETS;
 constexpr int TC_THREADS = (2 + TC_UNPACK_WARPS + 4 + 1) * 32;
@@ -59,31 +55,37 @@ struct TcShared {
     int failed;
 };
 
-// Stages of 64 K-elements: an unpacked weight tile and an activation tile that share one pair of barriers, so that
-// the issuing warp waits once per stage (a wait costs it about 150 cycles even when the stage is ready, and four MMAs
-// of 32 tokens only 160).  What they leave of shared memory goes to the packed-weight slots, one quantisation group
-// each.  The slots are even in number: a slot is then read by one pair of sets only.  With three, a pair could
-// reach its next use of a slot while the group between, the other pair's, was still on its way - copies may land out
-// of order - and take the barrier's older phase for the one it waits for.
+// Stages of 64 K-elements: the weight tile in tensor memory, the activation tile in shared memory, with one pair of
+// barriers, so that the issuing warp waits once per stage (a wait costs it about 150 cycles even when the stage is
+// ready).  A weight tile in shared memory would be written and read there besides the activations, at 256 tokens 104
+// KB a stage instead of 72.  256 tokens leave room for one accumulator: the MMAs of a tile wait for the last one's to be stored.
+// The slots of packed weights, one quantisation group each, are even in number: a slot is then read by one pair of sets
+// only.  With three, a pair could reach its next use of a slot while the group between, the other pair's, was still on
+// its way - copies may land out of order - and take the barrier's older phase for the one it waits for.
 template <int NTOK>
-__host__ __device__ constexpr int tc_stages() { return NTOK > 128 ? 4 : NTOK > 32 ? 5 : 6; }
+__host__ __device__ constexpr int tc_stages() { return NTOK > 192 ? 5 : NTOK > 128 ? 4 : 6; }
 template <int NTOK>
-__host__ __device__ constexpr int tc_wslots() { return NTOK > 128 ? 2 : NTOK > 32 ? 6 : TC_MAX_WSLOTS; }
+__host__ __device__ constexpr int tc_wslots() { return NTOK > 192 ? 6 : TC_MAX_WSLOTS; }
+template <int NTOK>
+__host__ __device__ constexpr int tc_accs() { return NTOK > 192 ? 1 : 2; }
+template <int NTOK>
+__host__ __device__ constexpr uint32_t tc_cols() { return tc_accs<NTOK>() * NTOK + tc_stages<NTOK>() * TC_A_COLS > 256 ? 512 : 256; }
 
 template <int NTOK>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CUtensorMap xmap,
                      __nv_bfloat16 *__restrict__ y, int N, int K, int M, int *status, int ksplit, float *part) {
     constexpr int B_BYTES = NTOK * 128;
-    constexpr int TC_STAGES = tc_stages<NTOK>(), TC_WSLOTS = tc_wslots<NTOK>();
+    constexpr int TC_STAGES = tc_stages<NTOK>(), TC_WSLOTS = tc_wslots<NTOK>(), ACCS = tc_accs<NTOK>();
+    static_assert(ACCS * NTOK + TC_STAGES * TC_A_COLS <= 512, "tensor memory");
     static_assert(TC_WSLOTS % (TC_SETS / 2) == 0 && TC_STAGES >= TC_SETS, "one pair of sets per slot; no set a lap ahead of a stage");
     constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NTOK >> 3) << 17) | ((128u >> 4) << 24);
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t *a_st = smem;                                   // [TC_STAGES][TC_A_BYTES]
-    uint8_t *b_st = a_st + TC_STAGES * TC_A_BYTES;          // [TC_STAGES][B_BYTES]
-    uint8_t *w_ring = b_st + TC_STAGES * B_BYTES;                 // [TC_WSLOTS][TC_WSLOT_BYTES]
-    TcShared *sh = (TcShared *)(w_ring + TC_WSLOTS * TC_WSLOT_BYTES);
+    uint8_t *b_st = smem;                            // [TC_STAGES][B_BYTES]
+    uint8_t *w_ring = b_st + TC_STAGES * B_BYTES;    // [TC_WSLOTS][TC_WSLOT_BYTES]
+    __nv_bfloat16 *stage = (__nv_bfloat16 *)(w_ring + TC_WSLOTS * TC_WSLOT_BYTES);  // [4 epilogue warps][32 tokens][32 channels]
+    TcShared *sh = (TcShared *)((uint8_t *)stage + TC_OUT_BYTES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = K >> 7, tiles16 = (N + 15) >> 4;
@@ -107,13 +109,13 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     }
     if (warp == 1) {  // tensor-memory allocation is a whole-warp operation
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(sptr(&sh->tmem_base)), "r"((uint32_t)(2 * NTOK)));
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(sptr(&sh->tmem_base)), "r"(tc_cols<NTOK>()));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = sh->tmem_base;
+    const uint32_t tmem = sh->tmem_base, tmem_a = tmem + (uint32_t)(ACCS * NTOK);
 
     if (warp == 0) {
         // ---------------------------------------------------------- producer of the packed weights
@@ -155,16 +157,17 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
         // ---------------------------------------------------------- MMA issue
         uint32_t suse = 0, tuse = 0;
         for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x, ++tuse) {
-            const int ab = tuse & 1;
-            if (!bar_wait(&sh->accempty[ab], ((tuse >> 1) & 1) ^ 1, failed)) break;
+            const int ab = tuse % ACCS;
+            if (!bar_wait(&sh->accempty[ab], ((tuse / ACCS) & 1) ^ 1, failed)) break;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const uint32_t tacc = tmem + (uint32_t)(ab * NTOK);
             TC_ITEM(it)
             for (int ks = 2 * g0; ks < 2 * g1; ++ks, ++suse) {
                 const int st = suse % TC_STAGES;
-                if (!warp_wait(&sh->full[st], (suse / TC_STAGES) & 1, failed)) break;  // no tensor memory in a stage: no tcgen05 fence
+                if (!warp_wait(&sh->full[st], (suse / TC_STAGES) & 1, failed)) break;
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 if (elect_one()) {
-                    umma_stage(tacc, umma_desc(sptr(a_st + st * TC_A_BYTES)), umma_desc(sptr(b_st + st * B_BYTES)), IDESC, ks == 2 * g0);
+                    umma_stage_ts(tacc, tmem_a + (uint32_t)(st * TC_A_COLS), umma_desc(sptr(b_st + st * B_BYTES)), IDESC, ks == 2 * g0);
                     umma_commit(&sh->empty[st]);  // the stage is free when the MMAs retire
                 }
                 __syncwarp();
@@ -174,7 +177,7 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
         }
     } else if (warp < 2 + TC_UNPACK_WARPS) {
         // ---------------------------------------------------------- dequantise
-        const int t = (threadIdx.x - 64) & 127, set = (threadIdx.x - 64) >> 7;  // output channel within the 128-channel tile
+        const int t = (warp & 3) * 32 + lane, set = (warp - 2) >> 2;  // channel within the tile: the warp's lanes of tensor memory
         const int blk = t >> 4, r = t & 15, half = set & 1;
         uint32_t gbase = 0;  // groups before this tile
         uint32_t k_mask = 0x000F000Fu, k_magic = 0x43004300u;
@@ -195,23 +198,24 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
                 const uint32_t nz2 = __byte_perm(pr, pr, 0x3232);  // bf16x2 -(128 + z)
                 const uint32_t suse = 2 * wuse + half;
                 const int s = suse % TC_STAGES;
-                if (!bar_wait(&sh->empty[s], ((suse / TC_STAGES) & 1) ^ 1, failed)) break;
-                uint8_t *arow = a_st + s * TC_A_BYTES + t * 128;
+                if (!warp_wait(&sh->empty[s], ((suse / TC_STAGES) & 1) ^ 1, failed)) break;
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                uint32_t o[32];  // two bf16 each
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {  // chunk c = 8 consecutive k = one code word
                     const uint4 q4 = pw[c >> 2];
                     const uint32_t word = (c & 3) == 0 ? q4.x : (c & 3) == 1 ? q4.y : (c & 3) == 2 ? q4.z : q4.w;
-                    uint32_t o[4];
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         uint32_t v;
                         const uint32_t shv = j ? (word >> (4 * j)) : word;
                         asm("lop3.b32 %0, %1, %2, %3, 0xEA;\n" : "=r"(v) : "r"(shv), "r"(k_mask), "r"(k_magic));
-                        o[j] = bf16x2_mul_(bf16x2_add_(v, nz2), sc2);
+                        o[4 * c + j] = bf16x2_mul_(bf16x2_add_(v, nz2), sc2);
                     }
-                    *reinterpret_cast<uint4 *>(arow + ((c ^ (t & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
                 }
-                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                tmem_st32(tmem_a + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(s * TC_A_COLS), o);
+                asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
                 __syncwarp();
                 if (lane == 0) bar_arrive(&sh->full[s]);
             }
@@ -220,33 +224,41 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
     } else if (warp < TC_THREADS / 32 - 1) {
         // ---------------------------------------------------------- epilogue
         const int quad = warp & 3;
+        const bool aligned = (N & 7) == 0 && ((uintptr_t)y & 15) == 0;
         uint32_t tuse = 0;
         for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x, ++tuse) {
             TC_ITEM(it)
-            const int ab = tuse & 1;
-            if (!bar_wait(&sh->accfull[ab], (tuse >> 1) & 1, failed)) break;
+            const int ab = tuse % ACCS;
+            if (!bar_wait(&sh->accfull[ab], (tuse / ACCS) & 1, failed)) break;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const int n = nt * 128 + quad * 32 + lane;
 #pragma unroll 1
-            for (int c = 0; c < NTOK / 32; ++c) {
+            for (int c = 0; c < NTOK / 32 && mt * NTOK + c * 32 < M; ++c) {
                 uint32_t v[32];
                 const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(ab * NTOK + c * 32);
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                    "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
-                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                      "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-                      "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-                      "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                    : "r"(taddr));
-                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                if (n < N) {
+                __syncwarp();  // the tensor-memory load is a whole-warp operation
+                tmem_ld32(v, taddr);
+                if (ksplit > 1) {  // a split is chosen for whole vectors of N only
+                    float *out = reinterpret_cast<float *>(stage + quad * 1024);
+                    const int tok = mt * NTOK + c * 32, n0 = nt * 128 + quad * 32;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        out[(j & 15) * 32 + lane] = __uint_as_float(v[j]);
+                        if ((j & 15) == 15)
+                            flush_rows_f32<16>(out, [&](int i) { return part + ((size_t)ksp * M + tok + j - 15 + i) * N + n0; }, M - tok - (j - 15), N - n0, lane);
+                    }
+                } else if (aligned) {
+                    __nv_bfloat16 *out = stage + quad * 1024;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) out[j * 32 + lane] = __float2bfloat16_rn(__uint_as_float(v[j]));
+                    const int tok = mt * NTOK + c * 32, n0 = nt * 128 + quad * 32;
+                    flush_rows<32>(out, y + (size_t)tok * N + n0, N, M - tok, N - n0, lane);
+                } else if (n < N) {
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
                         const int tok = mt * NTOK + c * 32 + j;
                         if (tok < M) {
-                            if (ksplit > 1) part[((size_t)ksp * M + tok) * N + n] = __uint_as_float(v[j]);
-                            else y[(size_t)tok * N + n] = __float2bfloat16_rn(__uint_as_float(v[j]));
+                            y[(size_t)tok * N + n] = __float2bfloat16_rn(__uint_as_float(v[j]));
                         }
                     }
                 }
@@ -263,7 +275,7 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
     if (threadIdx.x == 0 && sh->failed) atomicExch(status, (int)AB2_ERR_TIMEOUT);
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"((uint32_t)(2 * NTOK)));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(tc_cols<NTOK>()));
     }
 }
 
@@ -289,14 +301,14 @@ __global__ void splitk_reduce_kernel(const float *__restrict__ part, __nv_bfloat
 constexpr size_t TC_SPLIT_MAX_BYTES = (size_t)128 << 20;
 
 template <int NTOK>
-int launch_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t s) {
+int launch_tc(const ab2_qweight *w, const void *x, int M, void *y, int ksplit, cudaStream_t s) {
     int *status = nullptr;
     int rc = device_status_word(&status);
     if (rc != AB2_OK) return rc;
     CUtensorMap map;
     rc = make_x_map(&map, x, M, w->K, NTOK);
     if (rc != AB2_OK) return rc;
-    const size_t smem = 1024 + tc_stages<NTOK>() * (TC_A_BYTES + NTOK * 128) + tc_wslots<NTOK>() * TC_WSLOT_BYTES + sizeof(TcShared);
+    const size_t smem = 1024 + tc_stages<NTOK>() * NTOK * 128 + tc_wslots<NTOK>() * TC_WSLOT_BYTES + TC_OUT_BYTES + sizeof(TcShared);
     static bool configured[64] = {false};  // the attribute is per device
     int dev = 0;
     AB2_CUDA(cudaGetDevice(&dev));
@@ -306,26 +318,15 @@ int launch_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t 
         configured[dev] = true;
     }
     const int tiles = ((w->N + 127) / 128) * ((M + NTOK - 1) / NTOK);
-    // Fewer tiles than about half the SMs: split K so that the machine is busy (512 tokens on the
-    // 14336 x 4096 weight are 64 tiles of 256 tokens).  The sums of the splits are f32; one rounding.
-    const int sms = device_sm_count(), G = w->K / 128;
-    int ksplit = 1;
     float *part = nullptr;
     ScratchLease ws(s);
-    static const bool no_split = getenv("AB2_GEMM_NO_SPLITK") != nullptr;
-    if (!no_split && tiles * 2 <= sms + sms / 4 && G >= 8 && w->N % 8 == 0) {
-        ksplit = std::max(1, std::min(4, std::min(G / 4, sms / tiles)));  // all items in one wave
-        const size_t bytes = (size_t)ksplit * M * w->N * sizeof(float);
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (bytes > TC_SPLIT_MAX_BYTES || cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) ksplit = 1;
-        if (ksplit > 1) {
-            rc = ws.take(bytes);
-            if (rc != AB2_OK) return rc;
-            part = (float *)ws.ptr;
-        }
+    if (ksplit > 1) {
+        rc = ws.take((size_t)ksplit * M * w->N * sizeof(float));
+        if (rc != AB2_OK) return rc;
+        part = (float *)ws.ptr;
     }
     const int items = tiles * ksplit;
-    const int grid = std::min(items, sms);
+    const int grid = std::min(items, device_sm_count());
     gemm_w4a16_tc_kernel<NTOK><<<grid, TC_THREADS, smem, s>>>((const uint32_t *)w->codes, map, (__nv_bfloat16 *)y, w->N, w->K, M, status, ksplit, part);
     if (ksplit > 1) launch_splitk_reduce(part, (__nv_bfloat16 *)y, M, w->N, ksplit, s);
     AB2_LAUNCH_CHECK();
@@ -343,12 +344,21 @@ void launch_splitk_reduce(const float *part, __nv_bfloat16 *y, int M, int N, int
 // Y[M][N] = X[M][K] . W^T on the tcgen05 path (W4A16, group 128, bf16).
 int qlinear_w4a16_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t s) {
     AB2_REQUIRE(((uintptr_t)x & 15) == 0 && (w->K * 2) % 16 == 0, AB2_ERR_BAD_ALIGN, "activations must be 16-byte aligned");
-    if (M <= 48) return launch_tc<32>(w, x, M, y, s);
-    // From 257 tokens on, 256-token tiles: an unpacked weight stage then feeds twice the MMA work, which
-    // is what bounds the kernel at 128 (512 tokens on the 4096 x 28672 weight: 139 against 228 us), even
-    // where fewer tiles than SMs remain (4096 x 4096 at 512 tokens: 45 against 43 us).
-    if (M <= 256) return launch_tc<128>(w, x, M, y, s);
-    return launch_tc<256>(w, x, M, y, s);
+    // Measured: rounds of 19.7 / 22.3 / 27.1 us of tiles of 128 / 192 / 256 tokens over K = 4096 (28672 channels, 2048 tokens),
+    // 68 / 73 / 85 over K = 14336; a tile of 32 takes what one of 128 does but for its stores.  Splitting K (few tiles:
+    // 512 tokens on the 4096 x 14336 weight are 64 of 256) needs N in whole vectors and a workspace that a recorded launch has not.
+    static const GemmTileCost costs[] = {{32, 0.5, 0.58}, {128, 1.0, 0.605}, {192, 2.2, 0.63}, {256, 4.0, 0.72}};
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool recorded = cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+    static const bool no_split = getenv("AB2_GEMM_NO_SPLITK") != nullptr;
+    const bool split = !recorded && !no_split && w->N % 8 == 0 && (size_t)4 * M * w->N * sizeof(float) <= TC_SPLIT_MAX_BYTES;
+    const GemmTileChoice c = choose_gemm_tile(costs, M, w->N, w->K / 128, device_sm_count(), split ? 4 : 1);
+    switch (c.ntok) {
+    case 32: return launch_tc<32>(w, x, M, y, c.ksplit, s);
+    case 128: return launch_tc<128>(w, x, M, y, c.ksplit, s);
+    case 192: return launch_tc<192>(w, x, M, y, c.ksplit, s);
+    default: return launch_tc<256>(w, x, M, y, c.ksplit, s);
+    }
 }
 
 }  // namespace ab2

@@ -171,6 +171,56 @@ __device__ __forceinline__ uint32_t bf16x2_mul_(uint32_t a, uint32_t b) {
 }
 
 
+// T tokens x the warp's 32 channels, rounded to bf16, wait in `stage` ([T][32], the warp's own) and go out to rows of
+// `ld` elements: `rows` and `cols` of them exist.  Stored straight from the lanes, 32 instructions of 64 bytes for 32
+// tokens, they took 50 to 60 ns a token, and those of the last round of tiles are not hidden behind MMAs.
+// y lies on a 16-byte boundary; ld and cols are multiples of 8.
+template <int T>
+__device__ __forceinline__ void flush_rows(const __nv_bfloat16 *stage, __nv_bfloat16 *y, long long ld, int rows, int cols, int lane) {
+    __syncwarp();
+    const int n = (lane & 3) * 8, row = lane >> 2;
+#pragma unroll
+    for (int i = 0; i < T; i += 8) {
+        const uint4 q = *reinterpret_cast<const uint4 *>(stage + (i + row) * 32 + n);
+        if (i + row < rows && n < cols) *reinterpret_cast<uint4 *>(y + (i + row) * ld + n) = q;
+    }
+    __syncwarp();
+}
+
+// The same for T tokens of f32 ([T][32]); row(j), called by the whole warp, is where token j's channels of the warp start.
+template <int T, class Row>
+__device__ __forceinline__ void flush_rows_f32(const float *stage, Row row, int rows, int cols, int lane) {
+    __syncwarp();
+    const int n = (lane & 7) * 4, r = lane >> 3;
+#pragma unroll
+    for (int i = 0; i < T; i += 4) {
+        const float4 q = *reinterpret_cast<const float4 *>(stage + (i + r) * 32 + n);
+        float *y = row(i + r);
+        if (i + r < rows && n < cols) *reinterpret_cast<float4 *>(y + n) = q;
+    }
+    __syncwarp();
+}
+
+// What a tile of ntok tokens by 128 channels takes: `fixed` us and `group` us per 128 of K.
+struct GemmTileCost { int ntok; double fixed, group; };
+// Tile and K split of a GEMM over G groups: rounds of items on the SMs times an item's time.  A split of at most `splits`
+// fits one round; its parts are written and read as f32 at about 4 TB/s by a pass that takes 4 us more.
+struct GemmTileChoice { int ntok, ksplit; };
+template <int COUNT>
+inline GemmTileChoice choose_gemm_tile(const GemmTileCost (&costs)[COUNT], int M, int N, int G, int sms, int splits) {
+    GemmTileChoice best = {costs[0].ntok, 1};
+    double best_us = 1e30;
+    for (const GemmTileCost &c : costs) {
+        const long long tiles = (long long)((N + 127) / 128) * ((M + c.ntok - 1) / c.ntok);
+        for (int ks = 1; ks <= splits && (ks == 1 || (tiles * ks <= sms && G / ks >= 4)); ++ks) {
+            const double rounds = (double)((tiles * ks + sms - 1) / sms);
+            const double us = rounds * (c.fixed + c.group * ((G + ks - 1) / ks)) + (ks > 1 ? 4.0 + (double)ks * M * N * 8 / 4e6 : 0.0);
+            if (us < best_us) { best_us = us; best = {c.ntok, ks}; }
+        }
+    }
+    return best;
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);

@@ -59,6 +59,21 @@ def test_q4km_many_tokens_streams_and_capture():
     assert torch.equal(y, alone[0])
 
 
+# tiles of 128 channels and 32, 128, 192 or 256 tokens, their edges; K split or not; rows stored in 16-byte pieces (N % 8 == 0,
+# y on a 16-byte boundary) or element by element.  W4A16: the MMA multiplies the weights rounded to bf16.
+@pytest.mark.parametrize("M", [9, 32, 33, 65, 128, 129, 192, 193, 257, 385, 520, 1100])
+@pytest.mark.parametrize("method,N,K", [("w4a16", 256, 512), ("w4a16", 2000, 1024), ("w4a16", 1004, 2048), ("w4a16", 4096, 384),
+                                        ("int8_channel", 130, 128), ("int8_channel", 2000, 1024), ("int8_channel", 6144, 256),
+                                        ("bf16", 136, 64), ("bf16", 2004, 512), ("bf16", 5120, 256)])
+def test_tensor_core_tiles(method, N, K, M):
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    w = torch.randn((N, K), generator=g, device="cuda")
+    lin = pkg().QuantLinear.from_bf16(w.to(torch.bfloat16)) if method == "bf16" else pkg().QuantLinear.quantise(w, method, 128)
+    x = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
+    check(lin, x, 2 * K + (2 ** 15 if method == "w4a16" else 0))
+    assert torch.equal(lin(x), lin(x))
+
+
 # tiles of 64 x 64 and 32 x 32 outputs, steps of 32 columns
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("method", ["int8_channel", "int4", "q4_k_m", "w4a16"])
