@@ -166,7 +166,8 @@ static int forward_launches(ab2_model *m, ab2_kv *kv, const uint32_t *ids, int S
                             int len_hint, cudaStream_t s) {
     if (m->stack) return stack_forward(m->stack, kv, ids, S, row0, nrows, logits_mode, (float *)logits, argmax_out, len_hint, s);
     const ab2_model_config &c = m->cfg;
-    const int T = nrows * S, d = c.d_model, hd = c.head_dim;
+    const int all = nrows * S, d = c.d_model, hd = c.head_dim;
+    int T = all;  // tokens that the launches from here on work on
     const size_t esz = dtype_size(m->dtype);
     const long long qkv_stride = (long long)(c.n_heads + 2 * c.n_kv_heads) * hd;
     const float scale = (float)(1.0 / std::sqrt((double)hd));
@@ -187,6 +188,9 @@ static int forward_launches(ab2_model *m, ab2_kv *kv, const uint32_t *ids, int S
         pending = false;
         return rc2;
     };
+    // one row whose last token alone matters at the end; its rows keep the alignment of the buffers
+    const bool last_alone = nrows == 1 && S > 1 && logits_mode != 2 && d * esz % 16 == 0 && (size_t)c.n_heads * hd * esz % 16 == 0;
+    void *x = m->x, *attn = m->attn;  // first of those tokens
     bool xn_ready = false;  // the preceding layer's last residual add also wrote RMSNorm(x; norm1) of this layer
     for (int l = 0; l < c.n_layers; ++l) {
         LayerWeights &L = m->layers[l];
@@ -218,6 +222,14 @@ static int forward_launches(ab2_model *m, ab2_kv *kv, const uint32_t *ids, int S
             STEP(attention_cached_device(kv, l, m->qkv, m->attn, S, S, row0, nrows, scale, m->dtype, st, len_hint, s));
         }
         const bool tp = m->tp && m->tp->world > 1;
+        // A prompt of one row of which only the last token's logits are wanted: nothing past the last layer's attention
+        // reads the other tokens, so the rest of that layer runs on the last one (4 layers, 3001 tokens: 6.24 -> 5.15 ms;
+        // 8 layers, 512 tokens: 2.53 -> 2.34).
+        if (l + 1 == c.n_layers && last_alone && !tp) {
+            x = (char *)m->x + (size_t)(S - 1) * d * esz;
+            attn = (char *)m->attn + (size_t)(S - 1) * c.n_heads * hd * esz;
+            T = 1;
+        }
         if (tp) {
             // row-parallel O and down produce partial sums: all-reduce, then the residual add
             const size_t nd = (size_t)T * d;
@@ -266,8 +278,8 @@ static int forward_launches(ab2_model *m, ab2_kv *kv, const uint32_t *ids, int S
             // tokens on this measured faster than the residual / SwiGLU epilogues of the decode GEMM:
             // 6330 against 6120 tok/s at 32 rows, 7360 against 6740 at 64; with the strip kernel on the
             // gate|up weight, 7980 against 7850 at 32 rows)
-            STEP(qlinear_dispatch(L.part[3], m->attn, T, m->dtype, m->proj, s));
-            STEP(launch_add_rms_norm(m->x, m->proj, L.norm2, m->xn, T, d, c.rms_eps, m->dtype, s));
+            STEP(qlinear_dispatch(L.part[3], attn, T, m->dtype, m->proj, s));
+            STEP(launch_add_rms_norm(x, m->proj, L.norm2, m->xn, T, d, c.rms_eps, m->dtype, s));
             STEP(qlinear_dispatch(L.wgu, m->xn, T, m->dtype, m->gu, s));
             {
                 size_t n8 = (size_t)T * (c.ffn_hidden / 8);
@@ -277,43 +289,46 @@ static int forward_launches(ab2_model *m, ab2_kv *kv, const uint32_t *ids, int S
             }
             STEP(qlinear_dispatch(L.part[6], m->hid, T, m->dtype, m->proj, s));
             if (l + 1 < c.n_layers) {  // the add and the next layer's first normalisation in one launch
-                STEP(launch_add_rms_norm(m->x, m->proj, m->layers[l + 1].norm1, m->xn, T, d, c.rms_eps, m->dtype, s));
+                STEP(launch_add_rms_norm(x, m->proj, m->layers[l + 1].norm1, m->xn, T, d, c.rms_eps, m->dtype, s));
                 xn_ready = true;
             } else {
-                STEP(launch_add(m->x, m->proj, m->x, (size_t)T * d, m->dtype, s));
+                STEP(launch_add(x, m->proj, x, (size_t)T * d, m->dtype, s));
             }
         } else if (m->fused_epilogues) {
-            STEP(qlinear_w4a16_mma_add(L.part[3], m->attn, T, m->x, m->x, s));
-            STEP(norm_linear(m, L.wgu, m->x, L.norm2, T, m->hid, 2, s));
-            STEP(qlinear_w4a16_mma_add(L.part[6], m->hid, T, m->x, m->x, s));
+            STEP(qlinear_w4a16_mma_add(L.part[3], attn, T, x, x, s));
+            STEP(norm_linear(m, L.wgu, x, L.norm2, T, m->hid, 2, s));
+            STEP(qlinear_w4a16_mma_add(L.part[6], m->hid, T, x, x, s));
         } else {
             // a few tokens over weights without a GEMV of their own: the norm, the gated unit and the residual additions
             // ride with the linears
             if (qlinear_step_eligible(L.part[3], m->dtype, T)) {
-                STEP(qlinear_step_add(L.part[3], m->attn, m->x, T, m->dtype, m->x, s));
+                STEP(qlinear_step_add(L.part[3], attn, x, T, m->dtype, x, s));
             } else {
-                STEP(qlinear_dispatch(L.part[3], m->attn, T, m->dtype, m->proj, s));
-                STEP(launch_add(m->x, m->proj, m->x, (size_t)T * d, m->dtype, s));
+                STEP(qlinear_dispatch(L.part[3], attn, T, m->dtype, m->proj, s));
+                STEP(launch_add(x, m->proj, x, (size_t)T * d, m->dtype, s));
             }
             if (qlinear_step_eligible(L.wgu, m->dtype, T)) {
-                STEP(qlinear_step_norm(L.wgu, m->x, L.norm2, c.rms_eps, T, m->dtype, true, m->hid, s));
+                STEP(qlinear_step_norm(L.wgu, x, L.norm2, c.rms_eps, T, m->dtype, true, m->hid, s));
             } else {
-                STEP(launch_rms_norm(m->x, L.norm2, m->xn, T, d, c.rms_eps, m->dtype, s));
+                STEP(launch_rms_norm(x, L.norm2, m->xn, T, d, c.rms_eps, m->dtype, s));
                 STEP(qlinear_dispatch(L.wgu, m->xn, T, m->dtype, m->gu, s));
                 STEP(launch_swiglu_fused(m->gu, m->hid, T, c.ffn_hidden, m->dtype, s));
             }
             if (qlinear_step_eligible(L.part[6], m->dtype, T)) {
-                STEP(qlinear_step_add(L.part[6], m->hid, m->x, T, m->dtype, m->x, s));
+                STEP(qlinear_step_add(L.part[6], m->hid, x, T, m->dtype, x, s));
             } else {
                 STEP(qlinear_dispatch(L.part[6], m->hid, T, m->dtype, m->proj, s));
-                STEP(launch_add(m->x, m->proj, m->x, (size_t)T * d, m->dtype, s));
+                STEP(launch_add(x, m->proj, x, (size_t)T * d, m->dtype, s));
             }
         }
     }
     if (logits_mode == 0 && argmax_out == nullptr) return AB2_OK;
     const void *hidden = xcur;
-    int rows = T;
-    if (logits_mode != 2 && S > 1) {  // only the last token of each row is needed
+    int rows = all;
+    if (T < all) {
+        hidden = x;
+        rows = T;
+    } else if (logits_mode != 2 && S > 1) {  // only the last token of each row is needed
         switch (m->dtype) {
         case AB2_F32: gather_last_kernel<float><<<nrows, 128, 0, s>>>((const float *)m->x, (float *)m->proj, S, d); break;
         case AB2_F16: gather_last_kernel<__half><<<nrows, 128, 0, s>>>((const __half *)m->x, (__half *)m->proj, S, d); break;
@@ -347,7 +362,7 @@ static int forward_launches(ab2_model *m, ab2_kv *kv, const uint32_t *ids, int S
     if (argmax_out) {
         // last token of each row
         const char *src = (const char *)lg;
-        if (rows == T && S > 1) {
+        if (rows == all && S > 1) {
             return fail(AB2_ERR_UNSUPPORTED, "argmax with all-token logits needs S == 1");
         }
         STEP(launch_argmax(src, nrows, c.vocab, m->dtype, argmax_out, s));

@@ -474,7 +474,8 @@ static int poly_ffn(Stack *st, StackLayer &L, const void *in, int T, cudaStream_
 
 int stack_forward(Stack *st, ab2_kv *kv, const uint32_t *ids, int S, int row0, int nrows, int logits_mode, float *logits,
                   uint32_t *argmax_out, int len_hint, cudaStream_t s) {
-    const int T = nrows * S, d = st->cfg.d_model;
+    const int all = nrows * S, d = st->cfg.d_model;
+    int T = all;  // tokens that the launches from here on work on
     int max_len = len_hint;
     if (max_len <= 0)
         for (int i = 0; i < nrows; ++i) max_len = std::max(max_len, kv->lens_host[kv_row_host(kv, row0, i)] + S);
@@ -514,7 +515,17 @@ int stack_forward(Stack *st, ab2_kv *kv, const uint32_t *ids, int S, int row0, i
             if (sp.mixer == AB2_MIX_LATENT) STEP(latent_mixer(st, L, kv, r, S, row0, nrows, max_len, s));
             else STEP(attention_mixer(st, L, kv, r, S, row0, nrows, max_len, s));
         }
-        STEP(linear_bf16(L.out, st->mixed, T, st->dtype, st->parts, LIN_F32, 0, s));
+        const void *mixed = st->mixed;
+        // A prompt of one row of which only the last token's logits are wanted: nothing past the last run's mixer reads
+        // the other tokens, so the rest of that run works on the last one.
+        if (r + 1 == n_runs && nrows == 1 && S > 1 && last && d % 8 == 0 && L.out->K % 8 == 0) {
+            T = 1;
+            n.x = st->x + (size_t)(S - 1) * d;
+            mixed = (const char *)st->mixed + (size_t)(S - 1) * L.out->K * dtype_size(st->dtype);
+            if (in == st->x) in = n.x;
+            if (sp.ffn == AB2_FFN_MOE && sp.routing == AB2_ROUTE_TABLE) STEP(moe_route_tables(st->route_tables, st->n_route_tables, ids + S - 1, st->cfg.vocab, 1, s));
+        }
+        STEP(linear_bf16(L.out, mixed, T, st->dtype, st->parts, LIN_F32, 0, s));
         n.w = L.norm1; n.parts = st->parts; n.nparts = 1; n.extra = nullptr;
         if (sp.ffn == AB2_FFN_NONE) end_of_run();
         else { n.add = nullptr; n.x0 = nullptr; n.w_next = pre ? L.pre2 : nullptr; }
@@ -527,10 +538,10 @@ int stack_forward(Stack *st, ab2_kv *kv, const uint32_t *ids, int S, int row0, i
         STEP(launch_residual_norm(n, RN_ADD, T, st->dtype, s));
     }
     if (!want_logits) return AB2_OK;
-    const int rows = last ? nrows : T;
+    const int rows = last ? nrows : all;
     AB2_REQUIRE(!argmax_out || last || S == 1, AB2_ERR_UNSUPPORTED, "argmax with all-token logits needs S == 1");
     if (!final_norm_rides) {
-        n.w = st->final_norm; n.step = last ? S : 1; n.out = st->head_in;
+        n.w = st->final_norm; n.step = last && T == all ? S : 1; n.out = st->head_in;
         STEP(launch_residual_norm(n, RN_FINAL, rows, st->dtype, s));
     }
     float *lg = logits ? logits : st->logits_scratch;
