@@ -13,13 +13,14 @@
 // dimension, one persistent CTA per SM:
 //   warp 0       producer of the codes: a TMA tile of 128 channels x one block per slot
 //   warp 1       MMA issue; two accumulators, a block each in turn
-//   warps 2-9    unpack, two sets of four warps on alternate stages of 64 K-elements, thread = channel
+//   warps 2-9    unpack, two sets of four warps on alternate stages of 64 K-elements, thread = channel; the integers go
+//                to tensor memory (through shared memory, which the MMAs read too, the kernel took 5 to 11 % longer)
 //   warps 10-17  epilogue, thread = channel and half of the tokens, running sums in registers
 //   warp 18      producer of the activation tiles and of X
 // With fewer tiles than SMs the blocks of a tile are divided over several CTAs; their f32 sums meet in a reduce pass.
 // What bounds it is the unpack and the per-block epilogue (about 450 cycles a stage against the MMA's 257 at 128
 // tokens).  14336 x 4096 at 300 tokens: 3329 us on CUDA cores,
-// 88 us here (400 TFLOP/s); 3072 x 2048: 421 -> 20 us, at 9 tokens 17 -> 11.
+// 76 us here (464 TFLOP/s); 3072 x 2048: 421 -> 20 us, at 9 tokens 17 -> 11.
 // Every wait on an mbarrier is bounded; on a time-out the CTA records AB2_ERR_TIMEOUT, stops issuing work, frees its
 // tensor memory and returns.
 #include <cuda.h>
@@ -39,7 +40,7 @@ void launch_splitk_reduce(const float *part, __nv_bfloat16 *y, int M, int N, int
 namespace {
 
 constexpr int QB_MAX_STAGES = 6, QB_MAX_WSLOTS = 6;
-constexpr int QB_A_BYTES = 128 * 128;      // 128 channels x 64 bf16
+constexpr int QB_A_COLS = 32;              // tensor-memory columns of 64 K-elements: two bf16 per column, a lane per channel
 constexpr int QB_WSLOT_BYTES = 128 * 128;  // 128 channels x 256 codes
 constexpr int QB_UNPACK_WARPS = 8, QB_EPI_WARPS = 8;
 constexpr int QB_OUT_BYTES = QB_EPI_WARPS * 16 * 32 * 2;  // an epilogue warp's 16 tokens x 32 channels on their way out
@@ -91,11 +92,11 @@ template <int NTOK>
 __global__ void __launch_bounds__(QB_THREADS, 1)
 gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, QbArgs a, int *status) {
     constexpr int STAGES = qb_stages<NTOK>(), WSLOTS = qb_wslots<NTOK>(), B_BYTES = NTOK * 128;
-    constexpr uint32_t TMEM_COLS = 2 * NTOK;
+    constexpr uint32_t ACC_COLS = 2 * NTOK, TMEM_COLS = ACC_COLS + STAGES * QB_A_COLS > 256 ? 512 : 256;
+    static_assert(ACC_COLS + STAGES * QB_A_COLS <= 512, "accumulators and operand stages fit");
     constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NTOK >> 3) << 17) | ((128u >> 4) << 24);
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *a_st = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);  // [STAGES][QB_A_BYTES]
-    uint8_t *b_st = a_st + STAGES * QB_A_BYTES;                                    // [STAGES][B_BYTES]
+    uint8_t *b_st = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);  // [STAGES][B_BYTES]
     uint8_t *w_ring = b_st + STAGES * B_BYTES;                                     // [WSLOTS][QB_WSLOT_BYTES]
     __nv_bfloat16 *stage = (__nv_bfloat16 *)(w_ring + WSLOTS * QB_WSLOT_BYTES);  // [QB_EPI_WARPS][16][32]
     QbShared *sh = (QbShared *)((uint8_t *)stage + QB_OUT_BYTES);
@@ -127,7 +128,7 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = sh->tmem_base;
+    const uint32_t tmem = sh->tmem_base, tmem_a = tmem + ACC_COLS;
     int nt, mt, sp, b0, b1;
 
     if (warp == 0) {
@@ -178,8 +179,9 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                     const int st = suse % STAGES;
                     ok = warp_wait(&sh->full[st], (suse / STAGES) & 1, failed);
                     if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                     if (elect_one()) {
-                        umma_stage(tmem + (uint32_t)(ab * NTOK), umma_desc(sptr(a_st + st * QB_A_BYTES)), umma_desc(sptr(b_st + st * B_BYTES)), IDESC, q == 0);
+                        umma_stage_ts(tmem + (uint32_t)(ab * NTOK), tmem_a + (uint32_t)(st * QB_A_COLS), umma_desc(sptr(b_st + st * B_BYTES)), IDESC, q == 0);
                         umma_commit(&sh->empty[st]);
                         if (q == 3) umma_commit(&sh->accfull[ab]);
                     }
@@ -189,7 +191,7 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         }
     } else if (warp < 2 + QB_UNPACK_WARPS) {
         // ---------------------------------------------------------- unpack: codes -> bf16 integers
-        const int t = (threadIdx.x - 64) & 127, set = (threadIdx.x - 64) >> 7;
+        const int t = (warp & 3) * 32 + lane, set = (warp - 2) >> 2;  // channel: the warp's lanes of tensor memory
         uint32_t wuse = 0;
         uint32_t k_mask = 0x000F000Fu, k_magic = 0x43004300u, k_off = 0xC300C300u;  // -128
         asm volatile("" : "+r"(k_mask), "+r"(k_magic), "+r"(k_off));
@@ -210,23 +212,24 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                 for (int h = 0; h < 2; ++h) {
                     const uint32_t suse = 4 * wuse + set + 2 * h;
                     const int st = suse % STAGES;
-                    if (!bar_wait(&sh->empty[st], ((suse / STAGES) & 1) ^ 1, failed)) break;
-                    uint8_t *arow = a_st + st * QB_A_BYTES + t * 128;
+                    if (!warp_wait(&sh->empty[st], ((suse / STAGES) & 1) ^ 1, failed)) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    uint32_t o[32];  // two bf16 each
 #pragma unroll
                     for (int c = 0; c < 8; ++c) {
                         const uint4 q4 = h ? raw[2 + (c >> 2)] : raw[c >> 2];
                         const uint32_t word = (c & 3) == 0 ? q4.x : (c & 3) == 1 ? q4.y : (c & 3) == 2 ? q4.z : q4.w;
-                        uint32_t o[4];
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {  // codes j and j + 4
                             uint32_t v;
                             const uint32_t shv = j ? (word >> (4 * j)) : word;
                             asm("lop3.b32 %0, %1, %2, %3, 0xEA;\n" : "=r"(v) : "r"(shv), "r"(k_mask), "r"(k_magic));
-                            o[j] = bf16x2_add_(v, k_off);
+                            o[4 * c + j] = bf16x2_add_(v, k_off);
                         }
-                        *reinterpret_cast<uint4 *>(arow + ((c ^ (t & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
                     }
-                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                    tmem_st32(tmem_a + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(st * QB_A_COLS), o);
+                    asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
                     __syncwarp();
                     if (lane == 0) bar_arrive(&sh->full[st]);
                 }
@@ -317,8 +320,8 @@ int launch_qb(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t 
     int rc = device_status_word(&status);
     if (rc != AB2_OK) return rc;
     const int N = w->N, K = w->K, KB = K / 256, Mp = (M + NTOK - 1) / NTOK * NTOK;
-    const size_t smem = 1024 + qb_stages<NTOK>() * (QB_A_BYTES + NTOK * 128) + qb_wslots<NTOK>() * QB_WSLOT_BYTES + QB_OUT_BYTES + sizeof(QbShared);
-    static_assert(1024 + qb_stages<NTOK>() * (QB_A_BYTES + NTOK * 128) + qb_wslots<NTOK>() * QB_WSLOT_BYTES + QB_OUT_BYTES + sizeof(QbShared) <= 227 * 1024, "shared memory of a CTA");
+    const size_t smem = 1024 + qb_stages<NTOK>() * NTOK * 128 + qb_wslots<NTOK>() * QB_WSLOT_BYTES + QB_OUT_BYTES + sizeof(QbShared);
+    static_assert(1024 + qb_stages<NTOK>() * NTOK * 128 + qb_wslots<NTOK>() * QB_WSLOT_BYTES + QB_OUT_BYTES + sizeof(QbShared) <= 227 * 1024, "shared memory of a CTA");
     static bool configured[64] = {false};  // the attribute is per device
     int dev = 0;
     AB2_CUDA(cudaGetDevice(&dev));
