@@ -1,4 +1,4 @@
-// W4A16 (group 128, bf16) decode GEMM for 2..32 tokens on the 5th-generation
+// W4A16 (group 128, bf16) decode GEMM for 2..64 tokens on the 5th-generation
 // tensor cores, built so that the packed weights cross HBM once and cost one
 // shift and one logic op per pair of codes whatever the token count.
 //
@@ -79,26 +79,16 @@ struct DgShared {
     int last_flag;
 };
 
-template <int NTOK>
-__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&v)[NTOK]);
-template <>
-__device__ __forceinline__ void tmem_ld<16>(uint32_t taddr, uint32_t (&v)[16]) {
+// 16 columns of the warp's lanes; the registers pass through the wait, so that nothing computed from them can move ahead of it.
+__device__ __forceinline__ void tmem_ld16(uint32_t (&v)[16], uint32_t taddr) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
           "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
         : "r"(taddr));
-}
-template <>
-__device__ __forceinline__ void tmem_ld<32>(uint32_t taddr, uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]),
+                   "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])::"memory");
 }
 
 // units [u0, u1) of this CTA; the first `rem` CTAs take base + 1 units
@@ -124,7 +114,7 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
                      int *counters, int *status) {
     constexpr int B_BYTES = NTOK * 128;
     constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NTOK >> 3) << 17) | ((128u >> 4) << 24);
-    constexpr uint32_t ACC_COLS = DG_ACC * NTOK, TMEM_COLS = 256u;
+    constexpr uint32_t ACC_COLS = DG_ACC * NTOK, TMEM_COLS = NTOK > 32 ? 512u : 256u;
     static_assert(ACC_COLS + DG_STAGES * DG_A_COLS <= TMEM_COLS, "accumulators and operand stages fit");
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -273,17 +263,22 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
             const int nt = u / G, g = u - nt * G;
             const int ab = use % DG_ACC;
             if (!bar_wait(&sh->accfull[ab], (use / DG_ACC) & 1, failed)) break;
+            __syncwarp();  // the tensor-memory load is a whole-warp operation
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            uint32_t d[NTOK];
-            tmem_ld<NTOK>(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(ab * NTOK), d);
-            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-            const uint32_t pr = sh->params[use % DG_PARAM_BUFS][row];
+            const float sc = __uint_as_float(sh->params[use % DG_PARAM_BUFS][row] << 16);
+            constexpr int COLS = NTOK < 32 ? 16 : 32;  // tokens at a time
+#pragma unroll
+            for (int c = 0; c < NTOK; c += COLS) {
+                uint32_t d[COLS];
+                const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(ab * NTOK + c);
+                if constexpr (COLS == 16) tmem_ld16(d, taddr);
+                else tmem_ld32(d, taddr);
+#pragma unroll
+                for (int j = 0; j < COLS; ++j) acc[c + j] = fmaf(sc, __uint_as_float(d[j]), acc[c + j]);
+            }
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
             __syncwarp();
             if (lane == 0) bar_arrive(&sh->accempty[ab]);
-            const float sc = __uint_as_float(pr << 16);
-#pragma unroll
-            for (int j = 0; j < NTOK; ++j) acc[j] = fmaf(sc, __uint_as_float(d[j]), acc[j]);
 
             if (g != G - 1 && u + 1 != rg.u1) continue;
             // ---- end of this CTA's share of channel tile nt
@@ -316,13 +311,6 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
             }
             if (finish) {
                 const int n = nt * 128 + row;
-                // the residual may alias the output: its values are all read before the first store
-                float rv[EPI == W4_EPI_ADD ? NTOK : 1];
-                if (EPI == W4_EPI_ADD) {
-#pragma unroll
-                    for (int j = 0; j < NTOK; ++j)
-                        rv[j] = (j < M && n < N) ? __bfloat162float(resid[(size_t)j * N + n]) : 0.f;
-                }
 #pragma unroll
                 for (int j = 0; j < NTOK; ++j) {
                     if (EPI == W4_EPI_SWIGLU) {
@@ -338,7 +326,8 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
                         if (EPI == W4_EPI_F32) {
                             reinterpret_cast<float *>(y)[o] = v;
                         } else {
-                            if (EPI == W4_EPI_ADD) v = rv[EPI == W4_EPI_ADD ? j : 0] + __bfloat162float(__float2bfloat16_rn(v));
+                            // the residual may alias the output: a thread reads and writes the same elements
+                            if (EPI == W4_EPI_ADD) v = __bfloat162float(resid[o]) + __bfloat162float(__float2bfloat16_rn(v));
                             y[o] = __float2bfloat16_rn(v);
                         }
                     }
@@ -394,14 +383,14 @@ int launch_dg(const ab2_qweight *w, const void *x, int M, void *y, const void *r
 
 }  // namespace
 
-// Scratch the kernel needs per CTA: two slots of [32 tokens][128 channels] f32.
-size_t gemv_w4a16_tc_partial_floats_per_cta() { return 2 * 32 * 128; }
+// Scratch the kernel needs per CTA: two slots of [64 tokens][128 channels] f32.
+size_t gemv_w4a16_tc_partial_floats_per_cta() { return 2 * 64 * 128; }
 
-// Y = epilogue(X[M][K] . W^T) for 2..32 tokens; partials / counters are the caller's
+// Y = epilogue(X[M][K] . W^T) for 2..64 tokens; partials / counters are the caller's
 // scratch (zeroed counters, one per 128-channel tile; partials for max_ctas CTAs).
 int qlinear_w4a16_tc_decode(const ab2_qweight *w, const void *x, int M, void *y, const void *resid, int epi,
                             float *partials, int *counters, int max_ctas, cudaStream_t s) {
-    AB2_REQUIRE(M >= 1 && M <= 32, AB2_ERR_BAD_SHAPE, "the decode GEMM serves 1..32 tokens, got %d", M);
+    AB2_REQUIRE(M >= 1 && M <= 64, AB2_ERR_BAD_SHAPE, "the decode GEMM serves 1..64 tokens, got %d", M);
     AB2_REQUIRE(((uintptr_t)x & 15) == 0 && (w->K * 2) % 16 == 0, AB2_ERR_BAD_ALIGN, "activations must be 16-byte aligned");
 #define AB2_DG(NT)                                                                                              \
     switch (epi) {                                                                                              \
@@ -412,7 +401,8 @@ int qlinear_w4a16_tc_decode(const ab2_qweight *w, const void *x, int M, void *y,
     default: return fail(AB2_ERR_BAD_ARG, "unsupported epilogue %d", epi);                                       \
     }
     if (M <= 16) { AB2_DG(16) }
-    AB2_DG(32)
+    if (M <= 32) { AB2_DG(32) }
+    AB2_DG(64)
 #undef AB2_DG
 }
 

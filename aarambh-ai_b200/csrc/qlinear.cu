@@ -283,7 +283,7 @@ static int launch_w4a16_stream(const ab2_qweight *w, const void *x, int M, void 
     if (!align_off && G % W4W_WARPS == 0 && G / W4W_WARPS >= 4 && tiles <= sc.max_ctas && tiles * 10 >= device_sm_count() * 17) grid = tiles;
     const uint32_t *wt = (const uint32_t *)w->codes;
     const int out_n = EPI == W4_EPI_SWIGLU ? w->N / 2 : w->N;
-    // More than 8 tokens go in chunks of up to 32:
+    // More than 8 tokens go in chunks of up to 32, from 33 to 64 in one:
     //   9..24 tokens (and 25..32 on a weight of 24576 rows or more): the strip kernel - a warp multiplies
     //     64 or 32 rows by all tokens, so the activations it loads serve several weight blocks and the
     //     codes are unpacked once for every token.  On the largest shape it takes 96 / 113 / 150 us for
@@ -296,15 +296,19 @@ static int launch_w4a16_stream(const ab2_qweight *w, const void *x, int M, void 
     if constexpr (EPI != W4_EPI_F32_PEER) {
         if (M >= 9 && !norm_w) {
             const bool tc_ok = w->N % 16 == 0;
-            // equal chunks, in whole token tiles: 40 tokens go as 24 + 16, not as 32 + 8
-            const int nchunks = (M + 31) / 32, chunk = ((M + nchunks - 1) / nchunks + 7) / 8 * 8;
+            // equal chunks, in whole token tiles
+            // 33..64 tokens go through the tensor-memory GEMM in one pass, whose weights are then fetched and unpacked once
+            // (64 tokens: 49 us on 4096 x 28672, 22.6 on 4096 x 6144, 20.6 on 4096 x 4096, 33 on 14336 x 4096, against 86,
+            // 34, 32 and 54 in two passes; 33 tokens 49, 21, 21, 33 against 66, 33, 29, 46)
+            const int most = tc_ok && M > 32 ? 64 : 32;
+            const int nchunks = (M + most - 1) / most, chunk = ((M + nchunks - 1) / nchunks + 7) / 8 * 8;
             for (int m0 = 0; m0 < M; m0 += chunk) {
                 const int mv = std::min(chunk, M - m0);
                 const __nv_bfloat16 *xp = (const __nv_bfloat16 *)x + (size_t)m0 * w->K;
                 __nv_bfloat16 *yp = EPI == W4_EPI_F32 ? (__nv_bfloat16 *)((float *)y + (size_t)m0 * out_n)
                                                       : (__nv_bfloat16 *)y + (size_t)m0 * out_n;
                 const __nv_bfloat16 *rp = resid ? (const __nv_bfloat16 *)resid + (size_t)m0 * out_n : nullptr;
-                if (!strip_off && mv >= 9 && (mv <= 24 || w->N >= strip_wide_n || !tc_ok)) {
+                if (!strip_off && mv >= 9 && mv <= 32 && (mv <= 24 || w->N >= strip_wide_n || !tc_ok)) {
                     cudaError_t e;
                     // token tiles, tiles per strip, strips x K slices of a CTA
                     switch ((mv + 7) / 8) {

@@ -61,7 +61,7 @@ def test_q4km_many_tokens_streams_and_capture():
 
 # tiles of 128 channels and 32, 128, 192 or 256 tokens, their edges; K split or not; rows stored in 16-byte pieces (N % 8 == 0,
 # y on a 16-byte boundary) or element by element.  W4A16: the MMA multiplies the weights rounded to bf16.
-@pytest.mark.parametrize("M", [9, 32, 33, 65, 128, 129, 192, 193, 257, 385, 520, 1100])
+@pytest.mark.parametrize("M", [9, 32, 33, 40, 64, 65, 128, 129, 192, 193, 257, 385, 520, 1100])
 @pytest.mark.parametrize("method,N,K", [("w4a16", 256, 512), ("w4a16", 2000, 1024), ("w4a16", 1004, 2048), ("w4a16", 4096, 384),
                                         ("int8_channel", 130, 128), ("int8_channel", 2000, 1024), ("int8_channel", 6144, 256),
                                         ("bf16", 136, 64), ("bf16", 2004, 512), ("bf16", 5120, 256)])
