@@ -116,8 +116,15 @@ __device__ __forceinline__ void pdl_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 }
 
-// Set by the decoder step around its launches.
+// Set by the decoder step around its launches, and by prompts.
 extern thread_local bool g_pdl_launch;
+struct ChainedLaunches {
+    const bool before = g_pdl_launch;
+    explicit ChainedLaunches(bool on) { g_pdl_launch = before || on; }
+    ChainedLaunches(const ChainedLaunches &) = delete;
+    ChainedLaunches &operator=(const ChainedLaunches &) = delete;
+    ~ChainedLaunches() { g_pdl_launch = before; }
+};
 
 template <typename... KArgs, typename... Args>
 static inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,

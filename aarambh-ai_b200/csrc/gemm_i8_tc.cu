@@ -101,6 +101,8 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const float *__restr
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    pdl_wait();  // the setup above overlaps the end of the preceding kernel
+    pdl_launch_dependents();
     const uint32_t tmem = sh->tmem_base, tmem_a = tmem + (uint32_t)(ACCS * NTOK);
 
     if (warp == 0) {
@@ -262,7 +264,8 @@ int launch_i8_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaStream
     }
     const int items = ((w->N + 127) / 128) * ((M + NTOK - 1) / NTOK);
     const int grid = std::min(items, device_sm_count());
-    gemm_i8_tc_kernel<NTOK><<<grid, TC_THREADS, smem, s>>>(wmap, (const float *)w->scales, xmap, (__nv_bfloat16 *)y, w->N, w->K, M, status);
+    cudaError_t e = launch_kernel(gemm_i8_tc_kernel<NTOK>, dim3(grid), dim3(TC_THREADS), smem, s, wmap, (const float *)w->scales, xmap, (__nv_bfloat16 *)y, w->N, w->K, M, status);
+    if (e != cudaSuccess) return fail(AB2_ERR_CUDA, "INT8 GEMM launch failed: %s", cudaGetErrorString(e));
     AB2_LAUNCH_CHECK();
     return AB2_OK;
 }

@@ -72,6 +72,8 @@ struct QbArgs {
 __global__ void __launch_bounds__(256) q4km_prepare_kernel(const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__restrict__ xp, float *__restrict__ xsum,
                                                            int M, int Mp, int K) {
     const int b = blockIdx.x, t = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    pdl_wait();
+    pdl_launch_dependents();
     if (t >= Mp) return;
     float sum = 0.f;
     if (t < M) {
@@ -128,6 +130,8 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    pdl_wait();  // the setup above overlaps the end of the preceding kernel
+    pdl_launch_dependents();
     const uint32_t tmem = sh->tmem_base, tmem_a = tmem + ACC_COLS;
     int nt, mt, sp, b0, b1;
 
@@ -344,9 +348,10 @@ int launch_qb(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t 
     rc = make_x_map(&xmap, xp, M, K, NTOK);
     if (rc == AB2_OK) rc = make_bytes_map(&wmap, w->codes, N, K / 2);
     if (rc != AB2_OK) return rc;
-    q4km_prepare_kernel<<<dim3(KB, (Mp + 7) / 8), 256, 0, s>>>((const __nv_bfloat16 *)x, xp, xsum, M, Mp, K);
+    launch_kernel(q4km_prepare_kernel, dim3(KB, (Mp + 7) / 8), dim3(256), 0, s, (const __nv_bfloat16 *)x, xp, xsum, M, Mp, K);  // checked with the next
     const QbArgs a = {w->block_params, xsum, (__nv_bfloat16 *)y, part, N, KB, M, Mp, ksplit};
-    gemm_q4km_tc_kernel<NTOK><<<std::min(tiles * ksplit, sms), QB_THREADS, smem, s>>>(wmap, xmap, a, status);
+    cudaError_t e = launch_kernel(gemm_q4km_tc_kernel<NTOK>, dim3(std::min(tiles * ksplit, sms)), dim3(QB_THREADS), smem, s, wmap, xmap, a, status);
+    if (e != cudaSuccess) return fail(AB2_ERR_CUDA, "Q4_K_M GEMM launch failed: %s", cudaGetErrorString(e));
     if (ksplit > 1) launch_splitk_reduce(part, (__nv_bfloat16 *)y, M, N, ksplit, s);
     AB2_LAUNCH_CHECK();
     return AB2_OK;

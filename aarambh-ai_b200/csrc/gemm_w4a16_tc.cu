@@ -115,6 +115,8 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    pdl_wait();  // the setup above overlaps the end of the preceding kernel
+    pdl_launch_dependents();
     const uint32_t tmem = sh->tmem_base, tmem_a = tmem + (uint32_t)(ACCS * NTOK);
 
     if (warp == 0) {
@@ -281,6 +283,8 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
 
 // y[i] = bf16(sum over splits of part[s][i]): eight elements per thread
 __global__ void splitk_reduce_kernel(const float *__restrict__ part, __nv_bfloat16 *__restrict__ y, size_t n8, size_t stride, int ksplit) {
+    pdl_wait();
+    pdl_launch_dependents();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n8) return;
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -327,7 +331,9 @@ int launch_tc(const ab2_qweight *w, const void *x, int M, void *y, int ksplit, c
     }
     const int items = tiles * ksplit;
     const int grid = std::min(items, device_sm_count());
-    gemm_w4a16_tc_kernel<NTOK><<<grid, TC_THREADS, smem, s>>>((const uint32_t *)w->codes, map, (__nv_bfloat16 *)y, w->N, w->K, M, status, ksplit, part);
+    cudaError_t e = launch_kernel(gemm_w4a16_tc_kernel<NTOK>, dim3(grid), dim3(TC_THREADS), smem, s, (const uint32_t *)w->codes, map, (__nv_bfloat16 *)y, w->N, w->K, M,
+                                  status, ksplit, part);
+    if (e != cudaSuccess) return fail(AB2_ERR_CUDA, "W4A16 GEMM launch failed: %s", cudaGetErrorString(e));
     if (ksplit > 1) launch_splitk_reduce(part, (__nv_bfloat16 *)y, M, w->N, ksplit, s);
     AB2_LAUNCH_CHECK();
     return AB2_OK;
@@ -338,7 +344,7 @@ int launch_tc(const ab2_qweight *w, const void *x, int M, void *y, int ksplit, c
 // y[M][N] = bf16(sum of the splits' part[ksplit][M][N]); N is a multiple of 8
 void launch_splitk_reduce(const float *part, __nv_bfloat16 *y, int M, int N, int ksplit, cudaStream_t s) {
     const size_t n8 = (size_t)M * N / 8;
-    splitk_reduce_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, s>>>(part, y, n8, (size_t)M * N, ksplit);
+    launch_kernel(splitk_reduce_kernel, dim3((unsigned)((n8 + 255) / 256)), dim3(256), 0, s, part, y, n8, (size_t)M * N, ksplit);  // checked by the caller
 }
 
 // Y[M][N] = X[M][K] . W^T on the tcgen05 path (W4A16, group 128, bf16).

@@ -164,6 +164,10 @@ static int norm_linear(ab2_model *m, const ab2_qweight *w, const void *x, const 
 static int forward_launches(ab2_model *m, ab2_kv *kv, const uint32_t *ids, int S, int row0, int nrows,
                             const int *rope_base, int logits_mode, void *logits, uint32_t *argmax_out,
                             int len_hint, cudaStream_t s) {
+    // A prompt's launches are chained too: what a kernel sets up (barriers, tensor memory) and the launch itself overlap the
+    // end of the one before.  Ahead of its wait a kernel reads constant weights only.  4 layers of 2048, 300 tokens: 667 -> 526 us;
+    // 8 layers of 4096, 512 tokens: 2.30 -> 2.18 ms.  (Tensor parallel: the collectives are not ours.)
+    const ChainedLaunches chained(S > 1 && !(m->tp && m->tp->world > 1));
     if (m->stack) return stack_forward(m->stack, kv, ids, S, row0, nrows, logits_mode, (float *)logits, argmax_out, len_hint, s);
     const ab2_model_config &c = m->cfg;
     const int all = nrows * S, d = c.d_model, hd = c.head_dim;
