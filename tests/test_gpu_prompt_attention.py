@@ -1,0 +1,33 @@
+"""Prompt attention over bf16 and INT8 caches (the tcgen05 kernel from 16 queries on): edges of its tiles of 128 queries and
+128 keys, a cached prefix, head sizes that fill one and two boxes of 64, heads per KV head; against 64 bits over exactly what
+the cache holds.  The weights enter as two bf16 parts (2^-16), the output is rounded once (2^-9 of each value): the norm of the
+error is below 2^-8 of the result's."""
+import math
+
+import pytest
+import torch
+
+from helpers import pkg
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kv", ["bf16", "int8"])
+@pytest.mark.parametrize("h,kvh,hd", [(8, 2, 128), (6, 3, 64), (4, 4, 96)])
+@pytest.mark.parametrize("lens,S", [([16], 16), ([17, 144], 17), ([127], 127), ([256, 129], 128), ([129], 129), ([385], 257), ([700], 16)])
+def test_prompt_attention(kv, h, kvh, hd, lens, S):
+    g = torch.Generator(device="cuda").manual_seed(S + hd)
+    p = pkg()
+    cache = p.KVCache(max(lens), kvh, hd, h, batch=len(lens), dtype=kv)
+    for row, n in enumerate(lens):
+        k, v = (torch.randn((1, n, kvh, hd), generator=g, device="cuda") for _ in range(2))
+        cache.update(k, v, row0=row)
+    q = torch.randn((len(lens), S, h, hd), generator=g, device="cuda").to(torch.bfloat16)
+    got = p.dispatch.attention_cached(cache, q, hd ** -0.5).double()
+    assert p.device_status() == 0
+    for row, n in enumerate(lens):
+        k, v = (t.cuda().double().repeat_interleave(h // kvh, 1) for t in cache.read(row))  # [n, h, hd]
+        s = torch.einsum("thd,khd->htk", q[row].double(), k) / math.sqrt(hd)
+        hidden = torch.arange(n, device="cuda")[None] > torch.arange(n - S, n, device="cuda")[:, None]
+        want = torch.einsum("htk,khd->thd", torch.softmax(s.masked_fill(hidden, -math.inf), -1), v)
+        assert float((got[row] - want).norm()) <= 2.0 ** -8 * float(want.norm()), row
