@@ -198,7 +198,7 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const float *__restr
     } else if (warp < TC_THREADS / 32 - 1) {
         // ---------------------------------------------------------- epilogue
         const int quad = warp & 3;
-        const bool aligned = (N & 7) == 0 && ((uintptr_t)y & 15) == 0;
+        const bool aligned = rows_in_16_bytes(y, N);
         uint32_t tuse = 0;
         for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x, ++tuse) {
             const int nt = it / m_tiles, mt = it % m_tiles;

@@ -242,7 +242,7 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
     } else {
         // ---------------------------------------------------------- epilogue
         constexpr int COLS = NTOK / 2;  // tokens of a thread
-        const bool aligned = (a.N & 7) == 0 && ((uintptr_t)a.y & 15) == 0;  // rows go out in 16-byte pieces
+        const bool aligned = rows_in_16_bytes(a.y, a.N);
         const int quad = warp & 3, half = (warp - 2 - QB_UNPACK_WARPS) >> 2;
         uint32_t buse = 0;
         bool ok = true;
@@ -334,9 +334,9 @@ int launch_qb(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t 
         AB2_CUDA(cudaFuncSetAttribute(gemm_q4km_tc_kernel<NTOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         configured[dev] = true;
     }
-    // as many shares of K as make one wave of items, at least two blocks each
+    // as many shares of K as make one wave of items, at least two blocks each; the reduce pass stores rows in 16-byte pieces
     const int tiles = ((N + 127) / 128) * (Mp / NTOK), sms = device_sm_count();
-    const int ksplit = N % 8 == 0 ? std::max(1, std::min(std::min(8, KB / 2), sms / tiles)) : 1;
+    const int ksplit = rows_in_16_bytes(y, N) ? std::max(1, std::min(std::min(8, KB / 2), sms / tiles)) : 1;
     const size_t xp_bytes = ((size_t)M * K * 2 + 255) & ~(size_t)255, xs_bytes = ((size_t)KB * Mp * 4 + 255) & ~(size_t)255;
     const size_t part_bytes = ksplit > 1 ? (size_t)ksplit * M * N * 4 : 0;
     ScratchLease ws(s);

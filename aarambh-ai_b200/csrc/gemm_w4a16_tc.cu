@@ -226,7 +226,7 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
     } else if (warp < TC_THREADS / 32 - 1) {
         // ---------------------------------------------------------- epilogue
         const int quad = warp & 3;
-        const bool aligned = (N & 7) == 0 && ((uintptr_t)y & 15) == 0;
+        const bool aligned = rows_in_16_bytes(y, N);
         uint32_t tuse = 0;
         for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x, ++tuse) {
             TC_ITEM(it)
@@ -240,7 +240,7 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
                 const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(ab * NTOK + c * 32);
                 __syncwarp();  // the tensor-memory load is a whole-warp operation
                 tmem_ld32(v, taddr);
-                if (ksplit > 1) {  // a split is chosen for whole vectors of N only
+                if (ksplit > 1) {  // a split is chosen for rows_in_16_bytes only
                     float *out = reinterpret_cast<float *>(stage + quad * 1024);
                     const int tok = mt * NTOK + c * 32, n0 = nt * 128 + quad * 32;
 #pragma unroll
@@ -341,7 +341,7 @@ int launch_tc(const ab2_qweight *w, const void *x, int M, void *y, int ksplit, c
 
 }  // namespace
 
-// y[M][N] = bf16(sum of the splits' part[ksplit][M][N]); N is a multiple of 8
+// y[M][N] = bf16(sum of the splits' part[ksplit][M][N]); rows_in_16_bytes(y, N)
 void launch_splitk_reduce(const float *part, __nv_bfloat16 *y, int M, int N, int ksplit, cudaStream_t s) {
     const size_t n8 = (size_t)M * N / 8;
     launch_kernel(splitk_reduce_kernel, dim3((unsigned)((n8 + 255) / 256)), dim3(256), 0, s, part, y, n8, (size_t)M * N, ksplit);  // checked by the caller
@@ -352,12 +352,13 @@ int qlinear_w4a16_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaSt
     AB2_REQUIRE(((uintptr_t)x & 15) == 0 && (w->K * 2) % 16 == 0, AB2_ERR_BAD_ALIGN, "activations must be 16-byte aligned");
     // Measured: rounds of 19.7 / 22.3 / 27.1 us of tiles of 128 / 192 / 256 tokens over K = 4096 (28672 channels, 2048 tokens),
     // 68 / 73 / 85 over K = 14336; a tile of 32 takes what one of 128 does but for its stores.  Splitting K (few tiles:
-    // 512 tokens on the 4096 x 14336 weight are 64 of 256) needs N in whole vectors and a workspace that a recorded launch has not.
+    // 512 tokens on the 4096 x 14336 weight are 64 of 256) needs rows that the reduce pass can store in 16-byte
+    // pieces and a workspace that a recorded launch has not.
     static const GemmTileCost costs[] = {{32, 0.5, 0.58}, {128, 1.0, 0.605}, {192, 2.2, 0.63}, {256, 4.0, 0.72}};
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     const bool recorded = cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
     static const bool no_split = getenv("AB2_GEMM_NO_SPLITK") != nullptr;
-    const bool split = !recorded && !no_split && w->N % 8 == 0 && (size_t)4 * M * w->N * sizeof(float) <= TC_SPLIT_MAX_BYTES;
+    const bool split = !recorded && !no_split && rows_in_16_bytes(y, w->N) && (size_t)4 * M * w->N * sizeof(float) <= TC_SPLIT_MAX_BYTES;
     const GemmTileChoice c = choose_gemm_tile(costs, M, w->N, w->K / 128, device_sm_count(), split ? 4 : 1);
     switch (c.ntok) {
     case 32: return launch_tc<32>(w, x, M, y, c.ksplit, s);

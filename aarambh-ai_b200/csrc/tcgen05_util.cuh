@@ -171,6 +171,9 @@ __device__ __forceinline__ uint32_t bf16x2_mul_(uint32_t a, uint32_t b) {
 }
 
 
+// Whether rows of N bf16 at y can be stored in pieces of 16 bytes.  A caller's y need only lie on an element.
+__host__ __device__ __forceinline__ bool rows_in_16_bytes(const void *y, int N) { return (N & 7) == 0 && ((uintptr_t)y & 15) == 0; }
+
 // T tokens x the warp's 32 channels, rounded to bf16, wait in `stage` ([T][32], the warp's own) and go out to rows of
 // `ld` elements: `rows` and `cols` of them exist.  Stored straight from the lanes, 32 instructions of 64 bytes for 32
 // tokens, they took 50 to 60 ns a token, and those of the last round of tiles are not hidden behind MMAs.

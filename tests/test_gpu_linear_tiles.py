@@ -10,9 +10,9 @@ from helpers import pkg
 pytestmark = pytest.mark.gpu
 
 
-def check(lin, x, terms):
+def check(lin, x, terms, weight=None):
     y = lin(x).double()
-    w = lin.dequantise().double()
+    w = (weight or lin).dequantise().double()
     ref, size = x.double() @ w.T, x.double().abs() @ w.abs().T
     rounding = {torch.float32: 0.0, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[x.dtype]
     assert torch.isfinite(y).all()
@@ -90,3 +90,21 @@ def test_generic_tiles_short_rows(method):
     g = torch.Generator(device="cuda").manual_seed(1)
     lin = pkg().QuantLinear.quantise(torch.randn((50, 72), generator=g, device="cuda"), method, 16)
     check(lin, torch.randn((35, 72), generator=g, device="cuda"), 64)
+
+
+# y need only lie on an element: few tiles, for which a y on 16 bytes would have its K split and reduced in 16-byte pieces, and many
+@pytest.mark.parametrize("M", [9, 40, 65, 130, 300])
+@pytest.mark.parametrize("method,N,K", [("q4_k_m", 128, 2048), ("q4_k_m", 4096, 512), ("w4a16", 256, 4096), ("w4a16", 4096, 512),
+                                        ("int8_channel", 256, 512)])
+def test_output_off_a_16_byte_boundary(method, N, K, M):
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    p = pkg()
+    lin = p.QuantLinear.quantise(torch.randn((N, K), generator=g, device="cuda"), method, 128)
+    x = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
+    for off in (1, 4):
+        buf = torch.full((M * N + 16,), 7.0, dtype=torch.bfloat16, device="cuda")
+        assert buf.data_ptr() % 16 == 0
+        y = buf[off:off + M * N].view(M, N)
+        p._lib.check(p._lib.lib.ab2_qlinear_forward(lin._h, x.data_ptr(), M, p.qlinear.dtype_code(x.dtype), y.data_ptr(), p.qlinear.stream_ptr()))
+        assert bool((buf[:off] == 7).all()) and bool((buf[off + M * N:] == 7).all())
+        check(lambda _: y, x, 16 * (512 + K // 256) if method == "q4_k_m" else 2 * K + (2 ** 15 if method == "w4a16" else 0), lin)
