@@ -291,7 +291,7 @@ prompt_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
         asm volatile("barrier.cta.sync 1, 256;\n" ::: "memory");
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        if (!*failed) {
+        if (!__any_sync(0xffffffffu, *failed)) {
             // both halves of the warps store: value boxes of 64 dimensions in turn
             const float t0 = sh->top[0][r], t1 = sh->top[1][r], t = fmaxf(t0, t1);
             float f0 = ex2(t0 - t), f1 = tiles > 1 ? ex2(t1 - t) : 0.f;

@@ -154,14 +154,16 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
     } else if (warp == 1) {
         // ---------------------------------------------------------- MMA issue
         uint32_t use = 0, tuse = 0;
-        for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x, ++tuse) {
+        bool ok = true;
+        for (int it = blockIdx.x; it < items && ok; it += gridDim.x, ++tuse) {
             const int ab = tuse & 1;
-            if (!bar_wait(&sh->accempty[ab], ((tuse >> 1) & 1) ^ 1, failed)) break;
+            ok = warp_wait(&sh->accempty[ab], ((tuse >> 1) & 1) ^ 1, failed);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const uint32_t tacc = tmem + (uint32_t)(ab * ACC_COLS);
-            for (int ks = 0; ks < KS; ++ks, ++use) {
+            for (int ks = 0; ks < KS && ok; ++ks, ++use) {
                 const int s = use % STAGES;
-                if (!warp_wait(&sh->full[s], (use / STAGES) & 1, failed)) break;  // no tensor memory in a stage: no tcgen05 fence
+                ok = warp_wait(&sh->full[s], (use / STAGES) & 1, failed);
+                if (!ok) break;  // no tensor memory in a stage: no tcgen05 fence
                 if (elect_one()) {
                     const uint32_t a0 = sptr(ring + s * STAGE_BYTES);
                     const uint64_t xd = umma_desc(a0 + (DUAL ? 2 : 1) * GB_A_BYTES);
@@ -171,6 +173,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                 }
                 __syncwarp();
             }
+            if (!ok) break;
             if (elect_one()) umma_commit(&sh->accfull[ab]);
             __syncwarp();
         }
@@ -178,14 +181,16 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         // ---------------------------------------------------------- epilogue
         const int quad = warp & 3, first_block = (warp - 2) >> 2;
         uint32_t tuse = 0;
-        for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x, ++tuse) {
+        bool ok = true;
+        for (int it = blockIdx.x; it < items && ok; it += gridDim.x, ++tuse) {
             int nt, mt;
             cur.find(sh, it, n_tiles, nt, mt);
             const int ab = tuse & 1;
             const int r0 = GROUPED ? a.r.offset[cur.e] : 0;
             const int cnt = (GROUPED ? a.r.offset[cur.e + 1] - r0 : a.M) - mt * NTOK;  // rows of this tile that exist
             const int row0 = r0 + mt * NTOK;
-            if (!bar_wait(&sh->accfull[ab], (tuse >> 1) & 1, failed)) break;
+            ok = warp_wait(&sh->accfull[ab], (tuse >> 1) & 1, failed);
+            if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const int n = nt * 128 + quad * 32 + lane;
             constexpr int CW = DUAL ? 16 : 32;  // tokens per register block

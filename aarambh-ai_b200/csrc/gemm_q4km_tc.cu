@@ -199,11 +199,12 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         uint32_t wuse = 0;
         uint32_t k_mask = 0x000F000Fu, k_magic = 0x43004300u, k_off = 0xC300C300u;  // -128
         asm volatile("" : "+r"(k_mask), "+r"(k_magic), "+r"(k_off));
-        for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x) {
+        bool ok = true;
+        for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
             item(it, nt, mt, sp, b0, b1);
-            for (int b = b0; b < b1 && !*failed; ++b, ++wuse) {
+            for (int b = b0; b < b1 && ok; ++b, ++wuse) {
                 const int ws = wuse % WSLOTS;
-                if (!bar_wait(&sh->wfull[ws], (wuse / WSLOTS) & 1, failed)) break;
+                const bool here = bar_wait(&sh->wfull[ws], (wuse / WSLOTS) & 1, failed);
                 // row t of the slot: 256 codes in eight 16-byte chunks, chunk c stored at c ^ (t & 7); the set takes quarters
                 // set and set + 2 of the block
                 const uint8_t *wrow = w_ring + ws * QB_WSLOT_BYTES + t * 128;
@@ -216,7 +217,8 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                 for (int h = 0; h < 2; ++h) {
                     const uint32_t suse = 4 * wuse + set + 2 * h;
                     const int st = suse % STAGES;
-                    if (!warp_wait(&sh->empty[st], ((suse / STAGES) & 1) ^ 1, failed)) break;
+                    ok = warp_wait(&sh->empty[st], ((suse / STAGES) & 1) ^ 1, failed, here);
+                    if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                     uint32_t o[32];  // two bf16 each
 #pragma unroll

@@ -124,12 +124,12 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
         // One slot per quantisation group; lane b issues the bulk copy of block b, so the eight
         // copies of a group leave in parallel instead of one after the other from a single thread.
         uint32_t wuse = 0;
-        for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x) {
+        int ok = 1;
+        for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
             TC_ITEM(it)
             const int nblk = min(8, tiles16 - nt * 8);
-            for (int g = g0; g < g1 && !*failed; ++g, ++wuse) {
+            for (int g = g0; g < g1; ++g, ++wuse) {
                 const int ws = wuse % TC_WSLOTS;
-                int ok = 1;
                 if (lane == 0) {
                     ok = bar_wait(&sh->wempty[ws], ((wuse / TC_WSLOTS) & 1) ^ 1, failed) ? 1 : 0;
                     if (ok) bar_expect_tx(&sh->wfull[ws], (uint32_t)nblk * TC_BLOCK_WORDS * 4);
@@ -158,15 +158,17 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
     } else if (warp == 1) {
         // ---------------------------------------------------------- MMA issue
         uint32_t suse = 0, tuse = 0;
-        for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x, ++tuse) {
+        bool ok = true;
+        for (int it = blockIdx.x; it < items && ok; it += gridDim.x, ++tuse) {
             const int ab = tuse % ACCS;
-            if (!bar_wait(&sh->accempty[ab], ((tuse / ACCS) & 1) ^ 1, failed)) break;
+            ok = warp_wait(&sh->accempty[ab], ((tuse / ACCS) & 1) ^ 1, failed);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const uint32_t tacc = tmem + (uint32_t)(ab * NTOK);
             TC_ITEM(it)
-            for (int ks = 2 * g0; ks < 2 * g1; ++ks, ++suse) {
+            for (int ks = 2 * g0; ks < 2 * g1 && ok; ++ks, ++suse) {
                 const int st = suse % TC_STAGES;
-                if (!warp_wait(&sh->full[st], (suse / TC_STAGES) & 1, failed)) break;
+                ok = warp_wait(&sh->full[st], (suse / TC_STAGES) & 1, failed);
+                if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 if (elect_one()) {
                     umma_stage_ts(tacc, tmem_a + (uint32_t)(st * TC_A_COLS), umma_desc(sptr(b_st + st * B_BYTES)), IDESC, ks == 2 * g0);
@@ -174,6 +176,7 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
                 }
                 __syncwarp();
             }
+            if (!ok) break;
             if (elect_one()) umma_commit(&sh->accfull[ab]);
             __syncwarp();
         }
@@ -184,12 +187,13 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
         uint32_t gbase = 0;  // groups before this tile
         uint32_t k_mask = 0x000F000Fu, k_magic = 0x43004300u;
         asm volatile("" : "+r"(k_mask), "+r"(k_magic));
-        for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x) {
+        bool ok = true;
+        for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
             TC_ITEM(it)
             // the set's groups: every (TC_SETS / 2)-th of the CTA's sequence of groups
-            for (uint32_t wuse = gbase + ((set >> 1) + TC_SETS - gbase % (TC_SETS / 2)) % (TC_SETS / 2); wuse < gbase + (uint32_t)(g1 - g0) && !*failed; wuse += TC_SETS / 2) {
+            for (uint32_t wuse = gbase + ((set >> 1) + TC_SETS - gbase % (TC_SETS / 2)) % (TC_SETS / 2); wuse < gbase + (uint32_t)(g1 - g0); wuse += TC_SETS / 2) {
                 const int ws = wuse % TC_WSLOTS;
-                if (!bar_wait(&sh->wfull[ws], (wuse / TC_WSLOTS) & 1, failed)) break;
+                const bool here = bar_wait(&sh->wfull[ws], (wuse / TC_WSLOTS) & 1, failed);
                 const uint32_t *bw = (const uint32_t *)(w_ring + ws * TC_WSLOT_BYTES) + blk * TC_BLOCK_WORDS;
                 const uint4 pw[2] = {*reinterpret_cast<const uint4 *>(bw + r * 16 + half * 8), *reinterpret_cast<const uint4 *>(bw + r * 16 + half * 8 + 4)};
                 const uint32_t pr = bw[256 + r];
@@ -200,7 +204,8 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
                 const uint32_t nz2 = __byte_perm(pr, pr, 0x3232);  // bf16x2 -(128 + z)
                 const uint32_t suse = 2 * wuse + half;
                 const int s = suse % TC_STAGES;
-                if (!warp_wait(&sh->empty[s], ((suse / TC_STAGES) & 1) ^ 1, failed)) break;
+                ok = warp_wait(&sh->empty[s], ((suse / TC_STAGES) & 1) ^ 1, failed, here);
+                if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 uint32_t o[32];  // two bf16 each
 #pragma unroll
@@ -228,10 +233,12 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
         const int quad = warp & 3;
         const bool aligned = rows_in_16_bytes(y, N);
         uint32_t tuse = 0;
-        for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x, ++tuse) {
+        bool ok = true;
+        for (int it = blockIdx.x; it < items && ok; it += gridDim.x, ++tuse) {
             TC_ITEM(it)
             const int ab = tuse % ACCS;
-            if (!bar_wait(&sh->accfull[ab], (tuse / ACCS) & 1, failed)) break;
+            ok = warp_wait(&sh->accfull[ab], (tuse / ACCS) & 1, failed);
+            if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const int n = nt * 128 + quad * 32 + lane;
 #pragma unroll 1

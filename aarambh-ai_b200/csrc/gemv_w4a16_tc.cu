@@ -167,7 +167,7 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
         // Lane b fetches block b of a unit (blocks 2q and 2q + 1 go to ring q); issuing a copy occupies a
         // warp for a few hundred cycles, which the unpack warps used to pay once per unit each.
         const int n_units = rg.u1 - rg.u0;
-        for (int use = 0; use < n_units && !*failed; ++use) {
+        for (int use = 0; use < n_units; ++use) {
             const int u = rg.u0 + use, nt = u / G, g = u - nt * G, ws = use % DG_WSLOTS;
             int ok = 1;
             if (use >= DG_WSLOTS && lane < 4) ok = bar_wait(&sh->wempty[lane][ws], ((use / DG_WSLOTS) & 1) ^ 1, failed) ? 1 : 0;
@@ -189,16 +189,18 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
         // ---------------------------------------------------------- MMA issue (alternate units per warp)
         const uint32_t my_id = warp == 1 ? 0u : (uint32_t)(warp - 13);
         uint32_t use = 0;
-        for (int u = rg.u0; u < rg.u1 && !*failed; ++u, ++use) {
+        bool ok = true;
+        for (int u = rg.u0; u < rg.u1 && ok; ++u, ++use) {
             if (use % DG_MMA_WARPS != my_id) continue;
             const int ab = use % DG_ACC;
-            if (!bar_wait(&sh->accempty[ab], ((use / DG_ACC) & 1) ^ 1, failed)) break;
+            ok = warp_wait(&sh->accempty[ab], ((use / DG_ACC) & 1) ^ 1, failed);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const uint32_t td = tmem + (uint32_t)(ab * NTOK);
-            for (int half = 0; half < 2 && !*failed; ++half) {
+            for (int half = 0; half < 2 && ok; ++half) {
                 const uint32_t suse = 2 * use + half;
                 const int s = suse % DG_STAGES, xs = suse % DG_XSTAGES;
-                if (!warp_wait(&sh->xfull[xs], (suse / DG_XSTAGES) & 1, failed) || !warp_wait(&sh->afull[s], (suse / DG_STAGES) & 1, failed)) break;
+                ok = warp_wait(&sh->xfull[xs], (suse / DG_XSTAGES) & 1, failed) && warp_wait(&sh->afull[s], (suse / DG_STAGES) & 1, failed);
+                if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 if (elect_one()) {
                     umma_stage_ts(td, tmem_a + (uint32_t)(s * DG_A_COLS), umma_desc(sptr(b_st + xs * B_BYTES)), IDESC, half == 0);
@@ -207,6 +209,7 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
                 }
                 __syncwarp();
             }
+            if (!ok) break;
             if (elect_one()) umma_commit(&sh->accfull[ab]);
             __syncwarp();
         }
@@ -222,9 +225,9 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
         uint32_t k_mask = 0x000F000Fu, k_magic = 0x43004300u;
         asm volatile("" : "+r"(k_mask), "+r"(k_magic));
         uint32_t use = 0;
-        for (int u = rg.u0; u < rg.u1 && !*failed; ++u, ++use) {
+        for (int u = rg.u0; u < rg.u1; ++u, ++use) {
             const int ws = use % DG_WSLOTS;
-            if (!bar_wait(&sh->wfull[q][ws], (use / DG_WSLOTS) & 1, failed)) break;
+            const bool here = bar_wait(&sh->wfull[q][ws], (use / DG_WSLOTS) & 1, failed);
             const uint32_t *bw = (const uint32_t *)(ring + ws * DG_WSLOT_BYTES) + (blk & 1) * W4_BLOCK_WORDS;
             const uint4 p0 = *reinterpret_cast<const uint4 *>(bw + r * 16 + half * 8);
             const uint4 p1 = *reinterpret_cast<const uint4 *>(bw + r * 16 + half * 8 + 4);
@@ -236,7 +239,7 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
             if (lane == 0) bar_arrive_after(&sh->wempty[q][ws], held, (uint32_t)K & 1u);
             const uint32_t suse = 2 * use + half;
             const int s = suse % DG_STAGES;
-            if (!warp_wait(&sh->sempty[s], ((suse / DG_STAGES) & 1) ^ 1, failed)) break;
+            if (!warp_wait(&sh->sempty[s], ((suse / DG_STAGES) & 1) ^ 1, failed, here)) break;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const uint32_t words[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
             uint32_t o[32];
@@ -259,11 +262,13 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
 #pragma unroll
         for (int j = 0; j < NTOK; ++j) acc[j] = 0.f;
         uint32_t use = 0;
-        for (int u = rg.u0; u < rg.u1 && !*failed; ++u, ++use) {
+        // After a time-out the warps go through their remaining units without waiting: they share barriers, and the
+        // counters of cut tiles have to come back to zero.
+        bool ok = true;
+        for (int u = rg.u0; u < rg.u1; ++u, ++use) {
             const int nt = u / G, g = u - nt * G;
             const int ab = use % DG_ACC;
-            if (!bar_wait(&sh->accfull[ab], (use / DG_ACC) & 1, failed)) break;
-            __syncwarp();  // the tensor-memory load is a whole-warp operation
+            if (ok) ok = warp_wait(&sh->accfull[ab], (use / DG_ACC) & 1, failed);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const float sc = __uint_as_float(sh->params[use % DG_PARAM_BUFS][row] << 16);
             constexpr int COLS = NTOK < 32 ? 16 : 32;  // tokens at a time
