@@ -435,6 +435,7 @@ int prompt_tc_cached(const ab2_kv *kv, int layer, const void *q, void *out, int 
                      ab2_dtype dtype, const AttnStrides &st, cudaStream_t s) {
     const int hd = kv->hd;
     const bool int8 = kv->dtype == AB2_KV_INT8;
+    if (hd != 64 && hd != 128) return AB2_ERR_UNSUPPORTED;  // as for decode and fewer queries over such a cache: refused
     if (S < PT_MIN_QUERIES || dtype != AB2_BF16 || kv->dtype == AB2_KV_F32 || st.q_h != hd || st.o_h != hd || !lengths_known(s)) return AB2_ERR_UNSUPPORTED;
     const KvView v = kv_view(kv, layer);
     for (int i = 0; i < nrows; ++i) {

@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("kv", ["bf16", "int8"])
-@pytest.mark.parametrize("h,kvh,hd", [(8, 2, 128), (6, 3, 64), (4, 4, 96)])
+@pytest.mark.parametrize("h,kvh,hd", [(8, 2, 128), (6, 3, 64)])
 @pytest.mark.parametrize("lens,S", [([16], 16), ([17, 144], 17), ([127], 127), ([256, 129], 128), ([129], 129), ([385], 257), ([700], 16)])
 def test_prompt_attention(kv, h, kvh, hd, lens, S):
     g = torch.Generator(device="cuda").manual_seed(S + hd)
@@ -31,3 +31,17 @@ def test_prompt_attention(kv, h, kvh, hd, lens, S):
         hidden = torch.arange(n, device="cuda")[None] > torch.arange(n - S, n, device="cuda")[:, None]
         want = torch.einsum("htk,khd->thd", torch.softmax(s.masked_fill(hidden, -math.inf), -1), v)
         assert float((got[row] - want).norm()) <= 2.0 ** -8 * float(want.norm()), row
+
+
+@pytest.mark.parametrize("kv", ["bf16", "int8"])
+@pytest.mark.parametrize("hd", [32, 96, 192])
+@pytest.mark.parametrize("S", [1, 15, 16, 40])
+def test_head_sizes_are_refused_alike(kv, hd, S):
+    """A cache whose head size the attention over caches does not serve is refused for any number of queries."""
+    p = pkg()
+    cache = p.KVCache(S, 2, hd, 4, dtype=kv)
+    k, v = (torch.randn((1, S, 2, hd), device="cuda") for _ in range(2))
+    cache.append(0, k, v)
+    cache.commit(S)
+    with pytest.raises(p.Ab2Error, match="head_dim 64 and 128"):
+        p.dispatch.attention_cached(cache, torch.randn((1, S, 4, hd), device="cuda").to(torch.bfloat16), hd ** -0.5)
