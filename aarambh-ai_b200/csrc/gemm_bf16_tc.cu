@@ -200,27 +200,8 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                 if (c * CW >= cnt) break;
                 const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(ab * ACC_COLS + c * CW);
                 uint32_t v[32];
-                if (DUAL) {
-#pragma unroll
-                    for (int h = 0; h < 2; ++h)
-                        asm volatile(
-                            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-                            : "=r"(v[16 * h]), "=r"(v[16 * h + 1]), "=r"(v[16 * h + 2]), "=r"(v[16 * h + 3]), "=r"(v[16 * h + 4]),
-                              "=r"(v[16 * h + 5]), "=r"(v[16 * h + 6]), "=r"(v[16 * h + 7]), "=r"(v[16 * h + 8]), "=r"(v[16 * h + 9]),
-                              "=r"(v[16 * h + 10]), "=r"(v[16 * h + 11]), "=r"(v[16 * h + 12]), "=r"(v[16 * h + 13]),
-                              "=r"(v[16 * h + 14]), "=r"(v[16 * h + 15])
-                            : "r"(taddr + (uint32_t)(h * NTOK)));
-                } else {
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
-                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-                          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-                          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                        : "r"(taddr));
-                }
-                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                if (DUAL) tmem_ld16_pair(v, taddr, taddr + (uint32_t)NTOK);
+                else tmem_ld32(v, taddr);
                 if (MODE == LIN_DENSE) {
                     if (n >= a.N) continue;
                     if (a.epi == LIN_F32) {

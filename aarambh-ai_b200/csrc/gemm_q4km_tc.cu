@@ -268,11 +268,7 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
 #pragma unroll
                 for (int c = 0; c < COLS / 8; ++c) {
                     uint32_t v[8];
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-                        : "r"(taddr + 8 * c));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                    tmem_ld8(v, taddr + 8 * c);
 #pragma unroll
                     for (int j = 0; j < 8; j += 4) {
                         const float4 X = *reinterpret_cast<const float4 *>(xs + 8 * c + j);

@@ -79,18 +79,6 @@ struct DgShared {
     int last_flag;
 };
 
-// 16 columns of the warp's lanes; the registers pass through the wait, so that nothing computed from them can move ahead of it.
-__device__ __forceinline__ void tmem_ld16(uint32_t (&v)[16], uint32_t taddr) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;\n"
-                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]),
-                   "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])::"memory");
-}
-
 // units [u0, u1) of this CTA; the first `rem` CTAs take base + 1 units
 struct DgRange { int base, rem, u0, u1; };
 __device__ __forceinline__ DgRange dg_range(int total, int ctas, int cta) {

@@ -134,11 +134,23 @@ __device__ __forceinline__ void umma_stage_ts(uint32_t tmem_d, uint32_t tmem_a, 
 #pragma unroll
     for (int k = 0; k < 4; ++k) umma_bf16_ts(tmem_d, tmem_a + (uint32_t)(8 * k), bdesc + (uint64_t)(2 * k), idesc, !first || k > 0);
 }
+#define AB2_REGS8(c, v) c(v[0]), c(v[1]), c(v[2]), c(v[3]), c(v[4]), c(v[5]), c(v[6]), c(v[7])
+#define AB2_REGS16(c, v) AB2_REGS8(c, v), c(v[8]), c(v[9]), c(v[10]), c(v[11]), c(v[12]), c(v[13]), c(v[14]), c(v[15])
 #define AB2_REGS32(c, v) \
     c(v[0]), c(v[1]), c(v[2]), c(v[3]), c(v[4]), c(v[5]), c(v[6]), c(v[7]), c(v[8]), c(v[9]), c(v[10]), c(v[11]), c(v[12]), c(v[13]), c(v[14]), c(v[15]), \
     c(v[16]), c(v[17]), c(v[18]), c(v[19]), c(v[20]), c(v[21]), c(v[22]), c(v[23]), c(v[24]), c(v[25]), c(v[26]), c(v[27]), c(v[28]), c(v[29]), c(v[30]), c(v[31])
-// 32 columns of the warp's lanes; the registers pass through the wait, so that nothing computed from them can move
-// ahead of it.
+// 8, 16 or 32 columns of the warp's lanes; the registers pass through the wait, so that nothing computed from them can
+// move ahead of it.
+__device__ __forceinline__ void tmem_ld8(uint32_t (&v)[8], uint32_t addr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n" : AB2_REGS8("=r", v) : "r"(addr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" : AB2_REGS8("+r", v)::"memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t (&v)[16], uint32_t addr) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+        : AB2_REGS16("=r", v) : "r"(addr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" : AB2_REGS16("+r", v)::"memory");
+}
 __device__ __forceinline__ void tmem_ld32_start(uint32_t (&v)[32], uint32_t addr) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -148,6 +160,16 @@ __device__ __forceinline__ void tmem_ld32_start(uint32_t (&v)[32], uint32_t addr
 __device__ __forceinline__ void tmem_ld32_wait(uint32_t (&v)[32]) { asm volatile("tcgen05.wait::ld.sync.aligned;\n" : AB2_REGS32("+r", v)::"memory"); }
 __device__ __forceinline__ void tmem_ld32(uint32_t (&v)[32], uint32_t addr) {
     tmem_ld32_start(v, addr);
+    tmem_ld32_wait(v);
+}
+// 16 columns from each of two places
+__device__ __forceinline__ void tmem_ld16_pair(uint32_t (&v)[32], uint32_t addr, uint32_t addr2) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+        : AB2_REGS16("=r", v) : "r"(addr));
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+        : AB2_REGS16("=r", (v + 16)) : "r"(addr2));
     tmem_ld32_wait(v);
 }
 __device__ __forceinline__ void tmem_st32(uint32_t addr, const uint32_t (&v)[32]) {
