@@ -18,8 +18,8 @@
 // same tile list out from them (prefix sums in shared memory).  Rows of a tile past its expert's
 // last pair belong to the next expert; they are multiplied and not stored.  The pair's weight
 // multiplies the f32 sums, which is the sum over the weighted input without rounding it.
-// Every wait on an mbarrier is bounded; on a time-out the CTA records AB2_ERR_TIMEOUT, stops
-// issuing work, frees its tensor memory and returns.
+// Every wait on an mbarrier is bounded; on a time-out the CTA records AB2_ERR_TIMEOUT, walks
+// through the rest of its work, frees its tensor memory and returns.
 #include <cuda.h>
 
 #include <algorithm>
@@ -154,16 +154,14 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
     } else if (warp == 1) {
         // ---------------------------------------------------------- MMA issue
         uint32_t use = 0, tuse = 0;
-        bool ok = true;
-        for (int it = blockIdx.x; it < items && ok; it += gridDim.x, ++tuse) {
+        for (int it = blockIdx.x; it < items; it += gridDim.x, ++tuse) {
             const int ab = tuse & 1;
-            ok = warp_wait(&sh->accempty[ab], ((tuse >> 1) & 1) ^ 1, failed);
+            bar_wait(&sh->accempty[ab], ((tuse >> 1) & 1) ^ 1, failed);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const uint32_t tacc = tmem + (uint32_t)(ab * ACC_COLS);
-            for (int ks = 0; ks < KS && ok; ++ks, ++use) {
+            for (int ks = 0; ks < KS; ++ks, ++use) {
                 const int s = use % STAGES;
-                ok = warp_wait(&sh->full[s], (use / STAGES) & 1, failed);
-                if (!ok) break;  // no tensor memory in a stage: no tcgen05 fence
+                warp_wait(&sh->full[s], (use / STAGES) & 1, failed);  // no tensor memory in a stage: no tcgen05 fence
                 if (elect_one()) {
                     const uint32_t a0 = sptr(ring + s * STAGE_BYTES);
                     const uint64_t xd = umma_desc(a0 + (DUAL ? 2 : 1) * GB_A_BYTES);
@@ -173,7 +171,6 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                 }
                 __syncwarp();
             }
-            if (!ok) break;
             if (elect_one()) umma_commit(&sh->accfull[ab]);
             __syncwarp();
         }
@@ -181,16 +178,14 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         // ---------------------------------------------------------- epilogue
         const int quad = warp & 3, first_block = (warp - 2) >> 2;
         uint32_t tuse = 0;
-        bool ok = true;
-        for (int it = blockIdx.x; it < items && ok; it += gridDim.x, ++tuse) {
+        for (int it = blockIdx.x; it < items; it += gridDim.x, ++tuse) {
             int nt, mt;
             cur.find(sh, it, n_tiles, nt, mt);
             const int ab = tuse & 1;
             const int r0 = GROUPED ? a.r.offset[cur.e] : 0;
             const int cnt = (GROUPED ? a.r.offset[cur.e + 1] - r0 : a.M) - mt * NTOK;  // rows of this tile that exist
             const int row0 = r0 + mt * NTOK;
-            ok = warp_wait(&sh->accfull[ab], (tuse >> 1) & 1, failed);
-            if (!ok) break;
+            bar_wait(&sh->accfull[ab], (tuse >> 1) & 1, failed);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const int n = nt * 128 + quad * 32 + lane;
             constexpr int CW = DUAL ? 16 : 32;  // tokens per register block

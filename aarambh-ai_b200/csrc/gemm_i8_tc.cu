@@ -18,8 +18,8 @@
 //   warps 18-21 the epilogue multiplies the f32 accumulator by the channel's f32 scale - the
 //               product is rounded once, where the reference rounds q * scale to the model
 //               dtype before its matmul.
-// Every wait on an mbarrier is bounded; on a time-out the CTA records AB2_ERR_TIMEOUT, stops
-// issuing work, still frees its tensor memory and returns.
+// Every wait on an mbarrier is bounded; on a time-out the CTA records AB2_ERR_TIMEOUT, walks
+// through the rest of its work, frees its tensor memory and returns.
 #include <cuda.h>
 
 #include <algorithm>
@@ -136,16 +136,14 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const float *__restr
     } else if (warp == 1) {
         // ---------------------------------------------------------- MMA issue
         uint32_t suse = 0, tuse = 0;
-        bool ok = true;
-        for (int it = blockIdx.x; it < items && ok; it += gridDim.x, ++tuse) {
+        for (int it = blockIdx.x; it < items; it += gridDim.x, ++tuse) {
             const int ab = tuse % ACCS;
-            ok = warp_wait(&sh->accempty[ab], ((tuse / ACCS) & 1) ^ 1, failed);
+            bar_wait(&sh->accempty[ab], ((tuse / ACCS) & 1) ^ 1, failed);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const uint32_t tacc = tmem + (uint32_t)(ab * NTOK);
-            for (int ks = 0; ks < 2 * G && ok; ++ks, ++suse) {
+            for (int ks = 0; ks < 2 * G; ++ks, ++suse) {
                 const int st = suse % TC_STAGES;
-                ok = warp_wait(&sh->full[st], (suse / TC_STAGES) & 1, failed);
-                if (!ok) break;
+                warp_wait(&sh->full[st], (suse / TC_STAGES) & 1, failed);
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 if (elect_one()) {
                     umma_stage_ts(tacc, tmem_a + (uint32_t)(st * TC_A_COLS), umma_desc(sptr(b_st + st * B_BYTES)), IDESC, ks == 0);
@@ -153,7 +151,6 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const float *__restr
                 }
                 __syncwarp();
             }
-            if (!ok) break;
             if (elect_one()) umma_commit(&sh->accfull[ab]);
             __syncwarp();
         }
@@ -162,11 +159,10 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const float *__restr
         // a set of four warps takes the same half (64 K-elements, one stage) of every second group
         const int t = (warp & 3) * 32 + lane, set = (warp - 2) >> 2, half = set & 1;  // channel: the warp's lanes of tensor memory
         uint32_t gbase = 0;  // groups before this tile
-        bool ok = true;
-        for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+        for (int it = blockIdx.x; it < items; it += gridDim.x) {
             for (uint32_t wuse = gbase + ((set >> 1) + TC_SETS - gbase % (TC_SETS / 2)) % (TC_SETS / 2); wuse < gbase + (uint32_t)G; wuse += TC_SETS / 2) {
                 const int ws = wuse % TC_WSLOTS;
-                const bool here = bar_wait(&sh->wfull[ws], (wuse / TC_WSLOTS) & 1, failed);
+                bar_wait(&sh->wfull[ws], (wuse / TC_WSLOTS) & 1, failed);
                 // row t of the slot: 128 codes in eight 16-byte chunks, chunk c stored at c ^ (t & 7)
                 const uint8_t *wrow = w_ring + ws * TC_WSLOT_BYTES + t * 128;
                 uint4 raw[4];
@@ -177,8 +173,7 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const float *__restr
                 if (lane == 0) bar_arrive_after(&sh->wempty[ws], held, (uint32_t)K & 1u);
                 const uint32_t suse = 2 * wuse + half;
                 const int s = suse % TC_STAGES;
-                ok = warp_wait(&sh->empty[s], ((suse / TC_STAGES) & 1) ^ 1, failed, here);
-                if (!ok) break;
+                const bool free = warp_wait(&sh->empty[s], ((suse / TC_STAGES) & 1) ^ 1, failed);
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 uint32_t o[32];  // two bf16 each
 #pragma unroll
@@ -196,7 +191,7 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const float *__restr
                 asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
                 __syncwarp();
-                if (lane == 0) bar_arrive(&sh->full[s]);
+                if (lane == 0 && free) bar_arrive(&sh->full[s]);
             }
             gbase += (uint32_t)G;
         }
@@ -205,12 +200,10 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const float *__restr
         const int quad = warp & 3;
         const bool aligned = rows_in_16_bytes(y, N);
         uint32_t tuse = 0;
-        bool ok = true;
-        for (int it = blockIdx.x; it < items && ok; it += gridDim.x, ++tuse) {
+        for (int it = blockIdx.x; it < items; it += gridDim.x, ++tuse) {
             const int nt = it / m_tiles, mt = it % m_tiles;
             const int ab = tuse % ACCS;
-            ok = warp_wait(&sh->accfull[ab], (tuse / ACCS) & 1, failed);
-            if (!ok) break;
+            bar_wait(&sh->accfull[ab], (tuse / ACCS) & 1, failed);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const int n = nt * 128 + quad * 32 + lane;
             const float sc = n < N ? __ldg(scales + n) : 0.f;

@@ -21,8 +21,8 @@
 // What bounds it is the unpack and the per-block epilogue (about 450 cycles a stage against the MMA's 257 at 128
 // tokens).  14336 x 4096 at 300 tokens: 3329 us on CUDA cores,
 // 76 us here (464 TFLOP/s); 3072 x 2048: 421 -> 20 us, at 9 tokens 17 -> 11.
-// Every wait on an mbarrier is bounded; on a time-out the CTA records AB2_ERR_TIMEOUT, stops issuing work, frees its
-// tensor memory and returns.
+// Every wait on an mbarrier is bounded; on a time-out the CTA records AB2_ERR_TIMEOUT, walks through the rest
+// of its work, frees its tensor memory and returns.
 #include <cuda.h>
 
 #include <algorithm>
@@ -172,17 +172,15 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
     } else if (warp == 1) {
         // ---------------------------------------------------------- MMA issue
         uint32_t suse = 0, buse = 0;
-        bool ok = true;
-        for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+        for (int it = blockIdx.x; it < items; it += gridDim.x) {
             item(it, nt, mt, sp, b0, b1);
-            for (int b = b0; b < b1 && ok; ++b, ++buse) {
+            for (int b = b0; b < b1; ++b, ++buse) {
                 const int ab = buse & 1;
-                ok = warp_wait(&sh->accempty[ab], ((buse >> 1) & 1) ^ 1, failed);
+                bar_wait(&sh->accempty[ab], ((buse >> 1) & 1) ^ 1, failed);
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                for (int q = 0; q < 4 && ok; ++q, ++suse) {
+                for (int q = 0; q < 4; ++q, ++suse) {
                     const int st = suse % STAGES;
-                    ok = warp_wait(&sh->full[st], (suse / STAGES) & 1, failed);
-                    if (!ok) break;
+                    warp_wait(&sh->full[st], (suse / STAGES) & 1, failed);
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                     if (elect_one()) {
                         umma_stage_ts(tmem + (uint32_t)(ab * NTOK), tmem_a + (uint32_t)(st * QB_A_COLS), umma_desc(sptr(b_st + st * B_BYTES)), IDESC, q == 0);
@@ -199,12 +197,11 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         uint32_t wuse = 0;
         uint32_t k_mask = 0x000F000Fu, k_magic = 0x43004300u, k_off = 0xC300C300u;  // -128
         asm volatile("" : "+r"(k_mask), "+r"(k_magic), "+r"(k_off));
-        bool ok = true;
-        for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+        for (int it = blockIdx.x; it < items; it += gridDim.x) {
             item(it, nt, mt, sp, b0, b1);
-            for (int b = b0; b < b1 && ok; ++b, ++wuse) {
+            for (int b = b0; b < b1; ++b, ++wuse) {
                 const int ws = wuse % WSLOTS;
-                const bool here = bar_wait(&sh->wfull[ws], (wuse / WSLOTS) & 1, failed);
+                bar_wait(&sh->wfull[ws], (wuse / WSLOTS) & 1, failed);
                 // row t of the slot: 256 codes in eight 16-byte chunks, chunk c stored at c ^ (t & 7); the set takes quarters
                 // set and set + 2 of the block
                 const uint8_t *wrow = w_ring + ws * QB_WSLOT_BYTES + t * 128;
@@ -217,8 +214,7 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                 for (int h = 0; h < 2; ++h) {
                     const uint32_t suse = 4 * wuse + set + 2 * h;
                     const int st = suse % STAGES;
-                    ok = warp_wait(&sh->empty[st], ((suse / STAGES) & 1) ^ 1, failed, here);
-                    if (!ok) break;
+                    const bool free = warp_wait(&sh->empty[st], ((suse / STAGES) & 1) ^ 1, failed);
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                     uint32_t o[32];  // two bf16 each
 #pragma unroll
@@ -237,7 +233,7 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                     asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
                     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
                     __syncwarp();
-                    if (lane == 0) bar_arrive(&sh->full[st]);
+                    if (lane == 0 && free) bar_arrive(&sh->full[st]);
                 }
             }
         }
@@ -247,8 +243,7 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         const bool aligned = rows_in_16_bytes(a.y, a.N);
         const int quad = warp & 3, half = (warp - 2 - QB_UNPACK_WARPS) >> 2;
         uint32_t buse = 0;
-        bool ok = true;
-        for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+        for (int it = blockIdx.x; it < items; it += gridDim.x) {
             item(it, nt, mt, sp, b0, b1);
             const int n = nt * 128 + quad * 32 + lane;
             const uint32_t *prm = a.params + (size_t)min(n, a.N - 1) * a.KB;
@@ -260,8 +255,8 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                 const int ab = buse & 1;
                 const float s = f16_bits_to_f32((uint16_t)(next & 0xffffu)), m = f16_bits_to_f32((uint16_t)(next >> 16));
                 if (b + 1 < b1) next = __ldg(prm + b + 1);
-                ok = warp_wait(&sh->xsfull[ab], (buse >> 1) & 1, failed) && warp_wait(&sh->accfull[ab], (buse >> 1) & 1, failed);
-                if (!ok) break;
+                bar_wait(&sh->xsfull[ab], (buse >> 1) & 1, failed);
+                warp_wait(&sh->accfull[ab], (buse >> 1) & 1, failed);
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 const float *xs = sh->xsum[ab] + half * COLS;
                 const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(ab * NTOK + half * COLS);
@@ -292,13 +287,13 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
 #pragma unroll
                 for (int j = 0; j < COLS; ++j) {
                     out[(j & 15) * 32 + lane] = __float2bfloat16_rn(acc[j]);
-                    if ((j & 15) == 15) flush_rows<16>(out, a.y + (size_t)(t0 + j - 15) * a.N + n - lane, a.N, ok ? a.M - t0 - (j - 15) : 0, a.N - (n - lane), lane);
+                    if ((j & 15) == 15) flush_rows<16>(out, a.y + (size_t)(t0 + j - 15) * a.N + n - lane, a.N, a.M - t0 - (j - 15), a.N - (n - lane), lane);
                 }
                 continue;
             }
 #pragma unroll
             for (int j = 0; j < COLS; ++j)
-                if (ok && n < a.N && t0 + j < a.M) {
+                if (n < a.N && t0 + j < a.M) {
                     if (a.ksplit > 1) a.part[((size_t)sp * a.M + t0 + j) * a.N + n] = acc[j];
                     else a.y[(size_t)(t0 + j) * a.N + n] = __float2bfloat16_rn(acc[j]);
                 }

@@ -20,7 +20,7 @@
 //               operand-A stage in tensor memory, a lane per channel
 //   warps 18-21 epilogue: tcgen05.ld of the accumulator, bf16 rows of Y by way of shared memory
 // Every wait on an mbarrier is bounded; on a time-out the CTA records
-// AB2_ERR_TIMEOUT, stops issuing work, still frees its tensor memory and returns.
+// AB2_ERR_TIMEOUT, walks through the rest of its work, frees its tensor memory and returns.
 #include <cuda.h>
 
 #include <algorithm>
@@ -158,17 +158,15 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
     } else if (warp == 1) {
         // ---------------------------------------------------------- MMA issue
         uint32_t suse = 0, tuse = 0;
-        bool ok = true;
-        for (int it = blockIdx.x; it < items && ok; it += gridDim.x, ++tuse) {
+        for (int it = blockIdx.x; it < items; it += gridDim.x, ++tuse) {
             const int ab = tuse % ACCS;
-            ok = warp_wait(&sh->accempty[ab], ((tuse / ACCS) & 1) ^ 1, failed);
+            bar_wait(&sh->accempty[ab], ((tuse / ACCS) & 1) ^ 1, failed);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const uint32_t tacc = tmem + (uint32_t)(ab * NTOK);
             TC_ITEM(it)
-            for (int ks = 2 * g0; ks < 2 * g1 && ok; ++ks, ++suse) {
+            for (int ks = 2 * g0; ks < 2 * g1; ++ks, ++suse) {
                 const int st = suse % TC_STAGES;
-                ok = warp_wait(&sh->full[st], (suse / TC_STAGES) & 1, failed);
-                if (!ok) break;
+                warp_wait(&sh->full[st], (suse / TC_STAGES) & 1, failed);
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 if (elect_one()) {
                     umma_stage_ts(tacc, tmem_a + (uint32_t)(st * TC_A_COLS), umma_desc(sptr(b_st + st * B_BYTES)), IDESC, ks == 2 * g0);
@@ -176,7 +174,6 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
                 }
                 __syncwarp();
             }
-            if (!ok) break;
             if (elect_one()) umma_commit(&sh->accfull[ab]);
             __syncwarp();
         }
@@ -187,13 +184,12 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
         uint32_t gbase = 0;  // groups before this tile
         uint32_t k_mask = 0x000F000Fu, k_magic = 0x43004300u;
         asm volatile("" : "+r"(k_mask), "+r"(k_magic));
-        bool ok = true;
-        for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+        for (int it = blockIdx.x; it < items; it += gridDim.x) {
             TC_ITEM(it)
             // the set's groups: every (TC_SETS / 2)-th of the CTA's sequence of groups
             for (uint32_t wuse = gbase + ((set >> 1) + TC_SETS - gbase % (TC_SETS / 2)) % (TC_SETS / 2); wuse < gbase + (uint32_t)(g1 - g0); wuse += TC_SETS / 2) {
                 const int ws = wuse % TC_WSLOTS;
-                const bool here = bar_wait(&sh->wfull[ws], (wuse / TC_WSLOTS) & 1, failed);
+                bar_wait(&sh->wfull[ws], (wuse / TC_WSLOTS) & 1, failed);
                 const uint32_t *bw = (const uint32_t *)(w_ring + ws * TC_WSLOT_BYTES) + blk * TC_BLOCK_WORDS;
                 const uint4 pw[2] = {*reinterpret_cast<const uint4 *>(bw + r * 16 + half * 8), *reinterpret_cast<const uint4 *>(bw + r * 16 + half * 8 + 4)};
                 const uint32_t pr = bw[256 + r];
@@ -204,8 +200,7 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
                 const uint32_t nz2 = __byte_perm(pr, pr, 0x3232);  // bf16x2 -(128 + z)
                 const uint32_t suse = 2 * wuse + half;
                 const int s = suse % TC_STAGES;
-                ok = warp_wait(&sh->empty[s], ((suse / TC_STAGES) & 1) ^ 1, failed, here);
-                if (!ok) break;
+                const bool free = warp_wait(&sh->empty[s], ((suse / TC_STAGES) & 1) ^ 1, failed);
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 uint32_t o[32];  // two bf16 each
 #pragma unroll
@@ -224,7 +219,7 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
                 asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
                 __syncwarp();
-                if (lane == 0) bar_arrive(&sh->full[s]);
+                if (lane == 0 && free) bar_arrive(&sh->full[s]);
             }
             gbase += (uint32_t)(g1 - g0);
         }
@@ -233,12 +228,10 @@ gemm_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
         const int quad = warp & 3;
         const bool aligned = rows_in_16_bytes(y, N);
         uint32_t tuse = 0;
-        bool ok = true;
-        for (int it = blockIdx.x; it < items && ok; it += gridDim.x, ++tuse) {
+        for (int it = blockIdx.x; it < items; it += gridDim.x, ++tuse) {
             TC_ITEM(it)
             const int ab = tuse % ACCS;
-            ok = warp_wait(&sh->accfull[ab], (tuse / ACCS) & 1, failed);
-            if (!ok) break;
+            bar_wait(&sh->accfull[ab], (tuse / ACCS) & 1, failed);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const int n = nt * 128 + quad * 32 + lane;
 #pragma unroll 1

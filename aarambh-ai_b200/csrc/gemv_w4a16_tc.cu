@@ -38,7 +38,7 @@
 //                 (eight bulk copies in parallel; issuing one keeps a warp busy for
 //                 a few hundred cycles, which the unpack warps cannot afford)
 // Every wait on an mbarrier is bounded; on a time-out the CTA records
-// AB2_ERR_TIMEOUT, stops issuing work, still frees its tensor memory and returns.
+// AB2_ERR_TIMEOUT, walks through the rest of its work, frees its tensor memory and returns.
 #include <algorithm>
 
 #include "common.cuh"
@@ -177,18 +177,17 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
         // ---------------------------------------------------------- MMA issue (alternate units per warp)
         const uint32_t my_id = warp == 1 ? 0u : (uint32_t)(warp - 13);
         uint32_t use = 0;
-        bool ok = true;
-        for (int u = rg.u0; u < rg.u1 && ok; ++u, ++use) {
+        for (int u = rg.u0; u < rg.u1; ++u, ++use) {
             if (use % DG_MMA_WARPS != my_id) continue;
             const int ab = use % DG_ACC;
-            ok = warp_wait(&sh->accempty[ab], ((use / DG_ACC) & 1) ^ 1, failed);
+            bar_wait(&sh->accempty[ab], ((use / DG_ACC) & 1) ^ 1, failed);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const uint32_t td = tmem + (uint32_t)(ab * NTOK);
-            for (int half = 0; half < 2 && ok; ++half) {
+            for (int half = 0; half < 2; ++half) {
                 const uint32_t suse = 2 * use + half;
                 const int s = suse % DG_STAGES, xs = suse % DG_XSTAGES;
-                ok = warp_wait(&sh->xfull[xs], (suse / DG_XSTAGES) & 1, failed) && warp_wait(&sh->afull[s], (suse / DG_STAGES) & 1, failed);
-                if (!ok) break;
+                bar_wait(&sh->xfull[xs], (suse / DG_XSTAGES) & 1, failed);
+                warp_wait(&sh->afull[s], (suse / DG_STAGES) & 1, failed);
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 if (elect_one()) {
                     umma_stage_ts(td, tmem_a + (uint32_t)(s * DG_A_COLS), umma_desc(sptr(b_st + xs * B_BYTES)), IDESC, half == 0);
@@ -197,7 +196,6 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
                 }
                 __syncwarp();
             }
-            if (!ok) break;
             if (elect_one()) umma_commit(&sh->accfull[ab]);
             __syncwarp();
         }
@@ -215,7 +213,7 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
         uint32_t use = 0;
         for (int u = rg.u0; u < rg.u1; ++u, ++use) {
             const int ws = use % DG_WSLOTS;
-            const bool here = bar_wait(&sh->wfull[q][ws], (use / DG_WSLOTS) & 1, failed);
+            bar_wait(&sh->wfull[q][ws], (use / DG_WSLOTS) & 1, failed);
             const uint32_t *bw = (const uint32_t *)(ring + ws * DG_WSLOT_BYTES) + (blk & 1) * W4_BLOCK_WORDS;
             const uint4 p0 = *reinterpret_cast<const uint4 *>(bw + r * 16 + half * 8);
             const uint4 p1 = *reinterpret_cast<const uint4 *>(bw + r * 16 + half * 8 + 4);
@@ -227,7 +225,7 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
             if (lane == 0) bar_arrive_after(&sh->wempty[q][ws], held, (uint32_t)K & 1u);
             const uint32_t suse = 2 * use + half;
             const int s = suse % DG_STAGES;
-            if (!warp_wait(&sh->sempty[s], ((suse / DG_STAGES) & 1) ^ 1, failed, here)) break;
+            warp_wait(&sh->sempty[s], ((suse / DG_STAGES) & 1) ^ 1, failed);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const uint32_t words[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
             uint32_t o[32];
@@ -250,13 +248,12 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
 #pragma unroll
         for (int j = 0; j < NTOK; ++j) acc[j] = 0.f;
         uint32_t use = 0;
-        // After a time-out the warps go through their remaining units without waiting: they share barriers, and the
-        // counters of cut tiles have to come back to zero.
-        bool ok = true;
+        // that these warps do not leave after a time-out also brings the counters of cut tiles back to zero
         for (int u = rg.u0; u < rg.u1; ++u, ++use) {
             const int nt = u / G, g = u - nt * G;
             const int ab = use % DG_ACC;
-            if (ok) ok = warp_wait(&sh->accfull[ab], (use / DG_ACC) & 1, failed);
+            bar_wait(&sh->accfull[ab], (use / DG_ACC) & 1, failed);
+            __syncwarp();  // the tensor-memory load is a whole-warp operation
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const float sc = __uint_as_float(sh->params[use % DG_PARAM_BUFS][row] << 16);
             constexpr int COLS = NTOK < 32 ? 16 : 32;  // tokens at a time

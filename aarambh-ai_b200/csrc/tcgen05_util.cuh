@@ -178,12 +178,13 @@ __device__ __forceinline__ void tmem_st32(uint32_t addr, const uint32_t (&v)[32]
         "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31};\n" ::AB2_REGS32("r", v), "r"(addr)
         : "memory");
 }
-// A wait of a whole warp, with one answer for it: lanes that gave up while others went on would leave those waiting for them in
-// the warp's next collective instruction for good.  So a warp that executes any takes every decision to stop - a wait, *failed -
-// by such a vote.  `so_far` is what a lane's earlier wait gave it, where the two share a vote.
-__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volatile int *failed, bool so_far = true) {
-    return __all_sync(0xffffffffu, so_far && bar_wait(bar, parity, failed));
-}
+// A wait of a whole warp, with one answer for it.  Lanes that left a loop after a wait while others went on would leave those
+// waiting for them in the warp's next collective instruction for good.  So the warps of the GEMMs that execute any do not
+// leave: after a time-out they walk through the rest of their work, whose waits then give up at once, over whatever the
+// buffers hold, and the status word says that the output is void.  (They do not arrive at a barrier with copies under way
+// unless the stage was theirs: arrivals beyond its count are undefined.)  Leaving by a vote after each wait is sound too, but the INT8
+// GEMM took 225 us with it on 14336 x 4096 at 2048 tokens, 213 with lanes that left alone, and takes 205 so.
+__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volatile int *failed) { return __all_sync(0xffffffffu, bar_wait(bar, parity, failed)); }
 
 __device__ __forceinline__ uint32_t bf16x2_add_(uint32_t a, uint32_t b) {
     uint32_t d;
