@@ -385,11 +385,11 @@ __global__ void __launch_bounds__(256) prompt_gather_kernel(PtGather a) {
     *reinterpret_cast<uint4 *>(a.dst[w] + ((size_t)blockIdx.y * a.n + r) * a.ld[w] + c) = v;
 }
 
-// Fills in the gathered keys and values; `heads` of them.
+// Fills in the gathered keys and values; `heads` of them.  AB2_ERR_UNSUPPORTED where there is no memory for them: the kernels
+// that read the cache as it is need none.
 int gather_rows(PtGather g, bool int8, int heads, ScratchLease &ws, PromptAttnArgs &p, cudaStream_t s) {
     const size_t kb = (size_t)heads * g.n * g.ld[0] * 2, vb = (size_t)heads * g.n * g.ld[1] * 2;
-    int rc = ws.take(kb + vb);  // both are multiples of 16 bytes
-    if (rc != AB2_OK) return rc;
+    if (!ws.take(kb + vb)) return AB2_ERR_UNSUPPORTED;  // both are multiples of 16 bytes
     g.dst[0] = (__nv_bfloat16 *)ws.ptr;
     g.dst[1] = (__nv_bfloat16 *)((char *)ws.ptr + kb);
     const dim3 grid((unsigned)(((size_t)g.n * (std::max(g.ld[0], g.ld[1]) / 8) + 255) / 256), heads, 2);

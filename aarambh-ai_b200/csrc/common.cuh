@@ -74,7 +74,8 @@ struct ScratchLease {
     ScratchLease(const ScratchLease &) = delete;
     ScratchLease &operator=(const ScratchLease &) = delete;
     ~ScratchLease();
-    int take(size_t bytes);
+    // false where the memory is not to be had; no CUDA error stays behind, and the caller goes on without
+    bool take(size_t bytes);
 };
 
 static inline size_t ceil_div(size_t a, size_t b) { return (a + b - 1) / b; }

@@ -329,12 +329,11 @@ int launch_qb(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t 
     }
     // as many shares of K as make one wave of items, at least two blocks each; the reduce pass stores rows in 16-byte pieces
     const int tiles = ((N + 127) / 128) * (Mp / NTOK), sms = device_sm_count();
-    const int ksplit = rows_in_16_bytes(y, N) ? std::max(1, std::min(std::min(8, KB / 2), sms / tiles)) : 1;
+    int ksplit = rows_in_16_bytes(y, N) ? std::max(1, std::min(std::min(8, KB / 2), sms / tiles)) : 1;
     const size_t xp_bytes = ((size_t)M * K * 2 + 255) & ~(size_t)255, xs_bytes = ((size_t)KB * Mp * 4 + 255) & ~(size_t)255;
-    const size_t part_bytes = ksplit > 1 ? (size_t)ksplit * M * N * 4 : 0;
     ScratchLease ws(s);
-    rc = ws.take(xp_bytes + xs_bytes + part_bytes);
-    if (rc != AB2_OK) return rc;
+    if (ksplit > 1 && !ws.take(xp_bytes + xs_bytes + (size_t)ksplit * M * N * 4)) ksplit = 1;
+    if (!ws.ptr && !ws.take(xp_bytes + xs_bytes)) return AB2_ERR_UNSUPPORTED;  // the CUDA-core kernel needs none
     __nv_bfloat16 *xp = (__nv_bfloat16 *)ws.ptr;
     float *xsum = (float *)((char *)ws.ptr + xp_bytes), *part = (float *)((char *)ws.ptr + xp_bytes + xs_bytes);
     CUtensorMap wmap, xmap;
@@ -354,6 +353,7 @@ int launch_qb(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t 
 
 bool qlinear_q4km_tc_eligible(const ab2_qweight *w, ab2_dtype dtype) { return w->fmt == FMT_Q4KM && dtype == AB2_BF16 && w->K % 256 == 0; }
 
+// AB2_ERR_UNSUPPORTED where its scratch is not to be had.
 int qlinear_q4km_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t s) {
     // the token tile that leaves the fewest padded tokens in the fewest waves, larger tiles unpacking less
     if (M <= 32) return launch_qb<32>(w, x, M, y, s);

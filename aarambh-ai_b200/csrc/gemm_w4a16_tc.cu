@@ -305,7 +305,7 @@ __global__ void splitk_reduce_kernel(const float *__restrict__ part, __nv_bfloat
 constexpr size_t TC_SPLIT_MAX_BYTES = (size_t)128 << 20;
 
 template <int NTOK>
-int launch_tc(const ab2_qweight *w, const void *x, int M, void *y, int ksplit, cudaStream_t s) {
+int launch_tc(const ab2_qweight *w, const void *x, int M, void *y, int ksplit, float *part, cudaStream_t s) {
     int *status = nullptr;
     int rc = device_status_word(&status);
     if (rc != AB2_OK) return rc;
@@ -322,13 +322,6 @@ int launch_tc(const ab2_qweight *w, const void *x, int M, void *y, int ksplit, c
         configured[dev] = true;
     }
     const int tiles = ((w->N + 127) / 128) * ((M + NTOK - 1) / NTOK);
-    float *part = nullptr;
-    ScratchLease ws(s);
-    if (ksplit > 1) {
-        rc = ws.take((size_t)ksplit * M * w->N * sizeof(float));
-        if (rc != AB2_OK) return rc;
-        part = (float *)ws.ptr;
-    }
     const int items = tiles * ksplit;
     const int grid = std::min(items, device_sm_count());
     cudaError_t e = launch_kernel(gemm_w4a16_tc_kernel<NTOK>, dim3(grid), dim3(TC_THREADS), smem, s, (const uint32_t *)w->codes, map, (__nv_bfloat16 *)y, w->N, w->K, M,
@@ -359,12 +352,16 @@ int qlinear_w4a16_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaSt
     const bool recorded = cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
     static const bool no_split = getenv("AB2_GEMM_NO_SPLITK") != nullptr;
     const bool split = !recorded && !no_split && rows_in_16_bytes(y, w->N) && (size_t)4 * M * w->N * sizeof(float) <= TC_SPLIT_MAX_BYTES;
-    const GemmTileChoice c = choose_gemm_tile(costs, M, w->N, w->K / 128, device_sm_count(), split ? 4 : 1);
+    GemmTileChoice c = choose_gemm_tile(costs, M, w->N, w->K / 128, device_sm_count(), split ? 4 : 1);
+    ScratchLease ws(s);
+    if (c.ksplit > 1 && !ws.take((size_t)c.ksplit * M * w->N * sizeof(float)))
+        c = choose_gemm_tile(costs, M, w->N, w->K / 128, device_sm_count(), 1);
+    float *part = (float *)ws.ptr;
     switch (c.ntok) {
-    case 32: return launch_tc<32>(w, x, M, y, c.ksplit, s);
-    case 128: return launch_tc<128>(w, x, M, y, c.ksplit, s);
-    case 192: return launch_tc<192>(w, x, M, y, c.ksplit, s);
-    default: return launch_tc<256>(w, x, M, y, c.ksplit, s);
+    case 32: return launch_tc<32>(w, x, M, y, c.ksplit, part, s);
+    case 128: return launch_tc<128>(w, x, M, y, c.ksplit, part, s);
+    case 192: return launch_tc<192>(w, x, M, y, c.ksplit, part, s);
+    default: return launch_tc<256>(w, x, M, y, c.ksplit, part, s);
     }
 }
 

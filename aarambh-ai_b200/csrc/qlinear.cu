@@ -444,7 +444,10 @@ int qlinear_dispatch(const ab2_qweight *w, const void *x, int M, ab2_dtype dtype
     // Q4_K_M blocks (GGUF-loaded models), bf16 activations, a few tokens: the streaming GEMV over the two planes
     if (qlinear_q4km_stream_eligible(w, dtype, M)) return qlinear_q4km_stream(w, x, M, y, s);
     // more tokens: tcgen05 GEMM, scale and minimum applied in f32 per block
-    if (qlinear_q4km_tc_eligible(w, dtype)) return qlinear_q4km_tc(w, x, M, y, s);
+    if (qlinear_q4km_tc_eligible(w, dtype)) {
+        const int rc = qlinear_q4km_tc(w, x, M, y, s);
+        if (rc != AB2_ERR_UNSUPPORTED) return rc;
+    }
     return qlinear_generic(w, x, M, dtype, y, s);
 }
 

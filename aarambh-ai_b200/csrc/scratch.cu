@@ -11,25 +11,37 @@ constexpr unsigned long long SCRATCH_KEPT_BYTES = 160ull << 20;
 static std::mutex g_pool_mutex;
 static cudaMemPool_t g_pool[64] = {nullptr};
 
-int ScratchLease::take(size_t bytes) {
-    int dev = 0;
-    AB2_CUDA(cudaGetDevice(&dev));
-    AB2_REQUIRE(dev >= 0 && dev < 64, AB2_ERR_BAD_ARG, "device index %d out of range", dev);
-    {
-        std::lock_guard<std::mutex> lock(g_pool_mutex);
-        if (!g_pool[dev]) {
-            cudaMemPoolProps props = {};
-            props.allocType = cudaMemAllocationTypePinned;
-            props.handleTypes = cudaMemHandleTypeNone;
-            props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = dev;
-            AB2_CUDA(cudaMemPoolCreate(&g_pool[dev], &props));
-            unsigned long long kept = SCRATCH_KEPT_BYTES;
-            AB2_CUDA(cudaMemPoolSetAttribute(g_pool[dev], cudaMemPoolAttrReleaseThreshold, &kept));
-        }
+static cudaError_t pool_of(int dev, cudaMemPool_t *out) {
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    if (!g_pool[dev]) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.handleTypes = cudaMemHandleTypeNone;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaError_t e = cudaMemPoolCreate(&g_pool[dev], &props);
+        if (e != cudaSuccess) { g_pool[dev] = nullptr; return e; }
+        unsigned long long kept = SCRATCH_KEPT_BYTES;
+        cudaMemPoolSetAttribute(g_pool[dev], cudaMemPoolAttrReleaseThreshold, &kept);
     }
-    AB2_CUDA(cudaMallocFromPoolAsync(&ptr, bytes, g_pool[dev], stream));
-    return AB2_OK;
+    *out = g_pool[dev];
+    return cudaSuccess;
+}
+
+bool ScratchLease::take(size_t bytes) {
+    // for hosts that keep the device's memory to themselves: no lease is larger
+    static const char *most = getenv("AB2_SCRATCH_MAX_BYTES");
+    if (most && bytes > strtoull(most, nullptr, 10)) return false;
+    int dev = 0;
+    cudaMemPool_t pool = nullptr;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess && (dev < 0 || dev >= 64)) return false;
+    if (e == cudaSuccess) e = pool_of(dev, &pool);
+    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&ptr, bytes, pool, stream);
+    if (e == cudaSuccess) return true;
+    ptr = nullptr;
+    cudaGetLastError();
+    return false;
 }
 
 ScratchLease::~ScratchLease() {
