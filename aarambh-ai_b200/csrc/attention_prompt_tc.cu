@@ -20,6 +20,8 @@
 // MMAs.  32 / 8 heads of 128: 3001 tokens over an INT8 cache 787 us on the warp-level tensor cores, 222 + 11 (widening) here;
 // 1000 tokens behind 500 over a bf16 cache 1344 us on CUDA cores, 50 here; 2048 tokens of 16 / 4 heads with a window of
 // 1024: 114 -> 48.  Below 16 queries a CTA would be nearly empty.
+// The MMA multiplies a tile of values whole, a hidden one by a weight of 0, so an Inf or a NaN in it would reach queries
+// that do not see it.  A query whose sums came out as either is computed again on CUDA cores over the keys in its sight.
 // Every wait on an mbarrier is bounded; on a time-out the CTA records AB2_ERR_TIMEOUT, stops issuing
 // work, frees its tensor memory and returns.
 #include <algorithm>
@@ -45,6 +47,7 @@ struct PtShared {
     uint32_t tmem_base;
     int failed;
     float top[2][PT_Q], sum[2][PT_Q];
+    uint32_t again[2][4];  // queries to compute again, a bit each: by half of the warps and quarter of the queries
     // scales of a tile's keys and values: a half's tile is read from one buffer while its next is written to the other
     alignas(16) float ks[2][2][PT_KEYS], vs[2][2][PT_KEYS];
 };
@@ -139,9 +142,48 @@ __device__ __forceinline__ void softmax_tile(uint32_t s_addr, uint32_t o_addr, f
     sum += (part_sum[0] + part_sum[1]) + (part_sum[2] + part_sum[3]);
 }
 
+// A query's output over the keys of rows [from, to], by one warp: a lane has every 32nd dimension.  Where the fast path's
+// sums were sound this gives the same value, otherwise what a sum over the keys in sight alone gives.
+__device__ __noinline__ void attend_again(const PromptAttnArgs &a, int head, int kv_head, int qi, int from, int to, int lane) {
+    constexpr int QD = 6, VD = 4;  // dim + tail_dims <= 192 (what shared memory holds), vdim <= 128
+    const int dims = a.dim + a.tail_dims;
+    const size_t z = a.k_z ? kv_head : 0;
+    const __nv_bfloat16 *q = a.q + (size_t)qi * a.q_stride + (size_t)head * dims;
+    const __nv_bfloat16 *k = a.k + z * a.k_z + (size_t)kv_head * a.k_head, *v = a.v + z * a.v_z + (size_t)kv_head * a.v_head;
+    float qv[QD], acc[VD] = {}, top = -INFINITY, sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < QD; ++i) qv[i] = lane + 32 * i < dims ? __bfloat162float(q[lane + 32 * i]) : 0.f;
+    for (int key = from; key <= to; ++key) {
+        float s = 0.f, vv[VD];
+#pragma unroll
+        for (int i = 0; i < QD; ++i) {
+            const int d = lane + 32 * i;
+            if (d < dims) s = fmaf(qv[i], __bfloat162float(d < a.dim ? k[(size_t)key * a.k_stride + d] : a.tail[(size_t)key * a.tail_stride + d - a.dim]), s);
+        }
+#pragma unroll
+        for (int i = 0; i < VD; ++i) vv[i] = lane + 32 * i < a.vdim ? __bfloat162float(v[(size_t)key * a.v_stride + lane + 32 * i]) : 0.f;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        s *= a.scale;
+        if (a.k_scale) s *= a.k_scale[(size_t)kv_head * a.scale_z + key];
+        const float best = fmaxf(top, s), keep = top == best ? 1.f : expf(top - best);
+        float w = s == -INFINITY ? 0.f : expf(s - best);
+        sum = sum * keep + w;
+        if (a.v_scale) w *= a.v_scale[(size_t)kv_head * a.scale_z + key];
+#pragma unroll
+        for (int i = 0; i < VD; ++i) acc[i] = fmaf(w, vv[i], acc[i] * keep);
+        top = best;
+    }
+    float scale = sum > 0.f ? 1.f / sum : 1.f;  // a NaN is in acc
+    if (a.gate) scale /= 1.f + expf(-__bfloat162float(a.gate[(size_t)qi * a.gate_stride + head]));
+#pragma unroll
+    for (int i = 0; i < VD; ++i)
+        if (lane + 32 * i < a.vdim) a.out[(size_t)qi * a.out_stride + (size_t)head * a.vdim + lane + 32 * i] = __float2bfloat16_rn(acc[i] * scale);
+}
+
 template <bool SCALED>
 __global__ void __launch_bounds__(PT_THREADS, 1)
-prompt_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap vmap, PtArgs p, int *status) {
+prompt_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap vmap, const __grid_constant__ PtArgs p, int *status) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *qbuf = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const PromptAttnArgs &a = p.a;
@@ -291,7 +333,9 @@ prompt_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
         asm volatile("barrier.cta.sync 1, 256;\n" ::: "memory");
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        uint32_t again = 0;
         if (!__any_sync(0xffffffffu, *failed)) {
+            float poison = 0.f;  // stays 0 unless an output is Inf or NaN
             // both halves of the warps store: value boxes of 64 dimensions in turn
             const float t0 = sh->top[0][r], t1 = sh->top[1][r], t = fmaxf(t0, t1);
             float f0 = ex2(t0 - t), f1 = tiles > 1 ? ex2(t1 - t) : 0.f;
@@ -316,13 +360,24 @@ prompt_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         const int n = k + 2 * e;
-                        const __nv_bfloat162 q = __floats2bfloat162_rn(f0 * __uint_as_float(v[n]) + f1 * __uint_as_float(w[n]), f0 * __uint_as_float(v[n + 1]) + f1 * __uint_as_float(w[n + 1]));
+                        const float x = f0 * __uint_as_float(v[n]) + f1 * __uint_as_float(w[n]), y = f0 * __uint_as_float(v[n + 1]) + f1 * __uint_as_float(w[n + 1]);
+                        poison = fmaf(y, 0.f, fmaf(x, 0.f, poison));
+                        const __nv_bfloat162 q = __floats2bfloat162_rn(x, y);
                         o[e] = *reinterpret_cast<const uint32_t *>(&q);
                     }
                     if (qi < a.S && 32 * c + k < a.vdim) *reinterpret_cast<uint4 *>(dst + 32 * c + k) = make_uint4(o[0], o[1], o[2], o[3]);
                 }
             }
+            again = __ballot_sync(0xffffffffu, qi < a.S && poison != 0.f);  // NaN is not 0
         }
+        if (lane == 0) sh->again[part][quad] = again;
+        asm volatile("barrier.cta.sync 1, 256;\n" ::: "memory");
+        for (int i = 0, n = 0; i < 4; ++i)
+            for (uint32_t rows_left = sh->again[0][i] | sh->again[1][i]; rows_left; rows_left &= rows_left - 1, ++n)
+                if ((n & 7) == warp - 4) {
+                    const int at = q_lo + 32 * i + __ffs(rows_left) - 1, to = first + at;
+                    attend_again(a, head, kv_head, at, a.window ? max(0, to - a.window + 1) : 0, to, lane);
+                }
     }
 
     // ---- teardown: every warp arrives here (all waits are bounded)

@@ -45,3 +45,34 @@ def test_head_sizes_are_refused_alike(kv, hd, S):
     cache.commit(S)
     with pytest.raises(p.Ab2Error, match="head_dim 64 and 128"):
         p.dispatch.attention_cached(cache, torch.randn((1, S, 4, hd), device="cuda").to(torch.bfloat16), hd ** -0.5)
+
+
+@pytest.mark.parametrize("kv", ["bf16", "int8"])
+@pytest.mark.parametrize("h,kvh,hd", [(8, 2, 128), (6, 3, 64)])
+@pytest.mark.parametrize("where", ["keys", "values"])
+@pytest.mark.parametrize("bad", [math.inf, math.nan])
+def test_tokens_that_are_not_finite_stay_behind_the_mask(kv, h, kvh, hd, where, bad):
+    """A token with an Inf or NaN in its key or value changes nothing for the queries before it, in its own tile of 128 keys too."""
+    n, S, tokens = 500, 300, (230, 499)  # cached tokens, queries, tokens that are not finite: in the middle of a tile and at the end
+    g = torch.Generator(device="cuda").manual_seed(hd)
+    p = pkg()
+    k, v = (torch.randn((1, n, kvh, hd), generator=g, device="cuda") for _ in range(2))
+    q = torch.randn((1, S, h, hd), generator=g, device="cuda").to(torch.bfloat16)
+    for t in tokens:
+        (k if where == "keys" else v)[0, t, 0, 5] = bad
+    cache = p.KVCache(n, kvh, hd, h, dtype=kv)
+    cache.append(0, k, v)
+    cache.commit(n)
+    got = p.dispatch.attention_cached(cache, q, hd ** -0.5)[0].double()
+    assert p.device_status() == 0
+    kc, vc = (t.cuda().double() for t in cache.read(0))
+    for head in range(h):
+        kh, vh = kc[:, head * kvh // h], vc[:, head * kvh // h]
+        for qi in (0, 29, 30, 31, 127, 298, 299):
+            seen = n - S + qi + 1
+            w = torch.softmax(kh[:seen] @ q[0, qi, head].double() / math.sqrt(hd), 0)
+            want, out = w @ vh[:seen], got[qi, head]
+            ok = torch.isfinite(want)
+            assert torch.equal(ok, torch.isfinite(out)), (head, qi)
+            if ok.any():
+                assert float((out[ok] - want[ok]).norm()) <= 2.0 ** -8 * float(want[ok].norm()), (head, qi)
