@@ -312,8 +312,8 @@ int attention_cached_device(const ab2_kv *kv, int layer, const void *q, void *ou
         return AB2_OK;
     }
     if (S > 1) {
-        // prefill chunk of a bf16 model: the tcgen05 kernel (attention_prompt_tc.cu); few queries, or a recorded launch,
-        // over an INT8 cache: the warp-level tensor-core kernel (attention_mma.cu)
+        // prefill chunk of a bf16 model: the tcgen05 kernel (attention_prompt_tc.cu) where it is the faster one; few queries, short
+        // contexts, or a recorded launch, over an INT8 cache: the warp-level tensor-core kernel (attention_mma.cu)
         static const bool scalar_prefill = getenv("AB2_SCALAR_PREFILL_ATTN") != nullptr;  // measurement switch
         if (!scalar_prefill) {
             int rc = prompt_tc_cached(kv, layer, q, out, S, pending, row0, nrows, scale, dtype, st, s);

@@ -96,11 +96,18 @@ struct PromptAttnArgs {
     int S, heads, first, dim, tail_dims, vdim;   // `first`: position of the first query
     float scale;
     // what only attention_prompt_tc.cu reads: `rep` query heads (0: one) share a head of keys and values, whose heads
-    // lie k_z and v_z elements apart (0: side by side in a row); row 0 of the keys is position `base`; a query sees
-    // `window` keys (0: all before it); with k_scale and v_scale the key of row j is that row times
-    // k_scale[head scale_z + j], the value times v_scale[...] (codes of an INT8 cache)
-    long long k_z, v_z, scale_z;
-    int rep, base, window;
+    // lie k_z and v_z elements apart (0: side by side in a row); a query sees `window` keys (0: all before it).
+    // Sequences: `nrows` of them (0: one), queries and outputs q_row and out_row elements apart, each with its heads' keys at
+    // matrices (cache row) * kv heads + head, of `mats` in all.  The cache row of sequence i is rows[row0 + i], or row0 + i; the position
+    // of its first query is lens[row] + pending - S, or `first` without lens.  A matrix has key_rows rows; its row 0 is position
+    // 0 or, with `ring`, that of slot 0 of a ring of so many slots in which no sequence's keys in sight wrap.  With
+    // `gathered` the matrices are copies, counted by sequence, that start with the first key in sight.  With k_scale and
+    // v_scale the key of row j is that row times k_scale[matrix of the cache * scale_z + j], the value times v_scale[...] (codes of an
+    // INT8 cache).
+    long long k_z, v_z, scale_z, q_row, out_row;
+    int rep, window, nrows, row0, pending, mats, key_rows, ring;
+    bool gathered;
+    const int *lens, *rows;
     const float *k_scale, *v_scale;
 };
 bool prompt_attention_serves(int dim, int tail, int vdim);
