@@ -76,7 +76,19 @@ struct ScratchLease {
     ~ScratchLease();
     // false where the memory is not to be had; no CUDA error stays behind, and the caller goes on without
     bool take(size_t bytes);
+
+private:
+    bool pooled = false;
 };
+// Set by the decoder step while it records its graph: leases are this memory then, one lease after the other as their launches are,
+// since a graph would hold a lease from the pool as nodes of its own, which launches cannot be chained across.
+struct RecordedScratch {
+    void *ptr;
+    size_t bytes;
+};
+extern thread_local const RecordedScratch *g_recorded_scratch;
+bool scratch_allowed(size_t bytes);   // by the environment's limit
+int scratch_prepare();                // the device's pool, which cannot be made while a graph is recorded
 
 static inline size_t ceil_div(size_t a, size_t b) { return (a + b - 1) / b; }
 

@@ -311,12 +311,33 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
     }
 }
 
+// Tokens of a tile: one tile of 32 or 64 where it takes all of them; else 128, which unpack a weight for the most tokens.
+int qb_tokens(int M) { return M <= 32 ? 32 : M <= 64 ? 64 : 128; }
+
+struct QbPlan {
+    int Mp, tiles, ksplit;
+    size_t xp_bytes, xs_bytes, part_bytes;
+};
+QbPlan qb_plan(const ab2_qweight *w, int M, int ntok, bool whole_rows) {
+    const int KB = w->K / 256;
+    QbPlan p;
+    p.Mp = (M + ntok - 1) / ntok * ntok;
+    p.tiles = ((w->N + 127) / 128) * (p.Mp / ntok);
+    // as many shares of K as make one wave of items, at least two blocks each; the reduce pass stores rows in 16-byte pieces
+    p.ksplit = whole_rows ? std::max(1, std::min(std::min(8, KB / 2), device_sm_count() / p.tiles)) : 1;
+    p.xp_bytes = ((size_t)M * w->K * 2 + 255) & ~(size_t)255;
+    p.xs_bytes = ((size_t)KB * p.Mp * 4 + 255) & ~(size_t)255;
+    p.part_bytes = p.ksplit > 1 ? (size_t)p.ksplit * M * w->N * 4 : 0;
+    return p;
+}
+
 template <int NTOK>
 int launch_qb(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t s) {
     int *status = nullptr;
     int rc = device_status_word(&status);
     if (rc != AB2_OK) return rc;
-    const int N = w->N, K = w->K, KB = K / 256, Mp = (M + NTOK - 1) / NTOK * NTOK;
+    const QbPlan p = qb_plan(w, M, NTOK, rows_in_16_bytes(y, w->N));
+    const int N = w->N, K = w->K, KB = K / 256, Mp = p.Mp, tiles = p.tiles, sms = device_sm_count();
     const size_t smem = 1024 + qb_stages<NTOK>() * NTOK * 128 + qb_wslots<NTOK>() * QB_WSLOT_BYTES + QB_OUT_BYTES + sizeof(QbShared);
     static_assert(1024 + qb_stages<NTOK>() * NTOK * 128 + qb_wslots<NTOK>() * QB_WSLOT_BYTES + QB_OUT_BYTES + sizeof(QbShared) <= 227 * 1024, "shared memory of a CTA");
     static bool configured[64] = {false};  // the attribute is per device
@@ -327,15 +348,12 @@ int launch_qb(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t 
         AB2_CUDA(cudaFuncSetAttribute(gemm_q4km_tc_kernel<NTOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         configured[dev] = true;
     }
-    // as many shares of K as make one wave of items, at least two blocks each; the reduce pass stores rows in 16-byte pieces
-    const int tiles = ((N + 127) / 128) * (Mp / NTOK), sms = device_sm_count();
-    int ksplit = rows_in_16_bytes(y, N) ? std::max(1, std::min(std::min(8, KB / 2), sms / tiles)) : 1;
-    const size_t xp_bytes = ((size_t)M * K * 2 + 255) & ~(size_t)255, xs_bytes = ((size_t)KB * Mp * 4 + 255) & ~(size_t)255;
+    int ksplit = p.ksplit;
     ScratchLease ws(s);
-    if (ksplit > 1 && !ws.take(xp_bytes + xs_bytes + (size_t)ksplit * M * N * 4)) ksplit = 1;
-    if (!ws.ptr && !ws.take(xp_bytes + xs_bytes)) return AB2_ERR_UNSUPPORTED;  // the CUDA-core kernel needs none
+    if (ksplit > 1 && !ws.take(p.xp_bytes + p.xs_bytes + p.part_bytes)) ksplit = 1;
+    if (!ws.ptr && !ws.take(p.xp_bytes + p.xs_bytes)) return AB2_ERR_UNSUPPORTED;  // the CUDA-core kernel needs none
     __nv_bfloat16 *xp = (__nv_bfloat16 *)ws.ptr;
-    float *xsum = (float *)((char *)ws.ptr + xp_bytes), *part = (float *)((char *)ws.ptr + xp_bytes + xs_bytes);
+    float *xsum = (float *)((char *)ws.ptr + p.xp_bytes), *part = (float *)((char *)ws.ptr + p.xp_bytes + p.xs_bytes);
     CUtensorMap wmap, xmap;
     rc = make_x_map(&xmap, xp, M, K, NTOK);
     if (rc == AB2_OK) rc = make_bytes_map(&wmap, w->codes, N, K / 2);
@@ -355,10 +373,17 @@ bool qlinear_q4km_tc_eligible(const ab2_qweight *w, ab2_dtype dtype) { return w-
 
 // AB2_ERR_UNSUPPORTED where its scratch is not to be had.
 int qlinear_q4km_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t s) {
-    // the token tile that leaves the fewest padded tokens in the fewest waves, larger tiles unpacking less
-    if (M <= 32) return launch_qb<32>(w, x, M, y, s);
-    if (M <= 64) return launch_qb<64>(w, x, M, y, s);
-    return launch_qb<128>(w, x, M, y, s);
+    switch (qb_tokens(M)) {
+    case 32: return launch_qb<32>(w, x, M, y, s);
+    case 64: return launch_qb<64>(w, x, M, y, s);
+    default: return launch_qb<128>(w, x, M, y, s);
+    }
+}
+
+// The most that a call of M tokens leases.
+size_t qlinear_q4km_tc_scratch(const ab2_qweight *w, int M) {
+    const QbPlan p = qb_plan(w, M, qb_tokens(M), w->N % 8 == 0);
+    return p.xp_bytes + p.xs_bytes + p.part_bytes;
 }
 
 }  // namespace ab2

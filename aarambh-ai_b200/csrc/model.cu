@@ -33,6 +33,7 @@ int qlinear_w4a16_mma_add(const ab2_qweight *w, const void *x, int M, void *y, c
 int qlinear_w4a16_mma_swiglu(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t s);
 int qlinear_w4a16_mma_f32(const ab2_qweight *w, const void *x, int M, float *y, cudaStream_t s);
 int qlinear_w4a16_mma_f32_peer(const ab2_qweight *w, const void *x, int M, ab2_tp *tp, cudaStream_t s);
+size_t qlinear_recorded_scratch(const ab2_qweight *w, int M, ab2_dtype dtype);
 bool qlinear_step_eligible(const ab2_qweight *w, ab2_dtype dtype, int M);
 int qlinear_step_norm(const ab2_qweight *w, const void *x, const float *norm_w, float eps, int M, ab2_dtype dtype, bool swiglu, void *y, cudaStream_t s);
 int qlinear_step_add(const ab2_qweight *w, const void *x, const void *resid, int M, ab2_dtype dtype, void *y, cudaStream_t s);
@@ -74,6 +75,9 @@ struct ab2_model {
     // device copies of the token ids and greedy tokens of ab2_model_decode_step_host
     uint32_t *host_step_ids, *host_step_out;
     int host_step_rows;
+    // what the linears of recorded steps lease; a larger one takes its place for later graphs
+    ab2::RecordedScratch step_scratch;
+    std::vector<void *> old_step_scratch;
 };
 
 namespace ab2 {
@@ -166,8 +170,11 @@ static int forward_launches(ab2_model *m, ab2_kv *kv, const uint32_t *ids, int S
                             int len_hint, cudaStream_t s) {
     // A prompt's launches are chained too: what a kernel sets up (barriers, tensor memory) and the launch itself overlap the
     // end of the one before.  Ahead of its wait a kernel reads constant weights only.  4 layers of 2048, 300 tokens: 667 -> 526 us;
-    // 8 layers of 4096, 512 tokens: 2.30 -> 2.18 ms.  (Tensor parallel: the collectives are not ours.)
-    const ChainedLaunches chained(S > 1 && !(m->tp && m->tp->world > 1));
+    // 8 layers of 4096, 512 tokens: 2.30 -> 2.18 ms.  (Tensor parallel: the collectives are not ours.  A caller's graph: leases are
+    // nodes of it, which launches cannot be chained across.)
+    cudaStreamCaptureStatus recording = cudaStreamCaptureStatusNone;
+    const bool recorded = S > 1 && (cudaStreamIsCapturing(s, &recording) != cudaSuccess || recording != cudaStreamCaptureStatusNone);
+    const ChainedLaunches chained(S > 1 && !recorded && !(m->tp && m->tp->world > 1));
     if (m->stack) return stack_forward(m->stack, kv, ids, S, row0, nrows, logits_mode, (float *)logits, argmax_out, len_hint, s);
     const ab2_model_config &c = m->cfg;
     const int all = nrows * S, d = c.d_model, hd = c.head_dim;
@@ -374,6 +381,21 @@ static int forward_launches(ab2_model *m, ab2_kv *kv, const uint32_t *ids, int S
     return AB2_OK;
 }
 
+// Memory for the leases of a recorded step of `nrows` rows; without it their linears take the kernels that need none.
+static void prepare_step_scratch(ab2_model *m, int nrows) {
+    size_t need = 0;
+    auto linear = [&](const ab2_qweight *w) { if (w) need = std::max(need, qlinear_recorded_scratch(w, nrows, m->dtype)); };
+    for (const LayerWeights &L : m->layers) {
+        linear(L.wqkv); linear(L.part[3]); linear(L.wgu); linear(L.part[6]);
+    }
+    linear(m->lm_head);
+    if (need <= m->step_scratch.bytes || !scratch_allowed(need)) return;
+    void *p = nullptr;
+    if (cudaMalloc(&p, need) != cudaSuccess) { cudaGetLastError(); return; }
+    if (m->step_scratch.ptr) m->old_step_scratch.push_back(m->step_scratch.ptr);  // earlier graphs use it
+    m->step_scratch = {p, need};
+}
+
 static int check_forward(ab2_model *m, ab2_kv *kv, const void *ids, int S, int row0, int nrows,
                          const int *offsets_host, int logits_mode, const void *logits) {
     AB2_REQUIRE(m && kv && ids, AB2_ERR_BAD_ARG, "null argument");
@@ -473,6 +495,8 @@ AB2_API int ab2_model_destroy(ab2_model *m) {
     if (!m) return AB2_OK;
     stack_destroy(m->stack);
     for (auto &g : m->graphs) cudaGraphExecDestroy(g.second.exec);
+    for (void *p : m->old_step_scratch) cudaFree(p);
+    cudaFree(m->step_scratch.ptr);
     persistent_step_destroy(m->persistent);
     for (auto &L : m->layers) {
         ab2_qweight_destroy(L.wqkv); ab2_qweight_destroy(L.wgu);
@@ -753,11 +777,14 @@ AB2_API int ab2_model_decode_step(ab2_model *m, ab2_kv *kv, const uint32_t *ids_
         cudaGraph_t graph = nullptr;
         if (!m->stack) rc = w4a16_prepare_stream(s);  // scratch of the GEMV is allocated outside the capture
         if (rc != AB2_OK) return rc;
+        prepare_step_scratch(m, nrows);
         AB2_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         // Chained launches: a kernel launched with the attribute waits for its predecessor itself, one launched without
         // waits as a whole.  (Tensor parallel keeps plain launches unless the fast path is taken: its collectives are not ours.)
         g_pdl_launch = m->fused_epilogues || m->stack || !m->tp;
+        g_recorded_scratch = &m->step_scratch;
         rc = forward_launches(m, kv, ids_dev, 1, row0, nrows, kv->lens_dev, logits_dev ? 1 : 0, logits_dev, argmax_dev, len_bound, s);
+        g_recorded_scratch = nullptr;
         if (rc == AB2_OK) {
             // lengths advance inside the graph; the host mirror is advanced per replay
             std::vector<int> keep(kv->lens_host, kv->lens_host + kv->B);

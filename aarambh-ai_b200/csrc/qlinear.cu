@@ -451,6 +451,13 @@ int qlinear_dispatch(const ab2_qweight *w, const void *x, int M, ab2_dtype dtype
     return qlinear_generic(w, x, M, dtype, y, s);
 }
 
+size_t qlinear_q4km_tc_scratch(const ab2_qweight *w, int M);
+
+// The memory that qlinear_dispatch leases for M tokens in a recorded launch.
+size_t qlinear_recorded_scratch(const ab2_qweight *w, int M, ab2_dtype dtype) {
+    return qlinear_q4km_tc_eligible(w, dtype) && !qlinear_q4km_stream_eligible(w, dtype, M) ? qlinear_q4km_tc_scratch(w, M) : 0;
+}
+
 }  // namespace ab2
 
 AB2_API int ab2_qlinear_forward(const ab2_qweight *w, const void *x_dev, int M, ab2_dtype dtype,

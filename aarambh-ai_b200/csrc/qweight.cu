@@ -28,6 +28,10 @@ AB2_API const char *ab2_last_error(void) { return ab2::g_last_error.c_str(); }
 
 using namespace ab2;
 
+namespace ab2 {
+int device_status_word(int **out);
+}
+
 // ---------------------------------------------------------------------------
 // helpers
 // ---------------------------------------------------------------------------
@@ -184,6 +188,10 @@ static int make_q4km(ab2_qweight **out, int N, int K) {
     w->param_bytes = nb * 4;
     TRY_OR_FREE(w, dev_alloc(&w->codes, w->codes_bytes));
     TRY_OR_FREE(w, dev_alloc((void **)&w->block_params, nb * 4));
+    // what the first call would otherwise make, perhaps while it is recorded
+    int *status = nullptr;
+    TRY_OR_FREE(w, scratch_prepare());
+    TRY_OR_FREE(w, device_status_word(&status));
     return AB2_OK;
 }
 
