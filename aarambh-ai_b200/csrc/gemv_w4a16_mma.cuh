@@ -106,6 +106,9 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
 
 constexpr int W4_BLOCK_WORDS = 272;      // 16 rows x 16 code words + 16 parameter words
 
+// Partial sums of the decode GEMM (gemv_w4a16_tc.cu): two slots a CTA, each of at most 64 tokens x 128 channels f32.
+constexpr int W4DG_MAX_TOKENS = 64, W4DG_MAX_SLOT_FLOATS = W4DG_MAX_TOKENS * 128;
+
 // What the warp that finishes a 16-row tile stores: the projection
 // (W4_EPI_STORE), the residual plus the projection (W4_EPI_ADD; `resid` may
 // alias `y`), silu(gate) * up for a weight whose 16-row tiles hold 8 gate rows

@@ -104,6 +104,7 @@ gemv_w4a16_tc_kernel(const uint32_t *__restrict__ wt, const __grid_constant__ CU
     constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NTOK >> 3) << 17) | ((128u >> 4) << 24);
     constexpr uint32_t ACC_COLS = DG_ACC * NTOK, TMEM_COLS = NTOK > 32 ? 512u : 256u;
     static_assert(ACC_COLS + DG_STAGES * DG_A_COLS <= TMEM_COLS, "accumulators and operand stages fit");
+    static_assert(NTOK <= W4DG_MAX_TOKENS, "the caller's scratch holds two partial tiles per CTA");
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t *b_st = smem;                                    // [DG_XSTAGES][B_BYTES]
@@ -373,14 +374,11 @@ int launch_dg(const ab2_qweight *w, const void *x, int M, void *y, const void *r
 
 }  // namespace
 
-// Scratch the kernel needs per CTA: two slots of [64 tokens][128 channels] f32.
-size_t gemv_w4a16_tc_partial_floats_per_cta() { return 2 * 64 * 128; }
-
 // Y = epilogue(X[M][K] . W^T) for 2..64 tokens; partials / counters are the caller's
-// scratch (zeroed counters, one per 128-channel tile; partials for max_ctas CTAs).
+// scratch (zeroed counters, one per 128-channel tile; two slots of W4DG_MAX_SLOT_FLOATS for every SM).
 int qlinear_w4a16_tc_decode(const ab2_qweight *w, const void *x, int M, void *y, const void *resid, int epi,
                             float *partials, int *counters, int max_ctas, cudaStream_t s) {
-    AB2_REQUIRE(M >= 1 && M <= 64, AB2_ERR_BAD_SHAPE, "the decode GEMM serves 1..64 tokens, got %d", M);
+    AB2_REQUIRE(M >= 1 && M <= W4DG_MAX_TOKENS, AB2_ERR_BAD_SHAPE, "the decode GEMM serves 1..%d tokens, got %d", W4DG_MAX_TOKENS, M);
     AB2_REQUIRE(((uintptr_t)x & 15) == 0 && (w->K * 2) % 16 == 0, AB2_ERR_BAD_ALIGN, "activations must be 16-byte aligned");
 #define AB2_DG(NT)                                                                                              \
     switch (epi) {                                                                                              \

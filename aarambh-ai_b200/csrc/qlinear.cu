@@ -156,9 +156,9 @@ static int gemv_scratch_for(cudaStream_t s, GemvScratch *out) {
                         "on the stream before capturing (its scratch buffers are allocated then)");
         GemvScratch sc;
         sc.max_ctas = device_sm_count() * 3;
-        // two partial tiles per warp of the warp kernels, or two partial tile sets per CTA of the strip kernel
+        // two partial tiles per warp of the warp kernels, or per CTA of the strip kernel and the decode GEMM, one CTA per SM
         const size_t pbytes = std::max((size_t)sc.max_ctas * W4W_WARPS * 2 * W4W_SLOT_FLOATS,
-                                       (size_t)device_sm_count() * 2 * W4S_MAX_SLOT_FLOATS) * sizeof(float);
+                                       (size_t)device_sm_count() * 2 * std::max(W4S_MAX_SLOT_FLOATS, W4DG_MAX_SLOT_FLOATS)) * sizeof(float);
         AB2_CUDA(cudaMalloc((void **)&sc.partials, pbytes));
         AB2_CUDA(cudaMalloc((void **)&sc.counters, W4W_MAX_TILES * sizeof(int)));
         AB2_CUDA(cudaMemset(sc.counters, 0, W4W_MAX_TILES * sizeof(int)));
