@@ -2,9 +2,10 @@
 // crates/aarambh-studio-quant/src/gguf_quant.rs:39-49: w = q * scale + min), bf16 activations, many tokens: the
 // prompts and larger batches of a GGUF-loaded model on the 5th-generation tensor cores.
 //
-//   y[t][n] = sum over blocks b of  scale[n][b] * (sum_k q[n][k] x[t][k]) + min[n][b] * X[t][b],
+//   y[t][n] = sum over blocks b of  scale[n][b] * (sum_k (q[n][k] - 8) x[t][k]) + (min[n][b] + 8 scale[n][b]) * X[t][b],
 //
-// X the sum of a token's activations over a block.  The codes enter the MMA as exact small integers; a block is 256
+// X the sum of a token's activations over a block.  The codes enter the MMA as exact small integers, around 0 and not from 0 on: the
+// two parts would otherwise be sums of up to 16 times the result whose difference it is.  A block is 256
 // steps of K, after which its accumulator leaves tensor memory and the scale and the minimum are applied in f32, so
 // no weight is rounded.  A first kernel forms X and a copy of the activations whose groups of 8 are ordered
 // 0,4,1,5,2,6,3,7, the order in which one shift and one mask take codes out of a word of the reference's layout.
@@ -195,7 +196,7 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         // ---------------------------------------------------------- unpack: codes -> bf16 integers
         const int t = (warp & 3) * 32 + lane, set = (warp - 2) >> 2;  // channel: the warp's lanes of tensor memory
         uint32_t wuse = 0;
-        uint32_t k_mask = 0x000F000Fu, k_magic = 0x43004300u, k_off = 0xC300C300u;  // -128
+        uint32_t k_mask = 0x000F000Fu, k_magic = 0x43004300u, k_off = 0xC308C308u;  // -136: code - 8 from 128 + code
         asm volatile("" : "+r"(k_mask), "+r"(k_magic), "+r"(k_off));
         for (int it = blockIdx.x; it < items; it += gridDim.x) {
             item(it, nt, mt, sp, b0, b1);
@@ -253,7 +254,7 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
             uint32_t next = __ldg(prm + b0);
             for (int b = b0; b < b1; ++b, ++buse) {
                 const int ab = buse & 1;
-                const float s = f16_bits_to_f32((uint16_t)(next & 0xffffu)), m = f16_bits_to_f32((uint16_t)(next >> 16));
+                const float s = f16_bits_to_f32((uint16_t)(next & 0xffffu)), m = fmaf(8.f, s, f16_bits_to_f32((uint16_t)(next >> 16)));
                 if (b + 1 < b1) next = __ldg(prm + b + 1);
                 bar_wait(&sh->xsfull[ab], (buse >> 1) & 1, failed);
                 warp_wait(&sh->accfull[ab], (buse >> 1) & 1, failed);

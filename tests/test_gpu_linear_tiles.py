@@ -108,3 +108,17 @@ def test_output_off_a_16_byte_boundary(method, N, K, M):
         p._lib.check(p._lib.lib.ab2_qlinear_forward(lin._h, x.data_ptr(), M, p.qlinear.dtype_code(x.dtype), y.data_ptr(), p.qlinear.stream_ptr()))
         assert bool((buf[:off] == 7).all()) and bool((buf[off + M * N:] == 7).all())
         check(lambda _: y, x, 16 * (512 + K // 256) if method == "q4_k_m" else 2 * K + (2 ** 15 if method == "w4a16" else 0), lin)
+
+
+@pytest.mark.parametrize("M", [9, 40, 130])
+def test_q4km_codes_cancel_exactly(M):
+    """Weights scale * (code - 8) that sum to 0 in every block, and equal activations: the part with the minimum and the part with the
+    codes, each some thousand times larger than a weight's, have nothing to cancel, and the output is 0 to the last bit."""
+    scale = float(torch.tensor(0.0123, dtype=torch.float16))
+    codes = torch.tensor([-8, 7, 1] + [c for k in range(1, 8) for c in (k, -k)] * 18 + [0])
+    assert codes.numel() == 256 and int(codes.sum()) == 0
+    w = (codes.repeat(128, 2) * scale).cuda()
+    lin = pkg().QuantLinear.quantise(w, "q4_k_m")
+    assert torch.equal(lin.dequantise(), w)
+    x = torch.full((M, 512), 251.0, dtype=torch.bfloat16, device="cuda")
+    assert bool((lin(x) == 0).all())
