@@ -21,73 +21,75 @@ __global__ void __launch_bounds__(TM * TN / 16) gemm_generic_kernel(GemvArgs a, 
     constexpr int WV = TN * (GG_TK / 8) / THREADS, XV = TM * (GG_TK / 8) / THREADS;  // words of 8 per thread and step
     static_assert(WV * THREADS == TN * GG_TK / 8 && XV * THREADS == TM * GG_TK / 8, "whole words per thread");
     __shared__ __align__(16) float xs[GG_TK][TM + 4], ws[GG_TK][TN + 4];
-    const int tid = threadIdx.x, n0 = blockIdx.x * TN, m0 = blockIdx.y * TM;
+    const int tid = threadIdx.x, n0 = blockIdx.x * TN;
     const int words = a.K >> 3, steps = (words + GG_TK / 8 - 1) / (GG_TK / 8);
     const int tx = tid % (TN / 4), ty = tid / (TN / 4);
-    float wr[WV][8], xr[XV][8];
-    // a thread fetches word `i % 4` of row `i / 4`; what lies outside is zero
-    auto fetch = [&](int step) {
+    for (int m0 = blockIdx.y * TM; m0 < M; m0 += gridDim.y * TM) {  // once, but for more tokens than a grid has rows of tiles
+        float wr[WV][8], xr[XV][8];
+        // a thread fetches word `i % 4` of row `i / 4`; what lies outside is zero
+        auto fetch = [&](int step) {
 #pragma unroll
-        for (int u = 0; u < WV; ++u) {
-            const int i = tid + u * THREADS, word = step * (GG_TK / 8) + i % (GG_TK / 8), n = n0 + i / (GG_TK / 8);
-            if (word < words && n < a.N) dequant_word<FMT>(a, n, word, wr[u]);
-            else
+            for (int u = 0; u < WV; ++u) {
+                const int i = tid + u * THREADS, word = step * (GG_TK / 8) + i % (GG_TK / 8), n = n0 + i / (GG_TK / 8);
+                if (word < words && n < a.N) dequant_word<FMT>(a, n, word, wr[u]);
+                else
 #pragma unroll
-                for (int j = 0; j < 8; ++j) wr[u][j] = 0.f;
-        }
+                    for (int j = 0; j < 8; ++j) wr[u][j] = 0.f;
+            }
 #pragma unroll
-        for (int u = 0; u < XV; ++u) {
-            const int i = tid + u * THREADS, word = step * (GG_TK / 8) + i % (GG_TK / 8), m = m0 + i / (GG_TK / 8);
-            if (word < words && m < M) Vec8<T>::load(x + (size_t)m * a.K + (size_t)word * 8, xr[u]);
-            else
+            for (int u = 0; u < XV; ++u) {
+                const int i = tid + u * THREADS, word = step * (GG_TK / 8) + i % (GG_TK / 8), m = m0 + i / (GG_TK / 8);
+                if (word < words && m < M) Vec8<T>::load(x + (size_t)m * a.K + (size_t)word * 8, xr[u]);
+                else
 #pragma unroll
-                for (int j = 0; j < 8; ++j) xr[u][j] = 0.f;
-        }
-    };
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-    fetch(0);
-    for (int step = 0; step < steps; ++step) {
-#pragma unroll
-        for (int u = 0; u < WV; ++u)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) ws[((tid + u * THREADS) % (GG_TK / 8)) * 8 + j][(tid + u * THREADS) / (GG_TK / 8)] = wr[u][j];
-#pragma unroll
-        for (int u = 0; u < XV; ++u)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) xs[((tid + u * THREADS) % (GG_TK / 8)) * 8 + j][(tid + u * THREADS) / (GG_TK / 8)] = xr[u][j];
-        __syncthreads();
-        if (step + 1 < steps) fetch(step + 1);
-        float part[4][4];
+                    for (int j = 0; j < 8; ++j) xr[u][j] = 0.f;
+            }
+        };
+        float acc[4][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) part[i][j] = 0.f;
+            for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+        fetch(0);
+        for (int step = 0; step < steps; ++step) {
 #pragma unroll
-        for (int k = 0; k < GG_TK; ++k) {
-            const float4 xv = *reinterpret_cast<const float4 *>(&xs[k][ty * 4]), wv = *reinterpret_cast<const float4 *>(&ws[k][tx * 4]);
-            const float xa[4] = {xv.x, xv.y, xv.z, xv.w}, wa[4] = {wv.x, wv.y, wv.z, wv.w};
+            for (int u = 0; u < WV; ++u)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) ws[((tid + u * THREADS) % (GG_TK / 8)) * 8 + j][(tid + u * THREADS) / (GG_TK / 8)] = wr[u][j];
+#pragma unroll
+            for (int u = 0; u < XV; ++u)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) xs[((tid + u * THREADS) % (GG_TK / 8)) * 8 + j][(tid + u * THREADS) / (GG_TK / 8)] = xr[u][j];
+            __syncthreads();
+            if (step + 1 < steps) fetch(step + 1);
+            float part[4][4];
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) part[i][j] = fmaf(xa[i], wa[j], part[i][j]);
+                for (int j = 0; j < 4; ++j) part[i][j] = 0.f;
+#pragma unroll
+            for (int k = 0; k < GG_TK; ++k) {
+                const float4 xv = *reinterpret_cast<const float4 *>(&xs[k][ty * 4]), wv = *reinterpret_cast<const float4 *>(&ws[k][tx * 4]);
+                const float xa[4] = {xv.x, xv.y, xv.z, xv.w}, wa[4] = {wv.x, wv.y, wv.z, wv.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) part[i][j] = fmaf(xa[i], wa[j], part[i][j]);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j];
+            __syncthreads();
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j];
-        __syncthreads();
+            for (int j = 0; j < 4; ++j) {
+                const int m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
+                if (m < M && n < a.N) y[(size_t)m * a.N + n] = from_f32<T>(acc[i][j]);
+            }
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
-            if (m < M && n < a.N) y[(size_t)m * a.N + n] = from_f32<T>(acc[i][j]);
-        }
 }
 
 }  // namespace ab2

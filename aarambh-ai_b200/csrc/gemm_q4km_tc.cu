@@ -72,23 +72,24 @@ struct QbArgs {
 // A warp per (token, block): the block's sum and its activations in the order of the unpacked codes.
 __global__ void __launch_bounds__(256) q4km_prepare_kernel(const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__restrict__ xp, float *__restrict__ xsum,
                                                            int M, int Mp, int K) {
-    const int b = blockIdx.x, t = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int b = blockIdx.x, lane = threadIdx.x & 31;
     pdl_wait();
     pdl_launch_dependents();
-    if (t >= Mp) return;
-    float sum = 0.f;
-    if (t < M) {
-        const size_t at = (size_t)t * K + b * 256 + lane * 8;
-        const uint4 v = *reinterpret_cast<const uint4 *>(x + at);
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    for (int t = blockIdx.y * 8 + (threadIdx.x >> 5); t < Mp; t += gridDim.y * 8) {
+        float sum = 0.f;
+        if (t < M) {
+            const size_t at = (size_t)t * K + b * 256 + lane * 8;
+            const uint4 v = *reinterpret_cast<const uint4 *>(x + at);
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) sum += __uint_as_float(w[j] << 16) + __uint_as_float(w[j] & 0xffff0000u);
-        *reinterpret_cast<uint4 *>(xp + at) = make_uint4(__byte_perm(v.x, v.z, 0x5410), __byte_perm(v.x, v.z, 0x7632),
-                                                         __byte_perm(v.y, v.w, 0x5410), __byte_perm(v.y, v.w, 0x7632));
+            for (int j = 0; j < 4; ++j) sum += __uint_as_float(w[j] << 16) + __uint_as_float(w[j] & 0xffff0000u);
+            *reinterpret_cast<uint4 *>(xp + at) = make_uint4(__byte_perm(v.x, v.z, 0x5410), __byte_perm(v.x, v.z, 0x7632),
+                                                             __byte_perm(v.y, v.w, 0x5410), __byte_perm(v.y, v.w, 0x7632));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0) xsum[(size_t)b * Mp + t] = sum;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (lane == 0) xsum[(size_t)b * Mp + t] = sum;
 }
 
 template <int NTOK>
@@ -359,7 +360,7 @@ int launch_qb(const ab2_qweight *w, const void *x, int M, void *y, cudaStream_t 
     rc = make_x_map(&xmap, xp, M, K, NTOK);
     if (rc == AB2_OK) rc = make_bytes_map(&wmap, w->codes, N, K / 2);
     if (rc != AB2_OK) return rc;
-    launch_kernel(q4km_prepare_kernel, dim3(KB, (Mp + 7) / 8), dim3(256), 0, s, (const __nv_bfloat16 *)x, xp, xsum, M, Mp, K);  // checked with the next
+    launch_kernel(q4km_prepare_kernel, dim3(KB, std::min((Mp + 7) / 8, 65535)), dim3(256), 0, s, (const __nv_bfloat16 *)x, xp, xsum, M, Mp, K);  // checked with the next
     const QbArgs a = {w->block_params, xsum, (__nv_bfloat16 *)y, part, N, KB, M, Mp, ksplit};
     cudaError_t e = launch_kernel(gemm_q4km_tc_kernel<NTOK>, dim3(std::min(tiles * ksplit, sms)), dim3(QB_THREADS), smem, s, wmap, xmap, a, status);
     if (e != cudaSuccess) return fail(AB2_ERR_CUDA, "Q4_K_M GEMM launch failed: %s", cudaGetErrorString(e));

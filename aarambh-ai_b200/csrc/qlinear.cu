@@ -35,9 +35,9 @@ static int launch_generic(const ab2_qweight *w, const T *x, int M, T *y, cudaStr
     if (M > 8) {
         // 64 x 64 outputs where that gives at least a tile per SM, else 32 x 32
         if (((size_t)(w->N + 63) / 64) * ((M + 63) / 64) >= (size_t)device_sm_count())
-            gemm_generic_kernel<FMT, T, 64, 64><<<dim3((w->N + 63) / 64, (M + 63) / 64), 256, 0, s>>>(a, x, y, M);
+            gemm_generic_kernel<FMT, T, 64, 64><<<dim3((w->N + 63) / 64, std::min((M + 63) / 64, 65535)), 256, 0, s>>>(a, x, y, M);
         else
-            gemm_generic_kernel<FMT, T, 32, 32><<<dim3((w->N + 31) / 32, (M + 31) / 32), 64, 0, s>>>(a, x, y, M);
+            gemm_generic_kernel<FMT, T, 32, 32><<<dim3((w->N + 31) / 32, std::min((M + 31) / 32, 65535)), 64, 0, s>>>(a, x, y, M);
         AB2_LAUNCH_CHECK();
         return AB2_OK;
     }

@@ -122,3 +122,14 @@ def test_q4km_codes_cancel_exactly(M):
     assert torch.equal(lin.dequantise(), w)
     x = torch.full((M, 512), 251.0, dtype=torch.bfloat16, device="cuda")
     assert bool((lin(x) == 0).all())
+
+
+# more tokens than a grid has rows of tiles (65535): blocks of 8 tokens of the Q4_K_M preparation, tiles of 64 of the CUDA-core GEMM
+@pytest.mark.parametrize("method,dtype,K,M", [("q4_k_m", torch.bfloat16, 256, 8 * 65535 + 37), ("int8_channel", torch.float32, 8, 64 * 65535 + 100)])
+def test_more_tokens_than_rows_of_a_grid(method, dtype, K, M):
+    g = torch.Generator(device="cuda").manual_seed(1)
+    lin = pkg().QuantLinear.quantise(torch.randn((8, K), generator=g, device="cuda"), method, 128)
+    x = torch.randn((M, K), generator=g, device="cuda").to(dtype)
+    y = lin(x)
+    for part in (slice(0, 200), slice(M - 300, M)):
+        check(lambda _: y[part], x[part], 16 * (512 + K // 256), lin)
