@@ -112,16 +112,19 @@ def test_output_off_a_16_byte_boundary(method, N, K, M):
 
 @pytest.mark.parametrize("M", [9, 40, 130])
 def test_q4km_codes_cancel_exactly(M):
-    """Weights scale * (code - 8) that sum to 0 in every block, and equal activations: the part with the minimum and the part with the
-    codes, each some thousand times larger than a weight's, have nothing to cancel, and the output is 0 to the last bit."""
-    scale = float(torch.tensor(0.0123, dtype=torch.float16))
-    codes = torch.tensor([-8, 7, 1] + [c for k in range(1, 8) for c in (k, -k)] * 18 + [0])
-    assert codes.numel() == 256 and int(codes.sum()) == 0
+    """Weights scale * (code - 8) whose products with the activations, small integers, sum to 0 in every block: the part with the minimum and the
+    part with the codes have nothing to cancel, and the output is 0 to the last bit.  (scale * sum of codes is 27 bits long.)"""
+    scale = 2047 / 2 ** 17  # all 11 bits of an f16
+    groups = [(-8, 7, 1)] + [(k, -k) for k in range(1, 8)] * 18 + [(0,)]
+    codes = torch.tensor([c for group in groups for c in group])
+    assert codes.numel() == 256
     w = (codes.repeat(128, 2) * scale).cuda()
     lin = pkg().QuantLinear.quantise(w, "q4_k_m")
     assert torch.equal(lin.dequantise(), w)
-    x = torch.full((M, 512), 251.0, dtype=torch.bfloat16, device="cuda")
-    assert bool((lin(x) == 0).all())
+    each = torch.randint(1, 256, (M, 2, len(groups)), generator=torch.Generator().manual_seed(M))
+    x = each.repeat_interleave(torch.tensor([len(group) for group in groups]), -1).reshape(M, 512)
+    assert bool((x.view(M, 2, 256) * codes).sum(-1).eq(0).all())
+    assert bool((lin(x.to(torch.bfloat16).cuda()) == 0).all())
 
 
 # more tokens than a grid has rows of tiles (65535): blocks of 8 tokens of the Q4_K_M preparation, tiles of 64 of the CUDA-core GEMM
