@@ -346,7 +346,7 @@ int qlinear_w4a16_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaSt
     // Measured: rounds of 19.7 / 22.3 / 27.1 us of tiles of 128 / 192 / 256 tokens over K = 4096 (28672 channels, 2048 tokens),
     // 68 / 73 / 85 over K = 14336; a tile of 32 takes what one of 128 does but for its stores.  Splitting K (few tiles:
     // 512 tokens on the 4096 x 14336 weight are 64 of 256) needs rows that the reduce pass can store in 16-byte
-    // pieces and a workspace that a recorded launch has not.
+    // pieces and a workspace; a recorded launch, in whose graph that would be memory nodes, goes without.
     static const GemmTileCost costs[] = {{32, 0.5, 0.58}, {128, 1.0, 0.605}, {192, 2.2, 0.63}, {256, 4.0, 0.72}};
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     const bool recorded = cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;

@@ -5,7 +5,7 @@
 // A decoder of width 384 is bound by launches: its weights stream in less time than a launch takes.  A CTA is four
 // warps, a row (or a gate row and its up row) each; the warp requests its first words of the weight before the
 // dependency wait, and every CTA norms the tokens for itself.  One step of the 6-layer f32 decoder, with chained launches:
-// 171 us in 65 launches before, 90 us in 35.
+// 171 us in 65 launches before, 90 us in 33.
 #pragma once
 
 #include "gemv_generic.cuh"

@@ -61,7 +61,7 @@ constexpr int DG_WSLOT_BYTES = 2 * W4_BLOCK_WORDS * 4;  // per ring; four rings 
 constexpr int DG_A_COLS = 32;          // tensor-memory columns of 64 K-elements: two bf16 per column, a lane per channel
 constexpr int DG_MMA_WARPS = 2;        // MMA-issue warps, taking alternate units (warp 1 and the warps after the epilogue)
 constexpr int DG_THREADS = 448 + 32 * (DG_MMA_WARPS - 1) + 32;  // the last warp fetches the packed weights
-constexpr int DG_ACC = 4;             // accumulator pairs (D, S) in tensor memory
+constexpr int DG_ACC = 4;             // accumulators in tensor memory
 // An MMA-issue warp must see every phase of the barriers it waits on (a parity wait cannot tell
 // phase k from phase k + 2), so the stages, activation stages and accumulators a unit uses must come
 // back to the same warp: their counts are multiples of what DG_MMA_WARPS units use.

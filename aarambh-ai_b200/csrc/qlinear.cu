@@ -431,8 +431,8 @@ int qlinear_i8_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaStrea
 int qlinear_dispatch(const ab2_qweight *w, const void *x, int M, ab2_dtype dtype, void *y, cudaStream_t s) {
     if (w->fmt == FMT_BF16) return linear_bf16(w, x, M, dtype, y, LIN_STORE, 0, s);
     if (qlinear_w4a16_mma_eligible(w, dtype)) {
-        // Up to 64 tokens: the HBM-bound decode kernels (one token, 2..8 tokens, chunks of 9..32
-        // tokens).  The tcgen05 GEMM tiles 128 output channels per CTA, which leaves most SMs
+        // Up to 64 tokens: the HBM-bound decode kernels (one token, 2..8, 9..32, 33..64 in one pass).
+        // The tcgen05 GEMM tiles 128 output channels per CTA, which leaves most SMs
         // idle until the token count supplies the parallelism.
         if (M <= 64) return qlinear_w4a16_mma(w, x, M, y, s);
         return qlinear_w4a16_tc(w, x, M, y, s);
