@@ -21,7 +21,7 @@
 // With fewer tiles than SMs the blocks of a tile are divided over several CTAs; their f32 sums meet in a reduce pass.
 // What bounds it is the unpack and the per-block epilogue (about 450 cycles a stage against the MMA's 257 at 128
 // tokens).  14336 x 4096 at 300 tokens: 3329 us on CUDA cores,
-// 76 us here (464 TFLOP/s); 3072 x 2048: 421 -> 20 us, at 9 tokens 17 -> 11.
+// 73 us here (482 TFLOP/s); 3072 x 2048: 421 -> 20 us, at 9 tokens 17 -> 11.
 // Every wait on an mbarrier is bounded; on a time-out the CTA records AB2_ERR_TIMEOUT, walks through the rest
 // of its work, frees its tensor memory and returns.
 #include <cuda.h>
@@ -255,10 +255,11 @@ gemm_q4km_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
             uint32_t next = __ldg(prm + b0);
             for (int b = b0; b < b1; ++b, ++buse) {
                 const int ab = buse & 1;
-                const float s = f16_bits_to_f32((uint16_t)(next & 0xffffu)), m = fmaf(8.f, s, f16_bits_to_f32((uint16_t)(next >> 16)));
+                const uint32_t param = next;
                 if (b + 1 < b1) next = __ldg(prm + b + 1);
                 bar_wait(&sh->xsfull[ab], (buse >> 1) & 1, failed);
                 warp_wait(&sh->accfull[ab], (buse >> 1) & 1, failed);
+                const float s = f16_bits_to_f32((uint16_t)(param & 0xffffu)), m = fmaf(8.f, s, f16_bits_to_f32((uint16_t)(param >> 16)));
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 const float *xs = sh->xsum[ab] + half * COLS;
                 const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(ab * NTOK + half * COLS);
