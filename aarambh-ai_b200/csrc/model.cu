@@ -285,14 +285,14 @@ static int forward_launches(ab2_model *m, ab2_kv *kv, const uint32_t *ids, int S
                 STEP(launch_add(m->x, m->proj, m->x, nd, m->dtype, s));
             }
         } else if (m->fused_epilogues && T > 16) {
-            // many tokens: tensor-core GEMMs, then the element-wise steps as their own launches (from 17
-            // tokens on this measured faster than the residual / SwiGLU epilogues of the decode GEMM:
-            // 6330 against 6120 tok/s at 32 rows, 7360 against 6740 at 64; with the strip kernel on the
-            // gate|up weight, 7980 against 7850 at 32 rows)
+            // many tokens: the residual addition goes with the norm that follows it (8 layers of 32 rows: 811 us a step, 815 with
+            // additions in the GEMMs' epilogues), SwiGLU with the decode GEMM up to its 64 tokens (811 -> 805 us)
             STEP(qlinear_dispatch(L.part[3], attn, T, m->dtype, m->proj, s));
             STEP(launch_add_rms_norm(x, m->proj, L.norm2, m->xn, T, d, c.rms_eps, m->dtype, s));
-            STEP(qlinear_dispatch(L.wgu, m->xn, T, m->dtype, m->gu, s));
-            {
+            if (T <= 64) {
+                STEP(qlinear_w4a16_mma_swiglu(L.wgu, m->xn, T, m->hid, s));
+            } else {
+                STEP(qlinear_dispatch(L.wgu, m->xn, T, m->dtype, m->gu, s));
                 size_t n8 = (size_t)T * (c.ffn_hidden / 8);
                 cudaError_t e = launch_kernel(swiglu_interleaved8_kernel, dim3((unsigned)ceil_div(n8, 256)), dim3(256), 0, s,
                                               (const __nv_bfloat16 *)m->gu, (__nv_bfloat16 *)m->hid, (int)c.ffn_hidden, n8);

@@ -10,7 +10,6 @@
 #include "gemv_w4a16_mma.cuh"
 #include "gemv_w4a16_warp.cuh"
 #include "gemv_w4a16_m1.cuh"
-#include "gemv_w4a16_strip.cuh"
 #include "linear_bf16.cuh"
 
 using namespace ab2;
@@ -156,9 +155,9 @@ static int gemv_scratch_for(cudaStream_t s, GemvScratch *out) {
                         "on the stream before capturing (its scratch buffers are allocated then)");
         GemvScratch sc;
         sc.max_ctas = device_sm_count() * 3;
-        // two partial tiles per warp of the warp kernels, or per CTA of the strip kernel and the decode GEMM, one CTA per SM
+        // two partial tiles per warp of the warp kernels, or per CTA of the decode GEMM, one CTA per SM
         const size_t pbytes = std::max((size_t)sc.max_ctas * W4W_WARPS * 2 * W4W_SLOT_FLOATS,
-                                       (size_t)device_sm_count() * 2 * std::max(W4S_MAX_SLOT_FLOATS, W4DG_MAX_SLOT_FLOATS)) * sizeof(float);
+                                       (size_t)device_sm_count() * 2 * W4DG_MAX_SLOT_FLOATS) * sizeof(float);
         AB2_CUDA(cudaMalloc((void **)&sc.partials, pbytes));
         AB2_CUDA(cudaMalloc((void **)&sc.counters, W4W_MAX_TILES * sizeof(int)));
         AB2_CUDA(cudaMemset(sc.counters, 0, W4W_MAX_TILES * sizeof(int)));
@@ -221,29 +220,6 @@ static cudaError_t launch_w4a16_m1(const ab2_qweight *w, const __nv_bfloat16 *x,
     return launch_w4a16_m1_inst<EPI, 2, 8, false>(w, x, norm_w, eps, y, resid, grid, sc, status, s);
 }
 
-// 9..32 tokens: the register-tiled strip kernel (gemv_w4a16_strip.cuh), one CTA per SM.
-template <class S, int EPI>
-static cudaError_t launch_w4a16_strip(const ab2_qweight *w, const __nv_bfloat16 *x, int M, __nv_bfloat16 *y,
-                                      const __nv_bfloat16 *resid, const GemvScratch &sc, int *status,
-                                      cudaStream_t s) {
-    static_assert(S::SLOT_FLOATS <= W4S_MAX_SLOT_FLOATS, "the scratch holds two partial tile sets per CTA");
-    static_assert(S::SMEM <= 227 * 1024, "shared memory of a CTA");
-    static bool configured[64] = {false};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(gemv_w4a16_strip_kernel<S, EPI>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
-        if (e != cudaSuccess) return e;
-        configured[dev] = true;
-    }
-    const int tiles = (w->N + 15) / 16, sets = (tiles + S::WS * S::RT - 1) / (S::WS * S::RT);
-    const long long total = (long long)sets * (w->K / 128);
-    const int grid = (int)std::min<long long>(device_sm_count(), total);
-    return launch_kernel(gemv_w4a16_strip_kernel<S, EPI>, dim3(grid), dim3(S::WARPS * 32), S::SMEM, s,
-                         (const uint32_t *)w->codes, x, y, resid, w->N, w->K, M, sc.partials, sc.counters, status);
-}
-
 constexpr int W4M1_MAX_K = 16384;
 constexpr int W4M1_PLAIN_MAX_K = 8192;
 
@@ -283,58 +259,17 @@ static int launch_w4a16_stream(const ab2_qweight *w, const void *x, int M, void 
     if (!align_off && G % W4W_WARPS == 0 && G / W4W_WARPS >= 4 && tiles <= sc.max_ctas && tiles * 10 >= device_sm_count() * 17) grid = tiles;
     const uint32_t *wt = (const uint32_t *)w->codes;
     const int out_n = EPI == W4_EPI_SWIGLU ? w->N / 2 : w->N;
-    // More than 8 tokens go in chunks of up to 32, from 33 to 64 in one:
-    //   9..24 tokens (and 25..32 on a weight of 24576 rows or more): the strip kernel - a warp multiplies
-    //     64 or 32 rows by all tokens, so the activations it loads serve several weight blocks and the
-    //     codes are unpacked once for every token.  On the largest shape it takes 96 / 113 / 150 us for
-    //     16 / 24 / 32 tokens; the warp kernel needs 155 us per 16 tokens.
-    //   25..32 tokens on narrower weights: the tensor-memory decode GEMM, whose pass costs the same
-    //     whatever the token count (170 us on the largest shape, 15 / 26 / 27 us on 4096 x 4096,
-    //     4096 x 14336, 14336 x 4096 against the strip kernel's 17 / 29 / 30 us).
-    static const bool strip_off = getenv("AB2_GEMV_NO_STRIP") != nullptr;
-    static const int strip_wide_n = getenv("AB2_STRIP_WIDE_N") ? atoi(getenv("AB2_STRIP_WIDE_N")) : 24576;
+    // From 9 tokens on the tensor-memory decode GEMM, up to 64 in a pass: 9 / 16 / 32 / 64 tokens take 23 / 23 / 24.5 / 28 us on
+    // 4096 x 28672 and 9 / 9 / 10 / 11 on 4096 x 4096 (28 / 29 / 42 / 47 and 12 / 12 / 14 / 20 with warp-level MMAs and the form
+    // of it before).  At 2 to 8 tokens the warp kernel is as fast or faster (2 tokens 20.8, 7.8 us; 8 tokens 25.2, 8.6).
     if constexpr (EPI != W4_EPI_F32_PEER) {
         if (M >= 9 && !norm_w) {
-            const bool tc_ok = w->N % 16 == 0;
-            // equal chunks, in whole token tiles
-            // 33..64 tokens go through the tensor-memory GEMM in one pass, whose weights are then fetched and unpacked once
-            // (64 tokens: 49 us on 4096 x 28672, 22.6 on 4096 x 6144, 20.6 on 4096 x 4096, 33 on 14336 x 4096, against 86,
-            // 34, 32 and 54 in two passes; 33 tokens 49, 21, 21, 33 against 66, 33, 29, 46)
-            const int most = tc_ok && M > 32 ? 64 : 32;
-            const int nchunks = (M + most - 1) / most, chunk = ((M + nchunks - 1) / nchunks + 7) / 8 * 8;
-            for (int m0 = 0; m0 < M; m0 += chunk) {
-                const int mv = std::min(chunk, M - m0);
-                const __nv_bfloat16 *xp = (const __nv_bfloat16 *)x + (size_t)m0 * w->K;
-                __nv_bfloat16 *yp = EPI == W4_EPI_F32 ? (__nv_bfloat16 *)((float *)y + (size_t)m0 * out_n)
-                                                      : (__nv_bfloat16 *)y + (size_t)m0 * out_n;
-                const __nv_bfloat16 *rp = resid ? (const __nv_bfloat16 *)resid + (size_t)m0 * out_n : nullptr;
-                if (!strip_off && mv >= 9 && mv <= 32 && (mv <= 24 || w->N >= strip_wide_n || !tc_ok)) {
-                    cudaError_t e;
-                    // token tiles, tiles per strip, strips x K slices of a CTA
-                    switch ((mv + 7) / 8) {
-                    case 2: e = launch_w4a16_strip<W4sShape<2, 2, 8, 2>, EPI>(w, xp, mv, yp, rp, sc, status, s); break;
-                    case 3: e = launch_w4a16_strip<W4sShape<3, 4, 4, 2>, EPI>(w, xp, mv, yp, rp, sc, status, s); break;
-                    default: e = launch_w4a16_strip<W4sShape<4, 4, 4, 2>, EPI>(w, xp, mv, yp, rp, sc, status, s); break;
-                    }
-                    if (e != cudaSuccess) return fail(AB2_ERR_CUDA, "GEMV launch failed: %s", cudaGetErrorString(e));
-                } else if (tc_ok && mv >= 17) {
-                    rc = qlinear_w4a16_tc_decode(w, xp, mv, yp, rp, EPI, sc.partials, sc.counters, sc.max_ctas, s);
-                    if (rc != AB2_OK) return rc;
-                } else {
-                    for (int m1 = 0; m1 < mv; m1 += 16) {
-                        const int mw = std::min(16, mv - m1);
-                        const __nv_bfloat16 *xq = xp + (size_t)m1 * w->K;
-                        __nv_bfloat16 *yq = EPI == W4_EPI_F32 ? (__nv_bfloat16 *)((float *)yp + (size_t)m1 * out_n)
-                                                              : yp + (size_t)m1 * out_n;
-                        const __nv_bfloat16 *rq = rp ? rp + (size_t)m1 * out_n : nullptr;
-                        cudaError_t e =
-                            mw > 8 ? launch_kernel(gemv_w4a16_warp_kernel<2, EPI>, dim3(grid), dim3(256), 0, s, wt, xq, yq,
-                                                   rq, w->N, w->K, mw, sc.partials, sc.counters, status)
-                                   : launch_kernel(gemv_w4a16_warp_kernel<1, EPI>, dim3(grid), dim3(256), 0, s, wt, xq, yq,
-                                                   rq, w->N, w->K, mw, sc.partials, sc.counters, status);
-                        if (e != cudaSuccess) return fail(AB2_ERR_CUDA, "GEMV launch failed: %s", cudaGetErrorString(e));
-                    }
-                }
+            for (int m0 = 0; m0 < M; m0 += W4DG_MAX_TOKENS) {
+                const size_t in = (size_t)m0 * w->K, out = (size_t)m0 * out_n;
+                void *yp = EPI == W4_EPI_F32 ? (void *)((float *)y + out) : (void *)((__nv_bfloat16 *)y + out);
+                rc = qlinear_w4a16_tc_decode(w, (const __nv_bfloat16 *)x + in, std::min(W4DG_MAX_TOKENS, M - m0), yp,
+                                             resid ? (const __nv_bfloat16 *)resid + out : nullptr, EPI, sc.partials, sc.counters, sc.max_ctas, s);
+                if (rc != AB2_OK) return rc;
             }
             AB2_LAUNCH_CHECK();
             return AB2_OK;
@@ -431,7 +366,7 @@ int qlinear_i8_tc(const ab2_qweight *w, const void *x, int M, void *y, cudaStrea
 int qlinear_dispatch(const ab2_qweight *w, const void *x, int M, ab2_dtype dtype, void *y, cudaStream_t s) {
     if (w->fmt == FMT_BF16) return linear_bf16(w, x, M, dtype, y, LIN_STORE, 0, s);
     if (qlinear_w4a16_mma_eligible(w, dtype)) {
-        // Up to 64 tokens: the HBM-bound decode kernels (one token, 2..8, 9..32, 33..64 in one pass).
+        // Up to 64 tokens: the HBM-bound decode kernels (one token, 2..8, 9..64 in one pass).
         // The tcgen05 GEMM tiles 128 output channels per CTA, which leaves most SMs
         // idle until the token count supplies the parallelism.
         if (M <= 64) return qlinear_w4a16_mma(w, x, M, y, s);

@@ -75,6 +75,12 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
         "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n" ::
             "r"(sptr(dst)), "l"(map), "r"(sptr(bar)), "r"(x), "r"(y), "r"(z) : "memory");
 }
+// 4-D tile load: coordinates from the innermost on.
+__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, int x, int y, int z, int w, uint64_t *bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];\n" ::
+            "r"(sptr(dst)), "l"(map), "r"(sptr(bar)), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
 
 // Shared-memory matrix descriptor, K-major, 128-byte swizzle: 8-row groups are
 // 1024 bytes apart, the start address advances by 32 bytes per K = 16 step.
