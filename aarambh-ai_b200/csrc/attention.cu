@@ -265,20 +265,13 @@ static int launch_split_hd(const AttnArgs &a, dim3 grid, cudaStream_t s) {
 
 int device_sm_count();
 
-// Whether decode queries over this cache take the tensor-core flash-decode (attention_mma.cu).
-static bool decode_on_mma(const ab2_kv *kv) {
-    return kv->dtype == AB2_KV_INT8 && kv->hd == 128 && kv->h / kv->kvh <= 8;
-}
-
 // Context splits of a decode launch over `nrows` sequences of at most `max_len` tokens: enough
 // CTAs to fill the GPU a few times over, never a split shorter than a useful run of tokens.
 // One rule for every entry point, so that they return the same bits.
 static int decode_split_count(const ab2_kv *kv, int nrows, int max_len, int max_splits, bool mma) {
     const int sms = device_sm_count(), units = nrows * kv->kvh;
     if (mma) {
-        // short contexts with at least one (row, KV head) per SM: one CTA each and no merge launch
-        // (32 rows x 512 tokens: 4.35 ms per decode step against 4.62 with four splits)
-        if (units >= sms && max_len <= 1024) return 1;
+        // the most splits that a row may take; the launch deals them out by the rows' lengths (attention_mma.cu)
         const int want = (sms * 6 + units - 1) / units;
         return std::max(1, std::min(std::min(want, (max_len + 63) / 64), max_splits));
     }
@@ -298,18 +291,10 @@ int attention_cached_device(const ab2_kv *kv, int layer, const void *q, void *ou
     if (max_len <= 0)
         for (int i = 0; i < nrows; ++i) max_len = std::max(max_len, kv->lens_host[kv_row_host(kv, row0, i)] + pending);
     int nsplit = 1;
-    if (S == 1 && decode_on_mma(kv) && st.q_h == kv->hd && st.o_h == st.q_h && st.o_b == (long long)kv->h * kv->hd) {
-        // INT8 cache, head_dim 128: tensor-core flash-decode (attention_mma.cu)
+    if (S == 1 && attention_decode_mma_serves(kv, dtype) && st.q_h == kv->hd && st.o_h == st.q_h && st.o_b == (long long)kv->h * kv->hd) {
+        // INT8 or bf16 cache, head_dim 128: tensor-core flash-decode (attention_mma.cu)
         nsplit = decode_split_count(kv, nrows, max_len, kv->max_splits, true);
-        a.nsplit = nsplit;
-        int rc = attention_decode_mma_device(kv, layer, q, out, row0, nrows, scale, dtype, nsplit, kv->part_acc,
-                                             kv->part_ml, pending, st.q_b, s);
-        if (rc != AB2_OK) return rc;
-        if (nsplit > 1) {
-            cudaError_t e = launch_kernel(attn_merge_kernel, dim3(kv->h, nrows), dim3(kv->hd), 0, s, a, (int)kv->hd);
-            if (e != cudaSuccess) return fail(AB2_ERR_CUDA, "attention merge launch failed: %s", cudaGetErrorString(e));
-        }
-        return AB2_OK;
+        return attention_decode_mma_device(kv, layer, q, out, row0, nrows, scale, dtype, nsplit, kv->part_acc, kv->part_ml, pending, st.q_b, s);
     }
     if (S > 1) {
         // prefill chunk of a bf16 model: the tcgen05 kernel (attention_prompt_tc.cu) where it is the faster one; few queries, short
@@ -451,7 +436,7 @@ AB2_API int ab2_attention_decode_static(const ab2_kv *kv, int layer, const void 
     for (int r = row0; r < row0 + nrows; ++r) max_len = std::max(max_len, kv->lens_host[r]);
     // Kernel choice and split count come from the helpers ab2_attention_decode uses (with the
     // cache's own split limit), so both entry points return the same bits.
-    const bool mma_path = decode_on_mma(kv);
+    const bool mma_path = attention_decode_mma_serves(kv, dtype);
     a.nsplit = decode_split_count(kv, nrows, max_len, kv->max_splits, mma_path);
     // Partials are indexed by the absolute row, exactly as in the allocated scratch.
     const size_t parts = (size_t)(row0 + nrows) * kv->h * a.nsplit;
@@ -464,14 +449,9 @@ AB2_API int ab2_attention_decode_static(const ab2_kv *kv, int layer, const void 
     a.part_ml = g_static_attn_scratch_ptr[dev] + parts * kv->hd;
     cudaStream_t s = (cudaStream_t)stream;
     dim3 grid(a.nsplit, kv->kvh, nrows);
-    if (mma_path) {
-        rc = attention_decode_mma_device(kv, layer, q_dev, out_dev, row0, nrows, scale, dtype, a.nsplit, a.part_acc,
-                                         a.part_ml, 0, (long long)kv->h * kv->hd, s);
-        if (rc != AB2_OK) return rc;
-        if (a.nsplit > 1) attn_merge_kernel<<<dim3(kv->h, nrows), kv->hd, 0, s>>>(a, kv->hd);
-        AB2_LAUNCH_CHECK();
-        return AB2_OK;
-    }
+    if (mma_path)
+        return attention_decode_mma_device(kv, layer, q_dev, out_dev, row0, nrows, scale, dtype, a.nsplit, a.part_acc,
+                                           a.part_ml, 0, (long long)kv->h * kv->hd, s);
     if (kv->dtype == AB2_KV_F32) rc = launch_split_hd<AB2_KV_F32>(a, grid, s);
     else if (kv->dtype == AB2_KV_BF16) rc = launch_split_hd<AB2_KV_BF16>(a, grid, s);
     else rc = launch_split_hd<AB2_KV_INT8>(a, grid, s);

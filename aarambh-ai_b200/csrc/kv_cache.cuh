@@ -108,10 +108,11 @@ int attention_cached_device(const ab2_kv *kv, int layer, const void *q, void *ou
                             int row0, int nrows, float scale, ab2_dtype dtype, AttnStrides st,
                             int len_hint, cudaStream_t s);
 
-// Tensor-core INT8 flash-decode (head_dim 128): query head (row, head) sits at
+// Tensor-core flash-decode over INT8 or bf16 caches (head_dim 128): query head (row, head) sits at
 // row * q_stride + head * 128, out is [nrows][h][128]; `pending` appended but
 // uncommitted tokens per row are attended too; partials go to the given split
-// scratch, merged by the caller when nsplit > 1.
+// scratch and are merged by the same launch (kv's arrival counters).
+bool attention_decode_mma_serves(const ab2_kv *kv, ab2_dtype dtype);
 int attention_decode_mma_device(const ab2_kv *kv, int layer, const void *q, void *out, int row0, int nrows,
                                 float scale, ab2_dtype dtype, int nsplit, float *part_acc, float *part_ml,
                                 int pending, long long q_stride, cudaStream_t s);

@@ -133,14 +133,18 @@ __global__ void reorder_shards_kernel(const T *in, T *out, int rows, int vn, int
     out[i] = in[((size_t)r * rows + b) * vn + j];
 }
 
-// Decode attention as rotation + append + tensor-core flash-decode (+ merge) instead of the
-// one-launch CUDA-core kernels.  The one-launch kernels win while the launch count is what
-// matters; they are bound by the int8 -> float conversion once a step reads many cached tokens.
-static bool decode_attention_on_tensor_cores(const ab2_kv *kv, int nrows, int max_len) {
-    if (kv->dtype != AB2_KV_INT8 || kv->hd != 128 || kv->h / kv->kvh > 8) return false;
+// Decode attention as rotation + append + tensor-core flash-decode instead of the one-launch kernels on CUDA cores.  Those win
+// while the launch is what matters; they are bound by the conversions to f32 once a step reads many cached tokens, over bf16
+// caches sooner (their kernel there reads rows uncoalesced).  Steps of two 4096-wide layers, us, one launch / two: INT8 1 x 512
+// 147 / 154, 1 x 2048 165 / 158, 4 x 256 186 / 193, 2 x 512 190 / 184, 8 x 256 226 / 216, 16 x 64 207 / 207, 32 x 32 264 / 246; bf16
+// 1 x 32 144 / 141, 8 x 64 211 / 216, 2 x 512 189 / 186, 32 x 32 244 / 244, 32 x 700 322 / 269.
+static bool decode_attention_on_tensor_cores(const ab2_kv *kv, ab2_dtype dtype, int nrows, int max_len) {
+    if (!attention_decode_mma_serves(kv, dtype)) return false;
     static const char *force = getenv("AB2_DECODE_ATTN");
     if (force) return strcmp(force, "mma") == 0;
-    return nrows >= 2 ? nrows * (long long)max_len > 1024 : max_len > 6144;
+    const bool bf16 = kv->dtype == AB2_KV_BF16;
+    if (nrows == 1) return bf16 || max_len > 1200;
+    return nrows >= 16 || nrows * (long long)max_len > (bf16 ? 512 : 1024);
 }
 
 #define STEP(expr)                     \
@@ -211,7 +215,7 @@ static int forward_launches(ab2_model *m, ab2_kv *kv, const uint32_t *ids, int S
         int max_len = len_hint;
         if (S == 1 && max_len <= 0)
             for (int i = 0; i < nrows; ++i) max_len = std::max(max_len, kv->lens_host[kv_row_host(kv, row0, i)] + 1);
-        if (S == 1 && !decode_attention_on_tensor_cores(kv, nrows, max_len)) {
+        if (S == 1 && !decode_attention_on_tensor_cores(kv, m->dtype, nrows, max_len)) {
             // decode: RoPE, KV append, attention and split merge in one launch
             if (attention_decode_cluster_eligible(kv, m->dtype, max_len))
                 STEP(attention_decode_cluster_device(kv, l, m->qkv, qkv_stride, m->attn, row0, nrows, scale, m->cos_t,
