@@ -9,11 +9,13 @@
 // completion on an mbarrier per stage): there is no CTA-wide barrier, no shared
 // producer and no cross-warp reduction in shared memory.
 //
-// Arithmetic per block is that of gemv_w4a16_mma.cuh: nibbles become bf16 with
-// one shift and one LOP3 per pair (0x4300 | q == 128 + q exactly) and feed
+// Arithmetic per block: a pair of nibbles masked out of its word is a pair of bf16
+// subnormals (q 2^-133 or, four bits higher, q 2^-129), which one packed fma turns into
+// q / 128 - zero / 128, exactly; masks of two positions share a shift.  They feed
 // mma.sync.m16n8k16 (bf16 x bf16 -> f32) with the 16 weight rows as A and up to
-// 8 tokens as B; the zero point leaves by an exact bf16x2 add on the A registers;
-// the bf16 scale is applied per group in f32.
+// 8 tokens as B; the bf16 scale is applied per group in f32, and 128 at the end.
+// (0x4300 | q == 128 + q takes a shift for each pair but one: 4096 x 14336 13.4 us at
+// one token and 14.1 at two, 12.7 and 13.5 with subnormals; the results are the same.)
 //
 // A tile whose groups all lie inside one warp's range is finished by that warp.
 // A tile cut by a range boundary is finished by whichever of its contributors
@@ -143,6 +145,12 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
     return v;
 }
 
+__device__ __forceinline__ uint32_t bf16x2_fma(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("fma.rn.bf16x2 %0, %1, %2, %3;\n" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+
 // partials: [gridDim.x * 8 warps][2][W4W_SLOT_FLOATS] floats; counters: one int
 // per 16-row tile, zero on entry and on exit.
 //
@@ -193,8 +201,8 @@ gemv_w4a16_warp_kernel(const uint32_t *__restrict__ wt, const __nv_bfloat16 *__r
 
     const uint32_t hidden_zero = (uint32_t)K & 1u;  // K is a multiple of 128
     // Opaque register copies of the two constants of the nibble extraction.
-    uint32_t k_mask = 0x000F000Fu, k_magic = 0x43004300u;
-    asm volatile("" : "+r"(k_mask), "+r"(k_magic));
+    uint32_t k_lo = 0x000F000Fu, k_hi = 0x00F000F0u, up_lo = 0x7E807E80u, up_hi = 0x7C807C80u;  // 2^126, 2^122
+    asm volatile("" : "+r"(k_lo), "+r"(k_hi), "+r"(up_lo), "+r"(up_hi));
 
     const uint32_t code_off = (r * 16 + c * 4) * 4;  // this thread's 4 words of row r in a block
     const uint32_t param_off = (256 + r) * 4;
@@ -236,24 +244,18 @@ gemv_w4a16_warp_kernel(const uint32_t *__restrict__ wt, const __nv_bfloat16 *__r
             }
 
             const float sa = __uint_as_float(pa << 16), sb = __uint_as_float(pb << 16);
-            const uint32_t nza = __byte_perm(pa, pa, 0x3232), nzb = __byte_perm(pb, pb, 0x3232);
+            const uint32_t nza = bf16x2_fma(__byte_perm(pa, pa, 0x3232), 0x3C003C00u, 0x3F803F80u), nzb = bf16x2_fma(__byte_perm(pb, pb, 0x3232), 0x3C003C00u, 0x3F803F80u);
             float d[NT][4], dz[NT][4];
             const uint32_t words_a[4] = {wa.x, wa.y, wa.z, wa.w};
             const uint32_t words_b[4] = {wb.x, wb.y, wb.z, wb.w};
 #pragma unroll
             for (int wi = 0; wi < 4; ++wi) {
                 uint32_t a[8];
-#pragma unroll
-                for (int jj = 0; jj < 4; ++jj) {
-                    a[2 * jj] = w4_pair_bf16(words_a[wi], jj, k_mask, k_magic);
-                    a[2 * jj + 1] = w4_pair_bf16(words_b[wi], jj, k_mask, k_magic);
-                }
-                // the zero point leaves by an exact bf16x2 add: (128 + q) - (128 + z)
-#pragma unroll
-                for (int jj = 0; jj < 4; ++jj) {
-                    a[2 * jj] = bf16x2_add(a[2 * jj], nza);
-                    a[2 * jj + 1] = bf16x2_add(a[2 * jj + 1], nzb);
-                }
+                const uint32_t ua = words_a[wi], ub = words_b[wi], ua8 = ua >> 8, ub8 = ub >> 8;
+                a[0] = bf16x2_fma(ua & k_lo, up_lo, nza); a[1] = bf16x2_fma(ub & k_lo, up_lo, nzb);
+                a[2] = bf16x2_fma(ua & k_hi, up_hi, nza); a[3] = bf16x2_fma(ub & k_hi, up_hi, nzb);
+                a[4] = bf16x2_fma(ua8 & k_lo, up_lo, nza); a[5] = bf16x2_fma(ub8 & k_lo, up_lo, nzb);
+                a[6] = bf16x2_fma(ua8 & k_hi, up_hi, nza); a[7] = bf16x2_fma(ub8 & k_hi, up_hi, nzb);
 #pragma unroll
                 for (int t = 0; t < NT; ++t) {
                     // two independent accumulation chains (even / odd k-steps)
@@ -290,6 +292,10 @@ gemv_w4a16_warp_kernel(const uint32_t *__restrict__ wt, const __nv_bfloat16 *__r
             bar += 8;
             if (cur == ring_end) { cur = ring0; bar = bar0; parity ^= 1; }
         }
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[t][i] *= 128.f;
         b += n;
 
         // ---- end of this warp's share of the tile ---------------------------
