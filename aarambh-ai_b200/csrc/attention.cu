@@ -380,6 +380,7 @@ AB2_API int ab2_attention_decode(const ab2_kv *kv, int layer, const void *q_dev,
                                  int nrows, float scale, ab2_dtype dtype, ab2_stream stream) {
     int rc = check_attention(kv, layer, q_dev, out_dev, 1, row0, nrows, dtype);
     if (rc != AB2_OK) return rc;
+    AB2_FOLLOW(kv, stream);
     AttnStrides st;
     st.q_b = (long long)kv->h * kv->hd; st.q_s = 0; st.q_h = kv->hd;
     st.o_b = st.q_b; st.o_s = 0; st.o_h = kv->hd;
@@ -390,6 +391,7 @@ AB2_API int ab2_attention_cached(const ab2_kv *kv, int layer, const void *q_dev,
                                  int row0, int nrows, float scale, ab2_dtype dtype, ab2_stream stream) {
     int rc = check_attention(kv, layer, q_dev, out_dev, S, row0, nrows, dtype);
     if (rc != AB2_OK) return rc;
+    AB2_FOLLOW(kv, stream);
     AttnStrides st;  // q, out: [nrows][S][h][hd]
     st.q_h = kv->hd; st.q_s = (long long)kv->h * kv->hd; st.q_b = st.q_s * S;
     st.o_h = st.q_h; st.o_s = st.q_s; st.o_b = st.q_b;
@@ -415,6 +417,7 @@ AB2_API int ab2_attention_decode_static(const ab2_kv *kv, int layer, const void 
                                         ab2_stream stream) {
     int rc = check_attention(kv, layer, q_dev, out_dev, 1, row0, nrows, dtype);
     if (rc != AB2_OK) return rc;
+    AB2_FOLLOW(kv, stream);
     AB2_REQUIRE(kv->hd == 64 || kv->hd == 128, AB2_ERR_UNSUPPORTED, "attention supports head_dim 64 and 128, got %d", kv->hd);
     int dev = 0;
     AB2_CUDA(cudaGetDevice(&dev));

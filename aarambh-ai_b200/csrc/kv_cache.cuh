@@ -41,6 +41,10 @@ struct ab2_kv {
     int *high_host;   // [B] most tokens a row has held since it was last empty (which ring slots are intact)
     int *saved_len;   // [B] length ab2_kv_save_row recorded, -1 none
     size_t part_acc_bytes, part_ml_bytes, counter_bytes;
+    // The last truncation on `cut_stream`, for calls on other streams (kv_follow).
+    mutable cudaEvent_t cut_event;
+    mutable cudaStream_t cut_stream;
+    mutable bool cut_pending;
 };
 
 namespace ab2 {
@@ -68,6 +72,14 @@ static inline void kv_advance_host(ab2_kv *kv, int row, int S) {
 }
 
 KvView kv_view(const ab2_kv *kv, int layer);
+
+// Orders what is launched on `s` from here on after the last ab2_kv_truncate, whichever stream that was on.
+int kv_follow(const ab2_kv *kv, cudaStream_t s);
+#define AB2_FOLLOW(kv, stream)                                          \
+    do {                                                                \
+        const int _rc = ab2::kv_follow(kv, (cudaStream_t)(stream));     \
+        if (_rc != AB2_OK) return _rc;                                  \
+    } while (0)
 
 // One layer of a stack as kernels receive it.
 struct KvLayerView {

@@ -683,6 +683,7 @@ AB2_API int ab2_model_forward(ab2_model *m, ab2_kv *kv, const uint32_t *ids_dev,
                               uint32_t *argmax_dev, ab2_stream stream) {
     int rc = check_forward(m, kv, ids_dev, S, row0, nrows, offsets_host, logits_mode, logits_dev);
     if (rc != AB2_OK) return rc;
+    AB2_FOLLOW(kv, stream);
     cudaStream_t s = (cudaStream_t)stream;
     const int *rope_base = kv->lens_dev;
     if (offsets_host) {
@@ -747,6 +748,7 @@ AB2_API int ab2_model_decode_step(ab2_model *m, ab2_kv *kv, const uint32_t *ids_
                                   void *logits_dev, uint32_t *argmax_dev, ab2_stream stream) {
     int rc = check_forward(m, kv, ids_dev, 1, row0, nrows, nullptr, logits_dev ? 1 : 0, logits_dev);
     if (rc != AB2_OK) return rc;
+    AB2_FOLLOW(kv, stream);
     AB2_REQUIRE(logits_dev || argmax_dev, AB2_ERR_BAD_ARG, "decode step needs a logits or an argmax output");
     cudaStream_t s = (cudaStream_t)stream;
     if (s == nullptr || s == cudaStreamLegacy) {

@@ -585,6 +585,7 @@ AB2_API int ab2_window_attention(ab2_kv *kv, int layer, const ab2_layer_spec *sp
                                  const float *cos_dev, const float *sin_dev, float eps, void *out_dev, int S, int row0, int nrows,
                                  ab2_dtype dtype, ab2_stream stream) {
     STEP(check_mixer_call(kv, layer, spec, AB2_MIX_ATTENTION, qkv_dev, out_dev, S, row0, nrows, dtype));
+    AB2_FOLLOW(kv, stream);
     AB2_REQUIRE(spec->rot_dims == 0 || (cos_dev && sin_dev), AB2_ERR_BAD_ARG, "null rotation tables");
     AB2_REQUIRE(v_mode >= 0 && v_mode <= 2 && (v_mode == 0 || v_first_dev), AB2_ERR_BAD_ARG, "value mixing %d needs the first values", v_mode);
     WindowPrepArgs p = {};
@@ -604,6 +605,7 @@ AB2_API int ab2_window_attention(ab2_kv *kv, int layer, const ab2_layer_spec *sp
 AB2_API int ab2_lightning_attention(ab2_kv *kv, int layer, const ab2_layer_spec *spec, const float *decay_pow_dev, const void *qkv_dev,
                                     long long stride, float *scratch_dev, float *out_dev, int S, int row0, int nrows, ab2_dtype dtype, ab2_stream stream) {
     STEP(check_mixer_call(kv, layer, spec, AB2_MIX_LIGHTNING, qkv_dev, out_dev, S, row0, nrows, dtype));
+    AB2_FOLLOW(kv, stream);
     AB2_REQUIRE(decay_pow_dev != nullptr, AB2_ERR_BAD_ARG, "null decay table");
     AB2_REQUIRE(stride >= (long long)spec->heads * (2 * spec->dim + spec->vdim), AB2_ERR_BAD_SHAPE, "row stride %lld is too short", stride);
     LightningArgs a = {};
@@ -628,6 +630,7 @@ AB2_API int ab2_latent_attention(ab2_kv *kv, int layer, const ab2_layer_spec *sp
                                  const ab2_qweight *ukv, const float *cos_dev, const float *sin_dev, float eps, void *out_dev,
                                  void *workspace_dev, size_t workspace_bytes, int reuse, int S, int row0, int nrows, ab2_dtype dtype, ab2_stream stream) {
     STEP(check_mixer_call(kv, layer, spec, AB2_MIX_LATENT, proj_dev, out_dev, S, row0, nrows, dtype));
+    AB2_FOLLOW(kv, stream);
     const int H = spec->heads, D = spec->dim + spec->rot_dims;
     AB2_REQUIRE(norm_dev && ukv && workspace_dev && (spec->rot_dims == 0 || (cos_dev && sin_dev)), AB2_ERR_BAD_ARG, "null argument");
     AB2_REQUIRE(ukv->fmt == FMT_BF16 && ukv->N == H * (spec->dim + spec->vdim) && ukv->K == spec->kv_rank, AB2_ERR_BAD_SHAPE, "the up projection does not match the spec");
