@@ -1,7 +1,7 @@
 // Linear layers over dense bf16 weights, plain or grouped by expert (internal header).
 //
-// Three kernels serve them: a streaming GEMV for a few tokens (gemv_bf16.cu), a tcgen05 GEMM for
-// many (gemm_bf16_tc.cu) and a tiled CUDA-core kernel for f32 activations and odd shapes
+// Four kernels serve them: a streaming GEMV for the fewest tokens (gemv_bf16.cu), a tcgen05 GEMM that deals weights out
+// over the SMs for up to 32 (gemm_bf16_few.cu), a tcgen05 GEMM for more (gemm_bf16_tc.cu) and a tiled CUDA-core kernel for f32 activations and odd shapes
 // (linear_simt.cu), each in four modes.
 #pragma once
 
@@ -95,5 +95,25 @@ int linear_moe_down(const ab2_qweight *down, const void *act, ab2_dtype dtype, f
 int linear_simt(const LinArgs &a, int mode, ab2_dtype dtype, cudaStream_t s);
 int gemv_bf16(const LinArgs &a, int mode, cudaStream_t s);
 int gemm_bf16_tc(const LinArgs &a, int mode, cudaStream_t s);
+// Up to 32 tokens on the tensor cores (gemm_bf16_few.cu); false where another kernel has to serve.
+bool gemm_bf16_few(const LinArgs &a, int mode, cudaStream_t s, int *rc);
+
+// What that kernel hands parts of cut tiles over in: two slots of W4DG_MAX_SLOT_FLOATS for every SM and a zeroed counter per tile.
+// A layer stack has its own, which its recorded steps use on whatever stream they run.  Other calls share the
+// set of their stream with the W4A16 kernels; none while the stream is being recorded (the graph may run beside later work on
+// the stream), on the per-thread stream (one handle, several streams), or where memory is refused.
+struct DecodeGemmScratch {
+    float *partials;
+    int *counters;
+    int max_tiles;
+};
+extern thread_local const DecodeGemmScratch *g_decode_gemm_scratch;  // set by a layer stack around its launches
+struct DecodeGemmScratchOf {
+    explicit DecodeGemmScratchOf(const DecodeGemmScratch *own) { g_decode_gemm_scratch = own; }
+    DecodeGemmScratchOf(const DecodeGemmScratchOf &) = delete;
+    DecodeGemmScratchOf &operator=(const DecodeGemmScratchOf &) = delete;
+    ~DecodeGemmScratchOf() { g_decode_gemm_scratch = nullptr; }
+};
+bool decode_gemm_scratch(cudaStream_t s, DecodeGemmScratch *out);
 
 }  // namespace ab2

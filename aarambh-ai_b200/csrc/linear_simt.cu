@@ -107,6 +107,14 @@ cudaError_t launch_simt(const LinArgs &a, int mode, cudaStream_t s) {
 
 // Rows of the decode GEMV: beyond this many the tensor-memory GEMM's token tiles pay.
 constexpr int GEMV_MAX_ROWS = 32;
+// Whether the decode GEMM over clusters and cut tiles is the faster one for weights of so many elements.  Measured against
+// the GEMV in recorded launches, us (GEMV, decode GEMM): 17 to 32 tokens 2048 x 2048 7.4, 7.9 (but 8197, 8035 for 8 steps of 14
+// latent runs, whose launches are chained), 3664 x 2048 8.9, 8.4, 6144 x 4096 28, 16; 9 to 16 tokens 6144 x 2048 8.3, 9.9,
+// 4096 x 4096 11.1, 10.8, 8192 x 2048 13.6, 10.8; 8 tokens 4096 x 4096 10.6, 10.5, 4096 x 7168 15.8, 14.1, 32000 x 4096 56, 51,
+// but 32000 x 2048 28.6, 31.3; 4 tokens 4096 x 7168 14.9, 13.9, but 14336 x 4096 27.7, 28.7.
+bool few_pays(int M, int K, long long weights) {
+    return M > 16 ? weights >= 4LL << 20 : M > 8 ? weights >= 16LL << 20 : M > 4 && K >= 4096 && weights >= 28LL << 20;
+}
 
 bool rows_aligned(const void *w, const void *x, int K) { return K % 8 == 0 && (((uintptr_t)w | (uintptr_t)x) & 15) == 0; }
 
@@ -134,6 +142,8 @@ int linear_simt(const LinArgs &a, int mode, ab2_dtype dtype, cudaStream_t s) {
 
 int linear_dense(const LinArgs &a, ab2_dtype dtype, cudaStream_t s) {
     if (dtype != AB2_BF16 || !rows_aligned(a.w, a.x, a.K) || a.ldx % 8 != 0 || a.xb % 8 != 0 || a.wb % 8 != 0) return linear_simt(a, LIN_DENSE, dtype, s);
+    int rc;
+    if (few_pays(a.M, a.K, (long long)a.N * a.K) && gemm_bf16_few(a, LIN_DENSE, s, &rc)) return rc;
     return a.M <= GEMV_MAX_ROWS || a.batch > 1 || a.epi == LIN_GATE ? gemv_bf16(a, LIN_DENSE, s) : gemm_bf16_tc(a, LIN_DENSE, s);
 }
 
@@ -149,6 +159,8 @@ int linear_glu(const ab2_qweight *gate, const ab2_qweight *up, const void *x, in
     a.w = (const __nv_bfloat16 *)gate->codes; a.w2 = (const __nv_bfloat16 *)up->codes; a.x = x; a.y = act;
     a.N = gate->N; a.K = gate->K; a.M = M; a.glu = glu; a.limit = limit;
     if (dtype != AB2_BF16 || !rows_aligned(a.w, x, a.K)) return linear_simt(a, LIN_GLU, dtype, s);
+    int rc;
+    if (few_pays(M, a.K, 2LL * a.N * a.K) && gemm_bf16_few(a, LIN_GLU, s, &rc)) return rc;
     return M <= GEMV_MAX_ROWS ? gemv_bf16(a, LIN_GLU, s) : gemm_bf16_tc(a, LIN_GLU, s);
 }
 

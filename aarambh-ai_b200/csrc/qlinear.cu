@@ -138,8 +138,26 @@ struct GemvScratch {
     int *counters = nullptr;
     int max_ctas = 0;
 };
+constexpr size_t DECODE_GEMM_MAX_STREAMS = 64;  // linears of bf16 weights start no set beyond so many (11 MB each)
 static std::mutex g_scratch_mutex;
 static std::map<std::pair<int, cudaStream_t>, GemvScratch> g_scratch;
+
+static cudaError_t gemv_scratch_alloc(cudaStream_t s, GemvScratch *sc) {
+    sc->max_ctas = device_sm_count() * 3;
+    // two partial tiles per warp of the warp kernels, or per CTA of the decode GEMMs, one CTA per SM
+    const size_t pbytes = std::max((size_t)sc->max_ctas * W4W_WARPS * 2 * W4W_SLOT_FLOATS,
+                                   (size_t)device_sm_count() * 2 * W4DG_MAX_SLOT_FLOATS) * sizeof(float);
+    cudaError_t e = cudaMalloc((void **)&sc->partials, pbytes);
+    if (e == cudaSuccess) e = cudaMalloc((void **)&sc->counters, W4W_MAX_TILES * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemsetAsync(sc->counters, 0, W4W_MAX_TILES * sizeof(int), s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // a graph made with the set may be launched on another stream
+    if (e != cudaSuccess) {
+        cudaFree(sc->partials);
+        cudaFree(sc->counters);
+        (void)cudaGetLastError();
+    }
+    return e;
+}
 
 static int gemv_scratch_for(cudaStream_t s, GemvScratch *out) {
     int dev = 0;
@@ -154,18 +172,43 @@ static int gemv_scratch_for(cudaStream_t s, GemvScratch *out) {
                         "first quantised linear on this stream is inside a graph capture: run one launch "
                         "on the stream before capturing (its scratch buffers are allocated then)");
         GemvScratch sc;
-        sc.max_ctas = device_sm_count() * 3;
-        // two partial tiles per warp of the warp kernels, or per CTA of the decode GEMM, one CTA per SM
-        const size_t pbytes = std::max((size_t)sc.max_ctas * W4W_WARPS * 2 * W4W_SLOT_FLOATS,
-                                       (size_t)device_sm_count() * 2 * W4DG_MAX_SLOT_FLOATS) * sizeof(float);
-        AB2_CUDA(cudaMalloc((void **)&sc.partials, pbytes));
-        AB2_CUDA(cudaMalloc((void **)&sc.counters, W4W_MAX_TILES * sizeof(int)));
-        AB2_CUDA(cudaMemset(sc.counters, 0, W4W_MAX_TILES * sizeof(int)));
-        AB2_CUDA(cudaDeviceSynchronize());
+        AB2_CUDA(gemv_scratch_alloc(s, &sc));
         it = g_scratch.emplace(key, sc).first;
     }
     *out = it->second;
     return AB2_OK;
+}
+
+thread_local const DecodeGemmScratch *g_decode_gemm_scratch = nullptr;
+
+// The decode GEMM's parts and counters for launches on `s`; false where there are none to be had (linear_bf16.cuh).
+bool decode_gemm_scratch(cudaStream_t s, DecodeGemmScratch *out) {
+    if (g_decode_gemm_scratch) {
+        *out = *g_decode_gemm_scratch;
+        return out->partials != nullptr;
+    }
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (s == cudaStreamPerThread || cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    std::lock_guard<std::mutex> lock(g_scratch_mutex);
+    auto it = g_scratch.find(std::make_pair(dev, s));
+    if (it == g_scratch.end()) {
+        if (g_scratch.size() >= DECODE_GEMM_MAX_STREAMS) return false;
+        // another thread may be recording a graph: an allocation does not disturb it
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        (void)cudaThreadExchangeStreamCaptureMode(&mode);
+        GemvScratch sc;
+        const bool ok = gemv_scratch_alloc(s, &sc) == cudaSuccess;
+        (void)cudaThreadExchangeStreamCaptureMode(&mode);
+        if (!ok) return false;
+        it = g_scratch.emplace(std::make_pair(dev, s), sc).first;
+    }
+    *out = {it->second.partials, it->second.counters, W4W_MAX_TILES};
+    return true;
 }
 
 int w4a16_prepare_stream(cudaStream_t s) {

@@ -10,6 +10,7 @@
 #include <cstring>
 #include <map>
 
+#include "gemv_w4a16_mma.cuh"
 #include "ops.cuh"
 #include "stack.cuh"
 
@@ -17,6 +18,7 @@ using namespace ab2;
 
 namespace ab2 {
 int device_status_word(int **out);
+int device_sm_count();
 
 struct StackLayer {
     ab2_layer_spec spec;
@@ -54,6 +56,7 @@ struct Stack {
     // workspace, sized for max_tokens
     float *x, *x0, *mix32, *parts, *router_z, *shared_out;
     void *shared_act, *z, *latent_work;
+    DecodeGemmScratch few;
     size_t latent_bytes;
     void *xb, *proj, *mixed, *act, *gathered, *v_first, *head_in;
     int *route_int;
@@ -176,7 +179,7 @@ static void free_workspace(Stack *st) {
     void **all[] = {(void **)&st->x, (void **)&st->mix32, (void **)&st->parts, (void **)&st->router_z, &st->xb, &st->proj, &st->mixed,
                     &st->act, &st->gathered, &st->v_first, &st->head_in, (void **)&st->route_int, (void **)&st->route_score,
                     (void **)&st->logits_scratch, (void **)&st->seg_states, (void **)&st->x0, (void **)&st->shared_out, &st->shared_act,
-                    &st->z, &st->latent_work, (void **)&st->route_tables};
+                    &st->z, &st->latent_work, (void **)&st->route_tables, (void **)&st->few.partials, (void **)&st->few.counters};
     for (auto &L : st->layers) { cudaFree(L.route_int); L.route_int = nullptr; }
     for (void **p : all) { cudaFree(*p); *p = nullptr; }
 }
@@ -354,6 +357,20 @@ int stack_finalize(Stack *st) {
             }
         }
     }
+    if (st->dtype == AB2_BF16 && !st->few.partials) {
+        // refused, the linears of a few tokens take kernels that need none
+        const size_t slots = (size_t)device_sm_count() * 2 * W4DG_MAX_SLOT_FLOATS * 4;
+        st->few.max_tiles = 1 << 18;
+        cudaError_t e = cudaMalloc((void **)&st->few.partials, slots);
+        if (e == cudaSuccess) e = cudaMalloc((void **)&st->few.counters, st->few.max_tiles * 4);
+        if (e == cudaSuccess) e = cudaMemset(st->few.counters, 0, st->few.max_tiles * 4);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+        if (e != cudaSuccess) {
+            (void)cudaGetLastError();
+            cudaFree(st->few.partials); cudaFree(st->few.counters);
+            st->few = {};
+        }
+    }
     std::vector<MoeTable> tables;
     for (auto &L : st->layers) {
         const ab2_layer_spec &sp = L.spec;
@@ -474,6 +491,7 @@ static int poly_ffn(Stack *st, StackLayer &L, const void *in, int T, cudaStream_
 
 int stack_forward(Stack *st, ab2_kv *kv, const uint32_t *ids, int S, int row0, int nrows, int logits_mode, float *logits,
                   uint32_t *argmax_out, int len_hint, cudaStream_t s) {
+    const DecodeGemmScratchOf few(&st->few);
     const int all = nrows * S, d = st->cfg.d_model;
     int T = all;  // tokens that the launches from here on work on
     int max_len = len_hint;

@@ -276,7 +276,8 @@ inline int tensor_map_encoder(EncodeTiledFn *out) {
 
 // Tensor map of `rows` rows of `cols` elements that lie `ld` elements apart, read in boxes of 128 bytes x box_rows
 // (128-byte swizzle).
-inline int make_rows_map(CUtensorMap *map, CUtensorMapDataType type, int elem, const void *p, int rows, int cols, long long ld, int box_rows) {
+inline int make_rows_map(CUtensorMap *map, CUtensorMapDataType type, int elem, const void *p, int rows, int cols, long long ld, int box_rows,
+                         CUtensorMapL2promotion promotion = CU_TENSOR_MAP_L2_PROMOTION_L2_128B) {
     EncodeTiledFn encode;
     int rc = tensor_map_encoder(&encode);
     if (rc != AB2_OK) return rc;
@@ -285,7 +286,7 @@ inline int make_rows_map(CUtensorMap *map, CUtensorMapDataType type, int elem, c
     cuuint32_t box[2] = {(cuuint32_t)(128 / elem), (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = encode(map, type, 2, const_cast<void *>(p), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                        CU_TENSOR_MAP_SWIZZLE_128B, promotion, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     AB2_REQUIRE(r == CUDA_SUCCESS, AB2_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
     return AB2_OK;
 }
