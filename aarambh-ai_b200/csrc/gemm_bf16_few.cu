@@ -88,25 +88,8 @@ __device__ __forceinline__ uint32_t cluster_ctas() {
     asm volatile("mov.u32 %0, %%cluster_nctarank;\n" : "=r"(n));
     return n;
 }
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ uint32_t peer_addr(uint32_t local, uint32_t rank) {
-    uint32_t remote;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(local), "r"(rank));
-    return remote;
-}
 __device__ __forceinline__ void peer_store(uint32_t remote, uint32_t v) {
     asm volatile("st.shared::cluster.u32 [%0], %1;\n" ::"r"(remote), "r"(v) : "memory");
-}
-__device__ __forceinline__ void peer_arrive(uint32_t remote) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(remote) : "memory");
 }
 __device__ __forceinline__ void tensormap_prefetch(const CUtensorMap *map) {
     asm volatile("prefetch.tensormap [%0];\n" ::"l"(map) : "memory");

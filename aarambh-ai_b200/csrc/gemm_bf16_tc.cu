@@ -18,6 +18,16 @@
 // same tile list out from them (prefix sums in shared memory).  Rows of a tile past its expert's
 // last pair belong to the next expert; they are multiplied and not stored.  The pair's weight
 // multiplies the f32 sums, which is the sum over the weighted input without rounding it.
+//
+// What bounds it: operands out of L2.  A stage of one CTA's 128 x 256 tile is 48 KB for 512 cycles of MMAs, and an SM gets about
+// 56 bytes a cycle.  So where a launch has rounds enough, PAIRs of CTAs (clusters of two, cta_group::2) multiply one tile of 256
+// channels x 256 tokens (gate and up: 128): each loads its own 128 weight rows and half of the tokens, 32 KB a stage; the
+// first issues the MMAs for both, all copies of a stage count on its barrier, its commits arrive at both CTAs' barriers, and either
+// CTA's epilogue takes the 128 channels in its own tensor memory.  us, single CTAs -> pairs: 14336 x 4096, 2048 tokens 179 -> 165
+// (1.45 PFLOP/s), 4096 x 14336 183 -> 166, 8 experts' down products of 7168 x 4096, 256 rows each 154 -> 132, a shared expert's gate
+// and up products 193 -> 175; a latent stack's prompt of 2048 tokens 7500 -> 7110.  Measured and not kept: experts' last tiles
+// with fewer columns and 32-row loads, dealt out by a counter (no change); weights requested into L2 6 to 24 stages ahead
+// (a mixture's prompt 2723 -> 2816 to 2884).
 // Every wait on an mbarrier is bounded; on a time-out the CTA records AB2_ERR_TIMEOUT, walks
 // through the rest of its work, frees its tensor memory and returns.
 #include <cuda.h>
@@ -51,11 +61,11 @@ struct GbShared {
     int tile_start[GB_MAX_EXPERTS + 1];  // grouped modes: first token tile of each expert
 };
 
-template <int NTOK, int MODE>
-__host__ __device__ constexpr int gb_stage_bytes() { return (MODE == LIN_MOE_GLU || MODE == LIN_GLU ? 2 : 1) * GB_A_BYTES + NTOK * 128; }
-template <int NTOK, int MODE>
+template <int NTOK, int MODE, bool PAIR>
+__host__ __device__ constexpr int gb_stage_bytes() { return (MODE == LIN_MOE_GLU || MODE == LIN_GLU ? 2 : 1) * GB_A_BYTES + (PAIR ? NTOK / 2 : NTOK) * 128; }
+template <int NTOK, int MODE, bool PAIR>
 __host__ __device__ constexpr int gb_stages() {
-    return GB_RING_BYTES / gb_stage_bytes<NTOK, MODE>() < GB_MAX_STAGES ? GB_RING_BYTES / gb_stage_bytes<NTOK, MODE>() : GB_MAX_STAGES;
+    return GB_RING_BYTES / gb_stage_bytes<NTOK, MODE, PAIR>() < GB_MAX_STAGES ? GB_RING_BYTES / gb_stage_bytes<NTOK, MODE, PAIR>() : GB_MAX_STAGES;
 }
 
 // Walks the tile list: item -> (expert, channel tile, token tile).  Items of one CTA only grow, so
@@ -70,35 +80,42 @@ struct GbCursor {
     }
 };
 
-template <int NTOK, int MODE>
+template <int NTOK, int MODE, bool PAIR>
 __global__ void __launch_bounds__(GB_THREADS, 1)
 gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap w2map,
                     const __grid_constant__ CUtensorMap xmap, LinArgs a, int *status) {
     constexpr bool DUAL = MODE == LIN_MOE_GLU || MODE == LIN_GLU, GROUPED = MODE == LIN_MOE_GLU || MODE == LIN_MOE_DOWN;
-    constexpr int STAGES = gb_stages<NTOK, MODE>(), STAGE_BYTES = gb_stage_bytes<NTOK, MODE>();
+    constexpr int STAGES = gb_stages<NTOK, MODE, PAIR>(), STAGE_BYTES = gb_stage_bytes<NTOK, MODE, PAIR>();
+    constexpr int CTAS = PAIR ? 2 : 1;  // of a tile
     constexpr int ACC_COLS = DUAL ? 2 * NTOK : NTOK;  // tensor-memory columns of one accumulator set
     constexpr uint32_t TMEM_COLS = 2 * ACC_COLS;
     static_assert(TMEM_COLS <= 512, "two accumulator sets fit tensor memory");
-    constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NTOK >> 3) << 17) | ((128u >> 4) << 24);
+    constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NTOK >> 3) << 17) | ((CTAS * 128u >> 4) << 24);
     extern __shared__ uint8_t smem_raw[];
     uint8_t *ring = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     GbShared *sh = (GbShared *)(ring + STAGES * STAGE_BYTES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int KS = (a.K + 63) >> 6;
-    const int n_tiles = (a.N + 127) >> 7;
+    const int n_tiles = (a.N + CTAS * 128 - 1) / (CTAS * 128);
+    const int rank = PAIR ? (int)cluster_rank() : 0, first_item = (int)blockIdx.x / CTAS, item_step = (int)gridDim.x / CTAS;
     volatile int *failed = &sh->failed;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < STAGES; ++i) { bar_init(&sh->full[i], 1); bar_init(&sh->empty[i], 1); }
-        for (int i = 0; i < 2; ++i) { bar_init(&sh->accfull[i], 1); bar_init(&sh->accempty[i], GB_EPI_WARPS); }
+        for (int i = 0; i < 2; ++i) { bar_init(&sh->accfull[i], 1); bar_init(&sh->accempty[i], CTAS * GB_EPI_WARPS); }
         sh->failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     }
     if (warp == 1) {  // tensor-memory allocation is a whole-warp operation
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(sptr(&sh->tmem_base)), "r"(TMEM_COLS));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+        if (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(sptr(&sh->tmem_base)), "r"(TMEM_COLS));
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::);
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(sptr(&sh->tmem_base)), "r"(TMEM_COLS));
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+        }
     }
     pdl_wait();
     pdl_launch_dependents();
@@ -125,7 +142,9 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         if (lane == 0) sh->tile_start[E] = base;
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
+    __syncwarp();
+    if (PAIR) cluster_sync_all();  // the other CTA's copies and arrivals come to this one's barriers
+    else __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = sh->tmem_base;
     const int items = sh->tile_start[E] * n_tiles;
@@ -135,16 +154,25 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         // ---------------------------------------------------------- TMA producer
         if (lane == 0) {
             uint32_t use = 0;
-            for (int it = blockIdx.x; it < items && !*failed; it += gridDim.x) {
+            for (int it = first_item; it < items && !*failed; it += item_step) {
                 int nt, mt;
                 cur.find(sh, it, n_tiles, nt, mt);
-                const int wrow = (GROUPED ? cur.e * a.N : 0) + nt * 128;
-                const int xrow = (GROUPED ? a.r.offset[cur.e] : 0) + mt * NTOK;
+                const int wrow = (GROUPED ? cur.e * a.N : 0) + (nt * CTAS + rank) * 128;
+                const int xrow = (GROUPED ? a.r.offset[cur.e] : 0) + mt * NTOK + rank * (NTOK / CTAS);
                 for (int ks = 0; ks < KS && !*failed; ++ks, ++use) {
                     const int s = use % STAGES;
                     if (!bar_wait(&sh->empty[s], ((use / STAGES) & 1) ^ 1, failed)) break;
                     uint8_t *st = ring + s * STAGE_BYTES;
-                    bar_expect_tx(&sh->full[s], STAGE_BYTES);  // what lies past a tensor arrives as zeros and counts
+                    // what lies past a tensor arrives as zeros and counts
+                    if (PAIR) {  // the first CTA, which issues the MMAs, waits for both halves
+                        if (rank == 0) bar_expect_tx(&sh->full[s], 2 * STAGE_BYTES);
+                        const uint32_t full = peer_addr(sptr(&sh->full[s]), 0);
+                        tma_load_2d_pair(st, &wmap, ks * 64, wrow, full);
+                        if (DUAL) tma_load_2d_pair(st + GB_A_BYTES, &w2map, ks * 64, wrow, full);
+                        tma_load_2d_pair(st + (DUAL ? 2 : 1) * GB_A_BYTES, &xmap, ks * 64, xrow, full);
+                        continue;
+                    }
+                    bar_expect_tx(&sh->full[s], STAGE_BYTES);
                     tma_load_2d(st, &wmap, ks * 64, wrow, &sh->full[s]);
                     if (DUAL) tma_load_2d(st + GB_A_BYTES, &w2map, ks * 64, wrow, &sh->full[s]);
                     tma_load_2d(st + (DUAL ? 2 : 1) * GB_A_BYTES, &xmap, ks * 64, xrow, &sh->full[s]);
@@ -152,9 +180,9 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
             }
         }
     } else if (warp == 1) {
-        // ---------------------------------------------------------- MMA issue
+        // ---------------------------------------------------------- MMA issue (of a pair: by its first CTA)
         uint32_t use = 0, tuse = 0;
-        for (int it = blockIdx.x; it < items; it += gridDim.x, ++tuse) {
+        for (int it = first_item; rank == 0 && it < items; it += item_step, ++tuse) {
             const int ab = tuse & 1;
             bar_wait(&sh->accempty[ab], ((tuse >> 1) & 1) ^ 1, failed);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -165,20 +193,29 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                 if (elect_one()) {
                     const uint32_t a0 = sptr(ring + s * STAGE_BYTES);
                     const uint64_t xd = umma_desc(a0 + (DUAL ? 2 : 1) * GB_A_BYTES);
-                    umma_stage(tacc, umma_desc(a0), xd, IDESC, ks == 0);
-                    if (DUAL) umma_stage(tacc + NTOK, umma_desc(a0 + GB_A_BYTES), xd, IDESC, ks == 0);
-                    umma_commit(&sh->empty[s]);  // the stage is free when the MMAs retire
+                    if (PAIR) {
+                        umma_stage_pair(tacc, umma_desc(a0), xd, IDESC, ks == 0);
+                        if (DUAL) umma_stage_pair(tacc + NTOK, umma_desc(a0 + GB_A_BYTES), xd, IDESC, ks == 0);
+                        umma_commit_pair(&sh->empty[s]);
+                    } else {
+                        umma_stage(tacc, umma_desc(a0), xd, IDESC, ks == 0);
+                        if (DUAL) umma_stage(tacc + NTOK, umma_desc(a0 + GB_A_BYTES), xd, IDESC, ks == 0);
+                        umma_commit(&sh->empty[s]);  // the stage is free when the MMAs retire
+                    }
                 }
                 __syncwarp();
             }
-            if (elect_one()) umma_commit(&sh->accfull[ab]);
+            if (elect_one()) {
+                if (PAIR) umma_commit_pair(&sh->accfull[ab]);
+                else umma_commit(&sh->accfull[ab]);
+            }
             __syncwarp();
         }
     } else {
         // ---------------------------------------------------------- epilogue
         const int quad = warp & 3, first_block = (warp - 2) >> 2;
         uint32_t tuse = 0;
-        for (int it = blockIdx.x; it < items; it += gridDim.x, ++tuse) {
+        for (int it = first_item; it < items; it += item_step, ++tuse) {
             int nt, mt;
             cur.find(sh, it, n_tiles, nt, mt);
             const int ab = tuse & 1;
@@ -187,7 +224,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
             const int row0 = r0 + mt * NTOK;
             bar_wait(&sh->accfull[ab], (tuse >> 1) & 1, failed);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const int n = nt * 128 + quad * 32 + lane;
+            const int n = (nt * CTAS + rank) * 128 + quad * 32 + lane;
             constexpr int CW = DUAL ? 16 : 32;  // tokens per register block
 #pragma unroll 1
             for (int c = first_block; c < NTOK / CW; c += GB_EPI_WARPS / 4) {
@@ -241,21 +278,27 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
             }
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
             __syncwarp();
-            if (lane == 0) bar_arrive(&sh->accempty[ab]);
+            if (lane == 0) {
+                if (rank > 0) peer_arrive(peer_addr(sptr(&sh->accempty[ab]), 0));
+                else bar_arrive(&sh->accempty[ab]);
+            }
         }
     }
 
     // ---- teardown: every warp arrives here (all waits are bounded)
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
+    __syncwarp();
+    if (PAIR) cluster_sync_all();  // neither leaves while the other may arrive at its barriers
+    else __syncthreads();
     if (threadIdx.x == 0 && sh->failed) atomicExch(status, (int)AB2_ERR_TIMEOUT);
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS));
+        if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS));
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS));
     }
 }
 
-template <int NTOK, int MODE>
+template <int NTOK, int MODE, bool PAIR = false>
 int launch_tc(const LinArgs &a, cudaStream_t s) {
     int *status = nullptr;
     int rc = device_status_word(&status);
@@ -265,48 +308,64 @@ int launch_tc(const LinArgs &a, cudaStream_t s) {
     const int wrows = GROUPED ? a.N * a.r.E : a.N;
     rc = make_x_map(&wmap, a.w, wrows, a.K, 128);
     if (rc == AB2_OK) rc = make_x_map(&w2map, MODE == LIN_MOE_GLU || MODE == LIN_GLU ? a.w2 : a.w, wrows, a.K, 128);
-    if (rc == AB2_OK) rc = make_x_map(&xmap, a.x, a.M, a.K, NTOK, MODE == LIN_DENSE ? a.ldx : a.K);
+    if (rc == AB2_OK) rc = make_x_map(&xmap, a.x, a.M, a.K, PAIR ? NTOK / 2 : NTOK, MODE == LIN_DENSE ? a.ldx : a.K);
     if (rc != AB2_OK) return rc;
-    const size_t smem = 1024 + (size_t)gb_stages<NTOK, MODE>() * gb_stage_bytes<NTOK, MODE>() + sizeof(GbShared);
+    const size_t smem = 1024 + (size_t)gb_stages<NTOK, MODE, PAIR>() * gb_stage_bytes<NTOK, MODE, PAIR>() + sizeof(GbShared);
     static bool configured[64] = {false};  // the attribute is per device
     int dev = 0;
     AB2_CUDA(cudaGetDevice(&dev));
     AB2_REQUIRE(dev >= 0 && dev < 64, AB2_ERR_BAD_ARG, "device index %d out of range", dev);
     if (!configured[dev]) {
-        AB2_CUDA(cudaFuncSetAttribute(gemm_bf16_tc_kernel<NTOK, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        AB2_CUDA(cudaFuncSetAttribute(gemm_bf16_tc_kernel<NTOK, MODE, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         configured[dev] = true;
     }
     // at most this many tiles: every expert may leave one token tile part empty
     const long long m_tiles = (a.M + NTOK - 1) / NTOK + (GROUPED ? std::min(a.r.E, a.r.pairs) : 0);
-    const int grid = (int)std::min<long long>(m_tiles * ((a.N + 127) / 128), device_sm_count());
-    cudaError_t e = launch_kernel(gemm_bf16_tc_kernel<NTOK, MODE>, dim3(grid), dim3(GB_THREADS), smem, s, wmap, w2map, xmap, a, status);
+    constexpr int CTAS = PAIR ? 2 : 1;
+    const int grid = (int)std::min<long long>(m_tiles * ((a.N + CTAS * 128 - 1) / (CTAS * 128)), device_sm_count() / CTAS) * CTAS;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(GB_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CTAS; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_pdl_launch ? 2 : 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_bf16_tc_kernel<NTOK, MODE, PAIR>, wmap, w2map, xmap, a, status);
     if (e != cudaSuccess) return fail(AB2_ERR_CUDA, "bf16 GEMM launch failed: %s", cudaGetErrorString(e));
     return AB2_OK;
+}
+
+// Token tile, and one CTA or a pair for a tile: rounds of tiles over the SMs times what a tile costs.  That of one CTA is the
+// rows it streams through L2, its tokens and the 128 (gate and up: 256) weight rows.  A pair's tile costs as much as 350 of
+// them: 14336 x 4096, us by single CTAs and by pairs: 300 tokens 53, 46; 512 56, 50; 2048 178, 165; 4096 x 4096: 512 tokens 21, 26 (32
+// pair tiles for 74 pairs), 1024 28.1, 27.8; 2048 x 2048, 1024 tokens: 13.2, 15.9.  Over ten weights and eleven token counts
+// the rule took the slower form by 5 % at most.
+template <int MODE, int PAIR_TOK>
+int launch_best(const LinArgs &a, int groups, double rows, cudaStream_t s) {
+    constexpr bool DUAL = MODE == LIN_MOE_GLU || MODE == LIN_GLU;
+    const int sms = device_sm_count();
+    auto rounds = [&](int ntok, int channels, int units) { return std::ceil(std::ceil(rows / ntok) * ((a.N + channels - 1) / channels) * groups / units); };
+    auto cost = [&](int ntok) { return rounds(ntok, 128, sms) * (ntok + (DUAL ? 256 : 128)); };
+    int best = !DUAL && cost(256) <= cost(128) ? 256 : 128;
+    if (cost(64) < cost(best)) best = 64;
+    if (rounds(PAIR_TOK, 256, sms / 2) * 350 < cost(best)) return launch_tc<PAIR_TOK, MODE, true>(a, s);
+    if constexpr (!DUAL) if (best == 256) return launch_tc<256, MODE>(a, s);
+    return best == 128 ? launch_tc<128, MODE>(a, s) : launch_tc<64, MODE>(a, s);
 }
 
 }  // namespace
 
 int gemm_bf16_tc(const LinArgs &a, int mode, cudaStream_t s) {
-    // The token tile: waves of tiles over the SMs times what a tile costs, which is the rows it streams
-    // through L2 - its tokens and the 128 (gate and up: 256) weight rows.  An expert's rows are counted with what
-    // routing spreads around their mean.
-    const int sms = device_sm_count(), n_tiles = (a.N + 127) / 128;
-    const bool grouped = mode == LIN_MOE_GLU || mode == LIN_MOE_DOWN, dual = mode == LIN_MOE_GLU || mode == LIN_GLU;
+    // An expert's rows are counted with what routing spreads around their mean.
+    const bool grouped = mode == LIN_MOE_GLU || mode == LIN_MOE_DOWN;
     const int groups = grouped ? std::min(a.r.E, a.r.pairs) : 1;
     const double rows = !grouped ? a.M : (double)a.M / groups + std::sqrt((double)a.M / groups);
-    auto cost = [&](int ntok) {
-        const double tiles = std::ceil(rows / ntok) * n_tiles * groups;
-        return std::ceil(tiles / sms) * (ntok + (dual ? 256 : 128));
-    };
-    if (mode == LIN_DENSE) {
-        if (cost(256) <= cost(128) && cost(256) <= cost(64)) return launch_tc<256, LIN_DENSE>(a, s);
-        return cost(128) <= cost(64) ? launch_tc<128, LIN_DENSE>(a, s) : launch_tc<64, LIN_DENSE>(a, s);
-    }
-    if (mode == LIN_GLU) return cost(128) <= cost(64) ? launch_tc<128, LIN_GLU>(a, s) : launch_tc<64, LIN_GLU>(a, s);
+    if (mode == LIN_DENSE) return launch_best<LIN_DENSE, 256>(a, 1, rows, s);
+    if (mode == LIN_GLU) return launch_best<LIN_GLU, 128>(a, 1, rows, s);
     AB2_REQUIRE(a.r.E <= GB_MAX_EXPERTS, AB2_ERR_UNSUPPORTED, "%d experts exceed the %d the grouped GEMM serves", a.r.E, GB_MAX_EXPERTS);
-    if (mode == LIN_MOE_GLU) return cost(128) <= cost(64) ? launch_tc<128, LIN_MOE_GLU>(a, s) : launch_tc<64, LIN_MOE_GLU>(a, s);
-    if (cost(256) <= cost(128) && cost(256) <= cost(64)) return launch_tc<256, LIN_MOE_DOWN>(a, s);
-    return cost(128) <= cost(64) ? launch_tc<128, LIN_MOE_DOWN>(a, s) : launch_tc<64, LIN_MOE_DOWN>(a, s);
+    return mode == LIN_MOE_GLU ? launch_best<LIN_MOE_GLU, 128>(a, groups, rows, s) : launch_best<LIN_MOE_DOWN, 256>(a, groups, rows, s);
 }
 
 }  // namespace ab2

@@ -69,6 +69,32 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
             "r"(sptr(dst)), "l"(map), "r"(sptr(bar)), "r"(x), "r"(y) : "memory");
 }
 
+// ---- pairs of CTAs (a cluster of two) that multiply one tile: cta_group::2
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// The address of CTA `rank`'s variable that lies where `local` does in this CTA.
+__device__ __forceinline__ uint32_t peer_addr(uint32_t local, uint32_t rank) {
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(local), "r"(rank));
+    return remote;
+}
+__device__ __forceinline__ void peer_arrive(uint32_t remote) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(remote) : "memory");
+}
+// A tile into this CTA's memory, counted on a barrier of either CTA of the pair.
+__device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n" ::
+            "r"(sptr(dst)), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
+}
+
 // 3-D tile load: coordinates (element, row, matrix).
 __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int x, int y, int z, uint64_t *bar) {
     asm volatile(
@@ -127,6 +153,19 @@ __device__ __forceinline__ bool elect_one() {
 __device__ __forceinline__ void umma_stage(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, bool first) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) umma_bf16(tmem_d, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, !first || k > 0);
+}
+// The same by the first CTA of a pair for both: 256 rows of A and the columns of B, half of each in either's shared memory.
+__device__ __forceinline__ void umma_stage_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, bool first) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        asm volatile(
+            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+            " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::
+                "r"(tmem_d), "l"(adesc + (uint64_t)(2 * k)), "l"(bdesc + (uint64_t)(2 * k)), "r"(idesc), "r"((uint32_t)(!first || k > 0)) : "memory");
+}
+// Arrives at the barrier in both CTAs of the pair.
+__device__ __forceinline__ void umma_commit_pair(uint64_t *bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(sptr(bar)), "h"((uint16_t)3) : "memory");
 }
 // The first operand in tensor memory: 128 lanes, two bf16 per column.
 __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
