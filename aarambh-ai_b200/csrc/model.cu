@@ -315,17 +315,20 @@ static int forward_launches(ab2_model *m, ab2_kv *kv, const uint32_t *ids, int S
             STEP(qlinear_w4a16_mma_add(L.part[6], m->hid, T, x, x, s));
         } else {
             // a few tokens over weights without a GEMV of their own: the norm, the gated unit and the residual additions
-            // ride with the linears
+            // ride with the linears; with more, the residual addition goes with the norm that follows it
+            bool normed = false;
             if (qlinear_step_eligible(L.part[3], m->dtype, T)) {
                 STEP(qlinear_step_add(L.part[3], attn, x, T, m->dtype, x, s));
             } else {
                 STEP(qlinear_dispatch(L.part[3], attn, T, m->dtype, m->proj, s));
-                STEP(launch_add(x, m->proj, x, (size_t)T * d, m->dtype, s));
+                normed = !qlinear_step_eligible(L.wgu, m->dtype, T);
+                if (normed) STEP(launch_add_rms_norm(x, m->proj, L.norm2, m->xn, T, d, c.rms_eps, m->dtype, s));
+                else STEP(launch_add(x, m->proj, x, (size_t)T * d, m->dtype, s));
             }
             if (qlinear_step_eligible(L.wgu, m->dtype, T)) {
                 STEP(qlinear_step_norm(L.wgu, x, L.norm2, c.rms_eps, T, m->dtype, true, m->hid, s));
             } else {
-                STEP(launch_rms_norm(x, L.norm2, m->xn, T, d, c.rms_eps, m->dtype, s));
+                if (!normed) STEP(launch_rms_norm(x, L.norm2, m->xn, T, d, c.rms_eps, m->dtype, s));
                 STEP(qlinear_dispatch(L.wgu, m->xn, T, m->dtype, m->gu, s));
                 STEP(launch_swiglu_fused(m->gu, m->hid, T, c.ffn_hidden, m->dtype, s));
             }
@@ -333,7 +336,9 @@ static int forward_launches(ab2_model *m, ab2_kv *kv, const uint32_t *ids, int S
                 STEP(qlinear_step_add(L.part[6], m->hid, x, T, m->dtype, x, s));
             } else {
                 STEP(qlinear_dispatch(L.part[6], m->hid, T, m->dtype, m->proj, s));
-                STEP(launch_add(x, m->proj, x, (size_t)T * d, m->dtype, s));
+                xn_ready = l + 1 < c.n_layers && !qlinear_step_eligible(m->layers[l + 1].wqkv, m->dtype, T);
+                if (xn_ready) STEP(launch_add_rms_norm(x, m->proj, m->layers[l + 1].norm1, m->xn, T, d, c.rms_eps, m->dtype, s));
+                else STEP(launch_add(x, m->proj, x, (size_t)T * d, m->dtype, s));
             }
         }
     }
