@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <cstring>
+#include <mutex>
 
 #include "common.cuh"
 #include "kv_cache.cuh"
@@ -300,20 +301,43 @@ __global__ void kv_truncate_kernel(const __grid_constant__ KvCut c) {
     }
 }
 
+static std::mutex g_cut_mutex;  // the cut_* fields of every cache: rows of one cache may be cut and used from several threads
+
 int kv_follow(const ab2_kv *kv, cudaStream_t s) {
-    if (!kv || !kv->cut_pending || s == kv->cut_stream) return AB2_OK;
+    if (!kv) return AB2_OK;
     cudaStreamCaptureStatus recording = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &recording) != cudaSuccess) cudaGetLastError();
-    if (recording != cudaStreamCaptureStatusNone) {  // a recorded launch cannot wait for work outside its graph
-        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-        AB2_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
-        const cudaError_t e = cudaEventSynchronize(kv->cut_event);
-        AB2_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
-        AB2_CUDA(e);
-        kv->cut_pending = false;
-        return AB2_OK;
+    if (cudaStreamIsCapturing(s, &recording) != cudaSuccess) {
+        (void)cudaGetLastError();
+        recording = cudaStreamCaptureStatusNone;
     }
-    AB2_CUDA(cudaStreamWaitEvent(s, kv->cut_event, 0));
+    const bool in_graph = recording != cudaStreamCaptureStatusNone;
+    std::unique_lock<std::mutex> lock(g_cut_mutex);
+    if (in_graph) kv->recorded = true;
+    if (!kv->cut_pending) return AB2_OK;
+    // The stream that the cut was launched on keeps the order by itself.  Its id says which that is, its handle does not: the
+    // per-thread stream is one handle for a stream of every thread, and a destroyed stream's handle is used again.
+    if (!in_graph) {  // a recording stream is not asked
+        unsigned long long id = 0;
+        AB2_CUDA(cudaStreamGetId(s, &id));
+        if (id == kv->cut_stream_id) return AB2_OK;
+    }
+    // asking and waiting on the host would disturb a recording of this thread's or another's
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    AB2_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    cudaError_t e;
+    if (in_graph) {  // a recorded launch cannot wait for work outside its graph, which may be launched on any stream
+        lock.unlock();
+        e = cudaEventSynchronize(kv->cut_event);
+    } else {
+        e = cudaEventQuery(kv->cut_event);
+        if (e == cudaSuccess) kv->cut_pending = false;
+    }
+    AB2_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    if (e == cudaErrorNotReady) {
+        (void)cudaGetLastError();
+        e = cudaStreamWaitEvent(s, kv->cut_event, 0);
+    }
+    AB2_CUDA(e);
     return AB2_OK;
 }
 
@@ -548,8 +572,7 @@ AB2_API int ab2_kv_truncate(ab2_kv *kv, int row, int new_len, ab2_stream stream)
     cudaStreamCaptureStatus recording = cudaStreamCaptureStatusNone;
     AB2_CUDA(cudaStreamIsCapturing(s, &recording));
     AB2_REQUIRE(recording == cudaStreamCaptureStatusNone, AB2_ERR_CUDA, "a row cannot be cut while its stream is being captured");
-    int rc = kv_follow(kv, s);
-    if (rc != AB2_OK) return rc;
+    AB2_FOLLOW(kv, stream);
     KvCut cut;
     cut.len = kv->lens_dev + row; cut.new_len = new_len; cut.layers = 0;
     size_t most = 0;
@@ -583,13 +606,24 @@ AB2_API int ab2_kv_truncate(ab2_kv *kv, int row, int new_len, ab2_stream stream)
     }
     if (kv->layers && new_len == 0) { kv->high_host[row] = 0; kv->saved_len[row] = -1; }
     kv->lens_host[row] = new_len;
-    if (cut.len || cut.layers) launch();
-    AB2_LAUNCH_CHECK();
-    // stream-ordered like every other change of the cache; calls on other streams are ordered after it (kv_follow)
-    if (!kv->cut_event) AB2_CUDA(cudaEventCreateWithFlags(&kv->cut_event, cudaEventDisableTiming));
-    AB2_CUDA(cudaEventRecord(kv->cut_event, s));
-    kv->cut_stream = s;
-    kv->cut_pending = true;
+    bool recorded;
+    {
+        // stream-ordered like every other change of the cache; calls on other streams are ordered after it (kv_follow).  One event
+        // stands for all cuts: another thread's, since the call above, is waited for before the event moves on.
+        std::lock_guard<std::mutex> lock(g_cut_mutex);
+        if (!kv->cut_event) AB2_CUDA(cudaEventCreateWithFlags(&kv->cut_event, cudaEventDisableTiming));
+        unsigned long long id = 0;
+        AB2_CUDA(cudaStreamGetId(s, &id));
+        if (kv->cut_pending && id != kv->cut_stream_id) AB2_CUDA(cudaStreamWaitEvent(s, kv->cut_event, 0));
+        if (cut.len || cut.layers) launch();
+        AB2_LAUNCH_CHECK();
+        kv->cut_stream_id = id;
+        AB2_CUDA(cudaEventRecord(kv->cut_event, s));
+        kv->cut_pending = true;
+        recorded = kv->recorded;
+    }
+    // A caller's graph may hold calls on this cache; its launches are not seen here, and may come on any stream.
+    if (recorded) AB2_CUDA(cudaStreamSynchronize(s));
     return AB2_OK;
 }
 
@@ -627,7 +661,7 @@ static int clone_stack(ab2_kv **out, const ab2_kv *src, cudaStream_t s) {
     kv->part_acc = kv->part_ml = nullptr;
     kv->counters = nullptr;
     kv->rows_on = false;
-    kv->cut_event = nullptr; kv->cut_pending = false;
+    kv->cut_event = nullptr; kv->cut_pending = kv->recorded = false;
     cudaError_t e = cudaSuccess;
     auto dup = [&](void **dst, const void *from, size_t bytes, bool contents) {
         if (e == cudaSuccess && from) e = cudaMalloc(dst, bytes);

@@ -41,10 +41,11 @@ struct ab2_kv {
     int *high_host;   // [B] most tokens a row has held since it was last empty (which ring slots are intact)
     int *saved_len;   // [B] length ab2_kv_save_row recorded, -1 none
     size_t part_acc_bytes, part_ml_bytes, counter_bytes;
-    // The last truncation on `cut_stream`, for calls on other streams (kv_follow).
+    // The last truncation, for calls on other streams than its own (kv_follow).
     mutable cudaEvent_t cut_event;
-    mutable cudaStream_t cut_stream;
-    mutable bool cut_pending;
+    mutable unsigned long long cut_stream_id;
+    mutable bool cut_pending;  // not known to have been reached
+    mutable bool recorded;     // calls on this cache were recorded into a caller's graph
 };
 
 namespace ab2 {

@@ -268,7 +268,8 @@ int ab2_kv_append(ab2_kv *kv, int layer, const void *k_dev, const void *v_dev, i
                   const int *positions_dev, int max_seq, ab2_stream stream);
 int ab2_kv_commit(ab2_kv *kv, int S, int row0, int nrows, ab2_stream stream);
 /* KVCache::truncate (kvcache.rs:293-323): cannot grow (AB2_ERR_CAPACITY).  The call does not wait for the GPU: the cut takes
- * its place in `stream`, and calls on this cache from other streams are ordered after it. */
+ * its place in `stream`, and calls on this cache from other streams are ordered after it.  Once calls on the cache have been
+ * recorded into a graph of the caller's, whose launches are not seen here, a cut is waited for. */
 int ab2_kv_truncate(ab2_kv *kv, int row, int new_len, ab2_stream stream);
 /* KVCache::clear (kvcache.rs:284-290). */
 int ab2_kv_clear(ab2_kv *kv, ab2_stream stream);
