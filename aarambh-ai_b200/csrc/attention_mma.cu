@@ -10,8 +10,8 @@
 // fp16 by one shift or none and one logic op a pair (0x6400 | (code ^ 0x80) = 1152 + code, exact)
 // and one exact fp16 subtraction of 1152 on the otherwise idle FMA pipe; the
 // per-token K scale multiplies the f32 score, the per-token V scale is folded
-// into P.  Over a bf16 cache P enters as two bf16 terms, the rounded value and what rounding
-// left (relative error 2^-17), hence 16 MMAs for P.V.
+// into P.  Over a bf16 cache P enters as three bf16 terms, the rounded value and what rounding
+// left of it twice over (together all of its 24 bits), hence 24 MMAs for P.V.
 // Accumulation is f32; softmax is the same online form as the reference
 // (crates/aarambh-studio-kernel/src/cpu/parallel_attn.rs:189-234), in blocks of
 // 16 keys.
@@ -282,12 +282,18 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_co
         }
     }
 
-    float m_ref[2] = {-INFINITY, -INFINITY}, l_part[2] = {0.f, 0.f};  // of heads 2c, 2c+1: reference score; this lane's tokens' sum
-    float o[8][4];                                                     // [d chunk][fragment]: rows d, columns heads 2c, 2c+1
+    // Of heads 2c, 2c+1: reference score; this lane's tokens' sum.  The reference starts at the lowest finite value, so that blocks
+    // of scores of -inf weigh nothing.
+    float m_ref[2] = {-FLT_MAX, -FLT_MAX}, l_part[2] = {0.f, 0.f};
+    float o[8][4];               // [d chunk][fragment]: rows d, columns heads 2c, 2c+1
+    float rest[I8 ? 1 : 8][4];   // the same of what P's rounding to bf16 left: apart, since it is 0 or below 0 where a value may be infinite
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) o[i][j] = 0.f;
+        for (int j = 0; j < 4; ++j) {
+            o[i][j] = 0.f;
+            if constexpr (!I8) rest[i][j] = 0.f;
+        }
 
     const I8Pairs i8;
     // places in a block, from its start; further chunks are exclusive-ors away
@@ -340,20 +346,24 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_co
             if (base + g >= t1) sv[0] = sv[1] = -INFINITY;
             if (base + g + 8 >= t1) sv[2] = sv[3] = -INFINITY;
         }
-        // The reference moves when a score passes it, over bf16 rows by more than 2^8: rare after the first blocks.  (fp16 weights times
-        // their token's scale have no room above 1.)
-        constexpr float ROOM = I8 ? 0.f : 8.f;
-        if (__any_sync(0xffffffffu, !(fmaxf(sv[0], sv[2]) <= m_ref[0] + ROOM) || !(fmaxf(sv[1], sv[3]) <= m_ref[1] + ROOM))) {
+        // The reference moves when a score passes it; over bf16 rows 2^8 ahead, so that it seldom has to after the first blocks (fp16
+        // weights have no bits to spare for that).  No weight is above 1: it would overflow fp16 with its token's scale, and f32 sums
+        // of large bf16 values.
+        constexpr float AHEAD = I8 ? 0.f : 8.f;
+        if (__any_sync(0xffffffffu, !(fmaxf(sv[0], sv[2]) <= m_ref[0]) || !(fmaxf(sv[1], sv[3]) <= m_ref[1]))) {
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 float m = fmaxf(sv[e], sv[2 + e]);
 #pragma unroll
                 for (int x = 4; x < 32; x <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, x));
-                m = fmaxf(m, m_ref[e]);
+                m = m > m_ref[e] ? m + AHEAD : m_ref[e];
                 const float corr = exp2_approx(m_ref[e] - m);
                 l_part[e] *= corr;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) { o[i][e] *= corr; o[i][2 + e] *= corr; }
+                for (int i = 0; i < 8; ++i) {
+                    o[i][e] *= corr; o[i][2 + e] *= corr;
+                    if constexpr (!I8) { rest[i][e] *= corr; rest[i][2 + e] *= corr; }
+                }
                 m_ref[e] = m;
             }
         }
@@ -377,17 +387,31 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_co
                 mma_f16_16816(o[2 * dp + 1], i8.even(r2), i8.odd(r2), i8.even(r3), i8.odd(r3), pb0, pb1);
             }
         } else {
-            const uint32_t pb0 = transposed(pack_bf16(pv[0], pv[1])), pb1 = transposed(pack_bf16(pv[2], pv[3]));
-            const uint32_t pr0 = transposed(pack_bf16(bf16_rest(pv[0]), bf16_rest(pv[1]))), pr1 = transposed(pack_bf16(bf16_rest(pv[2]), bf16_rest(pv[3])));
+            uint32_t pb[3][2];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                pb[i][0] = transposed(pack_bf16(pv[0], pv[1]));
+                pb[i][1] = transposed(pack_bf16(pv[2], pv[3]));
+#pragma unroll
+                for (int j = 0; j < 4; ++j) pv[j] = bf16_rest(pv[j]);
+            }
 #pragma unroll
             for (int ch = 0; ch < 8; ++ch) {
                 uint32_t r0, r1, r2, r3;
                 ldmatrix_trans(r0, r1, r2, r3, (vs + (ch >> 2) * (AT_TOK * 128)) ^ ((ch & 3) << 5));
                 // rows g: d = chunk*16 + g; rows g+8: d + 8
-                mma_bf16_16816(o[ch], r0, r2, r1, r3, pb0, pb1);
-                mma_bf16_16816(o[ch], r0, r2, r1, r3, pr0, pr1);
+                mma_bf16_16816(o[ch], r0, r2, r1, r3, pb[0][0], pb[0][1]);
+                mma_bf16_16816(rest[ch], r0, r2, r1, r3, pb[2][0], pb[2][1]);
+                mma_bf16_16816(rest[ch], r0, r2, r1, r3, pb[1][0], pb[1][1]);
             }
         }
+    }
+    if constexpr (!I8) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (fabsf(o[i][j]) <= FLT_MAX) o[i][j] += rest[i][j];  // infinite: of an infinite value, as it stands
     }
 #pragma unroll
     for (int e = 0; e < 2; ++e)
@@ -416,12 +440,12 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_co
         float L = 0.f, A = 0.f;
 #pragma unroll
         for (int i2 = 0; i2 < S::WARPS; ++i2) {
-            const float e = (wm[i2][hh] == -INFINITY) ? 0.f : exp2f(wm[i2][hh] - M);
+            const float e = exp2f(wm[i2][hh] - M);
             L += e * wl[i2][hh];
             A += e * wacc[(i2 * 8 + hh) * HD + d];
         }
         if (w.splits == 1) {
-            st_out(a.out, a.dtype, ((size_t)rrow * a.h + kvhead * a.rep + hh) * HD + d, L > 0.f ? A * (1.0f / L) : A);
+            st_out(a.out, a.dtype, ((size_t)rrow * a.h + kvhead * a.rep + hh) * HD + d, A * (1.0f / L));
         } else {
             const size_t pi = pi0 + (size_t)hh * a.nsplit + w.split;
             a.part_acc[pi * HD + d] = A;
@@ -449,7 +473,7 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_co
         float L = ex * x.y + ey * y.y;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
-        const float inv = L > 0.f ? 1.0f / L : 1.0f;
+        const float inv = 1.0f / L;
         weight[hh][lane] = ex * inv;
         weight[hh][lane + 32] = ey * inv;
     }

@@ -44,3 +44,54 @@ def test_decode_attention(kv, h, kvh, lens):
         assert float((got[row] - want).norm()) <= 2.0 ** -8 * float(want.norm())
     again = p.dispatch.attention_decode(cache, q, 128 ** -0.5).double().view(len(lens), h, 128)
     assert torch.equal(got, again)  # the arrival counters are back at rest, and the merge does not depend on the order
+
+
+@pytest.mark.parametrize("n", [9, 700])
+def test_bf16_values_at_the_ends_of_the_range(n):
+    """Infinite values come out infinite; weighted sums of large ones do not overflow; keys whose scores are -inf weigh nothing,
+    a whole block of them ahead of the others too."""
+    p = pkg()
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    cache = p.KVCache(n + 3, 2, 128, 8, batch=3, dtype="bf16")
+    k, v = (torch.randn((3, n, 2, 128), generator=gen, device="cuda").bfloat16() for _ in range(2))
+    q = torch.randn((3, 8, 128), generator=gen, device="cuda").bfloat16()
+    q[:, :, 0] = 1
+    v[0, n // 2, 0, 5], v[0, n // 3, 1, 77] = math.inf, -math.inf
+    # scores that rise by 8 powers of two from one of a warp's blocks to the next; a weighted sum of the values has room for weights of
+    # up to 1 of a hundred tokens
+    k[1], q[1] = 0, 0
+    q[1, :, 1], k[1, :, :, 1] = 1, (torch.arange(n, device="cuda") // 64 * 60)[:, None].bfloat16()
+    v[1, :, :, 3] = 3e36
+    k[2, :min(n - 1, 80), :, 0] = -math.inf
+    for row in range(3):
+        cache.append(0, k[row:row + 1], v[row:row + 1], row0=row)
+        cache.commit(n, row0=row, nrows=1)
+    got = p.dispatch.attention_decode(cache, q, 128 ** -0.5).double().view(3, 8, 128)
+    for row in range(3):
+        want = attend(q[row], k[row], v[row])
+        if row == 0:
+            assert (got[0, :4, 5] == math.inf).all() and (got[0, 4:, 77] == -math.inf).all()
+            got[0, :4, 5] = got[0, 4:, 77] = want[:4, 5] = want[4:, 77] = 0
+        assert torch.isfinite(got[row]).all() and torch.isfinite(want).all()
+        for d in range(128):  # a column at a time: one of row 1 is far larger than the others
+            assert float((got[row, :, d] - want[:, d]).norm()) <= 2.0 ** -7 * float(want[:, d].norm()) + 2.0 ** -8
+
+
+@pytest.mark.parametrize("kv,dtype,shift", [("int8", torch.bfloat16, 1), ("bf16", torch.bfloat16, 3), ("int8", torch.float16, 0), ("int8", torch.float32, 0), ("int8", torch.float32, 1)])
+def test_queries_of_other_types_and_places(kv, dtype, shift):
+    """f32 and f16 queries, queries off 16 bytes, rows from the middle of a cache; rows that are split and rows that are not."""
+    p = pkg()
+    lens, row0, h, g = [5, 900, 2100, 31, 1500], 2, 12, 4
+    gen = torch.Generator(device="cuda").manual_seed(shift)
+    cache = p.KVCache(2200, g, 128, h, batch=row0 + len(lens), dtype=kv)
+    for row, n in enumerate(lens):
+        k, v = (torch.randn((1, n, g, 128), generator=gen, device="cuda").bfloat16() for _ in range(2))
+        cache.append(0, k, v, row0=row0 + row)
+        cache.commit(n, row0=row0 + row, nrows=1)
+    room = torch.randn(len(lens) * h * 128 + shift, generator=gen, device="cuda").bfloat16().to(dtype)
+    q = room[shift:].view(len(lens), h, 128)
+    got = p.dispatch.attention_decode(cache, q, 128 ** -0.5, row0=row0).double()
+    for row in range(len(lens)):
+        want = attend(q[row], *cache.read(row0 + row))
+        # weights of 11 bits over INT8 rows, and the output's rounding
+        assert float((got[row] - want).norm()) <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -10) * float(want.norm())
