@@ -294,7 +294,7 @@ int attention_cached_device(const ab2_kv *kv, int layer, const void *q, void *ou
     if (S == 1 && attention_decode_mma_serves(kv, dtype) && st.q_h == kv->hd && st.o_h == st.q_h && st.o_b == (long long)kv->h * kv->hd) {
         // INT8 or bf16 cache, head_dim 128: tensor-core flash-decode (attention_mma.cu)
         nsplit = decode_split_count(kv, nrows, max_len, kv->max_splits, true);
-        return attention_decode_mma_device(kv, layer, q, out, row0, nrows, scale, dtype, nsplit, kv->part_acc, kv->part_ml, pending, st.q_b, s);
+        return attention_decode_mma_device(kv, layer, q, out, row0, nrows, scale, dtype, max_len, nsplit, kv->part_acc, kv->part_ml, pending, st.q_b, s);
     }
     if (S > 1) {
         // prefill chunk of a bf16 model: the tcgen05 kernel (attention_prompt_tc.cu) where it is the faster one; few queries, short
@@ -453,7 +453,7 @@ AB2_API int ab2_attention_decode_static(const ab2_kv *kv, int layer, const void 
     cudaStream_t s = (cudaStream_t)stream;
     dim3 grid(a.nsplit, kv->kvh, nrows);
     if (mma_path)
-        return attention_decode_mma_device(kv, layer, q_dev, out_dev, row0, nrows, scale, dtype, a.nsplit, a.part_acc,
+        return attention_decode_mma_device(kv, layer, q_dev, out_dev, row0, nrows, scale, dtype, max_len, a.nsplit, a.part_acc,
                                            a.part_ml, 0, (long long)kv->h * kv->hd, s);
     if (kv->dtype == AB2_KV_F32) rc = launch_split_hd<AB2_KV_F32>(a, grid, s);
     else if (kv->dtype == AB2_KV_BF16) rc = launch_split_hd<AB2_KV_BF16>(a, grid, s);

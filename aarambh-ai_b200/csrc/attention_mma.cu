@@ -38,6 +38,7 @@ struct MmaAttnArgs {
     // CTAs of a KV head that are resident at once; most splits of a row; fewest tokens of a split; rows of up to that many are not split
     int slots, nsplit, min_tokens, whole_tokens;
     int pending;    // appended, not yet committed tokens per row: they are attended too
+    bool whole;     // no row is split: a CTA's row is its index
     float scale;
     float *part_acc, *part_ml;  // [row][head][nsplit]
     int *counters;  // [row][kv head] splits that have arrived, zero at rest
@@ -219,8 +220,14 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_co
     __syncthreads();
     pdl_wait();  // inputs come from the preceding kernel of the step
     pdl_launch_dependents();
-    const AtShare w = at_share(a, (int)blockIdx.x, lane);
-    if (w.rrow < 0) return;
+    AtShare w;
+    if (a.whole) {
+        w.rrow = (int)blockIdx.x; w.split = 0; w.splits = 1;
+        w.t0 = 0; w.t1 = a.kv.lens[kv_row(a.kv, a.row0, w.rrow)] + a.pending;
+    } else {
+        w = at_share(a, (int)blockIdx.x, lane);
+        if (w.rrow < 0) return;
+    }
     const int kvhead = blockIdx.y, rrow = w.rrow, row = kv_row(a.kv, a.row0, rrow), t0 = w.t0, t1 = w.t1;
     const size_t head_base = ((size_t)row * a.kv.kvh + kvhead) * a.kv.cap;
     uint8_t *ring = at_smem + warp * S::WARP;
@@ -751,7 +758,7 @@ bool attention_decode_mma_serves(const ab2_kv *kv, ab2_dtype dtype) {
 }
 
 int attention_decode_mma_device(const ab2_kv *kv, int layer, const void *q, void *out, int row0, int nrows,
-                                float scale, ab2_dtype dtype, int nsplit, float *part_acc, float *part_ml,
+                                float scale, ab2_dtype dtype, int max_len, int nsplit, float *part_acc, float *part_ml,
                                 int pending, long long q_stride, cudaStream_t s) {
     MmaAttnArgs a;
     a.kv = kv_view(kv, layer);
@@ -762,7 +769,9 @@ int attention_decode_mma_device(const ab2_kv *kv, int layer, const void *q, void
     a.min_tokens = 256; a.whole_tokens = 512;
     const int resident = device_sm_count() * (kv->dtype == AB2_KV_INT8 ? AtShape<AB2_KV_INT8>::CTAS : AtShape<AB2_KV_BF16>::CTAS);
     a.slots = std::max(1, resident / kv->kvh);
-    const dim3 grid((unsigned)std::max<long long>(nrows, std::min<long long>(a.slots, (long long)nrows * nsplit)), kv->kvh);
+    // What the launch would find from lengths that the host can bound: no CTA has to read all rows' lengths.
+    a.whole = nsplit == 1 || max_len <= a.whole_tokens;
+    const dim3 grid((unsigned)(a.whole ? nrows : std::max<long long>(nrows, std::min<long long>(a.slots, (long long)nrows * nsplit))), kv->kvh);
     return kv->dtype == AB2_KV_INT8 ? launch_decode_mma<AB2_KV_INT8>(a, grid, s) : launch_decode_mma<AB2_KV_BF16>(a, grid, s);
 }
 

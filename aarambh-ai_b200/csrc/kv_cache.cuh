@@ -127,7 +127,7 @@ int attention_cached_device(const ab2_kv *kv, int layer, const void *q, void *ou
 // scratch and are merged by the same launch (kv's arrival counters).
 bool attention_decode_mma_serves(const ab2_kv *kv, ab2_dtype dtype);
 int attention_decode_mma_device(const ab2_kv *kv, int layer, const void *q, void *out, int row0, int nrows,
-                                float scale, ab2_dtype dtype, int nsplit, float *part_acc, float *part_ml,
+                                float scale, ab2_dtype dtype, int max_len, int nsplit, float *part_acc, float *part_ml,
                                 int pending, long long q_stride, cudaStream_t s);
 // Causal attention of S > 1 new queries per row over an INT8 cache (head_dim 128, up to 4 query
 // heads per KV head) on the tensor cores; AB2_ERR_UNSUPPORTED for other layouts.
