@@ -279,6 +279,16 @@ static int decode_split_count(const ab2_kv *kv, int nrows, int max_len, int max_
     return std::max(1, std::min(std::min(want, (max_len + 255) / 256), max_splits));
 }
 
+// Whether a call of its own over one query per row takes the tensor-core kernel.  bf16 rows of a handful of tokens are served faster
+// by CUDA cores: us, CUDA cores / tensor cores, 24 x 4 at 8 / 8 heads 3.8 / 4.6, 128 x 16 6.4 / 8.1, 96 x 24 at 32 / 8 10.7 / 11.0, but
+// 37 x 16 at 8 / 8 4.9 / 4.8 and 16 / 2 heads, 200 x 4 10.3 / 9.9.
+static bool decode_on_tensor_cores(const ab2_kv *kv, ab2_dtype dtype, int nrows, int max_len) {
+    if (!attention_decode_mma_serves(kv, dtype)) return false;
+    if (kv->dtype != AB2_KV_BF16 || kv->h / kv->kvh > 4) return true;
+    return max_len > (nrows * kv->kvh > 2 * device_sm_count() ? 24 : 8);
+}
+
+// len_hint: what bounds the rows' lengths in a recorded step; 0 a step that is not, -1 a call of its own.
 int attention_cached_device(const ab2_kv *kv, int layer, const void *q, void *out, int S, int pending,
                             int row0, int nrows, float scale, ab2_dtype dtype, AttnStrides st,
                             int len_hint, cudaStream_t s) {
@@ -287,11 +297,12 @@ int attention_cached_device(const ab2_kv *kv, int layer, const void *q, void *ou
     a.q = q; a.out = out; a.st = st; a.S = S; a.pending = pending; a.row0 = row0; a.h = kv->h;
     a.rep = kv->h / kv->kvh;
     a.dtype = (int)dtype; a.scale = scale; a.part_acc = kv->part_acc; a.part_ml = kv->part_ml;
-    int max_len = len_hint;
-    if (max_len <= 0)
+    int max_len = std::max(0, len_hint);
+    if (max_len == 0)
         for (int i = 0; i < nrows; ++i) max_len = std::max(max_len, kv->lens_host[kv_row_host(kv, row0, i)] + pending);
     int nsplit = 1;
-    if (S == 1 && attention_decode_mma_serves(kv, dtype) && st.q_h == kv->hd && st.o_h == st.q_h && st.o_b == (long long)kv->h * kv->hd) {
+    const bool mma = len_hint < 0 ? decode_on_tensor_cores(kv, dtype, nrows, max_len) : attention_decode_mma_serves(kv, dtype);
+    if (S == 1 && mma && st.q_h == kv->hd && st.o_h == st.q_h && st.o_b == (long long)kv->h * kv->hd) {
         // INT8 or bf16 cache, head_dim 128: tensor-core flash-decode (attention_mma.cu)
         nsplit = decode_split_count(kv, nrows, max_len, kv->max_splits, true);
         return attention_decode_mma_device(kv, layer, q, out, row0, nrows, scale, dtype, max_len, nsplit, kv->part_acc, kv->part_ml, pending, st.q_b, s);
@@ -384,7 +395,7 @@ AB2_API int ab2_attention_decode(const ab2_kv *kv, int layer, const void *q_dev,
     AttnStrides st;
     st.q_b = (long long)kv->h * kv->hd; st.q_s = 0; st.q_h = kv->hd;
     st.o_b = st.q_b; st.o_s = 0; st.o_h = kv->hd;
-    return attention_cached_device(kv, layer, q_dev, out_dev, 1, 0, row0, nrows, scale, dtype, st, 0, (cudaStream_t)stream);
+    return attention_cached_device(kv, layer, q_dev, out_dev, 1, 0, row0, nrows, scale, dtype, st, -1, (cudaStream_t)stream);
 }
 
 AB2_API int ab2_attention_cached(const ab2_kv *kv, int layer, const void *q_dev, void *out_dev, int S,
@@ -395,7 +406,7 @@ AB2_API int ab2_attention_cached(const ab2_kv *kv, int layer, const void *q_dev,
     AttnStrides st;  // q, out: [nrows][S][h][hd]
     st.q_h = kv->hd; st.q_s = (long long)kv->h * kv->hd; st.q_b = st.q_s * S;
     st.o_h = st.q_h; st.o_s = st.q_s; st.o_b = st.q_b;
-    return attention_cached_device(kv, layer, q_dev, out_dev, S, 0, row0, nrows, scale, dtype, st, 0, (cudaStream_t)stream);
+    return attention_cached_device(kv, layer, q_dev, out_dev, S, 0, row0, nrows, scale, dtype, st, -1, (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -439,7 +450,7 @@ AB2_API int ab2_attention_decode_static(const ab2_kv *kv, int layer, const void 
     for (int r = row0; r < row0 + nrows; ++r) max_len = std::max(max_len, kv->lens_host[r]);
     // Kernel choice and split count come from the helpers ab2_attention_decode uses (with the
     // cache's own split limit), so both entry points return the same bits.
-    const bool mma_path = attention_decode_mma_serves(kv, dtype);
+    const bool mma_path = decode_on_tensor_cores(kv, dtype, nrows, max_len);
     a.nsplit = decode_split_count(kv, nrows, max_len, kv->max_splits, mma_path);
     // Partials are indexed by the absolute row, exactly as in the allocated scratch.
     const size_t parts = (size_t)(row0 + nrows) * kv->h * a.nsplit;
@@ -507,7 +518,7 @@ AB2_API int ab2_attention_causal(const void *q_dev, const void *k_dev, const voi
         st.q_s = head_dim; st.q_h = (long long)q_len * head_dim; st.q_b = st.q_h * h;
         st.o_s = st.q_s; st.o_h = st.q_h; st.o_b = st.q_b;
         // q_len queries over a context whose last q_len positions are theirs
-        rc = attention_cached_device(&view, 0, q_dev, out_dev, q_len, 0, 0, b, scale, dtype, st, 0, (cudaStream_t)stream);
+        rc = attention_cached_device(&view, 0, q_dev, out_dev, q_len, 0, 0, b, scale, dtype, st, -1, (cudaStream_t)stream);
     }
     if (rc == AB2_OK && cudaStreamSynchronize((cudaStream_t)stream) != cudaSuccess)
         rc = fail(AB2_ERR_CUDA, "attention kernel failed");

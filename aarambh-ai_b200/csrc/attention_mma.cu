@@ -120,15 +120,15 @@ __device__ __forceinline__ void ldmatrix_trans(uint32_t &r0, uint32_t &r1, uint3
 // 115 -> 86, 32 x 700 17.5 -> 15.6, 1 x 4096 24 -> 13, 1 x 512 8.8 -> 8.0; bf16 64 x 2048 215 -> 77 (0.94), 8 x 8192 159 -> 48,
 // 32 x 700 52 -> 19, 1 x 512 16 -> 10.
 constexpr int AT_STAGES = 3, AT_TOK = 16, AT_HD = 128;
-template <int KVD>
+template <int KVD, bool MANY>  // MANY: short rows, many of them
 struct AtShape {
     static constexpr bool I8 = KVD == AB2_KV_INT8;
-    static constexpr int WARPS = I8 ? 8 : 4, STRIDE = WARPS * AT_TOK;  // a warp takes every WARPS-th block
+    static constexpr int WARPS = (I8 ? 8 : 4) / (MANY ? 2 : 1), STRIDE = WARPS * AT_TOK;  // a warp takes every WARPS-th block
     static constexpr int TILES = I8 ? 1 : 2;                     // tiles of 16 tokens x 128 bytes that hold the keys, or values, of a block
     static constexpr int BLOCK = TILES * AT_TOK * 128, STAGE = 2 * BLOCK, WARP = AT_STAGES * STAGE;
     static constexpr int SCALES = I8 ? AT_STAGES * 2 * AT_TOK * 4 : 0;  // of a warp
     static constexpr int SMEM = 1024 + WARPS * (WARP + SCALES);
-    static constexpr int CTAS = 2;                               // of an SM
+    static constexpr int CTAS = MANY ? 4 : 2;                    // of an SM
     static_assert(WARP >= 8 * AT_HD * 4, "the warps' sums are merged in the rings' place");
 };
 
@@ -192,10 +192,10 @@ __device__ __forceinline__ AtShare at_share(const MmaAttnArgs &a, int cta, int l
 }
 
 // grid (CTAs of a KV head, kv heads); head_dim 128.
-template <int KVD>
-__global__ void __launch_bounds__(32 * AtShape<KVD>::WARPS, AtShape<KVD>::CTAS)
+template <int KVD, bool MANY>
+__global__ void __launch_bounds__(32 * AtShape<KVD, MANY>::WARPS, AtShape<KVD, MANY>::CTAS)
 attn_decode_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, MmaAttnArgs a, int *status) {
-    using S = AtShape<KVD>;
+    using S = AtShape<KVD, MANY>;
     constexpr int HD = AT_HD;
     constexpr bool I8 = S::I8;
     extern __shared__ uint8_t at_smem_raw[];
@@ -724,15 +724,16 @@ __global__ void __launch_bounds__(128) attn_prefill_mma_kernel(PrefillAttnArgs a
 
 }  // namespace
 
-template <int KVD>
+template <int KVD, bool MANY>
 static int launch_decode_mma(const MmaAttnArgs &a, dim3 grid, cudaStream_t s) {
-    constexpr int smem = AtShape<KVD>::SMEM;
+    using S = AtShape<KVD, MANY>;
+    constexpr int smem = S::SMEM;
     static bool configured[64] = {false};  // the attribute is per device
     int dev = 0;
     AB2_CUDA(cudaGetDevice(&dev));
     AB2_REQUIRE(dev >= 0 && dev < 64, AB2_ERR_BAD_ARG, "device index %d out of range", dev);
     if (!configured[dev]) {
-        AB2_CUDA(cudaFuncSetAttribute(attn_decode_mma_kernel<KVD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        AB2_CUDA(cudaFuncSetAttribute(attn_decode_mma_kernel<KVD, MANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         configured[dev] = true;
     }
     int *status = nullptr;
@@ -746,7 +747,7 @@ static int launch_decode_mma(const MmaAttnArgs &a, dim3 grid, cudaStream_t s) {
     rc = make_rows_map(&kmap, type, elem, a.kv.k, (int)rows, AT_HD, AT_HD, AT_TOK);
     if (rc == AB2_OK) rc = make_rows_map(&vmap, type, elem, a.kv.v, (int)rows, AT_HD, AT_HD, AT_TOK);
     if (rc != AB2_OK) return rc;
-    cudaError_t e = launch_kernel(attn_decode_mma_kernel<KVD>, grid, dim3(32 * AtShape<KVD>::WARPS), smem, s, kmap, vmap, a, status);
+    cudaError_t e = launch_kernel(attn_decode_mma_kernel<KVD, MANY>, grid, dim3(32 * S::WARPS), smem, s, kmap, vmap, a, status);
     if (e != cudaSuccess) return fail(AB2_ERR_CUDA, "decode attention launch failed: %s", cudaGetErrorString(e));
     return AB2_OK;
 }
@@ -767,12 +768,16 @@ int attention_decode_mma_device(const ab2_kv *kv, int layer, const void *q, void
     a.pending = pending; a.q_stride = q_stride;
     // A split costs its arrival and the merge, about 3 us: as long as 512 tokens of a CTA of its own.
     a.min_tokens = 256; a.whole_tokens = 512;
-    const int resident = device_sm_count() * (kv->dtype == AB2_KV_INT8 ? AtShape<AB2_KV_INT8>::CTAS : AtShape<AB2_KV_BF16>::CTAS);
-    a.slots = std::max(1, resident / kv->kvh);
+    // Short rows, more of them than the larger CTAs that are resident at once: CTAs of half the warps, twice as many.  us, 8 / 8 heads,
+    // larger and smaller: INT8 48 x 16 8.0, 5.0, 64 x 256 12.2, 10.8; bf16 96 x 4 11.2, 8.5, 64 x 256 17.0, 15.4; but long rows bf16 96 x 1500
+    // 93, 108, INT8 64 x 4096 ragged 72, 83.
+    const bool many = max_len <= a.whole_tokens && nrows * kv->kvh > 2 * device_sm_count();
+    a.slots = std::max(1, device_sm_count() * 2 / kv->kvh);
     // What the launch would find from lengths that the host can bound: no CTA has to read all rows' lengths.
     a.whole = nsplit == 1 || max_len <= a.whole_tokens;
     const dim3 grid((unsigned)(a.whole ? nrows : std::max<long long>(nrows, std::min<long long>(a.slots, (long long)nrows * nsplit))), kv->kvh);
-    return kv->dtype == AB2_KV_INT8 ? launch_decode_mma<AB2_KV_INT8>(a, grid, s) : launch_decode_mma<AB2_KV_BF16>(a, grid, s);
+    if (kv->dtype == AB2_KV_INT8) return many ? launch_decode_mma<AB2_KV_INT8, true>(a, grid, s) : launch_decode_mma<AB2_KV_INT8, false>(a, grid, s);
+    return many ? launch_decode_mma<AB2_KV_BF16, true>(a, grid, s) : launch_decode_mma<AB2_KV_BF16, false>(a, grid, s);
 }
 
 // S > 1 queries per row over an INT8 cache, head_dim 128, 1..4 query heads per KV head: the

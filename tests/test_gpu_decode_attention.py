@@ -25,6 +25,11 @@ def attend(q, k, v):
     (8, 2, [1, 3000, 40, 1025, 700]),
     (32, 8, [5000]),
     (16, 2, [(37 * r) % 900 + 1 for r in range(70)]),
+    (8, 8, [(5 * r) % 24 + 1 for r in range(40)]),      # more short rows than larger CTAs, the shortest over bf16 on CUDA cores
+    (8, 8, [(13 * r) % 512 + 1 for r in range(40)]),
+    (32, 8, [25 + r % 3 for r in range(64)]),
+    (8, 2, [3, 8, 1]),
+    (8, 2, [9, 8, 1]),
 ])
 def test_decode_attention(kv, h, kvh, lens):
     p = pkg()
@@ -95,3 +100,15 @@ def test_queries_of_other_types_and_places(kv, dtype, shift):
         want = attend(q[row], *cache.read(row0 + row))
         # weights of 11 bits over INT8 rows, and the output's rounding
         assert float((got[row] - want).norm()) <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -10) * float(want.norm())
+
+
+@pytest.mark.parametrize("n", [1, 5, 100, 3000])
+@pytest.mark.parametrize("b,h,kvh", [(2, 8, 2), (50, 8, 8)])
+def test_one_query_over_keys_and_values_of_the_caller(b, h, kvh, n):
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    n = min(n, 100) if b > 2 else n
+    q, k, v = (torch.randn((b, heads, t, 128), generator=gen, device="cuda").bfloat16() for heads, t in ((h, 1), (kvh, n), (kvh, n)))
+    got = pkg().dispatch.attention_forward_causal(q, k, v, 128 ** -0.5).double()
+    for row in range(b):
+        want = attend(q[row, :, 0], k[row].transpose(0, 1), v[row].transpose(0, 1))
+        assert float((got[row, :, 0] - want).norm()) <= 2.0 ** -8 * float(want.norm())
