@@ -451,14 +451,20 @@ AB2_API int ab2_attention_decode_static(const ab2_kv *kv, int layer, const void 
     // Kernel choice and split count come from the helpers ab2_attention_decode uses (with the
     // cache's own split limit), so both entry points return the same bits.
     const bool mma_path = decode_on_tensor_cores(kv, dtype, nrows, max_len);
-    a.nsplit = decode_split_count(kv, nrows, max_len, kv->max_splits, mma_path);
+    // The splits that have to fit, or the call is refused.  The tensor-core kernel may deal out more than these (over short rows of
+    // many sequences, and over bf16 caches, whose other kernel's count this is): those are cut down to what the scratch holds,
+    // and only then do the two entry points differ in the order of their sums.
+    const bool alone = mma_path && kv->dtype == AB2_KV_INT8 && nrows * kv->kvh >= device_sm_count() && max_len <= 1024;
+    const int least = alone ? 1 : decode_split_count(kv, nrows, max_len, kv->max_splits, mma_path && kv->dtype == AB2_KV_INT8);
     // Partials are indexed by the absolute row, exactly as in the allocated scratch.
-    const size_t parts = (size_t)(row0 + nrows) * kv->h * a.nsplit;
-    const size_t need = parts * ((size_t)kv->hd + 2);
-    AB2_REQUIRE(a.nsplit == 1 || need <= AB2_STATIC_SCRATCH_FLOATS, AB2_ERR_CAPACITY,
+    const size_t of_split = (size_t)(row0 + nrows) * kv->h * ((size_t)kv->hd + 2);
+    AB2_REQUIRE(least == 1 || of_split * least <= AB2_STATIC_SCRATCH_FLOATS, AB2_ERR_CAPACITY,
                 "decode attention needs %zu floats of split scratch (rows %d, heads %d, splits %d) but the "
                 "static scratch holds %u; use ab2_attention_decode",
-                need, row0 + nrows, kv->h, a.nsplit, (unsigned)AB2_STATIC_SCRATCH_FLOATS);
+                of_split * least, row0 + nrows, kv->h, least, (unsigned)AB2_STATIC_SCRATCH_FLOATS);
+    const int most = decode_split_count(kv, nrows, max_len, kv->max_splits, mma_path);
+    a.nsplit = std::max(1, (int)std::min<size_t>(most, AB2_STATIC_SCRATCH_FLOATS / of_split));
+    const size_t parts = (size_t)(row0 + nrows) * kv->h * a.nsplit;
     a.part_acc = g_static_attn_scratch_ptr[dev];
     a.part_ml = g_static_attn_scratch_ptr[dev] + parts * kv->hd;
     cudaStream_t s = (cudaStream_t)stream;

@@ -112,3 +112,24 @@ def test_one_query_over_keys_and_values_of_the_caller(b, h, kvh, n):
     for row in range(b):
         want = attend(q[row, :, 0], k[row].transpose(0, 1), v[row].transpose(0, 1))
         assert float((got[row, :, 0] - want).norm()) <= 2.0 ** -8 * float(want.norm())
+
+
+@pytest.mark.parametrize("kv,row0,rows,lens", [("bf16", 40, 1, 2048), ("bf16", 100, 3, 700), ("int8", 230, 20, 900), ("int8", 250, 38, 1024), ("bf16", 0, 2, 2048)])
+def test_fixed_scratch_serves_what_it_served(kv, row0, rows, lens):
+    """Rows far up in a cache: the most splits of the tensor-core kernel would not fit the fixed array, fewer do."""
+    p = pkg()
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    h, g = 32, 8
+    cache = p.KVCache(lens, g, 128, h, batch=row0 + rows, dtype=kv)
+    for row in range(row0, row0 + rows):
+        n = lens - 17 * (row - row0)
+        k, v = (torch.randn((1, n, g, 128), generator=gen, device="cuda").bfloat16() for _ in range(2))
+        cache.append(0, k, v, row0=row)
+        cache.commit(n, row0=row, nrows=1)
+    q = torch.randn((rows, h, 128), generator=gen, device="cuda").bfloat16()
+    got = p.dispatch.attention_decode_static(cache, q, 128 ** -0.5, torch.empty_like(q), row0=row0).double()
+    for row in range(rows):
+        want = attend(q[row], *cache.read(row0 + row))
+        assert float((got[row] - want).norm()) <= 2.0 ** -8 * float(want.norm())
+    if row0 == 0:
+        assert torch.equal(got, p.dispatch.attention_decode(cache, q, 128 ** -0.5).double())
