@@ -135,16 +135,17 @@ __global__ void reorder_shards_kernel(const T *in, T *out, int rows, int vn, int
 
 // Decode attention as rotation + append + tensor-core flash-decode instead of the one-launch kernels on CUDA cores.  Those win
 // while the launch is what matters; they are bound by the conversions to f32 once a step reads many cached tokens, over bf16
-// caches sooner (their kernel there reads rows uncoalesced).  Steps of two 4096-wide layers, us, one launch / two: INT8 1 x 512
-// 147 / 154, 1 x 2048 165 / 158, 4 x 256 186 / 193, 2 x 512 190 / 184, 8 x 256 226 / 216, 16 x 64 207 / 207, 32 x 32 264 / 246; bf16
-// 1 x 32 144 / 141, 8 x 64 211 / 216, 2 x 512 189 / 186, 32 x 32 244 / 244, 32 x 700 322 / 269.
+// caches sooner (their kernel there reads rows uncoalesced).  Over INT8 rows the tensor-core kernel takes weights times their
+// token's scale in 11 bits where the other takes 24: it serves what it pays for by a wide margin and has always served, not more
+// (1 x 5000 and 64 x 16 would gain).  Steps of two 4096-wide layers, us, one launch / two: INT8 1 x 512 134 / 141, 1 x 5000 168 / 150,
+// 1 x 7000 178 / 152, 2 x 500 166 / 165, 4 x 512 200 / 182, 8 x 128 192 / 188, 16 x 128 188 / 172, 64 x 16 274 / 234; bf16 1 x 16 133 / 128,
+// 1 x 512 148 / 141, 8 x 64 190 / 186, 2 x 500 174 / 167, 32 x 8 187 / 188, 64 x 128 246 / 239.
 static bool decode_attention_on_tensor_cores(const ab2_kv *kv, ab2_dtype dtype, int nrows, int max_len) {
     if (!attention_decode_mma_serves(kv, dtype)) return false;
     static const char *force = getenv("AB2_DECODE_ATTN");
     if (force) return strcmp(force, "mma") == 0;
-    const bool bf16 = kv->dtype == AB2_KV_BF16;
-    if (nrows == 1) return bf16 || max_len > 1200;
-    return nrows >= 16 || nrows * (long long)max_len > (bf16 ? 512 : 1024);
+    if (kv->dtype == AB2_KV_BF16) return nrows == 1 || nrows >= 16 || nrows * (long long)max_len > 512;
+    return nrows >= 2 ? nrows * (long long)max_len > 1024 : max_len > 6144;
 }
 
 #define STEP(expr)                     \

@@ -7,6 +7,7 @@ import pytest
 import torch
 
 from helpers import pkg
+from model_fixtures import SMALL, build_pair
 
 pytestmark = pytest.mark.gpu
 
@@ -133,3 +134,29 @@ def test_fixed_scratch_serves_what_it_served(kv, row0, rows, lens):
         assert float((got[row] - want).norm()) <= 2.0 ** -8 * float(want.norm())
     if row0 == 0:
         assert torch.equal(got, p.dispatch.attention_decode(cache, q, 128 ** -0.5).double())
+
+
+@pytest.mark.parametrize("rows,n", [(1, 1300), (1, 4000), (2, 300)])
+def test_steps_over_int8_rows_whose_scales_have_no_room_in_fp16(rows, n):
+    """Values of 10^7: a step takes their scales, times a weight, in f32.  Against an f32 cache of the same values."""
+    c = dict(SMALL, n_layers=1, n_heads=4, n_kv_heads=2, head_dim=128, max_seq=4100)
+    model, _, _ = build_pair(c, dtype=torch.bfloat16)
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    k, v = (torch.randn((rows, n, 2, 128), generator=gen, device="cuda").bfloat16() for _ in range(2))
+    v = (v.float() * 3e7).bfloat16()
+    out = []
+    for kv in ("int8", "f32"):
+        cache = pkg().KVCache(n + 4, 2, 128, 4, batch=rows, dtype=kv)
+        cache.append(0, k, v)
+        cache.commit(n)
+        ids = torch.arange(1, rows + 1, dtype=torch.int32, device="cuda")
+        logits = torch.empty((rows, 1, c["vocab"]), device="cuda", dtype=model.logits_dtype)
+        stream = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            model.decode_step(ids, cache, logits, None)
+        torch.cuda.synchronize()
+        out.append(logits.double())
+    assert torch.isfinite(out[0]).all() and torch.isfinite(out[1]).all()
+    # codes of 7 bits and a sign: a value's error is at most 2^-8 of its token's largest, about 3 standard deviations
+    assert float((out[0] - out[1]).norm()) <= 3 * 2.0 ** -8 * float(out[1].norm())
