@@ -72,10 +72,11 @@ static_assert(gf_stages<LIN_DENSE, false>() == GF_MAX_STAGES, "barriers for the 
 struct GfRange {
     int tiles, ks, ctas;
     bool whole;
-    __device__ __forceinline__ GfRange(int tiles_, int ks_, int ctas_) : tiles(tiles_), ks(ks_), ctas(ctas_) {
+    __host__ __device__ static bool in_whole(int tiles, int ctas) {
         const int rounds = (tiles + ctas - 1) / ctas;
-        whole = rounds == 1 ? tiles * 20 >= ctas * 13 : rounds * ctas * 5 <= tiles * 6;
+        return rounds == 1 ? tiles * 20 >= ctas * 13 : rounds * ctas * 5 <= tiles * 6;
     }
+    __device__ __forceinline__ GfRange(int tiles_, int ks_, int ctas_) : tiles(tiles_), ks(ks_), ctas(ctas_), whole(in_whole(tiles_, ctas_)) {}
     __device__ __forceinline__ int begin(int c) const {
         return whole ? (int)((long long)c * tiles / ctas) * ks : (int)((long long)c * tiles * ks / ctas);
     }
@@ -352,6 +353,17 @@ int clusters_at_once(int size, size_t smem) {
 }
 
 template <int MODE, bool CLUSTER>
+constexpr size_t gf_smem_bytes() { return 1024 + (size_t)gf_stages<MODE, CLUSTER>() * gf_stage_bytes<MODE>() + gf_part_bytes<MODE, CLUSTER>() + sizeof(GfShared); }
+
+// CTAs of a tile's cluster: the most of which all tiles' run side by side.
+template <int MODE>
+int gf_cluster(int tiles, int K) {
+    int cluster = GF_MAX_CLUSTER;
+    while (cluster > 2 && (cluster > (K + 63) / 64 || tiles > clusters_at_once<MODE>(cluster, gf_smem_bytes<MODE, true>()))) cluster >>= 1;
+    return cluster;
+}
+
+template <int MODE, bool CLUSTER>
 int launch_few(const LinArgs &a, int ctas, const DecodeGemmScratch &sc, cudaStream_t s) {
     int cluster = 1;
     int *status = nullptr;
@@ -362,7 +374,7 @@ int launch_few(const LinArgs &a, int ctas, const DecodeGemmScratch &sc, cudaStre
     if (rc == AB2_OK) rc = make_rows_map(&w2map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, gf_dual<MODE>() ? a.w2 : a.w, a.N, a.K, a.K, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
     if (rc == AB2_OK) rc = make_x_map(&xmap, a.x, a.M, a.K, GF_BOX_ROWS, MODE == LIN_DENSE ? a.ldx : a.K);
     if (rc != AB2_OK) return rc;
-    const size_t smem = 1024 + (size_t)gf_stages<MODE, CLUSTER>() * gf_stage_bytes<MODE>() + gf_part_bytes<MODE, CLUSTER>() + sizeof(GfShared);
+    constexpr size_t smem = gf_smem_bytes<MODE, CLUSTER>();
     static bool configured[64] = {false};  // the attribute is per device
     int dev = 0;
     AB2_CUDA(cudaGetDevice(&dev));
@@ -373,8 +385,7 @@ int launch_few(const LinArgs &a, int ctas, const DecodeGemmScratch &sc, cudaStre
     }
     if (CLUSTER) {
         const int n_tiles = (a.N + 127) / 128;
-        cluster = GF_MAX_CLUSTER;
-        while (cluster > 2 && (cluster > (a.K + 63) / 64 || n_tiles > clusters_at_once<MODE>(cluster, smem))) cluster >>= 1;
+        cluster = gf_cluster<MODE>(n_tiles, a.K);
         ctas = cluster * n_tiles;
     }
     cudaLaunchConfig_t cfg = {};
@@ -395,15 +406,24 @@ int launch_few(const LinArgs &a, int ctas, const DecodeGemmScratch &sc, cudaStre
 
 bool gemm_bf16_few(const LinArgs &a, int mode, cudaStream_t s, int *rc) {
     if (a.M < 1 || a.M > GF_TOK || (mode != LIN_DENSE && mode != LIN_GLU) || (mode == LIN_DENSE && (a.batch > 1 || a.epi == LIN_GATE))) return false;
-    const int tiles = (a.N + 127) / 128, KS = (a.K + 63) / 64, sms = device_sm_count();
+    const int tiles = (a.N + 127) / 128, KS = (a.K + 63) / 64, sms = device_sm_count(), k = (mode == LIN_GLU ? 2 : 1) * a.K;
     if (2 * tiles <= sms) {
         if (KS < 2) return false;
+        // Pairs of CTAs that leave a quarter of the SMs idle: us, GEMV / this kernel at 9 tokens, 4608 x 4096 15.0, 17.8, 6144 x 4096 16.9,
+        // 17.7, 5120 x 8192 25.6, 28.7, but 7168 x 4096 23.8, 18.3 (at 32 tokens 31, 18; 6144 x 4096 30, 18).
+        if (mode == LIN_DENSE && a.M <= 16 && 8 * tiles < 3 * sms && gf_cluster<LIN_DENSE>(tiles, a.K) == 2) return false;
         *rc = mode == LIN_DENSE ? launch_few<LIN_DENSE, true>(a, 0, {}, s) : launch_few<LIN_GLU, true>(a, 0, {}, s);
         return true;
     }
-    DecodeGemmScratch sc;
-    if ((long long)tiles * KS > 0x7fffffffll || !decode_gemm_scratch(s, &sc) || tiles > sc.max_tiles) return false;
-    const int ctas = tiles < sms && tiles * 20 >= sms * 13 ? tiles : sms;  // GfRange's rule for one round
+    const int ctas = tiles < sms && GfRange::in_whole(tiles, sms) ? tiles : sms;
+    DecodeGemmScratch sc = {};
+    if (!GfRange::in_whole(tiles, ctas)) {
+        // Handing parts over costs about 6 us, which short ranges do not win back.  us, GEMV / this kernel: 80 tiles, 1024 of K at 32 tokens
+        // 16.3, 18.3 (2048: 24.4, 20.5); 2048 of K at 9 tokens 16.0, 20.4 (4096: 27, 26.4); 4096 of K at 5 tokens 24.9, 26.4; 160
+        // tiles, 1024 of K at 9 tokens 15.9, 18.4 (2048: 24.0, 24.7; at 32 tokens 24.4, 18.5).
+        const int least = tiles < sms ? (a.M > 16 ? 1024 : a.M > 8 ? 2048 : 4096) : a.M > 16 ? 0 : 1024;
+        if (k <= least || (long long)tiles * KS > 0x7fffffffll || !decode_gemm_scratch(s, &sc) || tiles > sc.max_tiles) return false;
+    }
     *rc = mode == LIN_DENSE ? launch_few<LIN_DENSE, false>(a, ctas, sc, s) : launch_few<LIN_GLU, false>(a, ctas, sc, s);
     return true;
 }

@@ -107,13 +107,15 @@ cudaError_t launch_simt(const LinArgs &a, int mode, cudaStream_t s) {
 
 // Rows of the decode GEMV: beyond this many the tensor-memory GEMM's token tiles pay.
 constexpr int GEMV_MAX_ROWS = 32;
-// Whether the decode GEMM over clusters and cut tiles is the faster one for weights of so many elements.  Measured against
-// the GEMV in recorded launches, us (GEMV, decode GEMM): 17 to 32 tokens 2048 x 2048 7.4, 7.9 (but 8197, 8035 for 8 steps of 14
-// latent runs, whose launches are chained), 3664 x 2048 8.9, 8.4, 6144 x 4096 28, 16; 9 to 16 tokens 6144 x 2048 8.3, 9.9,
-// 4096 x 4096 11.1, 10.8, 8192 x 2048 13.6, 10.8; 8 tokens 4096 x 4096 10.6, 10.5, 4096 x 7168 15.8, 14.1, 32000 x 4096 56, 51,
-// but 32000 x 2048 28.6, 31.3; 4 tokens 4096 x 7168 14.9, 13.9, but 14336 x 4096 27.7, 28.7.
+// Whether the decode GEMM over clusters and cut tiles is the faster one for weights of so many elements; it refuses what it serves
+// slower for its shape itself.  us, GEMV and decode GEMM, launches one after another: 17 to 32 tokens, 2048 x 2048 8.4, 10.3 (but 8197,
+// 8035 for 8 steps of 14 latent runs, whose launches are chained), 4096 x 1024 8.2, 9.6, 1024 x 4096 13.8, 10.3, 2560 x 2048 10.3, 10.3, 4096
+// x 2048 10.3, 10.3, 6144 x 4096 30, 18; 9 to 16 tokens, 6144 x 2048 10.3, 12.3, 8192 x 2048 15.4, 13.4, 4096 x 4096 13.6, 13.6; 5 to 8 tokens,
+// 4096 x 4096 13.4, 13.6, 4096 x 7168 16.6, 16.4, 32000 x 4096 54, 48, 32000 x 2048 26.7, 27.4.
 bool few_pays(int M, int K, long long weights) {
-    return M > 16 ? weights >= 4LL << 20 : M > 8 ? weights >= 16LL << 20 : M > 4 && K >= 4096 && weights >= 28LL << 20;
+    const bool alone = g_decode_gemm_scratch == nullptr;  // not in a layer stack
+    if (M > 16) return weights >= (alone && K < 4096 ? 5LL : 4LL) << 20;
+    return M > 8 ? weights >= 16LL << 20 : M > 4 && K >= 4096 && weights >= 28LL << 20;
 }
 
 bool rows_aligned(const void *w, const void *x, int K) { return K % 8 == 0 && (((uintptr_t)w | (uintptr_t)x) & 15) == 0; }

@@ -20,9 +20,12 @@ def data(N, K, M):
 
 
 @pytest.mark.parametrize("N,K,M", [(N, K, M) for N, K in [(1000, 4200), (2048, 2048), (4104, 4096), (74 * 128, 1024), (75 * 128, 1800), (95 * 128 + 8, 1800),
-                                                         (12288, 1400), (149 * 128, 1024), (219 * 128 + 40, 640), (250 * 128, 544), (40000, 512), (8200, 8192)]
+                                                         (12288, 1400), (149 * 128, 1024), (219 * 128 + 40, 640), (250 * 128, 544), (40000, 512), (8200, 8192),
+                                                         (1536, 4096), (2560, 2048), (2048, 2560)]
                                    for M in (17, 31, 32)] +
-                         [(N, K, M) for N, K in [(1000, 17000), (4096, 4200), (149 * 128, 1024), (9600, 4100 // 8 * 8)] for M in (5, 8, 9, 15, 16)])
+                         [(N, K, M) for N, K in [(1000, 17000), (4096, 4200), (149 * 128, 1024), (9600, 4100 // 8 * 8), (149 * 128, 1400), (7168, 4096), (5120, 4096)]
+                          for M in (5, 8, 9, 15, 16)] +
+                         [(N, K, M) for N, K in [(4096, 7168), (10240, 4160), (14336, 4096)] for M in (5, 6, 7, 8)])
 def test_linear(N, K, M):
     w, x, want, bound = data(N, K, M)
     lin = pkg().QuantLinear.from_bf16(w)
@@ -33,7 +36,7 @@ def test_linear(N, K, M):
     assert pkg().device_status() == 0
 
 
-@pytest.mark.parametrize("N,K", [(2048, 2048), (149 * 128, 1024)])
+@pytest.mark.parametrize("N,K", [(2048, 2560), (149 * 128, 1024), (250 * 128, 544)])
 def test_rows_that_are_not_finite_stay_alone(N, K):
     w, x, want, bound = data(N, K, 32)
     x[3], x[31, 5] = float("nan"), float("inf")
@@ -43,7 +46,7 @@ def test_rows_that_are_not_finite_stay_alone(N, K):
     assert ((got[rest] - want[rest]).abs() <= bound[rest]).all()
 
 
-@pytest.mark.parametrize("N,K", [(2048, 2048), (149 * 128, 1024)])
+@pytest.mark.parametrize("N,K", [(2048, 2560), (149 * 128, 1024), (250 * 128, 544)])
 def test_recorded_and_on_several_streams(N, K):
     """A recorded call replays beside eager calls on the stream it was recorded on; streams have parts of their own."""
     w, x, want, bound = data(N, K, 32)
@@ -92,4 +95,33 @@ def test_gated_unit_and_capped_head_of_a_stack(tmp_path):
         many, one = (np.linalg.norm(x - want) / np.linalg.norm(want) for x in (got[r], steps([r])[0]))
         # the roundings of activations to bf16, which both have, fall differently: the GEMV's error is the measure
         assert many < 1.3 * one + 1e-3 and one < 3e-2, (many, one)
+    assert pkg().device_status() == 0
+
+
+@pytest.mark.parametrize("ff,rows", [(149 * 128 + 8, 17), (149 * 128 + 8, 32), (149 * 128 + 8, 9), (12800, 20), (80 * 128, 31), (54 * 128, 12)])
+def test_gated_unit_over_cut_and_whole_tiles(tmp_path, ff, rows):
+    """The gate and up products of a dense feed-forward in every form of more tiles than a cluster serves (and one that it does).  Rows
+    hold the same tokens, so that each has to be the others' equal to the bit."""
+    vocab = 512
+    cfg = fx.config([(fx.latent(8, 64, 32, 64, 128), fx.dense(ff))], width=1032, vocab=vocab, loop=None)
+    w = fx.weights(cfg, ff)
+    model = fx.load(tmp_path, cfg, w, torch.bfloat16, 64, 16)
+    tokens = np.random.default_rng(rows).integers(0, vocab, 3)
+
+    def steps(n):
+        cache = model.empty_kv_cache_with_capacity(16, batch=n)
+        logits = torch.empty((n, 1, vocab), device="cuda", dtype=model.logits_dtype)
+        out = []
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for t in tokens:
+                model.decode_step(torch.full((n,), int(t), dtype=torch.int32, device="cuda"), cache, logits, None)
+                out.append(logits[:, 0].clone())
+        torch.cuda.synchronize()
+        return torch.stack(out, 1)
+
+    got = steps(rows)
+    assert torch.equal(got, got[:1].expand_as(got)) and torch.equal(steps(rows), got)
+    want = fx.expected(cfg, w, tokens.tolist())
+    many, one = (np.linalg.norm(x[0].double().cpu().numpy() - want) / np.linalg.norm(want) for x in (got, steps(1)))
+    assert many < 1.3 * one + 1e-3 and one < 3e-2, (many, one)  # as above
     assert pkg().device_status() == 0
