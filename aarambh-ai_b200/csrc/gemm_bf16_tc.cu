@@ -346,8 +346,10 @@ int launch_tc(const LinArgs &a, cudaStream_t s) {
 // Token tile, and one CTA or a pair for a tile: rounds of tiles over the SMs times what a tile costs.  That of one CTA is the
 // rows it streams through L2, its tokens and the 128 (gate and up: 256) weight rows.  A pair's tile costs as much as 350 of
 // them: 14336 x 4096, us by single CTAs and by pairs: 300 tokens 53, 46; 512 56, 50; 2048 178, 165; 4096 x 4096: 512 tokens 21, 26 (32
-// pair tiles for 74 pairs), 1024 28.1, 27.8; 2048 x 2048, 1024 tokens: 13.2, 15.9.  Over ten weights and eleven token counts
-// the rule took the slower form by 5 % at most.
+// pair tiles for 74 pairs), 1024 28.1, 27.8; 2048 x 2048, 1024 tokens: 13.2, 15.9.  A plain linear by pairs pays for their launch besides,
+// as much as 100 rows over 1024 of K, which one round of short tiles does not win back: 6144 x 2048 at 700 tokens 18.7, 20.1, 3000 x
+// 1536 at 1024 15.6, 16.5; 7168 x 4096 at 300 30.7, 28.9, 8192 x 2048 at 700 (two rounds) 30.6, 28.9.  Over sixteen weights and fourteen
+// token counts the rule took the slower form by 2 % at most.
 template <int MODE, int PAIR_TOK>
 int launch_best(const LinArgs &a, int groups, double rows, cudaStream_t s) {
     constexpr bool DUAL = MODE == LIN_MOE_GLU || MODE == LIN_GLU;
@@ -356,7 +358,8 @@ int launch_best(const LinArgs &a, int groups, double rows, cudaStream_t s) {
     auto cost = [&](int ntok) { return rounds(ntok, 128, sms) * (ntok + (DUAL ? 256 : 128)); };
     int best = !DUAL && cost(256) <= cost(128) ? 256 : 128;
     if (cost(64) < cost(best)) best = 64;
-    if (rounds(PAIR_TOK, 256, sms / 2) * 350 < cost(best)) return launch_tc<PAIR_TOK, MODE, true>(a, s);
+    const double launch = MODE == LIN_DENSE ? 102400.0 / a.K : 0;
+    if (rounds(PAIR_TOK, 256, sms / 2) * 350 + launch < cost(best)) return launch_tc<PAIR_TOK, MODE, true>(a, s);
     if constexpr (!DUAL) if (best == 256) return launch_tc<256, MODE>(a, s);
     return best == 128 ? launch_tc<128, MODE>(a, s) : launch_tc<64, MODE>(a, s);
 }

@@ -10,8 +10,10 @@ from helpers import pkg
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("N,K", [(74 * 256, 1024), (75 * 256 - 128, 1000), (75 * 256 - 120, 200), (38 * 256 + 8, 64)])
-@pytest.mark.parametrize("M", [257, 400, 512, 513, 800])
+# short K by single CTAs, and by pairs where there are rounds enough
+@pytest.mark.parametrize("N,K,M", [(N, K, M) for N, K in [(74 * 256, 1024), (75 * 256 - 128, 1000), (75 * 256 - 120, 200), (38 * 256 + 8, 64)]
+                                   for M in (257, 400, 512, 513, 800)] +
+                         [(74 * 256, 4096, 257), (75 * 256 - 128, 4104, 513), (38 * 256 + 8, 4200, 400), (75 * 256 - 120, 1000, 801), (74 * 256 - 8, 200, 4100), (74 * 256, 136, 5890)])
 def test_linear(N, K, M):
     gen = torch.Generator("cuda").manual_seed(N + K + M)
     w = (torch.randn((N, K), generator=gen, device="cuda") * K ** -0.5).bfloat16()
