@@ -20,6 +20,7 @@
 using namespace ab2;
 
 namespace ab2 {
+int device_status_word(int **out);
 
 static size_t kv_elem_size(int dtype) { return dtype == AB2_KV_F32 ? 4 : dtype == AB2_KV_BF16 ? 2 : 1; }
 
@@ -360,6 +361,9 @@ AB2_API int ab2_kv_create(ab2_kv **out, int n_layers, int batch, int capacity, i
                 "query heads (%d) must be 1..8 times the kv heads (%d)", n_heads, kv_heads);
     AB2_REQUIRE(dtype == AB2_KV_F32 || dtype == AB2_KV_BF16 || dtype == AB2_KV_INT8, AB2_ERR_BAD_DTYPE,
                 "unsupported KV dtype %d", (int)dtype);
+    int *status = nullptr;  // what the first attention would otherwise make, perhaps while it is recorded
+    int rc = device_status_word(&status);
+    if (rc != AB2_OK) return rc;
     ab2_kv *kv = new ab2_kv();
     memset(kv, 0, sizeof(*kv));
     kv->L = n_layers; kv->B = batch; kv->cap = capacity; kv->kvh = kv_heads; kv->hd = head_dim; kv->h = n_heads;
