@@ -416,13 +416,14 @@ bool gemm_bf16_few(const LinArgs &a, int mode, cudaStream_t s, int *rc) {
         return true;
     }
     const int ctas = tiles < sms && GfRange::in_whole(tiles, sms) ? tiles : sms;
+    ScratchLease lease(s);  // given back once the launch stands
     DecodeGemmScratch sc = {};
     if (!GfRange::in_whole(tiles, ctas)) {
         // Handing parts over costs about 6 us, which short ranges do not win back.  us, GEMV / this kernel: 80 tiles, 1024 of K at 32 tokens
         // 16.3, 18.3 (2048: 24.4, 20.5); 2048 of K at 9 tokens 16.0, 20.4 (4096: 27, 26.4); 4096 of K at 5 tokens 24.9, 26.4; 160
         // tiles, 1024 of K at 9 tokens 15.9, 18.4 (2048: 24.0, 24.7; at 32 tokens 24.4, 18.5).
         const int least = tiles < sms ? (a.M > 16 ? 1024 : a.M > 8 ? 2048 : 4096) : a.M > 16 ? 0 : 1024;
-        if (k <= least || (long long)tiles * KS > 0x7fffffffll || !decode_gemm_scratch(s, &sc) || tiles > sc.max_tiles) return false;
+        if (k <= least || (long long)tiles * KS > 0x7fffffffll || !decode_gemm_scratch(s, tiles, &lease, &sc)) return false;
     }
     *rc = mode == LIN_DENSE ? launch_few<LIN_DENSE, false>(a, ctas, sc, s) : launch_few<LIN_GLU, false>(a, ctas, sc, s);
     return true;

@@ -99,9 +99,11 @@ int gemm_bf16_tc(const LinArgs &a, int mode, cudaStream_t s);
 bool gemm_bf16_few(const LinArgs &a, int mode, cudaStream_t s, int *rc);
 
 // What that kernel hands parts of cut tiles over in: two slots of W4DG_MAX_SLOT_FLOATS for every SM and a zeroed counter per tile.
-// A layer stack has its own, which its recorded steps use on whatever stream they run.  Other calls share the
-// set of their stream with the W4A16 kernels; none while the stream is being recorded (the graph may run beside later work on
-// the stream), on the per-thread stream (one handle, several streams), or where memory is refused.
+// A layer stack has its own, which its recorded steps use on whatever stream they run.  Other calls share the set of their
+// stream with the W4A16 kernels.  Where that would not do they lease one for the launch: while the stream is being recorded (the
+// graph may run beside later work on the stream), on the per-thread stream (one handle, several streams), on a handle that has
+// been another stream's, with many streams.  A
+// decoder's recorded step leases none, since zeroing the counters would break its chain of launches.
 struct DecodeGemmScratch {
     float *partials;
     int *counters;
@@ -114,6 +116,6 @@ struct DecodeGemmScratchOf {
     DecodeGemmScratchOf &operator=(const DecodeGemmScratchOf &) = delete;
     ~DecodeGemmScratchOf() { g_decode_gemm_scratch = nullptr; }
 };
-bool decode_gemm_scratch(cudaStream_t s, DecodeGemmScratch *out);
+bool decode_gemm_scratch(cudaStream_t s, int tiles, ScratchLease *lease, DecodeGemmScratch *out);
 
 }  // namespace ab2

@@ -137,6 +137,7 @@ struct GemvScratch {
     float *partials = nullptr;
     int *counters = nullptr;
     int max_ctas = 0;
+    unsigned long long stream_id = 0;
 };
 constexpr size_t DECODE_GEMM_MAX_STREAMS = 64;  // linears of bf16 weights start no set beyond so many (11 MB each)
 static std::mutex g_scratch_mutex;
@@ -147,7 +148,8 @@ static cudaError_t gemv_scratch_alloc(cudaStream_t s, GemvScratch *sc) {
     // two partial tiles per warp of the warp kernels, or per CTA of the decode GEMMs, one CTA per SM
     const size_t pbytes = std::max((size_t)sc->max_ctas * W4W_WARPS * 2 * W4W_SLOT_FLOATS,
                                    (size_t)device_sm_count() * 2 * W4DG_MAX_SLOT_FLOATS) * sizeof(float);
-    cudaError_t e = cudaMalloc((void **)&sc->partials, pbytes);
+    cudaError_t e = cudaStreamGetId(s, &sc->stream_id);
+    if (e == cudaSuccess) e = cudaMalloc((void **)&sc->partials, pbytes);
     if (e == cudaSuccess) e = cudaMalloc((void **)&sc->counters, W4W_MAX_TILES * sizeof(int));
     if (e == cudaSuccess) e = cudaMemsetAsync(sc->counters, 0, W4W_MAX_TILES * sizeof(int), s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // a graph made with the set may be launched on another stream
@@ -181,19 +183,10 @@ static int gemv_scratch_for(cudaStream_t s, GemvScratch *out) {
 
 thread_local const DecodeGemmScratch *g_decode_gemm_scratch = nullptr;
 
-// The decode GEMM's parts and counters for launches on `s`; false where there are none to be had (linear_bf16.cuh).
-bool decode_gemm_scratch(cudaStream_t s, DecodeGemmScratch *out) {
-    if (g_decode_gemm_scratch) {
-        *out = *g_decode_gemm_scratch;
-        return out->partials != nullptr;
-    }
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (s == cudaStreamPerThread || cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-        (void)cudaGetLastError();
-        return false;
-    }
+// The set of a stream that is not being recorded; false where there is none to be had.
+static bool stream_scratch(cudaStream_t s, DecodeGemmScratch *out) {
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    if (s == cudaStreamPerThread || cudaGetDevice(&dev) != cudaSuccess) return false;
     std::lock_guard<std::mutex> lock(g_scratch_mutex);
     auto it = g_scratch.find(std::make_pair(dev, s));
     if (it == g_scratch.end()) {
@@ -207,8 +200,32 @@ bool decode_gemm_scratch(cudaStream_t s, DecodeGemmScratch *out) {
         if (!ok) return false;
         it = g_scratch.emplace(std::make_pair(dev, s), sc).first;
     }
+    // a destroyed stream's handle is used again, perhaps while its launches are still to run: the set is that stream's
+    unsigned long long id = 0;
+    if (cudaStreamGetId(s, &id) != cudaSuccess || id != it->second.stream_id) return false;
     *out = {it->second.partials, it->second.counters, W4W_MAX_TILES};
     return true;
+}
+
+// The decode GEMM's parts and counters for a launch of `tiles` tiles on `s`; false where there are none to be had (linear_bf16.cuh).
+bool decode_gemm_scratch(cudaStream_t s, int tiles, ScratchLease *lease, DecodeGemmScratch *out) {
+    if (g_decode_gemm_scratch) {
+        *out = *g_decode_gemm_scratch;
+        return out->partials != nullptr && tiles <= out->max_tiles;
+    }
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    if (cap == cudaStreamCaptureStatusNone && stream_scratch(s, out) && tiles <= out->max_tiles) return true;
+    (void)cudaGetLastError();
+    const size_t slots = (size_t)device_sm_count() * 2 * W4DG_MAX_SLOT_FLOATS * sizeof(float);
+    if (g_recorded_scratch || !lease->take(slots + (size_t)tiles * sizeof(int))) return false;
+    *out = {(float *)lease->ptr, (int *)((char *)lease->ptr + slots), tiles};
+    if (cudaMemsetAsync(out->counters, 0, (size_t)tiles * sizeof(int), s) == cudaSuccess) return true;
+    (void)cudaGetLastError();
+    return false;
 }
 
 int w4a16_prepare_stream(cudaStream_t s) {

@@ -138,6 +138,7 @@ AB2_API int ab2_qweight_from_bf16(ab2_qweight **out, const uint16_t *weight, int
     }
     // what the first call would otherwise make, perhaps while it is recorded
     int *status = nullptr;
+    TRY_OR_FREE(w, scratch_prepare());
     TRY_OR_FREE(w, device_status_word(&status));
     return AB2_OK;
 }

@@ -1,5 +1,8 @@
 """Linears over bf16 weights of 5 to 32 tokens where the decode GEMM's shape changes: clusters of 8, 4 and 2 CTAs a tile, ranges
 that cut tiles, whole tiles, K and channels that do not fill theirs, and what a stream without its scratch memory takes."""
+import ctypes
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -69,6 +72,54 @@ def test_recorded_and_on_several_streams(N, K):
     torch.cuda.synchronize()
     for got in outs + [recorded]:
         assert ((got.double() - want).abs() <= bound).all()
+        assert torch.equal(got, outs[0])  # recorded or not, one kernel
+
+
+def test_a_stream_handle_that_is_used_again():
+    """A stream with launches still to run is destroyed, and another may get its handle."""
+    w, x, want, bound = data(149 * 128, 1024, 32)
+    lin, lib, cudart = pkg().QuantLinear.from_bf16(w), pkg()._lib.lib, ctypes.CDLL("libcudart.so.12")
+    eager = lin(x)
+    outs = [torch.full_like(eager, float("nan")) for _ in range(6)]
+    side, event, codes = torch.cuda.Stream(), torch.cuda.Event(), []
+    torch.cuda.synchronize()
+    for out in outs:
+        stream = ctypes.c_void_p()
+        codes.append(cudart.cudaStreamCreateWithFlags(ctypes.byref(stream), 1))
+        codes.append(lib.ab2_qlinear_forward(lin._h, x.data_ptr(), 32, 2, out.data_ptr(), stream))
+        if out is outs[0]:
+            with torch.cuda.stream(side):
+                torch.cuda._sleep(100_000_000)
+                event.record()
+        codes.append(cudart.cudaStreamWaitEvent(stream, ctypes.c_void_p(event.cuda_event), 0))
+        codes.append(lib.ab2_qlinear_forward(lin._h, x.data_ptr(), 32, 2, out.data_ptr(), stream))
+        codes.append(cudart.cudaStreamDestroy(stream))
+    torch.cuda.synchronize()
+    assert not any(codes) and all(torch.equal(out, eager) for out in outs)
+
+
+@pytest.mark.parametrize("N,K", [(149 * 128, 1024), (80 * 128, 1800)])
+def test_per_thread_stream(N, K):
+    """Cut tiles on the stream whose handle every thread shares: parts are leased for each launch."""
+    w, x, want, bound = data(N, K, 32)
+    lin = pkg().QuantLinear.from_bf16(w)
+    eager = lin(x)
+    torch.cuda.synchronize()
+    outs = [torch.full((32, N), float("nan"), device="cuda", dtype=torch.bfloat16) for _ in range(8)]
+    torch.cuda.synchronize()
+    lib, codes = pkg()._lib.lib, []
+
+    def work(mine):
+        for out in mine:
+            codes.append(lib.ab2_qlinear_forward(lin._h, x.data_ptr(), 32, 2, out.data_ptr(), ctypes.c_void_p(2)))
+
+    threads = [threading.Thread(target=work, args=(outs[i::2],)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert codes == [0] * 8 and all(torch.equal(out, eager) for out in outs)
 
 
 def test_gated_unit_and_capped_head_of_a_stack(tmp_path):

@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 HEAD = """
 import torch
 from helpers import pkg
-p, stream, graph = pkg(), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+p, stream, graph, same = pkg(), torch.cuda.Stream(), torch.cuda.CUDAGraph(), True
 gen = torch.Generator("cuda").manual_seed(1)
 randn = lambda *s: torch.randn(s, generator=gen, device="cuda").bfloat16()
 
@@ -24,7 +24,7 @@ def check(call, want):
     graph.replay()
     torch.cuda.synchronize()
     assert float((got.double() - want).norm()) <= 2.0 ** -8 * float(want.norm())
-    assert torch.equal(call(), got)  # recorded or not, the same kernel
+    assert torch.equal(call(), got) or not same  # recorded or not, one kernel
     assert p.device_status() == 0
 """
 ATTENTION = """
@@ -45,8 +45,8 @@ check(lambda: lin(x), x.double() @ w.double().T)
 """
 
 
-def alone(code):
-    env = dict(os.environ, PYTHONPATH=os.path.join(ROOT, "tests"))
+def alone(code, **more):
+    env = dict(os.environ, PYTHONPATH=os.path.join(ROOT, "tests"), **more)
     r = subprocess.run([sys.executable, "-c", HEAD + code], cwd=ROOT, env=env, capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-3000:]
 
@@ -56,6 +56,10 @@ def test_decode_attention(kv, n):
     alone(ATTENTION.format(kv=kv, n=n))
 
 
-@pytest.mark.parametrize("N,K,M", [(2560, 2048, 20), (250 * 128, 1024, 32), (4096, 4096, 300)])
+@pytest.mark.parametrize("N,K,M", [(2560, 2048, 20), (250 * 128, 1024, 32), (149 * 128, 1024, 32), (80 * 128, 4096, 9), (4096, 4096, 300)])
 def test_bf16_linears(N, K, M):
     alone(LINEAR.format(N=N, K=K, M=M))
+
+
+def test_refused_scratch_while_recording():
+    alone("same = False" + LINEAR.format(N=149 * 128, K=1024, M=32), AB2_SCRATCH_MAX_BYTES="0")
