@@ -279,7 +279,6 @@ __global__ void __launch_bounds__(128) lightning_chunk_kernel(LightningArgs a) {
                 if (v0 + n * 8 + 2 * c < a.vdim) *reinterpret_cast<float2 *>(dst + n * 8 + 2 * c) = make_float2(o[n][2 * h], o[n][2 * h + 1]);
         }
         }
-        if (!SUMS && seg != a.segs - 1 && t0 + C >= S_len) break;  // nobody takes this segment's last state
         // the state after the chunk
         const float dn = pw[n_tok];
 #pragma unroll
