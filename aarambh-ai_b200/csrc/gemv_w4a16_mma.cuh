@@ -1,8 +1,7 @@
 // Building blocks shared by the W4A16 (group 128) decode GEMV kernels: the
-// warp-level tensor-core MMA (m16n8k16, bf16 x bf16 -> f32), the nibble -> bf16
-// extraction (0x4300 | q == 128 + q exactly, one shift and one LOP3 per pair of
-// codes), and the mbarrier / bulk-copy primitives.  Every mbarrier wait is
-// bounded; a wait that runs out records AB2_ERR_TIMEOUT in the status word.
+// warp-level tensor-core MMA (m16n8k16, bf16 x bf16 -> f32) and the mbarrier / bulk-copy
+// primitives.  Every mbarrier wait is bounded; a wait that runs out records
+// AB2_ERR_TIMEOUT in the status word.
 #pragma once
 
 #include "common.cuh"
@@ -31,20 +30,9 @@ __device__ __forceinline__ void mma_bf16_16816_init(float (&d)[4], uint32_t a0, 
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
-// Pair j of a code word: elements (2j, 2j+1) as bf16x2 holding 128 + q:
-// ((word >> 4j) & 0x000F000F) | 0x43004300 as one shift and one three-input
-// logic op; mask and magic are passed in registers so the logic op stays single.
-__device__ __forceinline__ uint32_t w4_pair_bf16(uint32_t word, int j, uint32_t mask,
-                                                 uint32_t magic) {
+__device__ __forceinline__ uint32_t bf16x2_fma(uint32_t a, uint32_t b, uint32_t c) {
     uint32_t d;
-    const uint32_t sh = j ? (word >> (4 * j)) : word;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;\n" : "=r"(d) : "r"(sh), "r"(mask), "r"(magic));
-    return d;
-}
-
-__device__ __forceinline__ uint32_t bf16x2_add(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("add.rn.bf16x2 %0, %1, %2;\n" : "=r"(d) : "r"(a), "r"(b));
+    asm("fma.rn.bf16x2 %0, %1, %2, %3;\n" : "=r"(d) : "r"(a), "r"(b), "r"(c));
     return d;
 }
 

@@ -145,12 +145,6 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
     return v;
 }
 
-__device__ __forceinline__ uint32_t bf16x2_fma(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("fma.rn.bf16x2 %0, %1, %2, %3;\n" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-
 // partials: [gridDim.x * 8 warps][2][W4W_SLOT_FLOATS] floats; counters: one int
 // per 16-row tile, zero on entry and on exit.
 //

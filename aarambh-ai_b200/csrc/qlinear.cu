@@ -335,28 +335,23 @@ static int launch_w4a16_stream(const ab2_qweight *w, const void *x, int M, void 
             return AB2_OK;
         }
     }
-    for (int m0 = 0; m0 < M; m0 += 16) {
-        const __nv_bfloat16 *xp = (const __nv_bfloat16 *)x + (size_t)m0 * w->K;
-        __nv_bfloat16 *yp = EPI == W4_EPI_F32_PEER ? (__nv_bfloat16 *)y  // descriptor of the peer exchange (one pass)
-                            : EPI == W4_EPI_F32  ? (__nv_bfloat16 *)((float *)y + (size_t)m0 * out_n)
-                                                 : (__nv_bfloat16 *)y + (size_t)m0 * out_n;
-        const __nv_bfloat16 *rp = resid ? (const __nv_bfloat16 *)resid + (size_t)m0 * out_n : nullptr;
-        int mv = M - m0 < 16 ? M - m0 : 16;
-        cudaError_t e;
-        if (norm_w && !(M == 1 && w->K <= W4M1_MAX_K))
-            return fail(AB2_ERR_UNSUPPORTED, "the fused RMSNorm serves one token and K <= %d", W4M1_MAX_K);
-        // One token: the kernel that prepares the activations per CTA, while K is small
-        // next to the rows a CTA streams (or there is a norm to fuse); else the general one.
-        if (M == 1 && (norm_w || w->K <= W4M1_PLAIN_MAX_K) && w->K <= W4M1_MAX_K)
-            e = launch_w4a16_m1<EPI>(w, xp, norm_w, eps, yp, rp, grid, sc, status, s, peers, (__nv_bfloat16 *)x_out);
-        else if (mv > 8)
-            e = launch_kernel(gemv_w4a16_warp_kernel<2, EPI>, dim3(grid), dim3(256), 0, s, wt, xp, yp, rp, w->N,
-                              w->K, mv, sc.partials, sc.counters, status);
-        else
-            e = launch_kernel(gemv_w4a16_warp_kernel<1, EPI>, dim3(grid), dim3(256), 0, s, wt, xp, yp, rp, w->N,
-                              w->K, mv, sc.partials, sc.counters, status);
-        if (e != cudaSuccess) return fail(AB2_ERR_CUDA, "GEMV launch failed: %s", cudaGetErrorString(e));
-    }
+    // up to 8 tokens in a pass, up to 16 where the sums go to the peers
+    if (norm_w && !(M == 1 && w->K <= W4M1_MAX_K))
+        return fail(AB2_ERR_UNSUPPORTED, "the fused RMSNorm serves one token and K <= %d", W4M1_MAX_K);
+    const __nv_bfloat16 *xp = (const __nv_bfloat16 *)x, *rp = (const __nv_bfloat16 *)resid;
+    __nv_bfloat16 *yp = (__nv_bfloat16 *)y;  // for W4_EPI_F32_PEER the descriptor of the exchange
+    cudaError_t e = cudaErrorInvalidValue;
+    // One token: the kernel that prepares the activations per CTA, while K is small
+    // next to the rows a CTA streams (or there is a norm to fuse); else the general one.
+    if (M == 1 && (norm_w || w->K <= W4M1_PLAIN_MAX_K) && w->K <= W4M1_MAX_K)
+        e = launch_w4a16_m1<EPI>(w, xp, norm_w, eps, yp, rp, grid, sc, status, s, peers, (__nv_bfloat16 *)x_out);
+    else if (M <= 8)
+        e = launch_kernel(gemv_w4a16_warp_kernel<1, EPI>, dim3(grid), dim3(256), 0, s, wt, xp, yp, rp, w->N, w->K, M, sc.partials,
+                          sc.counters, status);
+    else if constexpr (EPI == W4_EPI_F32_PEER)
+        e = launch_kernel(gemv_w4a16_warp_kernel<2, EPI>, dim3(grid), dim3(256), 0, s, wt, xp, yp, rp, w->N, w->K, M, sc.partials,
+                          sc.counters, status);
+    if (e != cudaSuccess) return fail(AB2_ERR_CUDA, "GEMV launch failed: %s", cudaGetErrorString(e));
     AB2_LAUNCH_CHECK();
     return AB2_OK;
 }
