@@ -114,11 +114,14 @@ __device__ __forceinline__ void ldmatrix_trans(uint32_t &r0, uint32_t &r1, uint3
 // spent on a block that can be avoided: a warp's ring of AT_STAGES blocks of 16 tokens is filled by tensor-map copies of one
 // lane, two blocks ahead; their 128-byte swizzle keeps fragment reads free of bank conflicts; keys are the rows of the first
 // product, so that no half of an MMA is padding, and a transpose in registers makes its result the second one's operand; the
-// reference score moves rarely; exponentials are powers of two of scores scaled once.  408 instructions a block of INT8 tokens;
+// reference score moves rarely; exponentials are powers of two of scores scaled once.  394 instructions a block of INT8 tokens;
 // 583 with cp.async and queries as rows.  Sixteen warps of an INT8 launch share an SM, eight of a bf16 one.
-// us, 32 / 8 heads, the kernels before (for bf16 on CUDA cores) -> now: INT8 8 x 16384 71 -> 52 (0.81 of the copy rate), 64 x 4096
-// 115 -> 86, 32 x 700 17.5 -> 15.6, 1 x 4096 24 -> 13, 1 x 512 8.8 -> 8.0; bf16 64 x 2048 215 -> 77 (0.94), 8 x 8192 159 -> 48,
-// 32 x 700 52 -> 19, 1 x 512 16 -> 10.
+// us in a graph, 32 / 8 heads, the kernels before (for bf16 on CUDA cores) -> now: INT8 8 x 16384 74 -> 52 (0.82 of the copy rate; a call of
+// its own 75 -> 55), 64 x 4096 119 -> 93, 32 x 700 17.4 -> 15.6, 1 x 4096 24 -> 12.3, 1 x 256 7.9 -> 5.5; bf16 64 x 2048 225 -> 84 (0.99), 8 x 8192
+// 160 -> 49, 32 x 700 53 -> 20, 1 x 4096 27 -> 12.6, 1 x 256 14.7 -> 6.9.
+// Error against 64 bits over 40 drawn batches to that of the kernels before: bf16 rows 1.00000001 (two terms of the weights in one
+// accumulator 1.0000008; the third and accumulators of their own take 3 % of the time), INT8 rows with bf16 queries 0.999995, with f32
+// queries 1.0006, single batches 0.987 to 1.006.  Exponentials of scores scaled by log2 e, which are 2 ulp off, don't show in it.
 constexpr int AT_STAGES = 3, AT_TOK = 16, AT_HD = 128;
 template <int KVD, bool MANY>  // MANY: short rows, many of them
 struct AtShape {

@@ -21,9 +21,9 @@
 // counter per tile tells who is last, and the parts are added in the contributors' order.
 //
 // What bounds it: HBM for large weights (0.8 of the copy rate and 9 us a launch alone); for small ones the chain of launch,
-// first activations, products, exchange.  us, one launch after another from Python, GEMV -> this kernel, 9 / 32 tokens:
-// 4096 x 14336 31.5 / 48.9 -> 26.0 / 27.9; 14336 x 4096 34 / 57 -> 27 / 30; 32000 x 4096 61 / 101 -> 51 / 54.
-// With requests of 128 bytes to DRAM: 32000 x 4096 53.7 / 57.4.
+// first activations, products, exchange.  us, launches one after another over cold weights (channels x K), GEMV -> this kernel, 9 / 32
+// tokens: 4096 x 14336 30 / 46 -> 26 / 27; 14336 x 4096 34 / 56 -> 26 / 29; 32000 x 4096 58 / 98 -> 48 / 52.
+// With requests of 128 bytes to DRAM 32000 x 4096 took 3 us longer.
 // Built, measured and not kept: the experts' linears of a mixture in this form (units of all experts in one sequence, the
 // activations of all tokens multiplied and the pairs' columns picked from tensor memory): 8 rows x 8 layers of 32
 // experts 6170 -> 6370 us for 8 steps, 32 rows of the latent stack 7940 -> 8160.

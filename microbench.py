@@ -321,7 +321,8 @@ def bench_stack(pkg, args):
                 t = time_graph(lambda: [l(x) for l in w], 5, stream) / len(w)
                 byt, fl = 2 * (K * N + M * (K + N)), 2.0 * M * K * N
                 if M <= 32:
-                    report("gemv_bf16_kernel", t, byt=byt, K=K, N=N, M=M)
+                    few = M > 16 or M > 4 and K * N >= 28 << 20
+                    report("gemm_bf16_few_kernel" if few else "gemv_bf16_kernel", t, byt=byt, K=K, N=N, M=M)
                 else:
                     report("gemm_bf16_tc_kernel", t, flops=fl, K=K, N=N, M=M)
             del w
