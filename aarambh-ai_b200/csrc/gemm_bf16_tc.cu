@@ -108,6 +108,12 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     }
+    // A pair's tensor memory is allocated and given back by both CTAs together: either has to be running whenever the other asks.  (Before
+    // these barriers one CTA could leave while the other still gave back, and in rare launches that never ended.)
+    if (PAIR) {
+        __syncwarp();
+        cluster_sync_all();
+    }
     if (warp == 1) {  // tensor-memory allocation is a whole-warp operation
         if (PAIR) {
             asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(sptr(&sh->tmem_base)), "r"(TMEM_COLS));
@@ -181,6 +187,9 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                     tma_load_2d(st + (DUAL ? 2 : 1) * GB_A_BYTES, &xmap, ks * 64, xrow, &sh->full[s]);
                 }
             }
+            if (PAIR)  // the last stages' commits, which come from the other CTA's tensor core, have arrived
+                for (uint32_t u = use > STAGES ? use - STAGES : 0; u < use; ++u)
+                    if (!bar_wait(&sh->empty[u % STAGES], (u / STAGES) & 1, failed)) break;
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------- MMA issue (of a pair: by its first CTA)
@@ -301,6 +310,10 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS));
         else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS));
+    }
+    if (PAIR) {
+        __syncwarp();
+        cluster_sync_all();
     }
 }
 

@@ -65,3 +65,20 @@ def test_shared_expert_of_a_prompt(tmp_path):
     want = fx.expected(cfg, w, tokens.tolist())
     assert np.linalg.norm(got - want) < 2e-2 * np.linalg.norm(want)
     assert pkg().device_status() == 0
+
+
+def test_many_launches_of_pairs():
+    """Launch after launch: CTAs of one come and go while others of their pairs still set up or give back tensor memory."""
+    lins = [pkg().QuantLinear.from_bf16((torch.randn((n, k), device="cuda") * k ** -0.5).bfloat16()) for n, k in ((74 * 256, 256), (38 * 256 + 8, 1000))]
+    xs = [torch.randn((m, lin.in_features), device="cuda").bfloat16() for lin, m in zip(lins, (4096, 2600))]
+    first = [lin(x) for lin, x in zip(lins, xs)]
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        for _ in range(50):
+            got = [lin(x) for lin, x in zip(lins, xs)]
+    for _ in range(100):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(got, first)) and pkg().device_status() == 0
